@@ -66,13 +66,14 @@ EPI_PLAIN, EPI_SWIGLU, EPI_GEGLU = 0, 1, 2
 SWIGLU_BLOCK = 16  # gate/up rows alternate in blocks of this many for the fused epilogue
 
 
-def _simt(x, w, bias, residual, out):
+def _simt(x, w, bias, residual, out, tile: int = -1):
+    """``tile``: a tile of the kernel by index instead of its own choice (comparisons; the same bits)."""
     M, K = x.shape
     N = w.shape[0]
     L.check(L.core().dsp_gemm_simt(
         L.ptr(x), L.i64(x.stride(0)), L.ptr(w), L.ptr(bias), L.ptr(residual),
         L.i64(residual.stride(0) if residual is not None else 0), L.ptr(out), L.i64(out.stride(0)),
-        M, N, K, L.dtype_code(x.dtype), L.dtype_code(out.dtype), L.stream_handle()))
+        M, N, K, L.dtype_code(x.dtype), L.dtype_code(out.dtype), tile, L.stream_handle()))
     return out
 
 
