@@ -21,6 +21,10 @@
 // q:   element (t, head, d) at q[t * q_stride + head * D + d]
 // out: element (t, head, d) at out[t * out_stride + head * Dv + d]
 // pools: [num_pages, KVH, page_size, D] (keys) and [..., Dv] (values); page = page_table[seq * pt_stride + b / page_size]
+//
+// Two kernels.  `attn_rows_kernel` takes heads of up to 128 dimensions in rows of whole 16-byte (bfloat16: 8-byte)
+// pieces: several tokens of a portion share every key and value, which pass through shared memory.
+// `attn_generic_kernel` takes the rest, one block per (query token, KV head).
 #include "common.cuh"
 
 namespace {
@@ -187,6 +191,278 @@ attn_generic_kernel(const T* __restrict__ q, long q_stride, const T* __restrict_
     }
   }
 }
+
+// ------------------------------------------------------------------ heads of up to 128 dimensions
+// One block per (run of query tokens, KV head).  A run: tokens of one sequence at neighbouring positions, cut
+// where a position is a multiple of the `per` tokens whose G query heads fill the block's rows; the grid has a
+// block per token, and those whose token does not begin a run leave at once.  Row r of the block is head
+// g0 + r % gn of token r / gn.  A thread owns RI rows x KJ keys of the scores and RI rows x 4 DJ dimensions of
+// the result (the same rows, so the running maximum and sum stay in its registers); the keys of the next tile
+// are on their way while the values of this one are summed, and the other way round.
+//
+// What bounds it: shared-memory reads (eight 16-byte reads a thread per 64 products of the scores, twelve per
+// 128 of the sums).  260 tokens of a prompt beside four single tokens at 330, 12 heads of 128 on 2 KV heads:
+// 112 us; 299 with a block per token whose threads each walk a key of their own through global memory.
+constexpr int TILE_KEYS = 64, MAX_DIM = 128;
+
+struct RowsArgs {
+  const void *q, *k_pool, *v_pool;
+  const int *page_table, *positions, *seq_of_token;
+  void* out;
+  const float *sink_values, *turn_freq, *gate;
+  long q_stride, out_stride, ldg;
+  int pt_stride, T, H, KVH, D, Dv, page_size, num_pages, window, mask_mode, keep_first, sink, out_dtype;
+  float scale;
+  int* err;
+};
+
+// Four neighbouring elements as floats in shared memory: an asynchronous copy, or a load and a conversion.
+__device__ __forceinline__ void bring4(float* dst, const float* src, bool there) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void bring4(float* dst, const bf16* src, bool there) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (there) {
+    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(src);
+    const float2 a = __bfloat1622float2(p[0]), b = __bfloat1622float2(p[1]);
+    v = make_float4(a.x, a.y, b.x, b.y);
+  }
+  *reinterpret_cast<float4*>(dst) = v;
+}
+__device__ __forceinline__ void end_group() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void wait_groups() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// R rows on a grid of TY x TX threads.
+template <typename T, int R, int TY>
+__device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0, int n, int pos0, int seq, int kvh,
+                                          int g0, int gn) {
+  constexpr int TX = THREADS / TY, RI = R / TY, KJ = TILE_KEYS / TX, DJ = MAX_DIM / (4 * TX), LP = TILE_KEYS + 4;
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  const int D = a.D, Dv = a.Dv, LK = D + 4, LV = Dv + 4, G = a.H / a.KVH, rows = n * gn;
+  float* qs = smem;                     // [R][LK]
+  float* ks = qs + R * LK;              // [TILE_KEYS][LK]
+  float* vs = ks + TILE_KEYS * LK;      // [TILE_KEYS][LV]
+  float* ps = vs + TILE_KEYS * LV;      // [R][LP]
+  int* bad = (int*)(ps + R * LP);       // [2][TILE_KEYS] 1: the key's page id was outside the pool
+  const int* table = a.page_table + (size_t)seq * a.pt_stride;
+  const int last = pos0 + n - 1;
+
+  auto lowest = [&](int pos) {
+    return a.window > 0 ? (a.mask_mode == 1 ? pos / a.window * a.window : max(0, pos - a.window + 1)) : 0;
+  };
+  const int lo = lowest(pos0);  // (the first token sees the furthest back)
+  const int nfront = (min(a.keep_first, lo) + TILE_KEYS - 1) / TILE_KEYS;  // tiles of kept keys in front of the window
+  const int first = max(nfront, lo / TILE_KEYS), ntiles = nfront + last / TILE_KEYS - first + 1;
+  auto tile_start = [&](int i) { return (i < nfront ? i : first + i - nfront) * TILE_KEYS; };
+
+  __syncthreads();  // (a block of several groups of heads: the last one's reads are done)
+  for (int i = tid; i < R * (D / 4); i += THREADS) {
+    const int r = i / (D / 4), d = i % (D / 4) * 4;
+    const bool there = r < rows;
+    const T* src = (const T*)a.q;
+    if (there) src += (size_t)(t0 + r / gn) * a.q_stride + (size_t)(kvh * G + g0 + r % gn) * D + d;
+    bring4(qs + r * LK + d, src, there);
+  }
+  auto bring_keys = [&](int i) {
+    const int kt = tile_start(i);
+    for (int p = tid; p < TILE_KEYS * (D / 4); p += THREADS) {
+      const int j = p / (D / 4), d = p % (D / 4) * 4, key = kt + j;
+      const int page = key <= last ? table[key / a.page_size] : -1;
+      const bool there = page >= 0 && page < a.num_pages;
+      if (d == 0) {
+        bad[(i & 1) * TILE_KEYS + j] = !there;
+        // a page the window has passed is gone from the table; one that some token still sees must be there
+        if (!there && key <= last && (key >= lo || key < a.keep_first)) atomicOr(a.err, DSP_ERR_BAD_PAGE);
+      }
+      const T* src = (const T*)a.k_pool;
+      if (there) src += (((size_t)page * a.KVH + kvh) * a.page_size + key % a.page_size) * D + d;
+      bring4(ks + j * LK + d, src, there);
+    }
+    end_group();
+  };
+  auto bring_values = [&](int i) {
+    const int kt = tile_start(i);
+    for (int p = tid; p < TILE_KEYS * (Dv / 4); p += THREADS) {
+      const int j = p / (Dv / 4), d = p % (Dv / 4) * 4, key = kt + j;
+      const int page = key <= last ? table[key / a.page_size] : -1;
+      const bool there = page >= 0 && page < a.num_pages;
+      const T* src = (const T*)a.v_pool;
+      if (there) src += (((size_t)page * a.KVH + kvh) * a.page_size + key % a.page_size) * Dv + d;
+      bring4(vs + j * LV + d, src, there);
+    }
+    end_group();
+  };
+
+  float m[RI], l[RI], acc[RI][4 * DJ];
+  int pos[RI], low[RI];
+#pragma unroll
+  for (int i = 0; i < RI; ++i) {
+    const int r = ty + i * TY;
+    pos[i] = r < rows ? pos0 + r / gn : -1;
+    low[i] = r < rows ? lowest(pos[i]) : 0;
+    m[i] = a.sink ? ((a.sink_values && r < rows) ? a.sink_values[kvh * G + g0 + r % gn] : 0.f) : -INFINITY;
+    l[i] = a.sink ? 1.f : 0.f;
+#pragma unroll
+    for (int d = 0; d < 4 * DJ; ++d) acc[i][d] = 0.f;
+  }
+  bring_keys(0);
+  bring_values(0);
+  for (int t = 0; t < ntiles; ++t) {
+    const int kt = tile_start(t);
+    wait_groups<1>();
+    __syncthreads();
+    float s[RI][KJ];
+#pragma unroll
+    for (int i = 0; i < RI; ++i)
+#pragma unroll
+      for (int j = 0; j < KJ; ++j) s[i][j] = 0.f;
+#pragma unroll 2
+    for (int d = 0; d < D; d += 4) {
+      float4 x[RI];
+#pragma unroll
+      for (int i = 0; i < RI; ++i) x[i] = *reinterpret_cast<const float4*>(qs + (ty + i * TY) * LK + d);
+#pragma unroll
+      for (int j = 0; j < KJ; ++j) {
+        const float4 y = *reinterpret_cast<const float4*>(ks + (tx + j * TX) * LK + d);
+#pragma unroll
+        for (int i = 0; i < RI; ++i)
+          s[i][j] = fmaf(x[i].w, y.w, fmaf(x[i].z, y.z, fmaf(x[i].y, y.y, fmaf(x[i].x, y.x, s[i][j]))));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RI; ++i) {
+      float top = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < KJ; ++j) {
+        const int key = kt + tx + j * TX;
+        const bool seen = key <= pos[i] && (key >= low[i] || key < a.keep_first) && !bad[(t & 1) * TILE_KEYS + tx + j * TX];
+        s[i][j] = seen ? s[i][j] * a.scale : -INFINITY;
+        top = fmaxf(top, s[i][j]);
+      }
+#pragma unroll
+      for (int o = TX / 2; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      const float m_new = fmaxf(m[i], top);
+      // m_new stays -inf for rows that have seen no key yet
+      const float alpha = m_new == -INFINITY ? 1.f : expf(m[i] - m_new);
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < KJ; ++j) {
+        const float p = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - m_new);
+        ps[(ty + i * TY) * LP + tx + j * TX] = p;
+        sum += p;
+      }
+#pragma unroll
+      for (int o = TX / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      m[i] = m_new;
+      l[i] = l[i] * alpha + sum;
+#pragma unroll
+      for (int d = 0; d < 4 * DJ; ++d) acc[i][d] *= alpha;
+    }
+    __syncthreads();  // the keys have been read
+    if (t + 1 < ntiles) bring_keys(t + 1); else end_group();
+    wait_groups<1>();
+    __syncthreads();  // the values are there (and every row of ps)
+    // where some row does not see every key, a key that a row does not see must not reach it: 0 times a value that is
+    // no number is none either
+    const bool all_seen = kt + TILE_KEYS - 1 <= pos0 && kt >= lowest(last);
+#pragma unroll 2
+    for (int j = 0; j < TILE_KEYS; j += 4) {
+      float p[RI][4];
+#pragma unroll
+      for (int i = 0; i < RI; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(ps + (ty + i * TY) * LP + j);
+        p[i][0] = v.x, p[i][1] = v.y, p[i][2] = v.z, p[i][3] = v.w;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int dj = 0; dj < DJ; ++dj) {
+          const int d = (tx + dj * TX) * 4;
+          if (d >= Dv) continue;
+          const float4 v = *reinterpret_cast<const float4*>(vs + (j + e) * LV + d);
+#pragma unroll
+          for (int i = 0; i < RI; ++i) {
+            if (!all_seen && p[i][e] == 0.f) continue;
+            acc[i][4 * dj] = fmaf(p[i][e], v.x, acc[i][4 * dj]);
+            acc[i][4 * dj + 1] = fmaf(p[i][e], v.y, acc[i][4 * dj + 1]);
+            acc[i][4 * dj + 2] = fmaf(p[i][e], v.z, acc[i][4 * dj + 2]);
+            acc[i][4 * dj + 3] = fmaf(p[i][e], v.w, acc[i][4 * dj + 3]);
+          }
+        }
+    }
+    __syncthreads();  // the values have been read
+    if (t + 1 < ntiles) bring_values(t + 1); else end_group();
+  }
+  wait_groups<0>();
+  float* os = ks;  // [R][Dv] results before they are turned back (with turn_freq)
+#pragma unroll
+  for (int i = 0; i < RI; ++i) {
+    const int r = ty + i * TY;
+    if (r >= rows) continue;
+    const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
+    const int tok = t0 + r / gn;
+#pragma unroll
+    for (int dj = 0; dj < DJ; ++dj)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int d = (tx + dj * TX) * 4 + e;
+        if (d >= Dv) continue;
+        const size_t col = (size_t)(kvh * G + g0 + r % gn) * Dv + d;
+        float y = acc[i][4 * dj + e] * inv;
+        if (a.gate) y /= 1.f + expf(-a.gate[(size_t)tok * a.ldg + col]);
+        if (a.turn_freq)
+          os[r * Dv + d] = y;
+        else
+          st_any(a.out, a.out_dtype, (size_t)tok * a.out_stride + col, y);
+      }
+  }
+  if (a.turn_freq) {
+    __syncthreads();
+    const int half = Dv / 2;
+    for (int i = tid; i < rows * Dv; i += THREADS) {
+      const int r = i / Dv, d = i % Dv, mth = d < half ? d : d - half;
+      float sn, cn;
+      sincosf((float)(pos0 + r / gn) * a.turn_freq[mth], &sn, &cn);
+      // the inverse turn: (u, v) -> (u cos + v sin, v cos - u sin)
+      const float y = d < half ? os[i] * cn + os[i + half] * sn : os[i] * cn - os[i - half] * sn;
+      st_any(a.out, a.out_dtype, (size_t)(t0 + r / gn) * a.out_stride + (size_t)(kvh * G + g0 + r % gn) * Dv + d, y);
+    }
+  }
+}
+
+constexpr int ROWS = 32, FEW_ROWS = 8;
+
+template <typename T>
+__global__ void __launch_bounds__(THREADS) attn_rows_kernel(const RowsArgs a) {
+  extern __shared__ __align__(16) float rows_smem[];
+  const int t0 = blockIdx.x, kvh = blockIdx.y, pos0 = a.positions[t0];
+  if (pos0 < 0) return;
+  const int seq = a.seq_of_token[t0], G = a.H / a.KVH, per = max(1, ROWS / G);
+  if (pos0 % per && t0 > 0 && a.seq_of_token[t0 - 1] == seq && a.positions[t0 - 1] == pos0 - 1) return;  // inside a run
+  int n = 1;
+  while (n < per && (pos0 + n) % per && t0 + n < a.T && a.seq_of_token[t0 + n] == seq && a.positions[t0 + n] == pos0 + n) ++n;
+  if (n * G <= FEW_ROWS)
+    attn_rows<T, FEW_ROWS, 4>(a, rows_smem, t0, n, pos0, seq, kvh, 0, G);
+  else
+    for (int g0 = 0; g0 < G; g0 += ROWS) attn_rows<T, ROWS, 8>(a, rows_smem, t0, n, pos0, seq, kvh, g0, min(ROWS, G - g0));
+}
+
+template <typename T>
+int launch_rows(const RowsArgs& a, cudaStream_t stream) {
+  const size_t smem = (size_t)((ROWS + TILE_KEYS) * (a.D + 4) + TILE_KEYS * (a.Dv + 4) + ROWS * (TILE_KEYS + 4)) * sizeof(float) +
+                      2 * TILE_KEYS * sizeof(int);
+  DSP_CUDA(cudaFuncSetAttribute(attn_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  attn_rows_kernel<T><<<dim3(a.T, a.KVH), THREADS, smem, stream>>>(a);
+  DSP_CHECK_LAUNCH("dsp_attn_generic");
+  return 0;
+}
+
+// Whether rows of `width` elements at `stride` from `p` consist of whole pieces of four elements.
+bool whole_pieces(const void* p, long stride, int width, int dtype) {
+  return (uintptr_t)p % (dtype == DSP_F32 ? 16 : 8) == 0 && stride % 4 == 0 && width % 4 == 0;
+}
 }  // namespace
 
 extern "C" int dsp_attn_generic(const void* q, long q_stride, const void* k_pool,
@@ -208,6 +484,13 @@ extern "C" int dsp_attn_generic(const void* q, long q_stride, const void* k_pool
   DSP_REQUIRE(!turn_freq || Dv % 2 == 0, "dsp_attn_generic: values of an odd width %d cannot be turned", Dv);
   int* err = dsp_device_error_ptr();
   DSP_REQUIRE(err != nullptr, "dsp_attn_generic: no device error word");
+  if ((dtype == DSP_F32 || dtype == DSP_BF16) && D <= MAX_DIM && Dv <= MAX_DIM && whole_pieces(q, q_stride, D, dtype) &&
+      whole_pieces(k_pool, 0, D, dtype) && whole_pieces(v_pool, 0, Dv, dtype)) {
+    const RowsArgs a = {q, k_pool, v_pool, page_table, positions, seq_of_token, out, sink_values, turn_freq, gate,
+                        q_stride, out_stride, ldg, pt_stride, T, H, KVH, D, Dv, page_size, num_pages, window, mask_mode,
+                        keep_first, sink, out_dtype, scale, err};
+    return dtype == DSP_F32 ? launch_rows<float>(a, stream) : launch_rows<bf16>(a, stream);
+  }
   const size_t smem = (size_t)(GCHUNK * D + GCHUNK * THREADS + (turn_freq ? GCHUNK * Dv : 0)) * sizeof(float) +
                       THREADS * sizeof(long);
   dim3 grid(T, KVH);
