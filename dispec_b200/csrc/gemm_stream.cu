@@ -1,9 +1,9 @@
-// C[M,N] = A[M,K] * W[N,K]^T (+ bias) (+ residual) for up to 128 rows of A, bfloat16 in, 32-bit
+// C[M,N] = A[M,K] * W[N,K]^T (+ bias) (+ residual) for few rows of A, bfloat16 in, 32-bit
 // accumulation: the matrix product of decoding, bound by streaming W once from HBM, on TMA and
-// the fifth-generation tensor cores.
+// the fifth-generation tensor cores, and of portions of a few hundred rows where the output is narrow.
 //
 // Roles are swapped: 128 rows of W are the M side of tcgen05.mma, the few rows of A (padded to
-// 16, 32, 64 or 128) its N side, so the accumulator in tensor memory is 128 lanes (rows of W) by a
+// 16, 32, 64, 128 or 192; more are cut into chunks of equal size, tiles of their own) its N side, so the accumulator in tensor memory is 128 lanes (rows of W) by a
 // few columns (rows of A).  One thread streams W tiles of 128 rows x 64 k (16 KB a request)
 // and the matching slice of A by TMA into a ring of 4 to 5 stages (two CTAs per SM, about 180 KB
 // on its way per SM, which plain loads cannot keep in flight); one thread issues the products; four warps read
@@ -40,11 +40,13 @@ constexpr int MAX_SPLITS = 8;
 enum { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_GEGLU = 2 };
 
 template <int NB> struct Cfg {
+  static constexpr bool CHUNKED = NB > 64;  // there may be several chunks of rows
   static constexpr int X_BYTES = NB * BK * 2;
   static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
   // about 100 KB of ring per CTA, so that two CTAs fit an SM: the next kernel's CTA (programmatic
   // dependent launch) fills its ring with W while this kernel's CTA is still streaming
-  static constexpr int STAGES = NB == 16 ? 5 : NB == 32 ? 5 : NB == 64 ? 4 : 5;  // 128 rows of A: one CTA per SM
+  // (128 and 192 rows of A: one CTA per SM; at 192 the ring must also hold the partial tile and the inbox of a K split)
+  static constexpr int STAGES = NB == 64 ? 4 : 5;
   // One thread's turn of the ring (wait for the stage, fence, four products, commit) takes about
   // 0.3 us, of which the tensor pipe is busy a third (a product of 128 x 16 x 16 every 55 cycles from
   // one issuing thread, every 39 from two: `bench.py --only mma-rate`); a W tile of 16 KB per 0.3 us is
@@ -60,19 +62,23 @@ template <int NB> struct Cfg {
   static constexpr int PARTS = NB == 16 ? 4 : NB <= 64 ? 2 : 1;
   static constexpr int ISSUERS = PARTS;
   static constexpr int FIRST_EPI_WARP = 1 + ISSUERS;
-  static constexpr int THREADS = 32 * (1 + ISSUERS + 4);
+  // two epilogue warps per quarter of the lanes where a CTA has an SM to itself: they take the windows of the
+  // accumulator (the rows of a K split) in turn
+  static constexpr int EPI_GROUPS = NB <= 64 ? 1 : 2, EPI_WARPS = 4 * EPI_GROUPS;
+  static constexpr int THREADS = 32 * (1 + ISSUERS + EPI_WARPS);
   static constexpr int MIN_CTAS = NB <= 64 ? 2 : 1;  // CTAs per SM the registers are held down for
   // the epilogue takes the accumulator in windows of at most 64 columns (rows of A): what a thread holds at once
   static constexpr int WINDOW = NB <= 64 ? NB : 64;
   static constexpr int ACC_COLS = PARTS * NB;  // one accumulator buffer
-  static constexpr int TMEM_COLS = 2 * ACC_COLS < 32 ? 32 : 2 * ACC_COLS;
+  static constexpr int TMEM_COLS = 2 * ACC_COLS < 32 ? 32 : 2 * ACC_COLS <= 256 ? 2 * ACC_COLS : 512;  // a power of two
   // K split over a cluster: every CTA sends the rows of its partial tile to the CTA that finishes
   // them (row m to rank m % splits), into an inbox of [source rank][rows per CTA][128] floats.  Up
   // to 16 rows of A (at most 16 + 8 rows of inbox) it has room of its own behind the ring
   static constexpr bool PUSH = NB == 16;
   // behind the ring: that inbox, or 8 KB in which, without a split of K, an epilogue warp turns 16
   // columns of its accumulator around, so that a lane stores four outputs of one row
-  static constexpr int INBOX_BYTES = PUSH ? (16 + MAX_SPLITS) * ROWS_W * 4 : 4 * 16 * 32 * 4;
+  static constexpr int INBOX_BYTES = PUSH ? (16 + MAX_SPLITS) * ROWS_W * 4 : EPI_WARPS * 16 * 32 * 4;
+  static_assert(PUSH || STAGES * STAGE_BYTES >= (NB + NB + MAX_SPLITS) * ROWS_W * 4, "the drained ring holds tile and inbox");
 };
 
 // Timestamps for measurements, compiled in only with -DDSP_STAMPS (DISPEC_B200_STAMPS=1 at build
@@ -115,6 +121,17 @@ struct Args {
   const bf16* gain2;
   void* C2;
   long ldc2;
+};
+
+// More rows of A than a tile has columns are cut into chunks of equal size; the CTAs of a block of W take its
+// chunks side by side, so that the second one finds the tiles of W in the L2.
+struct Chunks {
+  int rows, count;
+  __host__ __device__ explicit Chunks(int M) {
+    count = (M + 191) / 192;
+    rows = (M + count - 1) / count;
+    count = (M + rows - 1) / rows;
+  }
 };
 
 template <typename TOut>
@@ -239,7 +256,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   if (!a.late_trigger) pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int splits = gridDim.y, split = blockIdx.y;
-  const int n_blocks = (a.N + ROWS_W - 1) / ROWS_W;
+  const Chunks ch(C::CHUNKED ? a.M : 1);
+  const int n_tiles = (a.N + ROWS_W - 1) / ROWS_W * (C::CHUNKED ? ch.count : 1);  // (block of W, chunk of rows), chunks innermost
   const int kb_total = (a.K + BK - 1) / BK;
   const int kb_begin = split * a.kb_per_split;
   const int kb_end = min(kb_total, kb_begin + a.kb_per_split);
@@ -252,7 +270,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&accum_full[b], C::ISSUERS);
-      mbar_init(&accum_empty[b], 4);
+      mbar_init(&accum_empty[b], C::EPI_WARPS);
     }
     mbar_init(&inbox_bar, 1);
     failed = 0;
@@ -275,15 +293,17 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   if (warp == 0) {
     if (lane == 0) {
       // the CTA's work as one flat sequence of (block of W, k block) items
-      const int my_tiles = blockIdx.x < n_blocks ? (n_blocks - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+      const int my_tiles = blockIdx.x < n_tiles ? (n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
       const int total = my_tiles * num_kb;
       const int first = total < C::STAGES ? total : C::STAGES;
-      auto w_row = [&](int it) { return ((int)blockIdx.x + (it / num_kb) * (int)gridDim.x) * ROWS_W; };
+      auto w_row = [&](int it) { return ((int)blockIdx.x + (it / num_kb) * (int)gridDim.x) / (C::CHUNKED ? ch.count : 1) * ROWS_W; };
+      auto x_row = [&](int it) { return C::CHUNKED ? ((int)blockIdx.x + (it / num_kb) * (int)gridDim.x) % ch.count * ch.rows : 0; };
       auto k_of = [&](int it) { return (kb_begin + it % num_kb) * BK; };
       // W does not depend on the kernel before this one: the ring is filled with W tiles first,
       // then the kernel waits for its predecessor and sends the matching slices of A after them
       // W is read once per call and is far larger than the L2 over a step: its lines leave first
-      const uint64_t once = l2_policy_evict_first();
+      // (with several chunks of rows it is read as often as there are chunks, and stays)
+      const uint64_t once = !C::CHUNKED || ch.count == 1 ? l2_policy_evict_first() : l2_policy_evict_normal();
       for (int it = 0; it < first; ++it) {
         mbar_expect_tx(&full_bar[it], C::STAGE_BYTES);
         tma_load_2d_hint(smem + it * C::STAGE_BYTES, &map_w, &full_bar[it], k_of(it), w_row(it), once);
@@ -292,7 +312,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       pdl_wait();
       STAMP(1);  // the predecessor is complete
       for (int it = 0; it < first; ++it)
-        tma_load_2d(smem + it * C::STAGE_BYTES + W_BYTES, &map_x, &full_bar[it], k_of(it), 0);
+        tma_load_2d(smem + it * C::STAGE_BYTES + W_BYTES, &map_x, &full_bar[it], k_of(it), x_row(it));
       for (int it = first; it < total; ++it) {
         const int s = it % C::STAGES;
         const uint32_t phase = (it / C::STAGES) & 1;
@@ -303,7 +323,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
         unsigned char* dst = smem + s * C::STAGE_BYTES;
         tma_load_2d_hint(dst, &map_w, &full_bar[s], k_of(it), w_row(it), once);
-        tma_load_2d(dst + W_BYTES, &map_x, &full_bar[s], k_of(it), 0);
+        tma_load_2d(dst + W_BYTES, &map_x, &full_bar[s], k_of(it), x_row(it));
       }
       STAMP(7);  // the last tile of W is requested
       if (a.late_trigger) pdl_launch_dependents();
@@ -314,7 +334,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       const int j = warp - 1;
       const uint32_t idesc = umma_idesc(ROWS_W, NB);
       int it = 0, local = 0;
-      for (int nb = blockIdx.x; nb < n_blocks && !failed; nb += gridDim.x, ++local) {
+      for (int tile = blockIdx.x; tile < n_tiles && !failed; tile += gridDim.x, ++local) {
         const int buf = local & 1;
         if (!mbar_wait(&accum_empty[buf], ((local >> 1) & 1) ^ 1)) {
           failed = 1;
@@ -446,7 +466,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       if constexpr (NB <= 32) compute_row_scales(0, 1);
       else compute_own_row_scales(0, 1);  // many rows: more loads in flight
       int local = 0;
-      for (int nb = blockIdx.x; nb < n_blocks; nb += gridDim.x, ++local) {
+      for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++local) {
+        const int nb = C::CHUNKED ? tile / ch.count : tile, base = C::CHUNKED ? tile % ch.count * ch.rows : 0;
+        const int rows = C::CHUNKED ? min(ch.rows, a.M - base) : a.M;
         const int buf = local & 1;
         if (!__all_sync(0xffffffffu, mbar_wait(&accum_full[buf], (local >> 1) & 1))) {
           failed = 1;
@@ -455,17 +477,20 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         tc_fence_after();
         if (threadIdx.x == 32 * C::FIRST_EPI_WARP) STAMP(4);  // an accumulator is complete (the last one stays)
         // the accumulator in windows of WIN columns (rows h0 .. h0 + WIN - 1 of A); one window up to 64 rows
-        constexpr int WIN = C::WINDOW;
-        for (int h0 = 0; h0 < NB && h0 < a.M; h0 += WIN) {
+        constexpr int WIN = C::WINDOW, STEP = WIN * C::EPI_GROUPS;
+        const int mine = C::EPI_GROUPS == 1 ? 0 : WIN * ((warp - C::FIRST_EPI_WARP) >> 2);  // this warp's first window
+        if (C::EPI_GROUPS > 1 && mine >= rows && lane == 0)  // (none: the accumulator is free as far as it is concerned)
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&accum_empty[buf])) : "memory");
+        for (int h0 = mine; h0 < NB && h0 < rows; h0 += STEP) {
         uint32_t v[WIN];
         load_accumulator<WIN, C::PARTS>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * C::ACC_COLS + h0), NB, v);
-        if (h0 + WIN >= NB || h0 + WIN >= a.M) {  // the last window: the accumulator is free again
+        if (h0 + STEP >= NB || h0 + STEP >= rows) {  // the last window: the accumulator is free again
           tc_fence_before();
           __syncwarp();
           if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&accum_empty[buf])) : "memory");
           if (threadIdx.x == 32 * C::FIRST_EPI_WARP) STAMP(5);  // the accumulator is in registers
         }
-        if (a.vec4 && !swiglu && a.residual == nullptr) {
+        if (a.vec4 && !swiglu && (C::CHUNKED || a.residual == nullptr)) {
           // Sixteen columns (rows of A) at a time go through shared memory and come back turned
           // around: a lane then holds four W rows of one row of A, the loop over the rows is rolled
           // (its instructions are fetched once) and a store carries four outputs.  (The output head
@@ -481,12 +506,22 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           }
 #pragma unroll
           for (int c0 = 0; c0 < WIN; c0 += 16) {
-            if (h0 + c0 >= a.M) break;
+            if (h0 + c0 >= rows) break;
+            float4 res4[C::CHUNKED ? 4 : 1];
+            if constexpr (C::CHUNKED) {
+#pragma unroll
+              for (int it = 0; it < 4; ++it) {
+                const int m = h0 + c0 + 4 * it + sub;
+                res4[it] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (a.residual && m < rows && n4 < a.N)
+                  res4[it] = load4(reinterpret_cast<const TOut*>(a.residual) + (size_t)(base + m) * a.ldr + n4);
+              }
+            }
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 16; ++j) stage[j * 32 + lane] = __uint_as_float(v[c0 + j]);
             __syncwarp();
-#pragma unroll 1
+#pragma unroll(C::CHUNKED ? 4 : 1)
             for (int it = 0; it < 4; ++it) {
               const int m = h0 + c0 + 4 * it + sub;
               float4 val = *reinterpret_cast<const float4*>(stage + (4 * it + sub) * 32 + 4 * l8);
@@ -494,12 +529,13 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 const float scale = row_scale[m];
                 val.x *= scale, val.y *= scale, val.z *= scale, val.w *= scale;
               }
-              if (m < a.M && n4 < a.N) {
+              if (m < rows && n4 < a.N) {
                 val.x += bias4.x, val.y += bias4.y, val.z += bias4.z, val.w += bias4.w;
-                store4(reinterpret_cast<TOut*>(a.C) + (size_t)m * a.ldc + n4, val);
+                if constexpr (C::CHUNKED) val.x += res4[it].x, val.y += res4[it].y, val.z += res4[it].z, val.w += res4[it].w;
+                store4(reinterpret_cast<TOut*>(a.C) + (size_t)(base + m) * a.ldc + n4, val);
                 if (a.C2) {
                   const float4 out = rounded4<TOut>(val);
-                  store4(reinterpret_cast<TOut*>(a.C2) + (size_t)m * a.ldc2 + n4,
+                  store4(reinterpret_cast<TOut*>(a.C2) + (size_t)(base + m) * a.ldc2 + n4,
                          make_float4(out.x * gain4.x, out.y * gain4.y, out.z * gain4.z, out.w * gain4.w));
                 }
               }
@@ -511,7 +547,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (a.norm_src) {
 #pragma unroll
           for (int m = 0; m < WIN; ++m)
-            if (h0 + m < a.M) v[m] = __float_as_uint(__uint_as_float(v[m]) * row_scale[h0 + m]);
+            if (h0 + m < rows) v[m] = __float_as_uint(__uint_as_float(v[m]) * row_scale[h0 + m]);
         }
         const int n = nb * ROWS_W + row;
         if (swiglu) {
@@ -527,13 +563,13 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             const float other = __shfl_xor_sync(0xffffffffu, low ? x1 : x0, 16);
             const float gate = low ? x0 : other, up = low ? other : x1;
             const int m = h0 + (low ? m0 : m0 + 1);
-            if (m < a.M && n_ok)
-              reinterpret_cast<TOut*>(a.C)[(size_t)m * a.ldc + col] = from_f32<TOut>(unit_times(gate, up, gelu));
+            if (m < rows && n_ok)
+              reinterpret_cast<TOut*>(a.C)[(size_t)(base + m) * a.ldc + col] = from_f32<TOut>(unit_times(gate, up, gelu));
           }
         } else {
 #pragma unroll
           for (int m = 0; m < WIN; ++m)
-            if (h0 + m < a.M && n < a.N) finish<TOut>(a, __uint_as_float(v[m]), h0 + m, n);
+            if (h0 + m < rows && n < a.N) finish<TOut>(a, __uint_as_float(v[m]), base + h0 + m, n);
         }
         }  // windows
         if (threadIdx.x == 32 * C::FIRST_EPI_WARP) STAMP(9);  // the block's stores are issued
@@ -557,16 +593,19 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     // from a tile ordered by rank 2.00 ms, its unrolled stores with computed addresses being the
     // cost.  8 rows: every thread sending its own 4-byte values, unrolled, 1.000 ms; this form
     // 0.988 ms; 1 row 0.989 -> 0.949 ms.)
-    const int rows_per = (a.M + splits - 1) / splits;
+    const unsigned nb = C::CHUNKED ? blockIdx.x / ch.count : blockIdx.x;
+    const int base = C::CHUNKED ? blockIdx.x % ch.count * ch.rows : 0;
+    const int rows = C::CHUNKED ? min(ch.rows, a.M - base) : a.M;
+    const int rows_per = (rows + splits - 1) / splits;
     float* tile = reinterpret_cast<float*>(smem);                    // [row of A][128]
     // [source rank][rows per CTA][128]: behind the ring where there is room for it (up to 16 rows)
     float* inbox = C::PUSH ? reinterpret_cast<float*>(smem + C::STAGES * C::STAGE_BYTES) : tile + NB * ROWS_W;
     if constexpr (C::PUSH) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // second half of the start barrier
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
-    const int rows_own = rank < a.M ? (a.M - rank + splits - 1) / splits : 0;
-    const int ew = warp - C::FIRST_EPI_WARP;                          // 0..3 in the epilogue warps
-    const int n4 = blockIdx.x * ROWS_W + 4 * lane;                    // this lane's four outputs of a row
+    const int rows_own = rank < rows ? (rows - rank + splits - 1) / splits : 0;
+    const int ew = warp - C::FIRST_EPI_WARP;                          // 0.. in the epilogue warps
+    const int n4 = nb * ROWS_W + 4 * lane;                            // this lane's four outputs of a row
     const bool n_ok = n4 < a.N;                                       // N is a multiple of 4 here
     // bias, and the residual of the first rows this warp finishes (its share at 64 or 128 rows over 8
     // ranks), are asked for while the products still run
@@ -580,16 +619,16 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       }
 #pragma unroll
       for (int i = 0; i < RES; ++i) {
-        const int m = rank + (ew + 4 * i) * splits;
+        const int m = rank + (ew + C::EPI_WARPS * i) * splits;
         res4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!swiglu && n_ok && a.residual && m < a.M)
-          res4[i] = load4(reinterpret_cast<const TOut*>(a.residual) + (size_t)m * a.ldr + n4);
+        if (!swiglu && n_ok && a.residual && m < rows)
+          res4[i] = load4(reinterpret_cast<const TOut*>(a.residual) + (size_t)(base + m) * a.ldr + n4);
       }
       compute_own_row_scales(rank, splits);
       if (!__all_sync(0xffffffffu, mbar_wait(&accum_full[0], 0))) failed = 1;
       tc_fence_after();
       if (threadIdx.x == 32 * C::FIRST_EPI_WARP) STAMP(4);  // the accumulator is complete
-      for (int h0 = 0; h0 < NB && h0 < a.M; h0 += C::WINDOW) {
+      for (int h0 = C::EPI_GROUPS == 1 ? 0 : C::WINDOW * (ew >> 2); h0 < NB && h0 < rows; h0 += C::WINDOW * C::EPI_GROUPS) {
         uint32_t v[C::WINDOW];
         load_accumulator<C::WINDOW, C::PARTS>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)h0, NB, v);
 #pragma unroll
@@ -609,7 +648,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       if (!failed) {
         // a warp sends whole rows of A, 16 bytes a lane: row m to rank m % splits, slot m / splits
 #pragma unroll 1
-        for (int m = ew; m < a.M; m += 4) {
+        for (int m = ew; m < rows; m += C::EPI_WARPS) {
           const uint32_t owner = (uint32_t)(m % splits);
           const int slot = m / splits;
           const float4 val = reinterpret_cast<const float4*>(tile + m * ROWS_W)[lane];
@@ -622,7 +661,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       if (threadIdx.x == 32 * C::FIRST_EPI_WARP) STAMP(5);  // every rank's rows have arrived
       if (!failed) {
 #pragma unroll 1
-        for (int slot = ew, i = 0; slot < rows_own; slot += 4, ++i) {
+        for (int slot = ew, i = 0; slot < rows_own; slot += C::EPI_WARPS, ++i) {
           const int m = rank + slot * splits;
           float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -645,8 +684,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             up.z = __shfl_down_sync(0xffffffffu, total.z, 4);
             up.w = __shfl_down_sync(0xffffffffu, total.w, 4);
             if ((lane & 4) == 0 && n4 + 16 < a.N) {
-              const int col = ((blockIdx.x * ROWS_W + (lane >> 3) * 32) >> 1) + 4 * (lane & 3);
-              store4(reinterpret_cast<TOut*>(a.C) + (size_t)m * a.ldc + col,
+              const int col = ((nb * ROWS_W + (lane >> 3) * 32) >> 1) + 4 * (lane & 3);
+              store4(reinterpret_cast<TOut*>(a.C) + (size_t)(base + m) * a.ldc + col,
                      make_float4(unit_times(total.x, up.x, gelu), unit_times(total.y, up.y, gelu),
                                  unit_times(total.z, up.z, gelu), unit_times(total.w, up.w, gelu)));
             }
@@ -655,14 +694,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
             for (int q = 1; q < RES; ++q)
               if (i == q) res = res4[q];
-            if (i >= RES && a.residual) res = load4(reinterpret_cast<const TOut*>(a.residual) + (size_t)m * a.ldr + n4);
+            if (i >= RES && a.residual) res = load4(reinterpret_cast<const TOut*>(a.residual) + (size_t)(base + m) * a.ldr + n4);
             // the same order of sums as finish(): bias, then residual
             total.x = (total.x + bias4.x) + res.x, total.y = (total.y + bias4.y) + res.y;
             total.z = (total.z + bias4.z) + res.z, total.w = (total.w + bias4.w) + res.w;
-            store4(reinterpret_cast<TOut*>(a.C) + (size_t)m * a.ldc + n4, total);
+            store4(reinterpret_cast<TOut*>(a.C) + (size_t)(base + m) * a.ldc + n4, total);
             if (a.C2) {
               const float4 out = rounded4<TOut>(total);
-              store4(reinterpret_cast<TOut*>(a.C2) + (size_t)m * a.ldc2 + n4,
+              store4(reinterpret_cast<TOut*>(a.C2) + (size_t)(base + m) * a.ldc2 + n4,
                      make_float4(out.x * gain4.x, out.y * gain4.y, out.z * gain4.z, out.w * gain4.w));
             }
           }
@@ -687,8 +726,37 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   }
 }
 
+// Clusters of `splits` CTAs that the device holds at once, for tiles that take an SM to themselves: a cluster
+// stays inside a group of SMs, and what does not fit waits for a second round (16 clusters of 8 in place
+// of 16 of 7: 14.9 us instead of 9.9 for 128 rows x 2,048 x 1,536).
 template <int NB, typename TOut>
-int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const Args& a, int n_blocks, int splits, int num_sms,
+int max_clusters(int splits) {
+  using C = Cfg<NB>;
+  static int known[MAX_SPLITS + 1] = {};
+  if (known[splits] == 0) {
+    const size_t smem = (size_t)C::STAGES * C::STAGE_BYTES + 1024 + C::INBOX_BYTES;
+    auto kernel = gemm_stream_kernel<NB, TOut>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, splits, 1);
+    cfg.blockDim = dim3(C::THREADS, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = splits;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) cudaGetLastError();
+    known[splits] = n > 0 ? n : 1;
+  }
+  return known[splits];
+}
+
+template <int NB, typename TOut>
+int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const Args& a, int tiles, int splits, int num_sms,
            int* err, cudaStream_t stream) {
   using C = Cfg<NB>;
   const size_t smem = (size_t)C::STAGES * C::STAGE_BYTES + 1024 + C::INBOX_BYTES;
@@ -700,7 +768,7 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const Args& a, in
   }
   cudaLaunchConfig_t cfg = {};
   const int resident = C::MIN_CTAS * num_sms;  // without a split the CTAs walk over the blocks of W
-  cfg.gridDim = dim3(splits > 1 ? n_blocks : (n_blocks < resident ? n_blocks : resident), splits, 1);
+  cfg.gridDim = dim3(splits > 1 ? tiles : (tiles < resident ? tiles : resident), splits, 1);
   cfg.blockDim = dim3(C::THREADS, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -717,7 +785,58 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const Args& a, in
   DSP_CUDA(cudaLaunchKernelEx(&cfg, kernel, map_w, map_x, a, err));
   return 0;
 }
+struct Plan {
+  int nb_rows;          // columns of a tile (rows of A, padded)
+  int tiles;            // blocks of W x chunks
+  int splits, kb_per_split;
+};
+
+Plan make_plan(int M, int N, int K, int out_dtype, int target_ctas, bool may_split) {
+  Plan p;
+  const Chunks ch(M);
+  p.nb_rows = ch.rows <= 16 ? 16 : ch.rows <= 32 ? 32 : ch.rows <= 64 ? 64 : ch.rows <= 128 ? 128 : 192;
+  p.tiles = (N + ROWS_W - 1) / ROWS_W * ch.count;
+  const int kb_total = (K + BK - 1) / BK;
+  int splits = may_split ? target_ctas / p.tiles : 1;
+  if (splits < 1) splits = 1;
+  if (splits > MAX_SPLITS) splits = MAX_SPLITS;
+  if (splits > kb_total) splits = kb_total;
+  if (p.nb_rows > 64) {
+    auto fits = [&](int n) {
+      if (p.nb_rows == 128) return out_dtype == DSP_BF16 ? max_clusters<128, bf16>(n) : max_clusters<128, float>(n);
+      return out_dtype == DSP_BF16 ? max_clusters<192, bf16>(n) : max_clusters<192, float>(n);
+    };
+    while (splits > 1 && fits(splits) < p.tiles) --splits;
+  }
+  p.kb_per_split = (kb_total + splits - 1) / splits;
+  p.splits = (kb_total + p.kb_per_split - 1) / p.kb_per_split;
+  return p;
+}
 }  // namespace
+
+// Whether this product beats the many-row one (gemm_tcgen05.cu) at M rows, which matters above 128: the
+// many-row kernel cuts C into tiles of 256 rows x 192 or 256 columns and does not split K, so a narrow product with
+// a long K (down_proj: 8 tiles of 140 k blocks) keeps a tenth of the SMs busy; this one has tiles of 128
+// columns x up to 192 rows and splits K over a cluster, but moves 40 KB for a product half as large.
+// Estimates in microseconds, fitted on launches that follow one another in a graph and read W from
+// memory.  This kernel and the many-row kernel, 1.5B sizes, qkv / o_proj / gate_up / down: 9.5 / 9.1 / 17.3 / 14.9 us
+// and 11.4 / 14.0 / 16.0 / 45.6 at 137 rows; 15.3 / 13.5 / 36.2 / 27.2 and 11.8 / 14.6 / 30.4 / 46.4 at 536; 16.3 /
+// 16.3 / 64 / 37.8 and 12.7 / 14.8 / 40.7 / 47.6 at 1,016.  7B sizes, qkv / o_proj / down: 17.5 / 15.4 / 36 and 21.4 /
+// 23.6 / 90 at 192; 22.1 / 23.1 / 66 and 22.8 / 24.1 / 91 at 384; 28.5 / 31.6 / 118 and 23.2 / 25.0 / 92 at 536.
+extern "C" int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas) {
+  if (M <= 0 || N <= 0 || K <= 0 || target_ctas <= 0) return 0;
+  const double few_fixed = 9.0, few_k_block = 0.39;     // 40 KB a k block of 64
+  const double many_fixed = 5.0, many_k_block = 0.31;   // a CTA pair that streams alone
+  const long pairs = target_ctas / 2 > 0 ? target_ctas / 2 : 1;
+  const long many_tiles = (long)((M + 255) / 256) * ((N + 255) / 256);
+  const int k_blocks = (K + BK - 1) / BK;
+  double many = many_fixed + (double)((many_tiles + pairs - 1) / pairs) * k_blocks * many_k_block;
+  if (2.0 * N * K / 6.5e6 > many) many = 2.0 * N * K / 6.5e6;  // W at the memory's rate
+  if (many <= few_fixed) return 0;
+  const Plan p = make_plan(M, N, K, DSP_BF16, target_ctas, N % 4 == 0);
+  const long rounds = p.splits > 1 ? 1 : (p.tiles + target_ctas - 1) / target_ctas;
+  return few_fixed + (double)rounds * p.kb_per_split * few_k_block < many;
+}
 
 #ifdef DSP_STAMPS
 namespace {
@@ -776,7 +895,6 @@ extern "C" int dsp_gemm_stream(const void* A, long lda, const void* W, const voi
               "dsp_gemm_stream: the rows under the norm must be 16-byte aligned (row stride %ld)", ld_src);
   DSP_REQUIRE(C2 == nullptr || (gain2 != nullptr && epilogue == EPI_PLAIN),
               "dsp_gemm_stream: the scaled second output needs a gain and the plain epilogue");
-  DSP_REQUIRE(M <= 128, "dsp_gemm_stream: M=%d above 128 rows", M);
   DSP_REQUIRE(M <= 64 || (norm_src == nullptr && C2 == nullptr),
               "dsp_gemm_stream: a norm split over two products takes at most 64 rows, got %d", M);
   DSP_REQUIRE(K > 0 && K % 8 == 0 && lda % 8 == 0, "dsp_gemm_stream: K=%d and the row stride must be multiples of 8", K);
@@ -793,17 +911,6 @@ extern "C" int dsp_gemm_stream(const void* A, long lda, const void* W, const voi
     DSP_CUDA(cudaGetDevice(&dev));
     DSP_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
   }
-  const int nb_rows = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
-  CUtensorMap map_w, map_x;
-  DSP_REQUIRE(make_map(&map_w, W, N, K, K, ROWS_W), "dsp_gemm_stream: cannot encode the tensor map of W");
-  DSP_REQUIRE(make_map(&map_x, A, M, K, lda, nb_rows), "dsp_gemm_stream: cannot encode the tensor map of A");
-  const int n_blocks = (N + ROWS_W - 1) / ROWS_W;
-  const int kb_total = (K + BK - 1) / BK;
-  if (target_ctas <= 0) target_ctas = num_sms;
-  int splits = target_ctas / n_blocks;
-  if (splits < 1) splits = 1;
-  if (splits > MAX_SPLITS) splits = MAX_SPLITS;
-  if (splits > kb_total) splits = kb_total;
   // the epilogues move four outputs at a time where rows and pointers allow 16-byte (32-bit output)
   // or 8-byte accesses; where they do not, K is not split and every thread stores single outputs
   const uintptr_t mask = out_dtype == DSP_F32 ? 15 : 7;
@@ -811,13 +918,15 @@ extern "C" int dsp_gemm_stream(const void* A, long lda, const void* W, const voi
                       (residual == nullptr || (ldr % 4 == 0 && ((uintptr_t)residual & mask) == 0)) &&
                       (bias == nullptr || ((uintptr_t)bias & 7) == 0) &&
                       (C2 == nullptr || (ldc2 % 4 == 0 && ((uintptr_t)C2 & mask) == 0 && ((uintptr_t)gain2 & 7) == 0));
-  if (!vec_ok) splits = 1;
-  const int kb_per_split = (kb_total + splits - 1) / splits;
-  splits = (kb_total + kb_per_split - 1) / kb_per_split;
+  const Plan plan = make_plan(M, N, K, out_dtype, target_ctas > 0 ? target_ctas : num_sms, vec_ok);
+  const int nb_rows = plan.nb_rows, tiles = plan.tiles, splits = plan.splits;
+  CUtensorMap map_w, map_x;
+  DSP_REQUIRE(make_map(&map_w, W, N, K, K, ROWS_W), "dsp_gemm_stream: cannot encode the tensor map of W");
+  DSP_REQUIRE(make_map(&map_x, A, M, K, lda, nb_rows), "dsp_gemm_stream: cannot encode the tensor map of A");
   Args a;
   a.stamp_base = -1;
 #ifdef DSP_STAMPS
-  a.stamp_base = stamp_next_base(splits > 1 ? (long)n_blocks * splits : (n_blocks < (nb_rows > 64 ? 1 : 2) * num_sms ? n_blocks : (nb_rows > 64 ? 1 : 2) * num_sms), N, K);
+  a.stamp_base = stamp_next_base(splits > 1 ? (long)tiles * splits : (tiles < (nb_rows > 64 ? 1 : 2) * num_sms ? tiles : (nb_rows > 64 ? 1 : 2) * num_sms), N, K);
 #endif
   a.bias = (const bf16*)bias;
   a.residual = residual;
@@ -827,7 +936,7 @@ extern "C" int dsp_gemm_stream(const void* A, long lda, const void* W, const voi
   a.M = M;
   a.N = N;
   a.K = K;
-  a.kb_per_split = kb_per_split;
+  a.kb_per_split = plan.kb_per_split;
   a.epilogue = epilogue;
   a.late_trigger = (late_trigger_bytes > 0 && (long)N * K * 2 >= late_trigger_bytes) ? 1 : 0;
   a.vec4 = vec_ok ? 1 : 0;
@@ -838,13 +947,15 @@ extern "C" int dsp_gemm_stream(const void* A, long lda, const void* W, const voi
   a.C2 = C2;
   a.ldc2 = ldc2;
   if (out_dtype == DSP_BF16) {
-    if (nb_rows == 16) return launch<16, bf16>(map_w, map_x, a, n_blocks, splits, num_sms, err, stream);
-    if (nb_rows == 32) return launch<32, bf16>(map_w, map_x, a, n_blocks, splits, num_sms, err, stream);
-    if (nb_rows == 64) return launch<64, bf16>(map_w, map_x, a, n_blocks, splits, num_sms, err, stream);
-    return launch<128, bf16>(map_w, map_x, a, n_blocks, splits, num_sms, err, stream);
+    if (nb_rows == 16) return launch<16, bf16>(map_w, map_x, a, tiles, splits, num_sms, err, stream);
+    if (nb_rows == 32) return launch<32, bf16>(map_w, map_x, a, tiles, splits, num_sms, err, stream);
+    if (nb_rows == 64) return launch<64, bf16>(map_w, map_x, a, tiles, splits, num_sms, err, stream);
+    if (nb_rows == 128) return launch<128, bf16>(map_w, map_x, a, tiles, splits, num_sms, err, stream);
+    return launch<192, bf16>(map_w, map_x, a, tiles, splits, num_sms, err, stream);
   }
-  if (nb_rows == 16) return launch<16, float>(map_w, map_x, a, n_blocks, splits, num_sms, err, stream);
-  if (nb_rows == 32) return launch<32, float>(map_w, map_x, a, n_blocks, splits, num_sms, err, stream);
-  if (nb_rows == 64) return launch<64, float>(map_w, map_x, a, n_blocks, splits, num_sms, err, stream);
-  return launch<128, float>(map_w, map_x, a, n_blocks, splits, num_sms, err, stream);
+  if (nb_rows == 16) return launch<16, float>(map_w, map_x, a, tiles, splits, num_sms, err, stream);
+  if (nb_rows == 32) return launch<32, float>(map_w, map_x, a, tiles, splits, num_sms, err, stream);
+  if (nb_rows == 64) return launch<64, float>(map_w, map_x, a, tiles, splits, num_sms, err, stream);
+  if (nb_rows == 128) return launch<128, float>(map_w, map_x, a, tiles, splits, num_sms, err, stream);
+  return launch<192, float>(map_w, map_x, a, tiles, splits, num_sms, err, stream);
 }
