@@ -32,6 +32,7 @@ CORE_SOURCES = [
     "gemm_stream.cu",
     "attn_generic.cu",
     "attn_combine.cu",
+    "dense_chain.cu",
     "sampling.cu",
     "random_fill.cu",
     "selftest.cu",

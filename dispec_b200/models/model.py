@@ -10,6 +10,7 @@ import torch
 
 from dispec_b200.cache.manager import CacheGroupSpec
 from dispec_b200.models.spec import LayerCall, ModelSpec
+from dispec_b200.ops import dense_chain
 from dispec_b200.parts.base import CacheNeed, Part, PartSpec, StateNeed
 from dispec_b200.registry import part_class
 
@@ -57,6 +58,7 @@ class DecoderModel:
             raise ValueError("the schedule marks the start of a pass but the model has no pass_entry part")
         self._parts = list(built.values())
         self.schedule: list[LayerCall] = list(spec.schedule)
+        self.dense_chain = False  # the layers run behind one call (ops/dense_chain.py), known once the weights are there
         self._plan_caches()
 
     # ------------------------------------------------------------------ cache planning
@@ -134,6 +136,7 @@ class DecoderModel:
         for part in self._parts:
             if hasattr(part, "prepare"):
                 part.prepare(device)
+        self.dense_chain = dense_chain.plan(self)
 
     # ----------------------------------------------------------------------- forward
     def forward(self, ctx):
@@ -141,6 +144,8 @@ class DecoderModel:
         output not yet added to it."""
         x = self.embedding.forward(ctx)
         pending = None
+        if self.dense_chain and getattr(ctx, "layer_trace", None) is None and dense_chain.run_layers(self, ctx, x):
+            return x, None
         # what the embedding gave, for passes that take it in again (the stream is updated in place)
         x0 = x.full.clone() if self.pass_entry is not None and self.pass_entry.needs_embedding else None
         trace = getattr(ctx, "layer_trace", None)

@@ -111,6 +111,11 @@ def raise_on_device_error(where: str) -> None:
         raise KernelError(f"{where}: device reported: {', '.join(names) or v}")
 
 
+def address_of(lib: ctypes.CDLL, name: str) -> int:
+    """Address of an entry point, for C code that calls it."""
+    return ctypes.cast(getattr(lib, name), ctypes.c_void_p).value
+
+
 def ptr(t) -> ctypes.c_void_p:
     return ctypes.c_void_p(0 if t is None else t.data_ptr())
 

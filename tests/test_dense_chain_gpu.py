@@ -1,0 +1,74 @@
+"""The layers behind one call give the bits that the parts give one by one."""
+import pytest
+import torch
+
+import replay_util as ru
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def model_of(**changes):
+    from dispec_b200 import load_model_config
+    from dispec_b200.weights import load_random_model
+    cfg = dict(ru.CONFIG_B)
+    cfg.update(changes)
+    return load_random_model(load_model_config(cfg), 3, 0.05, "bfloat16", DEV)
+
+
+def run(model, chain, lengths, steps, page_size, graph=False):
+    """A step that reads prompts of ``lengths`` together, then ``steps`` steps in which each takes a token, the last of
+    them beside a new prompt."""
+    from dispec_b200.engine import ModelRunner, SeqEntry
+    model.dense_chain = chain
+    runner = ModelRunner(model, page_size=page_size, num_pages=200, max_num_seqs=len(lengths) + 1, cuda_graph=graph)
+    ids = [ru.random_ids(n + steps + 1, model.spec.vocab_size, 5 + i) for i, n in enumerate(lengths)]
+    for i in range(len(lengths)):
+        runner.admit(i)
+    out = [runner.step([SeqEntry(i, s[:n], 0, [n - 1, n // 2]) for i, (s, n) in enumerate(zip(ids, lengths))]).clone()]
+    for t in range(steps):
+        entries = [SeqEntry(i, s[n + t:n + t + 1], n + t, [0]) for i, (s, n) in enumerate(zip(ids, lengths))]
+        if t == steps - 1:
+            runner.admit("late")
+            entries.append(SeqEntry("late", ru.random_ids(19, model.spec.vocab_size, 4), 0, [18]))
+        out.append(runner.step(entries).clone())
+    runner.check_device()
+    return out, runner
+
+
+@pytest.mark.parametrize("changes,lengths,page_size", [
+    ({}, [1], 16), ({}, [7, 3], 8), ({}, [63], 16), ({}, [64], 16), ({}, [65, 1], 32), ({}, [128], 16), ({}, [129], 8),
+    ({}, [300, 40, 2], 16),
+    (dict(tie_word_embeddings=True, num_attention_heads=4, num_key_value_heads=4), [33, 5], 16),
+    # a window in some layers, pages that the tiles of 128 rows do not take
+    (dict(use_sliding_window=True, sliding_window=24, max_window_layers=1), [90, 20], 16),
+    (dict(use_sliding_window=True, sliding_window=24, max_window_layers=1), [90, 20], 4),
+    (dict(head_dim=64, num_attention_heads=4, num_key_value_heads=2), [150, 9], 16),
+    (dict(head_dim=128, num_attention_heads=6, num_key_value_heads=1), [200], 16),
+    (dict(head_dim=80, num_attention_heads=4, num_key_value_heads=2), [70, 30], 16),
+])
+def test_same_bits_as_the_parts(changes, lengths, page_size):
+    from dispec_b200.ops.library import LaunchCounter
+    model = model_of(**changes)
+    assert model.dense_chain
+    n0 = LaunchCounter.n
+    mine, _ = run(model, True, lengths, 3, page_size)
+    n1 = LaunchCounter.n
+    parts, _ = run(model, False, lengths, 3, page_size)
+    assert LaunchCounter.n - n1 == n1 - n0
+    for a, b in zip(mine, parts):
+        assert torch.equal(a, b)
+
+
+def test_from_captured_steps():
+    model = model_of()
+    mine, runner = run(model, True, [40, 70, 12], 4, 16, graph=True)
+    assert runner._graphs
+    parts, _ = run(model, False, [40, 70, 12], 4, 16, graph=True)
+    for a, b in zip(mine, parts):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("changes", [dict(intermediate_size=232), dict(head_dim=24)])
+def test_sizes_that_stay_with_the_parts(changes):
+    assert not model_of(**changes).dense_chain
