@@ -165,6 +165,7 @@ def build_all(head_dims=(16, 32, 64, 128)) -> list[str]:
     libs += [mixer_library(name) for name in MIXER_LIBRARIES]
     # the attention with widths of their own for keys and values is compiled per pair of widths
     libs += [sink_attention_library(dk, dv) for dk, dv in ((64, 64), (128, 64), (128, 128))]
+    libs.append(latent_prompt_library(128, 128))
     return libs
 
 
@@ -179,6 +180,12 @@ def prefill_attention_library(head_dim: int) -> str:
 def sink_attention_library(key_dim: int, value_dim: int) -> str:
     """The tensor-core attention with a sink and widths of their own for keys and values."""
     return specialised_library(f"attn_sink_mma_k{key_dim}_v{value_dim}", "attn_sink_mma.cu",
+                               {"DSP_DK": key_dim, "DSP_DV": value_dim})
+
+
+def latent_prompt_library(key_dim: int, value_dim: int) -> str:
+    """The attention over a cached latent for portions of prompts, per unrotated key size and value size."""
+    return specialised_library(f"attn_latent_prompt_k{key_dim}_v{value_dim}", "attn_latent_prompt.cu",
                                {"DSP_DK": key_dim, "DSP_DV": value_dim})
 
 

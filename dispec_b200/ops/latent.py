@@ -125,10 +125,12 @@ def choose_key_splits(num_tiles: int, head_chunks: int, max_ctx: int, device) ->
 def latent_attention_tiles(ctx, q_absorbed: torch.Tensor, q: torch.Tensor, q_head_stride: int, qr_off: int,
                            inv_freq: torch.Tensor | None, rot: int, c_pool: torch.Tensor, r_pool: torch.Tensor,
                            page_table: torch.Tensor, num_heads: int, scale: float, layout: str = "interleaved",
-                           magnitude: float = 1.0, window: int = 0, sink: torch.Tensor | None = None) -> torch.Tensor:
+                           magnitude: float = 1.0, window: int = 0, sink: torch.Tensor | None = None,
+                           portions: bool = True) -> torch.Tensor:
     """The same attention on tensor cores (bfloat16 pools), over the step's tile list for
     ``mma_tokens_per_tile(num_heads)`` tokens a tile.  Single tokens (the first tiles) have their
-    keys cut into ranges that are merged by ``dsp_attn_combine``; portions of prompts run whole."""
+    keys cut into ranges that are merged by ``dsp_attn_combine``; portions of prompts run whole.
+    ``portions`` False: the rows are the step's single tokens only."""
     from dispec_b200.ops import attention as attn_ops
     num_pages, _, page_size, R = c_pool.shape
     r = r_pool.shape[3]
@@ -162,9 +164,70 @@ def latent_attention_tiles(ctx, q_absorbed: torch.Tensor, q: torch.Tensor, q_hea
                                               n_dec, num_heads, R, splits, L.dtype_code(out.dtype), L.stream_handle()))
         else:
             launch(0, n_dec, 1, None, None)
-    if n_tiles > n_dec:
+    if portions and n_tiles > n_dec:
         launch(n_dec, n_tiles - n_dec, 1, None, None)
     return out
+
+
+PROMPT_TOKENS_PER_TILE = 128  # tokens of one head of a tile of the kernel for portions of prompts
+PROMPT_ROT_DIM = 64  # size of the rotated key part it is built for
+PROMPT_MAX_BYTES = 1 << 30  # expanded keys and values a step may hold
+
+
+def prompt_supported(dim: int, rot_dim: int, vdim: int, kv_rank: int) -> bool:
+    """Sizes of the kernel that runs over expanded keys and values (``latent_attention_prompts``)."""
+    return dim in (64, 128) and vdim in (64, 128) and rot_dim == PROMPT_ROT_DIM and kv_rank % 8 == 0
+
+
+def expanded_keys(q_len: int, ctx_len: int, window: int) -> int:
+    """Keys of a sequence that a portion of ``q_len`` tokens has expanded."""
+    return ctx_len - (max(0, ctx_len - q_len - window + 1) // 64 * 64 if window > 0 else 0)
+
+
+def expanded_fits(q_lens: list, ctx_lens: list, row_bytes: int, window: int) -> bool:
+    """Whether a step's portions of prompts run on expanded keys and values: whenever those are no more than
+    ``PROMPT_MAX_BYTES``.  Measured on eight layers, 12 heads of 128 + 64 on latents of 512, a portion's whole step
+    (bound by the host below 1.8 ms): 2,048 tokens of a prompt 3.7 ms expanded and 5.9 on the latents, after 8,000
+    stored tokens 4.5 and 17.8; 128 tokens 1.74 and 1.80, after 8,000 2.0 and 5.6; 8 tokens after 2,000 1.8 and 2.1,
+    after 16,000 2.1 and 9.3; 8 tokens alone the same."""
+    return row_bytes * sum(expanded_keys(q, c, window) for q, c in zip(q_lens, ctx_lens)) <= PROMPT_MAX_BYTES
+
+
+def latent_attention_prompts(ctx, q: torch.Tensor, q_head_stride: int, qr_off: int, inv_freq: torch.Tensor | None,
+                             rot: int, c_pool: torch.Tensor, r_pool: torch.Tensor, page_table: torch.Tensor,
+                             w_kv: torch.Tensor, out: torch.Tensor, num_heads: int, dim: int, vdim: int, scale: float,
+                             layout: str = "interleaved", magnitude: float = 1.0, window: int = 0,
+                             sink: torch.Tensor | None = None, gate: torch.Tensor | None = None) -> None:
+    """The attention of the step's portions of prompts, with the value map applied, into their rows of ``out``
+    [T, H * vdim] (bfloat16).  ``w_kv`` [H * (dim + vdim), R]: every head's key map, then every head's value
+    map; the latents of the keys the portions see are gathered from the pages and expanded by one product."""
+    from dispec_b200.ops import gemm
+    num_pages, _, page_size, R = c_pool.shape
+    n_dec = ctx.num_decode_seqs
+    q_lens, ctx_lens = ctx.host_q_len[n_dec:], ctx.host_ctx_len[n_dec:]
+    keys = [expanded_keys(a, b, window) for a, b in zip(q_lens, ctx_lens)]
+    rows, max_tiles, S = sum(keys), max(-(-k // 64) for k in keys), len(keys)
+    assert q.dtype == out.dtype == c_pool.dtype == r_pool.dtype == w_kv.dtype == torch.bfloat16
+    assert q.stride(1) == 1 and out.stride(1) == 1 and c_pool.is_contiguous() and r_pool.is_contiguous()
+    assert w_kv.shape == (num_heads * (dim + vdim), R) and r_pool.shape[3] == PROMPT_ROT_DIM
+    assert page_table.dtype == torch.int32 and page_table.stride(1) == 1
+    assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1 and gate.shape == out.shape)
+    _checked_sink(sink, num_heads)
+    lib = L.latent_prompt_library(dim, vdim)
+    c_rows = torch.empty((rows, R), dtype=torch.bfloat16, device=q.device)
+    r_rows = torch.empty((rows, PROMPT_ROT_DIM), dtype=torch.bfloat16, device=q.device)
+    bad = torch.empty((S, max_tiles), dtype=torch.int64, device=q.device)
+    L.check(lib.dsp_latent_gather(
+        L.ptr(c_pool), L.ptr(r_pool), L.ptr(page_table), page_table.stride(0), L.ptr(ctx.q_start), L.ptr(ctx.ctx_len),
+        n_dec, S, int(window), L.ptr(c_rows), L.ptr(r_rows), L.ptr(bad), max_tiles, R, page_size, num_pages,
+        L.stream_handle()))
+    kv = gemm.linear(c_rows, w_kv)
+    tile_seq, tile_tok0, n_tiles = ctx.attention_tiles[PROMPT_TOKENS_PER_TILE]
+    L.check(lib.dsp_attn_latent_prompt(
+        L.ptr(q), L.i64(q.stride(0)), q_head_stride, qr_off, L.ptr(inv_freq), rot, _LAYOUTS[layout], L.f32(magnitude),
+        L.ptr(kv), L.ptr(r_rows), L.i64(rows), L.ptr(ctx.q_start), L.ptr(ctx.ctx_len), L.ptr(tile_seq), L.ptr(tile_tok0),
+        n_dec, n_tiles - n_dec, n_dec, int(window), L.ptr(bad), max_tiles, L.ptr(out), L.i64(out.stride(0)), L.ptr(gate),
+        L.i64(gate.stride(0) if gate is not None else 0), L.ptr(sink), num_heads, L.f32(scale), L.stream_handle()))
 
 
 def head_products_supported(x: torch.Tensor, head_stride: int, w: torch.Tensor) -> bool:

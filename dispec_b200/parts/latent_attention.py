@@ -50,7 +50,7 @@ class LatentAttention(JoinableMixer):
         self.window, self.gate = int(window), gate
         self.sink, self.own_latent = bool(sink), bool(own_latent)
         self.out_columns = num_heads * vdim
-        self.sink_values = self.c_gain = None
+        self.sink_values = self.c_gain = self.w_kv = None
 
     def tensor_specs(self):
         h, H, d, r, dv, R, Q = (self.hidden_size, self.num_heads, self.dim, self.rot_dim, self.vdim,
@@ -80,6 +80,10 @@ class LatentAttention(JoinableMixer):
         # qa_h = q_plain_h W_uk_h, i.e. x W^T with W = W_uk_h^T [R, d]
         self.w_uk_t = tensors["uk.weight"].view(H, d, R).transpose(1, 2).contiguous()
         self.w_uv = tensors["uv.weight"].view(H, self.vdim, R).contiguous()
+        # both maps as one product that expands latents to every head's key, then every head's value
+        self.w_kv = None
+        if tensors["uk.weight"].dtype == torch.bfloat16 and latent_ops.prompt_supported(d, self.rot_dim, self.vdim, R):
+            self.w_kv = torch.cat([tensors["uk.weight"], tensors["uv.weight"]], dim=0).contiguous()
         self.w_o = tensors["o.weight"]
 
     def cache_need(self):
@@ -87,7 +91,10 @@ class LatentAttention(JoinableMixer):
                          self.window)
 
     def tokens_per_attention_tile(self):
-        return latent_ops.mma_tokens_per_tile(self.num_heads)
+        tokens = latent_ops.mma_tokens_per_tile(self.num_heads)
+        if latent_ops.prompt_supported(self.dim, self.rot_dim, self.vdim, self.kv_rank):
+            return tokens, latent_ops.PROMPT_TOKENS_PER_TILE
+        return tokens
 
     def heads(self, ctx, down, cache, state, out):
         H, d, r, dv, R, Q = self.num_heads, self.dim, self.rot_dim, self.vdim, self.kv_rank, self.q_rank
@@ -106,6 +113,23 @@ class LatentAttention(JoinableMixer):
         else:
             cq = norm32_ops.sum_norm(down[:, :Q], self.q_gain, self.eps, out_dtype=out.dtype, want32=False)[1]
         q = ops.linear(cq, self.w_uq)  # [T, H * (d + r)]
+        gate = down[:, down.shape[1] - H * dv:] if self.gate else None
+        n_dec = ctx.num_decode_seqs
+        if (self.w_kv is not None and T > n_dec and c_pool.dtype == torch.bfloat16 and out.dtype == torch.bfloat16
+                and latent_ops.PROMPT_TOKENS_PER_TILE in ctx.attention_tiles
+                and latent_ops.mma_supported(R, r, c_pool.dtype) and latent_ops.mma_tokens_per_tile(H) in ctx.attention_tiles
+                and latent_ops.expanded_fits(ctx.host_q_len[n_dec:], ctx.host_ctx_len[n_dec:], 2 * H * (d + dv),
+                                             self.window)):
+            # portions of prompts on expanded keys and values; the single tokens, if any, on the latents
+            latent_ops.latent_attention_prompts(ctx, q, d + r, d, inv_freq, rot_n, c_pool, r_pool, cache.page_table,
+                                                self.w_kv, out, H, d, dv, scale, window=self.window,
+                                                sink=self.sink_values, gate=gate, **turn)
+            if n_dec == 0:
+                return
+            q, out, gate, T = q[:n_dec], out[:n_dec], gate[:n_dec] if gate is not None else None, n_dec
+            portions = False
+        else:
+            portions = True
         qa = torch.empty((T, H * R), dtype=torch.float32, device=down.device)
         if latent_ops.head_products_supported(q, d + r, self.w_uk_t):
             latent_ops.head_products(q, d + r, self.w_uk_t, qa, R)
@@ -116,12 +140,11 @@ class LatentAttention(JoinableMixer):
                 and latent_ops.mma_tokens_per_tile(H) in ctx.attention_tiles):
             mixed = latent_ops.latent_attention_tiles(ctx, qa, q, d + r, d, inv_freq, rot_n, c_pool, r_pool,
                                                       cache.page_table, H, scale, window=self.window,
-                                                      sink=self.sink_values, **turn)
+                                                      sink=self.sink_values, portions=portions, **turn)
         else:  # the 32-bit path, and sizes the tensor-core kernel is not built for
             mixed = latent_ops.latent_attention(qa, q, d + r, d, inv_freq, rot_n, c_pool, r_pool, cache.page_table,
                                                 ctx.positions, ctx.seq_of_token, H, scale, out.dtype,
                                                 window=self.window, sink=self.sink_values, **turn)
-        gate = down[:, down.shape[1] - H * dv:] if self.gate else None
         if latent_ops.head_products_supported(mixed, R, self.w_uv):
             latent_ops.head_products(mixed, R, self.w_uv, out, dv, gate=gate)  # the gate rides in the epilogue
         else:
