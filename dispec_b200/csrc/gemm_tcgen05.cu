@@ -587,6 +587,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 }  // namespace
 
 // bfloat16 A [M, K] (row stride lda) and W [N, K] (contiguous); C and residual bfloat16 or float32.
+// pair_mode 0: single CTAs; 1: CTA pairs; 2, 3: pairs with tiles 192, 256 wide (comparisons).
 // epilogue 1: SwiGLU (2: gelu in its tanh form instead of silu) over W rows alternating in blocks of 16 (16 gate rows, their 16 up rows):
 // C is [M, N/2], no bias, no residual.
 extern "C" int dsp_gemm_tcgen05(const void* A, long lda, const void* W, const void* bias, const void* residual,
@@ -621,15 +622,14 @@ extern "C" int dsp_gemm_tcgen05(const void* A, long lda, const void* W, const vo
     DSP_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
   }
   if (pair_mode) {
-    // tile width: 256, or 192 when that puts more of the CTA pairs to work in the last round
-    // (cost ~ rounds x width; N 1536 on 74 pairs: 48 tiles of 256 against 64 tiles of 192)
+    // Tile width: 256, or 192 where that takes no more rounds over the CTA pairs.  A round of the narrower tiles
+    // takes 0.92 of the time of a round of the wider ones, not 0.75: at full load the k blocks come at the pace
+    // of the L2 (0.355 and 0.387 us each).  192 and 256 wide: 1,024 rows x 1,536 x 1,536 (one round each) 15.2 and
+    // 17.1 us; 4,500 rows x 17,920 x 1,536 (23 rounds and 18) 196 and 167; 2,500 rows x 1,536 x 8,960 (2 and 1) 93 and 58.
     const long pairs_avail = num_sms / 2;
     const long m_tiles2 = (M + 2 * BM - 1) / (2 * BM);
-    auto cost = [&](int bn) {
-      const long tiles2 = (long)((N + bn - 1) / bn) * m_tiles2;
-      return ((tiles2 + pairs_avail - 1) / pairs_avail) * bn;
-    };
-    const int bnp = cost(192) < cost(256) ? 192 : 256;
+    auto rounds = [&](int bn) { return ((long)((N + bn - 1) / bn) * m_tiles2 + pairs_avail - 1) / pairs_avail; };
+    const int bnp = pair_mode == 2 ? 192 : pair_mode == 3 ? 256 : 0.92 * rounds(192) < rounds(256) ? 192 : 256;
     e.k_boxes = (make_map_k_blocks(&map_a, A, M, K, lda, BM, SUB) && make_map_k_blocks(&map_w, W, N, K, K, bnp / 2, SUB)) ? 1 : 0;
     if (!e.k_boxes) {
       DSP_REQUIRE(make_map(&map_a, A, M, K, lda, BM), "dsp_gemm_tcgen05: cannot encode the tensor map of A");
