@@ -15,7 +15,7 @@ int dsp_rmsnorm(void* x, const void* delta, const void* w, void* y, const int* r
                 int write_back, int dtype, cudaStream_t stream);
 int dsp_rope_kv_store(void* qkv, const int* positions, const int* seq_of_token, const int* page_table, int pt_stride,
                       void* k_pool, void* v_pool, const float* inv_freq, int T, int H, int KVH, int D, int rotary_dim,
-                      int page_size, int num_pages, int write_kv, int dtype, cudaStream_t stream);
+                      int page_size, int num_pages, int write_kv, int early, int dtype, cudaStream_t stream);
 int dsp_gemm_stream(const void* A, long lda, const void* W, const void* bias, const void* residual, long ldr, void* C,
                     long ldc, int M, int N, int K, int out_dtype, int target_ctas, int epilogue, long late_trigger_bytes,
                     const void* norm_src, long ld_src, float norm_eps, const void* gain2, void* C2, long ldc2,
@@ -106,7 +106,7 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
       DSP_STEP(dsp_rope_kv_store((bf16*)s.qkv + (size_t)first * wide, s.positions + first, s.seq_of_token + first,
                                  l.page_table, (int)l.pt_stride, l.write_kv ? l.k_pool : nullptr,
                                  l.write_kv ? l.v_pool : nullptr, l.inv_freq, T - first, H, KVH, D, (int)s.rotary_dim,
-                                 l.write_kv ? (int)s.page_size : 1, l.write_kv ? (int)l.num_pages : 0, (int)l.write_kv,
+                                 l.write_kv ? (int)s.page_size : 1, l.write_kv ? (int)l.num_pages : 0, (int)l.write_kv, 1,
                                  DSP_BF16, stream));
     auto mma = [&](int offset, int tiles, int splits, bool single) -> int {
       const bool fused = single && s.fused_rope, ranges = single && s.outer > 1;

@@ -82,7 +82,10 @@ def run_layers(model, ctx, x: torch.Tensor) -> bool:
     fused = attn_ops.decode_rope_fusable(ctx, H, KVH, D, rotary_dim, x.dtype)
 
     new = lambda columns: torch.empty((T, columns), dtype=x.dtype, device=dev)
-    h, qkv, heads, act = new(hidden), new((H + 2 * KVH) * D), new(H * D), new(inter)
+    # normed rows are dead when attention writes its heads, the q/k/v rows when the feed-forward writes its units:
+    # two buffers for the four keep more of a long portion in the L2
+    h = heads = new(max(hidden, H * D))
+    qkv = act = new(max((H + 2 * KVH) * D, inter))
     scaled_a = scaled_b = None
     if T <= gemm.NORM_SPLIT_MAX_ROWS:  # norms are split over the products around them
         scaled_a, scaled_b = new(hidden), new(hidden)

@@ -104,7 +104,7 @@ def rope_kv_store(qkv: torch.Tensor, positions: torch.Tensor, seq_of_token: torc
     L.check(L.core().dsp_rope_kv_store(
         L.ptr(qkv), L.ptr(positions), L.ptr(seq_of_token), L.ptr(page_table), page_table.stride(0),
         L.ptr(k_pool), L.ptr(v_pool), L.ptr(inv_freq), T, num_heads, num_kv_heads, head_dim,
-        rotary_dim, page_size, num_pages, int(write_kv), L.dtype_code(qkv.dtype), L.stream_handle()))
+        rotary_dim, page_size, num_pages, int(write_kv), 0, L.dtype_code(qkv.dtype), L.stream_handle()))
 
 
 def fill_normal(out: torch.Tensor, seed: int, ordinal: int, std: float, mean: float = 0.0,

@@ -1,4 +1,4 @@
-"""The norm of a sum four elements at a time, attention with a sink and a gate over tiles of 128 rows."""
+"""The norm of a sum four elements at a time, the RMS norm a warp a row, attention with a sink and a gate over tiles of 128 rows."""
 import pytest
 import torch
 
@@ -29,6 +29,42 @@ def test_sum_norm(width, x_dtype, off):
         tol = (width + 10) * U * (want.abs() + (alpha * x.double().abs().max() + delta.double().abs().max()) * U)
         assert ((y32.double() - want).abs() <= tol + 4 * U).all()
         assert torch.equal(y16, y32.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 4), (3, 2048), (2, 2052), (5, 8960), (2500, 60), (4, 66)])
+def test_xielu_rows(rows, cols):
+    from dispec_b200.ops import norm32
+    z = rnd((rows, cols + 4), 14, 3.0)[:, :cols]
+    p, q = 0.4, -0.7
+    y = norm32.xielu(z, torch.tensor([p, q], device=DEV), torch.bfloat16).double()
+    sp = lambda v: torch.log1p(torch.exp(torch.tensor(v, dtype=torch.float64, device=DEV)))
+    v = z.double()
+    want = torch.where(v > 0, sp(p) * v * v, (0.5 + sp(q)) * (torch.expm1(v.clamp(max=0)) - v)) + 0.5 * v
+    # rounded to bfloat16 once (2^-8 with what 32 bits leave open); the two terms below zero nearly cancel
+    assert ((y - want).abs() <= 2.0 ** -8 * want.abs() + 32 * U * (1 + v.abs())).all()
+
+
+@pytest.mark.parametrize("n,hidden", [(592, 1536), (593, 8), (600, 1032), (595, 1544), (700, 768), (591, 1536)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_rms_norm_of_many_rows(n, hidden, dtype):
+    from dispec_b200 import ops
+    x, w, delta = rnd((n, hidden), 11, 2.0, dtype), (1.0 + rnd((hidden,), 12, 0.2)).to(dtype), rnd((n, hidden), 13, 1.0, dtype)
+    rows = torch.arange(n - 1, -1, -1, dtype=torch.int32, device=DEV)
+
+    def want(v):
+        unit = (v.double() / torch.sqrt((v.double() ** 2).mean(-1, keepdim=True) + 1e-6)).to(dtype)
+        return w.double() * unit.double()
+
+    # a unit row may round the other way, which is one unit in its last place (2^-7 of it at most in bfloat16), and the
+    # product is rounded once (2^-8)
+    tol = (2.0 ** -7 + 2.0 ** -8 if dtype == torch.bfloat16 else (hidden + 10) * U)
+    close = lambda y, v: ((y.double() - want(v)).abs() <= tol * (want(v).abs() + 1e-3)).all()
+    assert close(ops.rms_norm(x, w, 1e-6), x)
+    assert torch.equal(ops.rms_norm(x, w, 1e-6, rows=rows), ops.rms_norm(x, w, 1e-6).flip(0))
+    total = (x.double() + delta.double()).to(dtype)
+    y = x.clone()
+    out = ops.rms_norm(y, w, 1e-6, delta=delta, write_back=True)
+    assert torch.equal(y, total) and close(out, total)
 
 
 @pytest.mark.parametrize("spans,H,G,D,page,window,sink,gate", [
