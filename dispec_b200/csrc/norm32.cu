@@ -168,29 +168,41 @@ xielu_kernel(const void* __restrict__ z, int z_dtype, long ldz, const float* __r
              void* __restrict__ y, int y_dtype, long ldy, long rows, int cols) {
   const float ap = softplus_f(pq[0]), an = 0.5f + softplus_f(pq[1]);
   auto act = [&](float v) { return v > 0.f ? fmaf(ap * v, v, 0.5f * v) : fmaf(an, expm1f(v) - v, 0.5f * v); };
-  // four elements a thread where rows are whole groups of four on 16-byte (8-byte) pieces
-  const bool vec = z_dtype == DSP_F32 && y_dtype == DSP_BF16 && cols % 4 == 0 && ldz % 4 == 0 && ldy % 4 == 0 &&
-                   ((uintptr_t)z % 16) == 0 && ((uintptr_t)y % 8) == 0;
-  if (vec) {
-    const int c4 = cols / 4;
-    const long n = rows * c4;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-      const long r = i / c4;
-      const int c = (int)(i % c4) * 4;
-      const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(z) + (size_t)r * ldz + c);
-      __nv_bfloat162 lo = __floats2bfloat162_rn(act(v.x), act(v.y)), hi = __floats2bfloat162_rn(act(v.z), act(v.w));
-      uint2 out;
-      out.x = *reinterpret_cast<uint32_t*>(&lo);
-      out.y = *reinterpret_cast<uint32_t*>(&hi);
-      *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(y) + (size_t)r * ldy + c) = out;
-    }
-    return;
-  }
   const long n = rows * cols;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const long r = i / cols;
     const int c = (int)(i % cols);
     st_any(y, y_dtype, (size_t)r * ldy + c, act(ld_any(z, z_dtype, (size_t)r * ldz + c)));
+  }
+}
+
+// The same from floats to bfloat16 where rows are whole groups of four on 16-byte (8-byte) pieces: a block takes
+// stretches of 4 * GROUPS * blockDim columns of rows blockIdx.y, blockIdx.y + gridDim.y, ..., a thread GROUPS groups
+// of a row at once (no division of an index; four loads on their way).  2,500 rows of 8,960: 135 MB in 40.9 us (45.5
+// with one group at a time from a running index, whose 64-bit divisions were most of its instructions).
+constexpr int XIELU_GROUPS = 4;
+__global__ void __launch_bounds__(128)
+xielu_rows_kernel(const float* __restrict__ z, long ldz, const float* __restrict__ pq, bf16* __restrict__ y, long ldy,
+                  long rows, int cols) {
+  const float ap = softplus_f(pq[0]), an = 0.5f + softplus_f(pq[1]);
+  auto act = [&](float v) { return v > 0.f ? fmaf(ap * v, v, 0.5f * v) : fmaf(an, expm1f(v) - v, 0.5f * v); };
+  const int c0 = (blockIdx.x * XIELU_GROUPS * blockDim.x + threadIdx.x) * 4, step = blockDim.x * 4;
+  for (long r = blockIdx.y; r < rows; r += gridDim.y) {
+    const float* src = z + (size_t)r * ldz;
+    bf16* dst = y + (size_t)r * ldy;
+    float4 v[XIELU_GROUPS];
+#pragma unroll
+    for (int g = 0; g < XIELU_GROUPS; ++g)
+      if (c0 + g * step < cols) v[g] = *reinterpret_cast<const float4*>(src + c0 + g * step);
+#pragma unroll
+    for (int g = 0; g < XIELU_GROUPS; ++g) {
+      if (c0 + g * step >= cols) break;
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(act(v[g].x), act(v[g].y)), hi = __floats2bfloat162_rn(act(v[g].z), act(v[g].w));
+      uint2 out;
+      out.x = *reinterpret_cast<const uint32_t*>(&lo);
+      out.y = *reinterpret_cast<const uint32_t*>(&hi);
+      *reinterpret_cast<uint2*>(dst + c0 + g * step) = out;
+    }
   }
 }
 
@@ -463,6 +475,14 @@ extern "C" int dsp_xielu(const void* z, int z_dtype, long ldz, const float* pq, 
   DSP_REQUIRE(z && pq && y, "dsp_xielu: missing operand");
   const long n = rows * cols;
   const int sms = dsp_num_sms();
+  if (z_dtype == DSP_F32 && y_dtype == DSP_BF16 && cols % 4 == 0 && whole_groups(z, z_dtype, ldz) && whole_groups(y, y_dtype, ldy)) {
+    const int across = (cols + 4 * XIELU_GROUPS * 128 - 1) / (4 * XIELU_GROUPS * 128);
+    const long fill = (long)(sms > 0 ? sms : 148) * 16 / across + 1, down = rows < fill ? rows : fill;
+    DSP_CUDA(launch_plain(xielu_rows_kernel, dim3(across, (unsigned)(down < 65535 ? down : 65535)), dim3(128), 0, stream,
+                          (const float*)z, ldz, pq, (bf16*)y, ldy, rows, cols));
+    DSP_CHECK_LAUNCH("dsp_xielu");
+    return 0;
+  }
   const long want = (n + 255) / 256, cap = (long)(sms > 0 ? sms : 148) * 16;
   DSP_CUDA(launch_plain(xielu_kernel, dim3((unsigned)(want < cap ? want : cap)), dim3(256), 0, stream, z,
                       z_dtype, ldz, pq, y, y_dtype, ldy, rows, cols));
