@@ -202,7 +202,8 @@ attn_generic_kernel(const T* __restrict__ q, long q_stride, const T* __restrict_
 //
 // What bounds it: shared-memory reads (eight 16-byte reads a thread per 64 products of the scores, twelve per
 // 128 of the sums).  260 tokens of a prompt beside four single tokens at 330, 12 heads of 128 on 2 KV heads:
-// 112 us; 299 with a block per token whose threads each walk a key of their own through global memory.
+// 93 us; 112 with the page table read and indices divided for every copied piece, 299 with a block per token whose
+// threads each walk a key of their own through global memory.
 constexpr int TILE_KEYS = 64, MAX_DIM = 128;
 
 struct RowsArgs {
@@ -245,7 +246,7 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
   float* ks = qs + R * LK;              // [TILE_KEYS][LK]
   float* vs = ks + TILE_KEYS * LK;      // [TILE_KEYS][LV]
   float* ps = vs + TILE_KEYS * LV;      // [R][LP]
-  int* bad = (int*)(ps + R * LP);       // [2][TILE_KEYS] 1: the key's page id was outside the pool
+  long* slot = (long*)(ps + R * LP);    // [2][TILE_KEYS] row of each key of a tile in the pools, -1: none
   const int* table = a.page_table + (size_t)seq * a.pt_stride;
   const int last = pos0 + n - 1;
 
@@ -265,35 +266,34 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
     if (there) src += (size_t)(t0 + r / gn) * a.q_stride + (size_t)(kvh * G + g0 + r % gn) * D + d;
     bring4(qs + r * LK + d, src, there);
   }
-  auto bring_keys = [&](int i) {
-    const int kt = tile_start(i);
-    for (int p = tid; p < TILE_KEYS * (D / 4); p += THREADS) {
-      const int j = p / (D / 4), d = p % (D / 4) * 4, key = kt + j;
-      const int page = key <= last ? table[key / a.page_size] : -1;
-      const bool there = page >= 0 && page < a.num_pages;
-      if (d == 0) {
-        bad[(i & 1) * TILE_KEYS + j] = !there;
-        // a page the window has passed is gone from the table; one that some token still sees must be there
-        if (!there && key <= last && (key >= lo || key < a.keep_first)) atomicOr(a.err, DSP_ERR_BAD_PAGE);
+  // Where the keys of tile i lie: thread j < TILE_KEYS asks the page table for key j (`find`) and writes the answer
+  // down for all (`note`), a tile ahead, so that nobody waits for the table between the tiles.
+  auto find = [&](int i) -> long {
+    const int key = tile_start(i) + tid;
+    if (tid >= TILE_KEYS || key > last) return -1;
+    const int page = table[key / a.page_size];
+    if (page >= 0 && page < a.num_pages) return ((long)page * a.KVH + kvh) * a.page_size + key % a.page_size;
+    // a page the window has passed is gone from the table; one that some token still sees must be there
+    if (key >= lo || key < a.keep_first) atomicOr(a.err, DSP_ERR_BAD_PAGE);
+    return -1;
+  };
+  auto note = [&](int i, long at) {
+    if (tid < TILE_KEYS) slot[(i & 1) * TILE_KEYS + tid] = at;
+  };
+  // a warp copies whole rows, a lane 16 bytes (8 of bfloat16) of each
+  const int lane = tid & 31, warp = tid >> 5;
+  auto bring = [&](int i, const T* pool, int width, float* to, int ld) {
+    if (lane < width / 4) {
+#pragma unroll 2
+      for (int j = warp; j < TILE_KEYS; j += THREADS / 32) {
+        const long at = slot[(i & 1) * TILE_KEYS + j];
+        bring4(to + j * ld + lane * 4, at >= 0 ? pool + at * width + lane * 4 : pool, at >= 0);
       }
-      const T* src = (const T*)a.k_pool;
-      if (there) src += (((size_t)page * a.KVH + kvh) * a.page_size + key % a.page_size) * D + d;
-      bring4(ks + j * LK + d, src, there);
     }
     end_group();
   };
-  auto bring_values = [&](int i) {
-    const int kt = tile_start(i);
-    for (int p = tid; p < TILE_KEYS * (Dv / 4); p += THREADS) {
-      const int j = p / (Dv / 4), d = p % (Dv / 4) * 4, key = kt + j;
-      const int page = key <= last ? table[key / a.page_size] : -1;
-      const bool there = page >= 0 && page < a.num_pages;
-      const T* src = (const T*)a.v_pool;
-      if (there) src += (((size_t)page * a.KVH + kvh) * a.page_size + key % a.page_size) * Dv + d;
-      bring4(vs + j * LV + d, src, there);
-    }
-    end_group();
-  };
+  auto bring_keys = [&](int i) { bring(i, (const T*)a.k_pool, D, ks, LK); };
+  auto bring_values = [&](int i) { bring(i, (const T*)a.v_pool, Dv, vs, LV); };
 
   float m[RI], l[RI], acc[RI][4 * DJ];
   int pos[RI], low[RI];
@@ -307,10 +307,13 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
 #pragma unroll
     for (int d = 0; d < 4 * DJ; ++d) acc[i][d] = 0.f;
   }
+  note(0, find(0));
+  __syncthreads();
   bring_keys(0);
   bring_values(0);
   for (int t = 0; t < ntiles; ++t) {
     const int kt = tile_start(t);
+    const long next = t + 1 < ntiles ? find(t + 1) : -1;
     wait_groups<1>();
     __syncthreads();
     float s[RI][KJ];
@@ -337,7 +340,7 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
 #pragma unroll
       for (int j = 0; j < KJ; ++j) {
         const int key = kt + tx + j * TX;
-        const bool seen = key <= pos[i] && (key >= low[i] || key < a.keep_first) && !bad[(t & 1) * TILE_KEYS + tx + j * TX];
+        const bool seen = key <= pos[i] && (key >= low[i] || key < a.keep_first) && slot[(t & 1) * TILE_KEYS + tx + j * TX] >= 0;
         s[i][j] = seen ? s[i][j] * a.scale : -INFINITY;
         top = fmaxf(top, s[i][j]);
       }
@@ -360,6 +363,7 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
 #pragma unroll
       for (int d = 0; d < 4 * DJ; ++d) acc[i][d] *= alpha;
     }
+    note(t + 1, next);  // (the slots of tile t - 1, which all have left)
     __syncthreads();  // the keys have been read
     if (t + 1 < ntiles) bring_keys(t + 1); else end_group();
     wait_groups<1>();
@@ -452,7 +456,7 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(const RowsArgs a) {
 template <typename T>
 int launch_rows(const RowsArgs& a, cudaStream_t stream) {
   const size_t smem = (size_t)((ROWS + TILE_KEYS) * (a.D + 4) + TILE_KEYS * (a.Dv + 4) + ROWS * (TILE_KEYS + 4)) * sizeof(float) +
-                      2 * TILE_KEYS * sizeof(int);
+                      2 * TILE_KEYS * sizeof(long);
   DSP_CUDA(cudaFuncSetAttribute(attn_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   attn_rows_kernel<T><<<dim3(a.T, a.KVH), THREADS, smem, stream>>>(a);
   DSP_CHECK_LAUNCH("dsp_attn_generic");
