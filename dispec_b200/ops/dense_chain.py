@@ -55,7 +55,11 @@ def plan(model) -> bool:
 
 
 def run_layers(model, ctx, x: torch.Tensor) -> bool:
-    """Runs the layers on the rows ``x`` in place; False (nothing has run) where this step is not for it."""
+    """Runs the layers on the rows ``x`` in place; False (nothing has run) where this step is not for it.  A step that
+    is being captured is not: its launches are replayed from the graph, whoever made them, and one row a step was
+    1.5 % slower on this function's buffers (950 us against 935) than on those of the parts."""
+    if ctx.graph_capture:
+        return False
     block = model.layers[model.schedule[0].layer]
     mixer, ff = block.mixer, block.feed_forward
     H, KVH, D, hidden, inter = (mixer.num_heads, mixer.num_kv_heads, mixer.head_dim, mixer.hidden_size,
