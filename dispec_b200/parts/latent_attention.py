@@ -114,22 +114,24 @@ class LatentAttention(JoinableMixer):
             cq = norm32_ops.sum_norm(down[:, :Q], self.q_gain, self.eps, out_dtype=out.dtype, want32=False)[1]
         q = ops.linear(cq, self.w_uq)  # [T, H * (d + r)]
         gate = down[:, down.shape[1] - H * dv:] if self.gate else None
-        n_dec = ctx.num_decode_seqs
+        n_dec, portions = ctx.num_decode_seqs, True
         if (self.w_kv is not None and T > n_dec and c_pool.dtype == torch.bfloat16 and out.dtype == torch.bfloat16
                 and latent_ops.PROMPT_TOKENS_PER_TILE in ctx.attention_tiles
                 and latent_ops.mma_supported(R, r, c_pool.dtype) and latent_ops.mma_tokens_per_tile(H) in ctx.attention_tiles
                 and latent_ops.expanded_fits(ctx.host_q_len[n_dec:], ctx.host_ctx_len[n_dec:], 2 * H * (d + dv),
                                              self.window)):
             # portions of prompts on expanded keys and values; the single tokens, if any, on the latents
-            latent_ops.latent_attention_prompts(ctx, q, d + r, d, inv_freq, rot_n, c_pool, r_pool, cache.page_table,
-                                                self.w_kv, out, H, d, dv, scale, window=self.window,
-                                                sink=self.sink_values, gate=gate, **turn)
-            if n_dec == 0:
+            try:
+                latent_ops.latent_attention_prompts(ctx, q, d + r, d, inv_freq, rot_n, c_pool, r_pool, cache.page_table,
+                                                    self.w_kv, out, H, d, dv, scale, window=self.window,
+                                                    sink=self.sink_values, gate=gate, **turn)
+                portions = False
+            except torch.OutOfMemoryError:
+                pass  # no room beside the pools for the expanded rows: on the latents, which need none
+            if not portions and n_dec == 0:
                 return
-            q, out, gate, T = q[:n_dec], out[:n_dec], gate[:n_dec] if gate is not None else None, n_dec
-            portions = False
-        else:
-            portions = True
+            if not portions:
+                q, out, gate, T = q[:n_dec], out[:n_dec], gate[:n_dec] if gate is not None else None, n_dec
         qa = torch.empty((T, H * R), dtype=torch.float32, device=down.device)
         if latent_ops.head_products_supported(q, d + r, self.w_uk_t):
             latent_ops.head_products(q, d + r, self.w_uk_t, qa, R)

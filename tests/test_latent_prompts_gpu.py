@@ -132,8 +132,8 @@ def test_a_bad_page_is_hidden_and_reported():
     assert (out[29].double().cpu() - want).abs().max() < 0.02 * max(1.0, want.abs().max().item())
 
 
-def test_mixers_of_both_kinds_agree():
-    """A small model's logits with its portions on expanded keys and on the latents."""
+def small_model_logits(expand):
+    """Logits of two steps of a small model with portions of prompts and single tokens."""
     from dispec_b200 import load_model_config
     from dispec_b200.engine import ModelRunner, SeqEntry
     from dispec_b200.ops import latent as LO
@@ -146,20 +146,32 @@ def test_mixers_of_both_kinds_agree():
     model = load_random_model(load_model_config(cfg), 1, 0.1, "bfloat16", DEV)
     g = torch.Generator().manual_seed(1)
     ids = [torch.randint(0, 300, (400,), generator=g).tolist() for _ in range(3)]
+    most, LO.PROMPT_MAX_BYTES = LO.PROMPT_MAX_BYTES, 1 << 30 if expand else 0
+    try:
+        r = ModelRunner(model, page_size=16, num_pages=100, max_num_seqs=3)
+        for i in range(3):
+            r.admit(i)
+        out = [r.step([SeqEntry(0, ids[0][:150], 0, [149]), SeqEntry(1, ids[1][:33], 0, [32])]).clone()]
+        out.append(r.step([SeqEntry(0, ids[0][150:151], 150, [0]), SeqEntry(1, ids[1][33:200], 33, [166, 1]),
+                           SeqEntry(2, ids[2][:70], 0, [69])]).clone())
+        r.check_device()
+        return torch.cat(out)
+    finally:
+        LO.PROMPT_MAX_BYTES = most
 
-    def logits(expand):
-        most, LO.PROMPT_MAX_BYTES = LO.PROMPT_MAX_BYTES, 1 << 30 if expand else 0
-        try:
-            r = ModelRunner(model, page_size=16, num_pages=100, max_num_seqs=3)
-            for i in range(3):
-                r.admit(i)
-            out = [r.step([SeqEntry(0, ids[0][:150], 0, [149]), SeqEntry(1, ids[1][:33], 0, [32])]).clone()]
-            out.append(r.step([SeqEntry(0, ids[0][150:151], 150, [0]), SeqEntry(1, ids[1][33:200], 33, [166, 1]),
-                               SeqEntry(2, ids[2][:70], 0, [69])]).clone())
-            r.check_device()
-            return torch.cat(out)
-        finally:
-            LO.PROMPT_MAX_BYTES = most
 
-    a, b = logits(True), logits(False)
+def test_mixers_of_both_kinds_agree():
+    """A small model's logits with its portions on expanded keys and on the latents."""
+    a, b = small_model_logits(True), small_model_logits(False)
     assert ((a - b).norm() / b.norm()).item() < 0.02 and not torch.equal(a, b)
+
+
+def test_without_room_for_the_expanded_rows(monkeypatch):
+    from dispec_b200.ops import latent as LO
+
+    def no_room(*args, **kwargs):
+        raise torch.OutOfMemoryError("no room")
+
+    a = small_model_logits(True)
+    monkeypatch.setattr(LO, "latent_attention_prompts", no_room)
+    assert torch.equal(small_model_logits(True), small_model_logits(False)) and not torch.equal(a, small_model_logits(True))
