@@ -7,12 +7,12 @@
 //
 // Two kernels, both fed by 16-byte asynchronous copies a few stages ahead.  `few_rows_kernel` (up to 16 rows)
 // streams W: it is bound by the bytes of W, or, where N is small, by the chain itself (K dependent FMAs of
-// four cycles).  4 rows x 17,920 x 1,536: 112 -> 44 us; x 1,536 x 8,960: 620 -> 62 us.
+// four cycles).  4 rows x 17,920 x 1,536: 44 us (210 with one 64 x 64 tile, single-float loads and no copies
+// ahead); x 1,536 x 8,960: 62 us (1,056).
 // `tile_kernel` holds BM x BN outputs in the registers of a block, 8 x 8 down to 4 x 2 a thread; it is bound
 // by the issue of FMAs (the 128 x 128 tile: FMA pipe 64 % of its peak, issue slots 76 %) and, for the small
-// tiles that few outputs need to reach all SMs, by shared-memory reads.  264 rows x 17,920 x 1,536: 383 us
-// (38 TFLOP/s); x 1,536 x 8,960: 275 us.  One tile of 64 x 64 with single-float loads and no copies ahead,
-// as it was: 1,150 and 700 us.
+// tiles that few outputs need to reach all SMs, by shared-memory reads.  264 rows x 17,920 x 1,536: 381 us
+// (38 TFLOP/s; 738 with that one tile); x 1,536 x 8,960: 275 us (1,026).
 #include "common.cuh"
 
 namespace {
