@@ -80,12 +80,6 @@ struct Params {
   int page_runs;  // the run maps are valid
   float scale_log2;
   int* err;
-  // a sink: one more key of score sink_values[head] (0 without them) and no value; a gate (float, laid out like the
-  // output): results times its sigmoid.  Read by the kernel that is built with them.
-  const float* sink_values;
-  const float* gate;
-  long ldg;
-  int sink;
 };
 
 // value tile as the B operand of O += P V: N (head dimension) contiguous, 64 per 128-byte row,
@@ -129,8 +123,6 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&t);
 }
 
-// EXTRA: with a sink, a gate or both.
-template <bool EXTRA>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_tcgen05_kernel(const Params p, int tile_offset, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap runs_k,
@@ -548,16 +540,10 @@ attn_tcgen05_kernel(const Params p, int tile_offset, const __grid_constant__ CUt
       tc_fence_after();
       const bool two = n_kt > 1;  // group 1 had tiles: O[1] holds its part
       const float m1 = two ? merge_m[r] : -INFINITY, l1 = two ? merge_l[r] : 0.f;
-      float M = fmaxf(m_run, m1), z = -INFINITY;
-      const int head = kvh * G + r % G;
-      if constexpr (EXTRA) {
-        if (p.sink) z = p.sink_values && row_ok ? p.sink_values[head] * 1.4426950408889634f : 0.f;
-        M = fmaxf(M, z);
-      }
+      const float M = fmaxf(m_run, m1);
       const float w0 = m_run == -INFINITY ? 0.f : ex2(m_run - M);
       const float w1 = m1 == -INFINITY ? 0.f : ex2(m1 - M);
-      float denom = l_run * w0 + l1 * w1;
-      if constexpr (EXTRA) denom += z == -INFINITY ? 0.f : ex2(z - M);
+      const float denom = l_run * w0 + l1 * w1;
       const float inv = denom > 0.f ? 1.f / denom : 0.f;
       const float f0 = w0 * inv, f1 = w1 * inv;
       bf16* dst = p.out;
@@ -576,13 +562,6 @@ attn_tcgen05_kernel(const Params p, int tile_offset, const __grid_constant__ CUt
         } else {
 #pragma unroll
           for (int c = 0; c < 32; ++c) ov[c] = __float_as_uint(__uint_as_float(ov[c]) * f0);
-        }
-        if constexpr (EXTRA) {
-          if (row_ok && p.gate) {
-            const float* gate = p.gate + (size_t)(qs + tok0 + r / G) * p.ldg + (size_t)head * D + c0;
-#pragma unroll
-            for (int c = 0; c < 32; ++c) ov[c] = __float_as_uint(__uint_as_float(ov[c]) / (1.f + expf(-gate[c])));
-          }
         }
         if (row_ok) {
 #pragma unroll
@@ -657,12 +636,17 @@ bool pool_map(const void* base, long num_pages, int heads, int page_size, CUtens
   *has_runs = k.has_runs;
   return true;
 }
-template <bool EXTRA>
-int launch(const void* q, long q_stride, const void* k_pool, const void* v_pool, const int* page_table, int pt_stride,
-           const int* q_start, const int* ctx_len, const int* tile_seq, const int* tile_tok0, int tile_offset,
-           int num_tiles, void* out, long out_stride, int H, int KVH, int tokens_per_tile, int page_size, int num_pages,
-           int window, float scale, int sink, const float* sink_values, const float* gate, long ldg, int* err,
-           cudaStream_t stream) {
+}  // namespace
+
+// Attention of the tiles tile_offset .. tile_offset + num_tiles - 1 of the step's tile list (tiles of
+// tokens_per_tile tokens, 128 / group size at most).  Returns 0, or: 1 launch failed, 2 unsupported
+// head/group counts or page size (a power of two from 8 to 64), 3 misaligned operands, 4 the
+// shared-memory opt-in or the tensor maps failed.
+extern "C" int DSP_CAT(dsp_attn_tcgen05_d, DSP_HEAD_DIM)(
+    const void* q, long q_stride, const void* k_pool, const void* v_pool, const int* page_table,
+    int pt_stride, const int* q_start, const int* ctx_len, const int* tile_seq, const int* tile_tok0,
+    int tile_offset, int num_tiles, void* out, long out_stride, int H, int KVH, int tokens_per_tile,
+    int page_size, int num_pages, int window, float scale, int* err, cudaStream_t stream) {
   if (num_tiles <= 0) return 0;
   if (KVH <= 0 || H % KVH != 0 || (H / KVH) * tokens_per_tile > BM || tokens_per_tile < 1 || KVH > 65535) return 2;
   if (page_size != 8 && page_size != 16 && page_size != 32 && page_size != 64) return 2;
@@ -690,10 +674,6 @@ int launch(const void* q, long q_stride, const void* k_pool, const void* v_pool,
   p.window = window;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.err = err;
-  p.sink_values = sink_values;
-  p.gate = gate;
-  p.ldg = ldg;
-  p.sink = sink;
   CUtensorMap map_k, map_v, runs_k, runs_v;
   bool has_runs_k = false, has_runs_v = false;
   if (!pool_map(k_pool, num_pages, KVH, page_size, &map_k, &runs_k, &has_runs_k) ||
@@ -702,7 +682,7 @@ int launch(const void* q, long q_stride, const void* k_pool, const void* v_pool,
   p.page_runs = has_runs_k && has_runs_v && page_runs_enabled();
   static bool configured = false;  // once; not repeated under graph capture
   if (!configured) {
-    if (cudaFuncSetAttribute(attn_tcgen05_kernel<EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
+    if (cudaFuncSetAttribute(attn_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
         cudaSuccess)
       return 4;
     configured = true;
@@ -717,32 +697,5 @@ int launch(const void* q, long q_stride, const void* k_pool, const void* v_pool,
   attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, attn_tcgen05_kernel<EXTRA>, p, tile_offset, map_k, map_v, runs_k, runs_v) == cudaSuccess ? 0 : 1;
-}
-}  // namespace
-
-// Attention of the tiles tile_offset .. tile_offset + num_tiles - 1 of the step's tile list (tiles of
-// tokens_per_tile tokens, 128 / group size at most).  Returns 0, or: 1 launch failed, 2 unsupported
-// head/group counts or page size (a power of two from 8 to 64), 3 misaligned operands, 4 the
-// shared-memory opt-in or the tensor maps failed.
-extern "C" int DSP_CAT(dsp_attn_tcgen05_d, DSP_HEAD_DIM)(
-    const void* q, long q_stride, const void* k_pool, const void* v_pool, const int* page_table,
-    int pt_stride, const int* q_start, const int* ctx_len, const int* tile_seq, const int* tile_tok0,
-    int tile_offset, int num_tiles, void* out, long out_stride, int H, int KVH, int tokens_per_tile,
-    int page_size, int num_pages, int window, float scale, int* err, cudaStream_t stream) {
-  return launch<false>(q, q_stride, k_pool, v_pool, page_table, pt_stride, q_start, ctx_len, tile_seq, tile_tok0,
-                       tile_offset, num_tiles, out, out_stride, H, KVH, tokens_per_tile, page_size, num_pages, window,
-                       scale, 0, nullptr, nullptr, 0, err, stream);
-}
-
-// The same with a sink and a gate (see Params).
-extern "C" int DSP_CAT(dsp_attn_tcgen05_sink_d, DSP_HEAD_DIM)(
-    const void* q, long q_stride, const void* k_pool, const void* v_pool, const int* page_table,
-    int pt_stride, const int* q_start, const int* ctx_len, const int* tile_seq, const int* tile_tok0,
-    int tile_offset, int num_tiles, void* out, long out_stride, int H, int KVH, int tokens_per_tile,
-    int page_size, int num_pages, int window, float scale, int sink, const float* sink_values, const float* gate,
-    long ldg, int* err, cudaStream_t stream) {
-  return launch<true>(q, q_stride, k_pool, v_pool, page_table, pt_stride, q_start, ctx_len, tile_seq, tile_tok0,
-                      tile_offset, num_tiles, out, out_stride, H, KVH, tokens_per_tile, page_size, num_pages, window,
-                      scale, sink, sink_values, gate, ldg, err, stream);
+  return cudaLaunchKernelEx(&cfg, attn_tcgen05_kernel, p, tile_offset, map_k, map_v, runs_k, runs_v) == cudaSuccess ? 0 : 1;
 }

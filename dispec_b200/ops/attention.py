@@ -413,14 +413,12 @@ def sink_attention_tiles(q, k_pool, v_pool, page_table, q_start, ctx_len, tile_s
                          num_heads, num_kv_heads, window, scale, sink, num_single: int = 0, splits: int = 1,
                          chunked: bool = False, sink_values: torch.Tensor | None = None,
                          turn_freq: torch.Tensor | None = None, positions: torch.Tensor | None = None,
-                         keep_first: int = 0, gate: torch.Tensor | None = None, big_tiles: tuple | None = None) -> torch.Tensor:
+                         keep_first: int = 0, gate: torch.Tensor | None = None) -> torch.Tensor:
     """The tensor-core kernel over a tile list (``tokens per tile`` = 64 // group).  The first
     ``num_single`` tiles are single tokens (the first rows of the batch): with ``splits`` > 1
     their keys are cut into that many shares, merged by the combine kernel.  ``chunked``,
     ``sink_values``, ``turn_freq``, ``keep_first``, ``gate``: as in ``paged_attention_generic``; ``positions`` (of the step's
-    tokens) is needed where split results are turned back.  ``big_tiles``: the step's tiles of 128 rows (single tokens
-    first as well); portions of prompts run on the tcgen05 kernel over them where it is built for what is asked
-    (1,024 tokens of a prompt, then 476 after them, 12 heads of 128 on 2 KV heads, sink and gate: 41 us a launch, 85 on mma.sync)."""
+    tokens) is needed where split results are turned back."""
     num_pages, G, page_size, dk = k_pool.shape
     dv = v_pool.shape[3]
     assert q.dtype == k_pool.dtype == v_pool.dtype == torch.bfloat16 and out.dtype in (torch.bfloat16, torch.float32)
@@ -456,24 +454,6 @@ def sink_attention_tiles(q, k_pool, v_pool, page_table, q_start, ctx_len, tile_s
                                                     num_single, num_heads, dv, splits, L.dtype_code(out.dtype),
                                                     L.ptr(gate), ldg, L.stream_handle()))
         first = num_single
-    if (big_tiles is not None and big_tiles[2] > num_single and dk == dv and not mask_mode and not keep_first
-            and turn_freq is None and out.dtype == torch.bfloat16
-            and tcgen05_supported(dk, num_heads // G, page_size, q.dtype)
-            and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0
-            and (q.data_ptr() | out.data_ptr() | k_pool.data_ptr() | v_pool.data_ptr()) % 16 == 0):
-        if num_single > first:
-            launch(first, num_single - first, 1, None, None)
-        lib = L.prefill_attention_library(dk)
-        rc = getattr(lib, f"dsp_attn_tcgen05_sink_d{dk}")(
-            L.ptr(q), L.i64(q.stride(0)), L.ptr(k_pool), L.ptr(v_pool), L.ptr(page_table), page_table.stride(0),
-            L.ptr(q_start), L.ptr(ctx_len), L.ptr(big_tiles[0]), L.ptr(big_tiles[1]), num_single,
-            big_tiles[2] - num_single, L.ptr(out), L.i64(out.stride(0)), num_heads, num_kv_heads,
-            prefill_tokens_per_tile(num_heads // G), page_size, num_pages, window, L.f32(scale), int(bool(sink)),
-            L.ptr(sink_values), L.ptr(gate), ldg, ctypes.c_void_p(_device_error_address(q.device)), L.stream_handle())
-        L.LaunchCounter.n += 1
-        if rc != 0:
-            raise L.KernelError(f"dsp_attn_tcgen05_sink_d{dk}: {_TCGEN05_ERRORS.get(rc, rc)}")
-        return out
     if num_tiles > first:
         launch(first, num_tiles - first, 1, None, None)
     return out
@@ -501,8 +481,7 @@ def sink_paged_attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, num_hea
                                     tile_seq, tile_tok0, num_tiles, out, num_heads, num_kv_heads, window, scale, sink,
                                     num_single=ctx.num_decode_seqs, splits=splits, chunked=chunked,
                                     sink_values=sink_values, turn_freq=turn_freq, positions=ctx.positions,
-                                    keep_first=keep_first, gate=gate,
-                                    big_tiles=ctx.attention_tiles.get(prefill_tokens_per_tile(group)))
+                                    keep_first=keep_first, gate=gate)
     return paged_attention_generic(q, q.stride(0), cache.key_pool, cache.value_pool, cache.page_table,
                                    ctx.positions, ctx.seq_of_token, out, num_heads, num_kv_heads, key_dim,
                                    window, scale, sink=sink, chunked=chunked, sink_values=sink_values,

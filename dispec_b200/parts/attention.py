@@ -228,12 +228,7 @@ class SinkAttention(JoinableMixer):
                           CacheTensor("value", self.num_kv_heads, self.value_dim)), self.window)
 
     def tokens_per_attention_tile(self):
-        group = self.num_heads // self.num_kv_heads
-        tokens = attn_ops.sink_tokens_per_tile(group, self.key_dim, self.value_dim)
-        if (tokens and self.key_dim == self.value_dim and self.key_dim in (64, 128) and self.mask == "window"
-                and self.value_theta is None):
-            return tokens, attn_ops.prefill_tokens_per_tile(group)  # portions of prompts: 128-row tiles
-        return tokens
+        return attn_ops.sink_tokens_per_tile(self.num_heads // self.num_kv_heads, self.key_dim, self.value_dim)
 
     def heads(self, ctx, z, cache, state, out):
         H, G, dk, dv = self.num_heads, self.num_kv_heads, self.key_dim, self.value_dim
