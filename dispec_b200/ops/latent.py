@@ -179,6 +179,16 @@ def prompt_supported(dim: int, rot_dim: int, vdim: int, kv_rank: int) -> bool:
     return dim in (64, 128) and vdim in (64, 128) and rot_dim == PROMPT_ROT_DIM and kv_rank % 8 == 0
 
 
+def prompt_operands_fit(q: torch.Tensor, q_head_stride: int, qr_off: int, c_pool: torch.Tensor, r_pool: torch.Tensor,
+                        out: torch.Tensor, gate: torch.Tensor | None) -> bool:
+    """Whether ``latent_attention_prompts`` takes these operands: bfloat16, rows of whole 16-byte pieces.  Where the
+    output's columns begin elsewhere (a mixer beside another one of an odd width), the latents are used as they are."""
+    return (all(t.dtype == torch.bfloat16 for t in (q, c_pool, r_pool, out)) and q_head_stride % 8 == 0 and qr_off % 8 == 0
+            and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0
+            and (q.data_ptr() | out.data_ptr() | c_pool.data_ptr() | r_pool.data_ptr()) % 16 == 0
+            and (gate is None or gate.dtype == torch.float32))
+
+
 def expanded_keys(q_len: int, ctx_len: int, window: int) -> int:
     """Keys of a sequence that a portion of ``q_len`` tokens has expanded."""
     return ctx_len - (max(0, ctx_len - q_len - window + 1) // 64 * 64 if window > 0 else 0)

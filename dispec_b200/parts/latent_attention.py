@@ -115,7 +115,7 @@ class LatentAttention(JoinableMixer):
         q = ops.linear(cq, self.w_uq)  # [T, H * (d + r)]
         gate = down[:, down.shape[1] - H * dv:] if self.gate else None
         n_dec, portions = ctx.num_decode_seqs, True
-        if (self.w_kv is not None and T > n_dec and c_pool.dtype == torch.bfloat16 and out.dtype == torch.bfloat16
+        if (self.w_kv is not None and T > n_dec and latent_ops.prompt_operands_fit(q, d + r, d, c_pool, r_pool, out, gate)
                 and latent_ops.PROMPT_TOKENS_PER_TILE in ctx.attention_tiles
                 and latent_ops.mma_supported(R, r, c_pool.dtype) and latent_ops.mma_tokens_per_tile(H) in ctx.attention_tiles
                 and latent_ops.expanded_fits(ctx.host_q_len[n_dec:], ctx.host_ctx_len[n_dec:], 2 * H * (d + dv),

@@ -175,3 +175,19 @@ def test_without_room_for_the_expanded_rows(monkeypatch):
     a = small_model_logits(True)
     monkeypatch.setattr(LO, "latent_attention_prompts", no_room)
     assert torch.equal(small_model_logits(True), small_model_logits(False)) and not torch.equal(a, small_model_logits(True))
+
+
+@pytest.mark.parametrize("first", [1, 4])
+def test_output_columns_that_begin_anywhere(monkeypatch, first):
+    """Heads whose output rows do not begin on 16 bytes (columns of a wider row): on the latents, as they were."""
+    from dispec_b200.parts.latent_attention import LatentAttention
+    heads = LatentAttention.heads
+
+    def shifted(self, ctx, z, cache, state, out):
+        wide = torch.empty((out.shape[0], out.shape[1] + 8), dtype=out.dtype, device=out.device)
+        heads(self, ctx, z, cache, state, wide[:, first:first + out.shape[1]])
+        out.copy_(wide[:, first:first + out.shape[1]])
+
+    monkeypatch.setattr(LatentAttention, "heads", shifted)
+    a, b = small_model_logits(True), small_model_logits(False)
+    assert torch.equal(a, b) and a.isfinite().all()
