@@ -16,6 +16,8 @@ from dispec_b200.cache.manager import CacheGroupSpec
 
 
 class CacheStorage:
+    ROOM_RETRY = 256  # times a want of memory is taken as given before it is tried again
+
     def __init__(self, groups: list[CacheGroupSpec], page_size: int, num_pages: list[int],
                  dtype: torch.dtype, device, poison: bool = False):
         self.page_size = page_size
@@ -30,6 +32,24 @@ class CacheStorage:
                 pool.fill_(float("nan") if poison else 0.0)
                 named[t.name] = pool
             self.pools.append(named)
+        self._no_room: int | None = None  # bytes of working memory that the device did not have when last asked
+        self._no_room_turns = 0
+
+    def room_beside(self, n_bytes: int) -> bool:
+        """Whether a part may ask for ``n_bytes`` of working memory beside the pools: no where that much was refused
+        lately.  A refusal empties the allocator's cache and takes milliseconds, so it is not asked for again in every
+        layer of every step; memory that others have given back is found after ``ROOM_RETRY`` questions."""
+        if self._no_room is None or n_bytes < self._no_room:
+            return True
+        self._no_room_turns += 1
+        if self._no_room_turns >= self.ROOM_RETRY:
+            self._no_room, self._no_room_turns = None, 0
+        return False
+
+    def no_room_beside(self, n_bytes: int) -> None:
+        """``n_bytes`` of working memory were refused."""
+        self._no_room = n_bytes if self._no_room is None else min(n_bytes, self._no_room)
+        self._no_room_turns = 0
 
     def layer_tensors(self, group: int, slot: int) -> dict:
         """name -> ``[page, head, offset in page, width]`` of one layer cache."""

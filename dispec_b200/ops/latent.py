@@ -171,7 +171,11 @@ def latent_attention_tiles(ctx, q_absorbed: torch.Tensor, q: torch.Tensor, q_hea
 
 PROMPT_TOKENS_PER_TILE = 128  # tokens of one head of a tile of the kernel for portions of prompts
 PROMPT_ROT_DIM = 64  # size of the rotated key part it is built for
-PROMPT_MAX_BYTES = 1 << 30  # expanded keys and values a step may hold
+# Gathered latents and expanded keys and values that a step may hold.  Measured on eight layers, 12 heads of 128 + 64 on
+# latents of 512, a portion's whole step (bound by the host below 1.8 ms): 2,048 tokens of a prompt 3.7 ms expanded and 5.9
+# on the latents, after 8,000 stored tokens 4.5 and 17.8; 128 tokens 1.74 and 1.80, after 8,000 2.0 and 5.6; 8 tokens after
+# 2,000 1.8 and 2.1, after 16,000 2.1 and 9.3; 8 tokens alone the same.
+PROMPT_MAX_BYTES = 1 << 30
 
 
 def prompt_supported(dim: int, rot_dim: int, vdim: int, kv_rank: int) -> bool:
@@ -194,13 +198,18 @@ def expanded_keys(q_len: int, ctx_len: int, window: int) -> int:
     return ctx_len - (max(0, ctx_len - q_len - window + 1) // 64 * 64 if window > 0 else 0)
 
 
-def expanded_fits(q_lens: list, ctx_lens: list, row_bytes: int, window: int) -> bool:
-    """Whether a step's portions of prompts run on expanded keys and values: whenever those are no more than
-    ``PROMPT_MAX_BYTES``.  Measured on eight layers, 12 heads of 128 + 64 on latents of 512, a portion's whole step
-    (bound by the host below 1.8 ms): 2,048 tokens of a prompt 3.7 ms expanded and 5.9 on the latents, after 8,000
-    stored tokens 4.5 and 17.8; 128 tokens 1.74 and 1.80, after 8,000 2.0 and 5.6; 8 tokens after 2,000 1.8 and 2.1,
-    after 16,000 2.1 and 9.3; 8 tokens alone the same."""
-    return row_bytes * sum(expanded_keys(q, c, window) for q, c in zip(q_lens, ctx_lens)) <= PROMPT_MAX_BYTES
+def expanded_room(rows: int) -> int:
+    """Rows that are allocated for ``rows`` expanded ones: rounded up to a quarter of a power of two, so that a request
+    that grows finds the last step's blocks in the allocator's cache (every step a new block of 400 MB otherwise, for
+    64 requests of 1,000 tokens)."""
+    step = max(64, 1 << max(0, rows.bit_length() - 3))
+    return -(-rows // step) * step
+
+
+def expanded_bytes(q_lens: list, ctx_lens: list, num_heads: int, dim: int, vdim: int, kv_rank: int, window: int) -> int:
+    """Bytes of the gathered latents and the expanded keys and values of a step's portions of prompts."""
+    rows = expanded_room(sum(expanded_keys(q, c, window) for q, c in zip(q_lens, ctx_lens)))
+    return 2 * rows * (num_heads * (dim + vdim) + kv_rank + PROMPT_ROT_DIM)
 
 
 def latent_attention_prompts(ctx, q: torch.Tensor, q_head_stride: int, qr_off: int, inv_freq: torch.Tensor | None,
@@ -224,14 +233,14 @@ def latent_attention_prompts(ctx, q: torch.Tensor, q_head_stride: int, qr_off: i
     assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1 and gate.shape == out.shape)
     _checked_sink(sink, num_heads)
     lib = L.latent_prompt_library(dim, vdim)
-    c_rows = torch.empty((rows, R), dtype=torch.bfloat16, device=q.device)
-    r_rows = torch.empty((rows, PROMPT_ROT_DIM), dtype=torch.bfloat16, device=q.device)
+    new = lambda columns: torch.empty((expanded_room(rows), columns), dtype=torch.bfloat16, device=q.device)[:rows]
+    c_rows, r_rows, kv = new(R), new(PROMPT_ROT_DIM), new(num_heads * (dim + vdim))
     bad = torch.empty((S, max_tiles), dtype=torch.int64, device=q.device)
     L.check(lib.dsp_latent_gather(
         L.ptr(c_pool), L.ptr(r_pool), L.ptr(page_table), page_table.stride(0), L.ptr(ctx.q_start), L.ptr(ctx.ctx_len),
         n_dec, S, int(window), L.ptr(c_rows), L.ptr(r_rows), L.ptr(bad), max_tiles, R, page_size, num_pages,
         L.stream_handle()))
-    kv = gemm.linear(c_rows, w_kv)
+    gemm.linear(c_rows, w_kv, out=kv)
     tile_seq, tile_tok0, n_tiles = ctx.attention_tiles[PROMPT_TOKENS_PER_TILE]
     L.check(lib.dsp_attn_latent_prompt(
         L.ptr(q), L.i64(q.stride(0)), q_head_stride, qr_off, L.ptr(inv_freq), rot, _LAYOUTS[layout], L.f32(magnitude),

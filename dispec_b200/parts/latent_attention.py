@@ -96,6 +96,18 @@ class LatentAttention(JoinableMixer):
             return tokens, latent_ops.PROMPT_TOKENS_PER_TILE
         return tokens
 
+    def _expanded_bytes(self, ctx, q, c_pool, r_pool, out, gate) -> int:
+        """Bytes of working memory with which the step's portions of prompts run on expanded keys and values; 0: they
+        stay on the latents."""
+        H, d, r, dv, R, first = self.num_heads, self.dim, self.rot_dim, self.vdim, self.kv_rank, ctx.num_decode_seqs
+        if not (latent_ops.prompt_operands_fit(q, d + r, d, c_pool, r_pool, out, gate)
+                and latent_ops.PROMPT_TOKENS_PER_TILE in ctx.attention_tiles
+                and latent_ops.mma_supported(R, r, c_pool.dtype) and latent_ops.mma_tokens_per_tile(H) in ctx.attention_tiles):
+            return 0
+        spans = ctx.host_q_len[first:], ctx.host_ctx_len[first:]
+        need = latent_ops.expanded_bytes(*spans, H, d, dv, R, self.window)
+        return need if need <= latent_ops.PROMPT_MAX_BYTES and ctx.storage.room_beside(need) else 0
+
     def heads(self, ctx, down, cache, state, out):
         H, d, r, dv, R, Q = self.num_heads, self.dim, self.rot_dim, self.vdim, self.kv_rank, self.q_rank
         T = down.shape[0]
@@ -115,19 +127,16 @@ class LatentAttention(JoinableMixer):
         q = ops.linear(cq, self.w_uq)  # [T, H * (d + r)]
         gate = down[:, down.shape[1] - H * dv:] if self.gate else None
         n_dec, portions = ctx.num_decode_seqs, True
-        if (self.w_kv is not None and T > n_dec and latent_ops.prompt_operands_fit(q, d + r, d, c_pool, r_pool, out, gate)
-                and latent_ops.PROMPT_TOKENS_PER_TILE in ctx.attention_tiles
-                and latent_ops.mma_supported(R, r, c_pool.dtype) and latent_ops.mma_tokens_per_tile(H) in ctx.attention_tiles
-                and latent_ops.expanded_fits(ctx.host_q_len[n_dec:], ctx.host_ctx_len[n_dec:], 2 * H * (d + dv),
-                                             self.window)):
+        need = self._expanded_bytes(ctx, q, c_pool, r_pool, out, gate) if self.w_kv is not None and T > n_dec else 0
+        if need:
             # portions of prompts on expanded keys and values; the single tokens, if any, on the latents
             try:
                 latent_ops.latent_attention_prompts(ctx, q, d + r, d, inv_freq, rot_n, c_pool, r_pool, cache.page_table,
                                                     self.w_kv, out, H, d, dv, scale, window=self.window,
                                                     sink=self.sink_values, gate=gate, **turn)
                 portions = False
-            except torch.OutOfMemoryError:
-                pass  # no room beside the pools for the expanded rows: on the latents, which need none
+            except torch.OutOfMemoryError:  # on the latents, which need no room
+                ctx.storage.no_room_beside(need)
             if not portions and n_dec == 0:
                 return
             if not portions:

@@ -191,3 +191,16 @@ def test_output_columns_that_begin_anywhere(monkeypatch, first):
     monkeypatch.setattr(LatentAttention, "heads", shifted)
     a, b = small_model_logits(True), small_model_logits(False)
     assert torch.equal(a, b) and a.isfinite().all()
+
+
+def test_a_refusal_is_asked_for_once(monkeypatch):
+    """Two layers and two steps without room: the expanded rows are asked for in the first layer of the first step."""
+    from dispec_b200.ops import latent as LO
+    asked = []
+
+    def no_room(*args, **kwargs):
+        asked.append(1)
+        raise torch.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(LO, "latent_attention_prompts", no_room)
+    assert torch.equal(small_model_logits(True), small_model_logits(False)) and len(asked) == 1
