@@ -212,6 +212,33 @@ def expanded_bytes(q_lens: list, ctx_lens: list, num_heads: int, dim: int, vdim:
     return 2 * rows * (num_heads * (dim + vdim) + kv_rank + PROMPT_ROT_DIM)
 
 
+def expanded_is_faster(q_lens: list, ctx_lens: list, num_heads: int, width: int, kv_rank: int, window: int, sms: int) -> bool:
+    """Whether a step's portions of prompts run faster on expanded keys and values (``width`` = dim + vdim) than on the
+    latents.  The latents need a walk over a request's keys for every tile of 64 rows, tiles side by side; expanding
+    costs every request's keys once, however few tokens attend to them: right for long portions and for few
+    requests, wrong for many requests that bring a few tokens each.  Estimates in microseconds a layer, fitted on
+    launches of 1, 4, 16 and 32 requests of 2 to 512 tokens after 0 to 8,000.  Measured, latents and expanded, 12 heads of
+    128 + 64 on latents of 512: one request of 2 tokens after 1,000 154 and 46, of 512 tokens 239 and 55; 16 requests
+    of 2 tokens 156 and 142; 32 requests of 2 tokens 158 and 219, of 16 tokens 177 and 221, of 32 tokens 336 and 226, of 128
+    tokens 1,082 and 250; 32 heads, 16 requests of 16 tokens 175 and 274, of 64 tokens 690 and 291.  Estimates that
+    close to one another (8 us) say nothing: expanded."""
+    per = mma_tokens_per_tile(num_heads)
+    tiles = blocks = rows = walks = longest = 0
+    for q, c in zip(q_lens, ctx_lens):
+        seen = min(c, window + q) if window > 0 else c
+        n = -(-q // per) * -(-num_heads // MMA_ROWS_PER_TILE)
+        tiles += n
+        walks += n * max(1, seen - q // 2)
+        longest = max(longest, seen)
+        blocks += num_heads * -(-q // PROMPT_TOKENS_PER_TILE)
+        rows += expanded_keys(q, c, window)
+    walk = max(longest, -(-tiles // sms) * walks / tiles)
+    latents = (14.0 + 0.04 * kv_rank + (0.064 + 0.000116 * kv_rank) * walk
+               + 2.5e-8 * sum(q_lens) * num_heads * width * kv_rank)
+    expanded = 22.0 + -(-blocks // sms) * (10.0 + 0.009 * longest) + 1e-6 * rows * num_heads * width * (0.4 + 0.002 * kv_rank)
+    return expanded <= latents + 8.0
+
+
 def latent_attention_prompts(ctx, q: torch.Tensor, q_head_stride: int, qr_off: int, inv_freq: torch.Tensor | None,
                              rot: int, c_pool: torch.Tensor, r_pool: torch.Tensor, page_table: torch.Tensor,
                              w_kv: torch.Tensor, out: torch.Tensor, num_heads: int, dim: int, vdim: int, scale: float,

@@ -28,6 +28,7 @@ import torch
 from dispec_b200 import ops
 from dispec_b200.ops import latent as latent_ops
 from dispec_b200.ops import norm32 as norm32_ops
+from dispec_b200.ops import tuning
 from dispec_b200.parts.base import CacheNeed, CacheTensor, JoinableMixer, TensorSpec
 from dispec_b200.registry import register_part
 
@@ -106,7 +107,12 @@ class LatentAttention(JoinableMixer):
             return 0
         spans = ctx.host_q_len[first:], ctx.host_ctx_len[first:]
         need = latent_ops.expanded_bytes(*spans, H, d, dv, R, self.window)
-        return need if need <= latent_ops.PROMPT_MAX_BYTES and ctx.storage.room_beside(need) else 0
+        if need > latent_ops.PROMPT_MAX_BYTES:
+            return 0
+        key = ("expanded_is_faster", H, d + dv, R, self.window)  # the layers of a step ask the same
+        if key not in ctx.scratch:
+            ctx.scratch[key] = latent_ops.expanded_is_faster(*spans, H, d + dv, R, self.window, tuning.sm_count(q.device))
+        return need if ctx.scratch[key] and ctx.storage.room_beside(need) else 0
 
     def heads(self, ctx, down, cache, state, out):
         H, d, r, dv, R, Q = self.num_heads, self.dim, self.rot_dim, self.vdim, self.kv_rank, self.q_rank
