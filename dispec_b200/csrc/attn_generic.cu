@@ -337,11 +337,13 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
       float top = -INFINITY;
+      unsigned hidden = 0;  // bit j: key j is not this row's
 #pragma unroll
       for (int j = 0; j < KJ; ++j) {
         const int key = kt + tx + j * TX;
         const bool seen = key <= pos[i] && (key >= low[i] || key < a.keep_first) && slot[(t & 1) * TILE_KEYS + tx + j * TX] >= 0;
         s[i][j] = seen ? s[i][j] * a.scale : -INFINITY;
+        hidden |= (seen ? 0u : 1u) << j;
         top = fmaxf(top, s[i][j]);
       }
 #pragma unroll
@@ -349,13 +351,19 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
       const float m_new = fmaxf(m[i], top);
       // m_new stays -inf for rows that have seen no key yet
       const float alpha = m_new == -INFINITY ? 1.f : expf(m[i] - m_new);
-      float sum = 0.f;
+      // a hidden key's weight is -0, which no seen key's is: below it is told from a weight that is merely small
+      float p[KJ];
 #pragma unroll
       for (int j = 0; j < KJ; ++j) {
-        const float p = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - m_new);
-        ps[(ty + i * TY) * LP + tx + j * TX] = p;
-        sum += p;
+        p[j] = s[i][j] == -INFINITY ? ((hidden >> j & 1u) ? -0.f : 0.f) : expf(s[i][j] - m_new);
+        ps[(ty + i * TY) * LP + tx + j * TX] = p[j];
       }
+      // keys l, l + 32 first, then their neighbours 16, 8, 4, 2 and 1 away, on either grid of threads: a token's sum is
+      // the same alone and among the others of a portion
+      float sum;
+      static_assert(KJ == 2 || KJ == 4, "32 or 16 threads a row");
+      if constexpr (KJ == 2) sum = p[0] + p[1];
+      else sum = (p[0] + p[2]) + (p[1] + p[3]);
 #pragma unroll
       for (int o = TX / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
       m[i] = m_new;
@@ -368,8 +376,8 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
     if (t + 1 < ntiles) bring_keys(t + 1); else end_group();
     wait_groups<1>();
     __syncthreads();  // the values are there (and every row of ps)
-    // where some row does not see every key, a key that a row does not see must not reach it: 0 times a value that is
-    // no number is none either
+    // where some row does not see every key, a key that a row does not see (weight -0) must not reach it: 0 times a
+    // value that is no number is none either
     const bool all_seen = kt + TILE_KEYS - 1 <= pos0 && kt >= lowest(last);
 #pragma unroll 2
     for (int j = 0; j < TILE_KEYS; j += 4) {
@@ -388,7 +396,7 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
           const float4 v = *reinterpret_cast<const float4*>(vs + (j + e) * LV + d);
 #pragma unroll
           for (int i = 0; i < RI; ++i) {
-            if (!all_seen && p[i][e] == 0.f) continue;
+            if (!all_seen && __float_as_uint(p[i][e]) == 0x80000000u) continue;
             acc[i][4 * dj] = fmaf(p[i][e], v.x, acc[i][4 * dj]);
             acc[i][4 * dj + 1] = fmaf(p[i][e], v.y, acc[i][4 * dj + 1]);
             acc[i][4 * dj + 2] = fmaf(p[i][e], v.z, acc[i][4 * dj + 2]);

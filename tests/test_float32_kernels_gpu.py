@@ -103,3 +103,33 @@ def test_attention_of_runs(H, G_heads, D, Dv, page, window, chunked, keep, sink)
     mine = 2 + last
     keepers = [i for i in range(T) if i != mine]
     assert torch.equal(again[keepers], out[keepers]) and again[mine].isnan().all()
+
+
+@pytest.mark.parametrize("H,G_heads,D,window,chunked,keep,sink", [
+    (12, 2, 128, 0, False, 0, False),   # one token: 8 rows on 32 lanes, five tokens: 32 rows on 16 lanes
+    (4, 4, 64, 0, False, 0, True),      # up to 8 tokens on 32 lanes
+    (9, 1, 32, 70, False, 0, False),    # always on 16 lanes
+    (8, 2, 48, 33, False, 5, True),
+    (6, 2, 16, 64, True, 0, False),
+])
+def test_attention_of_a_token_does_not_depend_on_its_portion(H, G_heads, D, window, chunked, keep, sink):
+    """Every token of a portion alone, in pairs, and with the portion cut elsewhere: the same bits."""
+    from dispec_b200.ops import attention as A
+    n, first, page = 300, 130, 16
+    kp, vp = (rnd((n // page + 1, G_heads, page, D), s) for s in (31, 32))
+    kp *= 3.0  # weights of very different sizes
+    vp[3, :, 2, 1] = float("inf")  # and a value that a weight which is merely small does not hide
+    table = torch.arange(kp.shape[0], dtype=torch.int32, device=DEV)[None]
+    q, z = rnd((n - first, H * D), 33), rnd((H,), 34)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+
+    def run(lo, hi):
+        out = torch.full((hi - lo, H * D), 7.0, device=DEV)
+        return A.paged_attention_generic(q[lo:hi], H * D, kp, vp, table, i32(list(range(first + lo, first + hi))),
+                                         i32([0] * (hi - lo)), out, H, G_heads, D, window, D ** -0.5, sink=sink, chunked=chunked,
+                                         sink_values=z if sink else None, keep_first=keep)
+
+    whole = run(0, n - first).view(torch.int32)
+    for cut in (1, 2, 7, 50):
+        parts = torch.cat([run(a, min(n - first, a + cut)) for a in range(0, n - first, cut)])
+        assert torch.equal(parts.view(torch.int32), whole), cut
