@@ -111,9 +111,6 @@ __global__ void rmsnorm_kernel(T* __restrict__ x, const T* __restrict__ delta,
 
 // Fast form of the same computation for rows whose bytes are a multiple of 16 and that fit in
 // registers (hidden <= 256 threads * 4 vectors): one read of x (and delta), one write of y.
-// (A warp per row with all of a lane's loads in flight, for the 2,048 rows of a prompt's portion,
-// was measured and dropped: alone as fast, the prefill step 2 % slower at a width of 1,536 and
-// 10 % at 3,584, where it needs 224 registers.)
 template <typename T> struct Vec16 {
   static constexpr int N = 16 / sizeof(T);
   T v[N];
@@ -182,9 +179,8 @@ rmsnorm_vec_kernel(T* __restrict__ x, const T* __restrict__ delta, const T* __re
   }
 }
 
-// The same with a warp a row, for many rows: no barrier, every row of a wave on its way at once, and the gains, which no
-// kernel of the step writes, are read before the wait.  2,048 rows of 1,536 bfloat16: 5.5 us, 6.1 with a block a
-// row (of one launch alone from a cold L2, with what it costs to start).
+// The same with a warp a row, for many rows: no barrier, every row of a wave on its way at once.  bfloat16 only: a warp adds
+// a row's squares in another order than a block, and a 32-bit row must not depend on how many there are.
 constexpr int RMS_WARPS = 4;
 template <typename T, int VPL>
 __global__ void __launch_bounds__(32 * RMS_WARPS)
@@ -192,12 +188,8 @@ rmsnorm_rows_kernel(T* __restrict__ x, const T* __restrict__ delta, const T* __r
                     const int* __restrict__ rows, int n_rows, int hidden, float eps, int write_back) {
   constexpr int N = Vec16<T>::N;
   pdl_launch_dependents();
-  const int lane = threadIdx.x & 31, r = blockIdx.x * RMS_WARPS + (threadIdx.x >> 5), nvec = hidden / N;
-  uint4 wv[VPL];
-#pragma unroll
-  for (int j = 0; j < VPL; ++j)
-    if (lane + j * 32 < nvec) wv[j] = __ldg(reinterpret_cast<const uint4*>(w) + lane + j * 32);
   pdl_wait();
+  const int lane = threadIdx.x & 31, r = blockIdx.x * RMS_WARPS + (threadIdx.x >> 5), nvec = hidden / N;
   if (r >= n_rows) return;
   const size_t in_row = rows ? (size_t)rows[r] : (size_t)r;
   uint4* xr = reinterpret_cast<uint4*>(x + in_row * hidden);
@@ -205,6 +197,10 @@ rmsnorm_rows_kernel(T* __restrict__ x, const T* __restrict__ delta, const T* __r
   uint4 v[VPL];
 #pragma unroll
   for (int j = 0; j < VPL; ++j) v[j] = lane + j * 32 < nvec ? xr[lane + j * 32] : make_uint4(0u, 0u, 0u, 0u);
+  uint4 wv[VPL];
+#pragma unroll
+  for (int j = 0; j < VPL; ++j)
+    if (lane + j * 32 < nvec) wv[j] = __ldg(reinterpret_cast<const uint4*>(w) + lane + j * 32);
   float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < VPL; ++j) {
@@ -243,13 +239,17 @@ static bool launch_rmsnorm_vec(void* x, const void* delta, const void* w, void* 
   const uintptr_t bits = (uintptr_t)x | (uintptr_t)delta | (uintptr_t)w | (uintptr_t)y;
   if (bits % 16 != 0) return false;
   const int nvec = hidden / N;
-  // A warp a row once every SM has several rows to work on, and while a lane's share of a row and its gains fit 90
-  // registers (3,584 bfloat16 would take 223: 1,016 rows 7.1 us, and 1 % of a step slower than a block a row).
-  if (n_rows >= 4 * (dsp_num_sms() > 0 ? dsp_num_sms() : 148) && nvec <= 192) {
+  // A warp a row from 12 rows an SM on.  Block and warp a row, us of a launch among others, rows from memory: 1,024 rows of
+  // 1,024 2.4 and 2.9, of 1,536 2.9 and 3.8; 2,048 rows of 256 3.4 and 2.3, of 1,536 4.5 and 4.4, of 3,072 7.9 and 7.3;
+  // 4,500 rows of 1,536 8.3 and 6.7, of 3,072 14.9 and 12.8.  Up to 3,072: twelve pieces of the row and of the gains a lane are
+  // what its registers hold (at 3,584 a launch with the gains read first took 223 and was the slower one).
+  if constexpr (sizeof(T) == 2) if (n_rows >= 12 * (dsp_num_sms() > 0 ? dsp_num_sms() : 148) && nvec <= 12 * 32) {
     const dim3 grid((n_rows + RMS_WARPS - 1) / RMS_WARPS);
 #define DSP_RMS_ROWS(V) launch_pdl(rmsnorm_rows_kernel<T, V>, grid, dim3(32 * RMS_WARPS), 0, stream, (T*)x, (const T*)delta, (const T*)w, (T*)y, rows, n_rows, hidden, eps, write_back)
-    if (nvec <= 128) DSP_RMS_ROWS(4);
-    else DSP_RMS_ROWS(6);
+    if (nvec <= 4 * 32) DSP_RMS_ROWS(4);
+    else if (nvec <= 6 * 32) DSP_RMS_ROWS(6);
+    else if (nvec <= 8 * 32) DSP_RMS_ROWS(8);
+    else DSP_RMS_ROWS(12);
 #undef DSP_RMS_ROWS
     return true;
   }

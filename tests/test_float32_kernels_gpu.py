@@ -133,3 +133,12 @@ def test_attention_of_a_token_does_not_depend_on_its_portion(H, G_heads, D, wind
     for cut in (1, 2, 7, 50):
         parts = torch.cat([run(a, min(n - first, a + cut)) for a in range(0, n - first, cut)])
         assert torch.equal(parts.view(torch.int32), whole), cut
+
+
+@pytest.mark.parametrize("hidden", [8, 512, 768, 772, 1536])
+def test_rms_norm_of_a_row_does_not_depend_on_the_others(hidden):
+    from dispec_b200 import ops
+    x, w = rnd((2500, hidden), 41), rnd((hidden,), 42)
+    whole = ops.rms_norm(x, w, 1e-6)
+    for n in (1, 3, 592, 1775, 1776):
+        assert torch.equal(ops.rms_norm(x[:n].contiguous(), w, 1e-6), whole[:n]), n

@@ -44,7 +44,10 @@ def test_xielu_rows(rows, cols):
     assert ((y - want).abs() <= 2.0 ** -8 * want.abs() + 32 * U * (1 + v.abs())).all()
 
 
-@pytest.mark.parametrize("n,hidden", [(592, 1536), (593, 8), (600, 1032), (595, 1544), (700, 768), (591, 1536)])
+@pytest.mark.parametrize("n,hidden", [(592, 1536), (593, 8), (600, 1032), (595, 1544), (700, 768), (591, 1536),
+                                      # a warp a row: each share of a row that a lane can have, full and not, and beyond it
+                                      (1776, 8), (1777, 1024), (1780, 1032), (1800, 1536), (1776, 1544), (1779, 2048),
+                                      (1790, 2056), (1801, 3072), (1776, 3080), (1775, 1536)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_rms_norm_of_many_rows(n, hidden, dtype):
     from dispec_b200 import ops
