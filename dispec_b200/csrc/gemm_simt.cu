@@ -5,7 +5,7 @@
 // one FMA chain over k = 0..K-1 in ascending order, so a row's result does not depend on
 // which other rows are in the batch, nor on which of the kernels below computes it.
 //
-// Two kernels, both fed by 16-byte asynchronous copies a few stages ahead.  `few_rows_kernel` (up to 16 rows)
+// Two kernels for floats, both fed by 16-byte asynchronous copies a few stages ahead, and one for bfloat16.  `few_rows_kernel` (up to 16 rows)
 // streams W: it is bound by the bytes of W, or, where N is small, by the chain itself (K dependent FMAs of
 // four cycles).  4 rows x 17,920 x 1,536: 44 us (210 with one 64 x 64 tile, single-float loads and no copies
 // ahead); x 1,536 x 8,960: 62 us (1,056).
@@ -41,11 +41,11 @@ constexpr int tile_stages() { return BM + BN > 192 ? 3 : 4; }
 template <int BM, int BN>
 constexpr int tile_smem() { return tile_stages<BM, BN>() * LDK * (BM + BN) * (int)sizeof(float); }
 
-// COPY16: A and W are float with rows of whole 16-byte pieces, which are copied asynchronously.
-template <typename TIn, typename TOut, int BM, int BN, int TM, int TN, bool COPY16>
+// COPY16: A and W have rows of whole 16-byte pieces, which are copied asynchronously.
+template <int BM, int BN, int TM, int TN, bool COPY16>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
-tile_kernel(const TIn* __restrict__ A, long lda, const TIn* __restrict__ W, const TIn* __restrict__ bias,
-            const TOut* __restrict__ residual, long ldr, TOut* __restrict__ C, long ldc, int M, int N, int K) {
+tile_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, const float* __restrict__ bias,
+            const float* __restrict__ residual, long ldr, float* __restrict__ C, long ldc, int M, int N, int K) {
   constexpr int TX = BN / TN, TY = BM / TM, THREADS = TX * TY, STAGES = tile_stages<BM, BN>(), STAGE = LDK * (BM + BN);
   static_assert(TX % 8 == 0 && TY % 4 == 0 && THREADS % 32 == 0, "warps are 4 x 8 threads of the tile");
   extern __shared__ __align__(16) float tile_buf[];
@@ -72,14 +72,14 @@ tile_kernel(const TIn* __restrict__ A, long lda, const TIn* __restrict__ W, cons
       const bool is_a = r < BM;
       const int row = is_a ? m0 + r : n0 + r - BM;
       const bool inside = row < (is_a ? M : N);
-      const TIn* src = is_a ? A + (size_t)row * lda + k : W + (size_t)row * K + k;
+      const float* src = is_a ? A + (size_t)row * lda + k : W + (size_t)row * K + k;
       float* dst = to + r * LDK + (k - k0);
       if constexpr (COPY16) {
         const bool there = inside && k < K;
         copy16(dst, there ? src : A, there);
       } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) dst[e] = inside && k + e < K ? to_f32(src[e]) : 0.f;
+        for (int e = 0; e < 4; ++e) dst[e] = inside && k + e < K ? src[e] : 0.f;
       }
     }
   };
@@ -142,6 +142,65 @@ tile_kernel(const TIn* __restrict__ A, long lda, const TIn* __restrict__ W, cons
   }
 }
 
+// ------------------------------------------------------------------ bfloat16 operands
+// The sizes the tensor-core kernels refuse (a width that is no multiple of 8): single elements, turned to floats and
+// stored k-major, 256 threads of 4 x 4 outputs.  Bound by the loads of single elements, which the many threads of a
+// block cover best: 8 rows x 151,936 x 1,537 1,166 us, 64 rows x 1,536 x 1,537 205; in the row-major tiles above, 128
+// threads of 8 x 4 outputs and stages that no asynchronous copy fills, 1,683 and 322.
+constexpr int BF_M = 64, BF_N = 64, BF_K = 16, BF_T = 4;
+
+template <typename TOut>
+__global__ void __launch_bounds__(256)
+bf16_kernel(const bf16* __restrict__ A, long lda, const bf16* __restrict__ W, const bf16* __restrict__ bias,
+            const TOut* __restrict__ residual, long ldr, TOut* __restrict__ C, long ldc, int M, int N, int K) {
+  __shared__ float as[BF_K][BF_M + 4], ws[BF_K][BF_N + 4];
+  const int tid = threadIdx.x, m0 = blockIdx.y * BF_M, n0 = blockIdx.x * BF_N;
+  const int tx = tid % 16, ty = tid / 16;  // outputs rows ty * 4 .., columns tx * 4 ..
+  float acc[BF_T][BF_T];
+#pragma unroll
+  for (int i = 0; i < BF_T; ++i)
+#pragma unroll
+    for (int j = 0; j < BF_T; ++j) acc[i][j] = 0.f;
+  for (int k0 = 0; k0 < K; k0 += BF_K) {
+#pragma unroll
+    for (int e = 0; e < BF_M * BF_K / 256; ++e) {
+      const int idx = tid + e * 256, r = idx / BF_K, c = idx % BF_K, m = m0 + r, n = n0 + r, k = k0 + c;
+      as[c][r] = m < M && k < K ? to_f32(A[(size_t)m * lda + k]) : 0.f;
+      ws[c][r] = n < N && k < K ? to_f32(W[(size_t)n * K + k]) : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < BF_K; ++k) {
+      float a[BF_T], w[BF_T];
+#pragma unroll
+      for (int i = 0; i < BF_T; ++i) a[i] = as[k][ty * BF_T + i];
+#pragma unroll
+      for (int j = 0; j < BF_T; ++j) w[j] = ws[k][tx * BF_T + j];
+#pragma unroll
+      for (int i = 0; i < BF_T; ++i)
+#pragma unroll
+        for (int j = 0; j < BF_T; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < BF_T; ++i)
+#pragma unroll
+    for (int j = 0; j < BF_T; ++j) {
+      const int m = m0 + ty * BF_T + i, n = n0 + tx * BF_T + j;
+      if (m < M && n < N) finish(acc[i][j], bias, residual, ldr, C, ldc, m, n);
+    }
+}
+
+template <typename TOut>
+int launch_bf16(const void* A, long lda, const void* W, const void* bias, const void* residual, long ldr, void* C, long ldc,
+                int M, int N, int K, cudaStream_t stream) {
+  bf16_kernel<TOut><<<dim3((N + BF_N - 1) / BF_N, (M + BF_M - 1) / BF_M), 256, 0, stream>>>(
+      (const bf16*)A, lda, (const bf16*)W, (const bf16*)bias, (const TOut*)residual, ldr, (TOut*)C, ldc, M, N, K);
+  DSP_CHECK_LAUNCH("dsp_gemm_simt");
+  return 0;
+}
+
 // ------------------------------------------------------------------ up to 16 rows
 constexpr int FEW_N = 16, FEW_K = 128, FEW_STAGES = 4, FEW_THREADS = 64;
 constexpr int FEW_LD = FEW_K + 4;  // a row's 16-byte pieces start in another bank group than its neighbour's
@@ -201,16 +260,16 @@ few_rows_kernel(const float* __restrict__ A, long lda, const float* __restrict__
   }
 }
 
-template <typename TIn, typename TOut, int BM, int BN, int TM, int TN, bool COPY16 = false>
+template <int BM, int BN, int TM, int TN, bool COPY16>
 int launch_tile(const void* A, long lda, const void* W, const void* bias, const void* residual, long ldr, void* C,
                 long ldc, int M, int N, int K, cudaStream_t stream) {
   const long blocks = (long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   DSP_REQUIRE(blocks < (1l << 31), "dsp_gemm_simt: M=%d, N=%d too large for one launch", M, N);
   constexpr int smem = tile_smem<BM, BN>();
-  auto* kernel = tile_kernel<TIn, TOut, BM, BN, TM, TN, COPY16>;
+  auto* kernel = tile_kernel<BM, BN, TM, TN, COPY16>;
   DSP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   kernel<<<(unsigned)blocks, (BM / TM) * (BN / TN), smem, stream>>>(
-      (const TIn*)A, lda, (const TIn*)W, (const TIn*)bias, (const TOut*)residual, ldr, (TOut*)C, ldc, M, N, K);
+      (const float*)A, lda, (const float*)W, (const float*)bias, (const float*)residual, ldr, (float*)C, ldc, M, N, K);
   DSP_CHECK_LAUNCH("dsp_gemm_simt");
   return 0;
 }
@@ -269,27 +328,27 @@ extern "C" int dsp_gemm_simt(const void* A, long lda, const void* W, const void*
   return launch_tile<__VA_ARGS__>(A, lda, W, bias, residual, ldr, C, ldc, M, N, K, stream)
 #define DSP_FEW(MR) return launch_few<MR>(A, lda, W, bias, residual, ldr, C, ldc, M, N, K, stream)
   if (in_dtype == DSP_F32 && out_dtype == DSP_F32) {
-    if (K % 4 || lda % 4 || (uintptr_t)A % 16 || (uintptr_t)W % 16) DSP_TILE(float, float, 64, 64, 8, 4);
+    if (K % 4 || lda % 4 || (uintptr_t)A % 16 || (uintptr_t)W % 16) DSP_TILE(64, 64, 8, 4, false);
     DSP_REQUIRE(tile != FEW_TILE || M <= FEW_MAX_ROWS, "dsp_gemm_simt: %d rows are too many for the kernel of few rows", M);
     if (tile < 0) tile = choose_tile(M, N);
     switch (tile) {
-      case 0: DSP_TILE(float, float, 128, 128, 8, 8, true);
-      case 1: DSP_TILE(float, float, 96, 128, 12, 4, true);
-      case 2: DSP_TILE(float, float, 64, 128, 8, 8, true);
-      case 3: DSP_TILE(float, float, 96, 64, 12, 4, true);
-      case 4: DSP_TILE(float, float, 64, 64, 8, 4, true);
-      case 5: DSP_TILE(float, float, 96, 32, 6, 4, true);
-      case 6: DSP_TILE(float, float, 64, 32, 4, 4, true);
-      case 7: DSP_TILE(float, float, 32, 64, 4, 4, true);
-      case 8: DSP_TILE(float, float, 32, 32, 4, 2, true);
+      case 0: DSP_TILE(128, 128, 8, 8, true);
+      case 1: DSP_TILE(96, 128, 12, 4, true);
+      case 2: DSP_TILE(64, 128, 8, 8, true);
+      case 3: DSP_TILE(96, 64, 12, 4, true);
+      case 4: DSP_TILE(64, 64, 8, 4, true);
+      case 5: DSP_TILE(96, 32, 6, 4, true);
+      case 6: DSP_TILE(64, 32, 4, 4, true);
+      case 7: DSP_TILE(32, 64, 4, 4, true);
+      case 8: DSP_TILE(32, 32, 4, 2, true);
       default:
         if (M <= 4) DSP_FEW(1);
         if (M <= 8) DSP_FEW(2);
         DSP_FEW(4);
     }
   }
-  if (in_dtype == DSP_BF16 && out_dtype == DSP_BF16) DSP_TILE(bf16, bf16, 64, 64, 8, 4);
-  if (in_dtype == DSP_BF16 && out_dtype == DSP_F32) DSP_TILE(bf16, float, 64, 64, 8, 4);
+  if (in_dtype == DSP_BF16 && out_dtype == DSP_BF16) return launch_bf16<bf16>(A, lda, W, bias, residual, ldr, C, ldc, M, N, K, stream);
+  if (in_dtype == DSP_BF16 && out_dtype == DSP_F32) return launch_bf16<float>(A, lda, W, bias, residual, ldr, C, ldc, M, N, K, stream);
 #undef DSP_TILE
 #undef DSP_FEW
   DSP_REQUIRE(false, "dsp_gemm_simt: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);

@@ -1,4 +1,4 @@
-"""The 32-bit product and the 32-bit attention alone, at the sizes where their tiles end."""
+"""The product and the attention on the FMA units alone, at the sizes where their tiles end."""
 import math
 
 import pytest
@@ -142,3 +142,20 @@ def test_rms_norm_of_a_row_does_not_depend_on_the_others(hidden):
     whole = ops.rms_norm(x, w, 1e-6)
     for n in (1, 3, 592, 1775, 1776):
         assert torch.equal(ops.rms_norm(x[:n].contiguous(), w, 1e-6), whole[:n]), n
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 3, 5), (7, 64, 17), (64, 65, 33), (65, 130, 15), (3, 1000, 515)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_bfloat16_widths_that_are_no_multiple_of_eight(M, N, K, out_dtype):
+    from dispec_b200.ops import gemm
+    x, w, b = (rnd(shape, s).bfloat16() for shape, s in (((M, K), 51), ((N, K), 52), ((N,), 53)))
+    r = rnd((M, N), 54).to(out_dtype)
+    out = gemm.linear(x, w, b, residual=r, out_dtype=out_dtype, backend="simt")
+    ref = x.double() @ w.double().T + b.double() + r.double()
+    bound = (K + 2) * U * (x.abs().double() @ w.abs().double().T + b.abs().double() + r.abs().double())
+    if out_dtype == torch.bfloat16:
+        bound = bound + 2.0 ** -8 * (ref.abs() + bound)  # the result is rounded once
+    assert ((out.double() - ref).abs() <= bound).all()
+    one = gemm.linear(x[M // 2:M // 2 + 1].contiguous(), w, b, residual=r[M // 2:M // 2 + 1].contiguous(), out_dtype=out_dtype,
+                      backend="simt")
+    assert torch.equal(out[M // 2:M // 2 + 1], one)
