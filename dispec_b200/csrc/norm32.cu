@@ -178,24 +178,26 @@ xielu_kernel(const void* __restrict__ z, int z_dtype, long ldz, const float* __r
 
 // The same from floats to bfloat16 where rows are whole groups of four on 16-byte (8-byte) pieces: a block takes
 // stretches of 4 * GROUPS * blockDim columns of rows blockIdx.y, blockIdx.y + gridDim.y, ..., a thread GROUPS groups
-// of a row at once (no division of an index; four loads on their way).  2,500 rows of 8,960: 135 MB in 40.9 us (45.5
-// with one group at a time from a running index, whose 64-bit divisions were most of its instructions).
+// of a row at once (no division of an index).  Four groups keep four loads on their way: 2,500 rows of 8,960, 135 MB
+// in 40.9 us (45.5 with one group at a time from a running index, whose 64-bit divisions were most of its instructions).
+// With few rows four groups leave SMs idle and pay their exponentials one after the other: one group a thread.
 constexpr int XIELU_GROUPS = 4;
+template <int GROUPS>
 __global__ void __launch_bounds__(128)
 xielu_rows_kernel(const float* __restrict__ z, long ldz, const float* __restrict__ pq, bf16* __restrict__ y, long ldy,
                   long rows, int cols) {
   const float ap = softplus_f(pq[0]), an = 0.5f + softplus_f(pq[1]);
   auto act = [&](float v) { return v > 0.f ? fmaf(ap * v, v, 0.5f * v) : fmaf(an, expm1f(v) - v, 0.5f * v); };
-  const int c0 = (blockIdx.x * XIELU_GROUPS * blockDim.x + threadIdx.x) * 4, step = blockDim.x * 4;
+  const int c0 = (blockIdx.x * GROUPS * blockDim.x + threadIdx.x) * 4, step = blockDim.x * 4;
   for (long r = blockIdx.y; r < rows; r += gridDim.y) {
     const float* src = z + (size_t)r * ldz;
     bf16* dst = y + (size_t)r * ldy;
-    float4 v[XIELU_GROUPS];
+    float4 v[GROUPS];
 #pragma unroll
-    for (int g = 0; g < XIELU_GROUPS; ++g)
+    for (int g = 0; g < GROUPS; ++g)
       if (c0 + g * step < cols) v[g] = *reinterpret_cast<const float4*>(src + c0 + g * step);
 #pragma unroll
-    for (int g = 0; g < XIELU_GROUPS; ++g) {
+    for (int g = 0; g < GROUPS; ++g) {
       if (c0 + g * step >= cols) break;
       const __nv_bfloat162 lo = __floats2bfloat162_rn(act(v[g].x), act(v[g].y)), hi = __floats2bfloat162_rn(act(v[g].z), act(v[g].w));
       uint2 out;
@@ -476,9 +478,13 @@ extern "C" int dsp_xielu(const void* z, int z_dtype, long ldz, const float* pq, 
   const long n = rows * cols;
   const int sms = dsp_num_sms();
   if (z_dtype == DSP_F32 && y_dtype == DSP_BF16 && cols % 4 == 0 && whole_groups(z, z_dtype, ldz) && whole_groups(y, y_dtype, ldy)) {
-    const int across = (cols + 4 * XIELU_GROUPS * 128 - 1) / (4 * XIELU_GROUPS * 128);
-    const long fill = (long)(sms > 0 ? sms : 148) * 16 / across + 1, down = rows < fill ? rows : fill;
-    DSP_CUDA(launch_plain(xielu_rows_kernel, dim3(across, (unsigned)(down < 65535 ? down : 65535)), dim3(128), 0, stream,
+    const int threads = cols >= 512 ? 128 : (cols / 4 + 31) / 32 * 32;
+    const long fill = (long)(sms > 0 ? sms : 148) * 16;  // blocks that are resident at once
+    const int groups = rows * ((cols + 4 * threads - 1) / (4 * threads)) <= fill ? 1 : XIELU_GROUPS;
+    const int across = (cols + 4 * groups * threads - 1) / (4 * groups * threads);
+    const long most = fill / across + 1, down = rows < most ? rows : most;
+    auto* kernel = groups == 1 ? xielu_rows_kernel<1> : xielu_rows_kernel<XIELU_GROUPS>;
+    DSP_CUDA(launch_plain(kernel, dim3(across, (unsigned)(down < 65535 ? down : 65535)), dim3(threads), 0, stream,
                           (const float*)z, ldz, pq, (bf16*)y, ldy, rows, cols));
     DSP_CHECK_LAUNCH("dsp_xielu");
     return 0;

@@ -31,7 +31,9 @@ def test_sum_norm(width, x_dtype, off):
         assert torch.equal(y16, y32.to(torch.bfloat16))
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 4), (3, 2048), (2, 2052), (5, 8960), (2500, 60), (4, 66)])
+@pytest.mark.parametrize("rows,cols", [(1, 4), (3, 2048), (2, 2052), (5, 8960), (2500, 60), (4, 66),
+                                       # one group a thread and four, and their last stretches
+                                       (2368, 512), (2369, 512), (64, 1536), (700, 2044), (800, 2052), (5000, 132)])
 def test_xielu_rows(rows, cols):
     from dispec_b200.ops import norm32
     z = rnd((rows, cols + 4), 14, 3.0)[:, :cols]
