@@ -84,7 +84,9 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
                      float eps, const void* gain, void* scaled_out, bool* prepared) -> int {
     const void* residual = add ? C : nullptr;
     if (prepared) *prepared = false;
-    if (T <= s.always_few || dsp_gemm_few_rows_faster(T, N, K, (int)s.target_ctas)) {
+    const int few = T <= s.always_few ? 1 : dsp_gemm_few_rows_faster(T, N, K, (int)s.target_ctas);
+    if (few < 0) return few;
+    if (few) {
       const bool prepare = gain && scaled_out;
       if (prepared) *prepared = prepare;
       return dsp_gemm_stream(scaled ? scaled : A, K, W, bias, residual, add ? N : 0, C, N, T, N, K, DSP_BF16,

@@ -24,6 +24,8 @@
 // Epilogues: bias[n], residual[m, n] (32-bit sum, rounded once), or SwiGLU over W rows that
 // alternate in blocks of 16 (16 gate rows, the 16 up rows of the same outputs): C is [M, N/2].
 // Every wait on an mbarrier is bounded; a wait that runs out is recorded in the device error word.
+#include <atomic>
+
 #include <cooperative_groups.h>
 
 #include "tcgen05_common.cuh"
@@ -728,31 +730,36 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
 // Clusters of `splits` CTAs that the device holds at once, for tiles that take an SM to themselves: a cluster
 // stays inside a group of SMs, and what does not fit waits for a second round (16 clusters of 8 in place
-// of 16 of 7: 14.9 us instead of 9.9 for 128 rows x 2,048 x 1,536).
+// of 16 of 7: 14.9 us instead of 9.9 for 128 rows x 2,048 x 1,536).  Asked once a kernel and size; an answer that does
+// not come is an error of this call (0, with the message set) and nothing that is remembered.
 template <int NB, typename TOut>
 int max_clusters(int splits) {
   using C = Cfg<NB>;
-  static int known[MAX_SPLITS + 1] = {};
-  if (known[splits] == 0) {
-    const size_t smem = (size_t)C::STAGES * C::STAGE_BYTES + 1024 + C::INBOX_BYTES;
-    auto kernel = gemm_stream_kernel<NB, TOut>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1, splits, 1);
-    cfg.blockDim = dim3(C::THREADS, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = splits;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) cudaGetLastError();
-    known[splits] = n > 0 ? n : 1;
+  static std::atomic<int> known[MAX_SPLITS + 1] = {};
+  int n = known[splits].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  const size_t smem = (size_t)C::STAGES * C::STAGE_BYTES + 1024 + C::INBOX_BYTES;
+  auto kernel = gemm_stream_kernel<NB, TOut>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, splits, 1);
+  cfg.blockDim = dim3(C::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = splits;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+  if (e != cudaSuccess || n <= 0) {
+    dsp_set_error("dsp_gemm_stream: how many clusters of %d CTAs fit is not known (%s)", splits, cudaGetErrorString(e));
+    cudaGetLastError();
+    return 0;
   }
-  return known[splits];
+  known[splits].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 template <int NB, typename TOut>
@@ -788,7 +795,7 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const Args& a, in
 struct Plan {
   int nb_rows;          // columns of a tile (rows of A, padded)
   int tiles;            // blocks of W x chunks
-  int splits, kb_per_split;
+  int splits, kb_per_split;  // splits 0: no plan (the message is set)
 };
 
 Plan make_plan(int M, int N, int K, int out_dtype, int target_ctas, bool may_split) {
@@ -806,7 +813,14 @@ Plan make_plan(int M, int N, int K, int out_dtype, int target_ctas, bool may_spl
       if (p.nb_rows == 128) return out_dtype == DSP_BF16 ? max_clusters<128, bf16>(n) : max_clusters<128, float>(n);
       return out_dtype == DSP_BF16 ? max_clusters<192, bf16>(n) : max_clusters<192, float>(n);
     };
-    while (splits > 1 && fits(splits) < p.tiles) --splits;
+    for (; splits > 1; --splits) {
+      const int n = fits(splits);
+      if (n == 0) {
+        p.splits = 0;
+        return p;
+      }
+      if (n >= p.tiles) break;
+    }
   }
   p.kb_per_split = (kb_total + splits - 1) / splits;
   p.splits = (kb_total + p.kb_per_split - 1) / p.kb_per_split;
@@ -814,7 +828,7 @@ Plan make_plan(int M, int N, int K, int out_dtype, int target_ctas, bool may_spl
 }
 }  // namespace
 
-// Whether this product beats the many-row one (gemm_tcgen05.cu) at M rows, which matters above 128: the
+// Whether this product beats the many-row one (gemm_tcgen05.cu) at M rows (-1: not known, the message is set), which matters above 128: the
 // many-row kernel cuts C into tiles of 256 rows x 192 or 256 columns and does not split K, so a narrow product with
 // a long K (down_proj: 8 tiles of 140 k blocks) keeps a tenth of the SMs busy; this one has tiles of 128
 // columns x up to 192 rows and splits K over a cluster, but moves 40 KB for a product half as large.
@@ -834,6 +848,7 @@ extern "C" int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas) {
   if (2.0 * N * K / 6.5e6 > many) many = 2.0 * N * K / 6.5e6;  // W at the memory's rate
   if (many <= few_fixed) return 0;
   const Plan p = make_plan(M, N, K, DSP_BF16, target_ctas, N % 4 == 0);
+  if (p.splits == 0) return -1;
   const long rounds = p.splits > 1 ? 1 : (p.tiles + target_ctas - 1) / target_ctas;
   return few_fixed + (double)rounds * p.kb_per_split * few_k_block < many;
 }
@@ -919,6 +934,7 @@ extern "C" int dsp_gemm_stream(const void* A, long lda, const void* W, const voi
                       (bias == nullptr || ((uintptr_t)bias & 7) == 0) &&
                       (C2 == nullptr || (ldc2 % 4 == 0 && ((uintptr_t)C2 & mask) == 0 && ((uintptr_t)gain2 & 7) == 0));
   const Plan plan = make_plan(M, N, K, out_dtype, target_ctas > 0 ? target_ctas : num_sms, vec_ok);
+  if (plan.splits == 0) return -1;
   const int nb_rows = plan.nb_rows, tiles = plan.tiles, splits = plan.splits;
   CUtensorMap map_w, map_x;
   DSP_REQUIRE(make_map(&map_w, W, N, K, K, ROWS_W), "dsp_gemm_stream: cannot encode the tensor map of W");

@@ -52,7 +52,10 @@ def rows_in_chunks_is_faster(M: int, N: int, K: int, device=None, chunk_rows: in
 @functools.lru_cache(maxsize=4096)
 def _few_rows_faster(M: int, N: int, K: int, sms: int) -> bool:
     from dispec_b200.ops import library
-    return bool(library.core().dsp_gemm_few_rows_faster(M, N, K, STREAM_CTAS_PER_SM * sms))
+    answer = library.core().dsp_gemm_few_rows_faster(M, N, K, STREAM_CTAS_PER_SM * sms)
+    if answer < 0:  # (an exception is not kept by the cache)
+        library.check(answer, launches=0)
+    return bool(answer)
 
 
 # ---- attention of single tokens (attn_mma.cu, decode kernel) ---------------------------------
