@@ -828,29 +828,36 @@ Plan make_plan(int M, int N, int K, int out_dtype, int target_ctas, bool may_spl
 }
 }  // namespace
 
-// Whether this product beats the many-row one (gemm_tcgen05.cu) at M rows (-1: not known, the message is set), which matters above 128: the
-// many-row kernel cuts C into tiles of 256 rows x 192 or 256 columns and does not split K, so a narrow product with
-// a long K (down_proj: 8 tiles of 140 k blocks) keeps a tenth of the SMs busy; this one has tiles of 128
-// columns x up to 192 rows and splits K over a cluster, but moves 40 KB for a product half as large.
-// Estimates in microseconds, fitted on launches that follow one another in a graph and read W from
-// memory.  This kernel and the many-row kernel, 1.5B sizes, qkv / o_proj / gate_up / down: 9.5 / 9.1 / 17.3 / 14.9 us
-// and 11.4 / 14.0 / 16.0 / 45.6 at 137 rows; 15.3 / 13.5 / 36.2 / 27.2 and 11.8 / 14.6 / 30.4 / 46.4 at 536; 16.3 /
-// 16.3 / 64 / 37.8 and 12.7 / 14.8 / 40.7 / 47.6 at 1,016.  7B sizes, qkv / o_proj / down: 17.5 / 15.4 / 36 and 21.4 /
-// 23.6 / 90 at 192; 22.1 / 23.1 / 66 and 22.8 / 24.1 / 91 at 384; 28.5 / 31.6 / 118 and 23.2 / 25.0 / 92 at 536.
+// Whether this product beats the many-row one (gemm_tcgen05.cu) at M rows, which matters above 128 (-1: not known,
+// the message is set): the many-row kernel cuts C into tiles of 256 rows x 192 or 256 columns and does not split K,
+// so a narrow product with a long K (down_proj: 8 tiles of 140 k blocks) keeps a tenth of the SMs busy; this one has
+// tiles of 128 columns x up to 192 rows and splits K over a cluster, but moves 40 KB for a product half as large.
+// Estimates in microseconds, fitted on launches that follow one another in a graph and read W from memory: 18
+// shapes from 512 x 4,096 to 3,584 x 18,944 and 17,920 x 1,536, 129 to 2,048 rows each; of the 342, five take the kernel
+// that is more than 2 % slower (at most 8 %: 17,920 x 1,536 at 129 rows).  This kernel and the many-row kernel, N x K 2,048 x 1,536 / 1,536 x 1,536 / 17,920 x 1,536 / 1,536 x 8,960 / 3,584 x 18,944: 9.4 / 8.9 /
+// 17.5 / 15.0 / 34 us and 11.5 / 12.5 / 19.0 / 43 / 86 at 129 rows; 12.9 / 11.7 / 30 / 20.5 / 62 and 11.6 / 12.9 / 25 / 44 / 89 at
+// 384; 15.1 / 12.9 / 37 / 27 / 109 and 11.7 / 12.9 / 32 / 44 / 89 at 536; 15.6 / 15.6 / 64 / 37 / 204 and 12.9 / 13.1 / 44 /
+// 46 / 106 at 1,016.
 extern "C" int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas) {
   if (M <= 0 || N <= 0 || K <= 0 || target_ctas <= 0) return 0;
-  const double few_fixed = 9.0, few_k_block = 0.39;     // 40 KB a k block of 64
-  const double many_fixed = 5.0, many_k_block = 0.31;   // a CTA pair that streams alone
-  const long pairs = target_ctas / 2 > 0 ? target_ctas / 2 : 1;
-  const long many_tiles = (long)((M + 255) / 256) * ((N + 255) / 256);
   const int k_blocks = (K + BK - 1) / BK;
-  double many = many_fixed + (double)((many_tiles + pairs - 1) / pairs) * k_blocks * many_k_block;
-  if (2.0 * N * K / 6.5e6 > many) many = 2.0 * N * K / 6.5e6;  // W at the memory's rate
-  if (many <= few_fixed) return 0;
+  const double w_us = 2.0 * N * K / 6.5e6;  // W at the memory's rate
+  // the many-row kernel: the rounds of its tiles over the CTA pairs, of the width that it would choose
+  const long pairs = target_ctas / 2 > 0 ? target_ctas / 2 : 1;
+  auto many_tiles = [&](int width) { return (long)((M + 255) / 256) * ((N + width - 1) / width); };
+  auto many_rounds = [&](int width) { return (many_tiles(width) + pairs - 1) / pairs; };
+  const int width = 0.92 * many_rounds(192) < many_rounds(256) ? 192 : 256;
+  const double many_busy = fmin(1.0, (double)many_tiles(width) / pairs);
+  const double many = 5.0 + many_rounds(width) * (1.2 + k_blocks * (0.23 + 0.056 * many_busy)) + 0.44 * w_us;
+  // this one: a k block costs more while more CTAs stream; storing a tile, and the partial rows a split sends and adds,
+  // go with the rows of a tile
   const Plan p = make_plan(M, N, K, DSP_BF16, target_ctas, N % 4 == 0);
   if (p.splits == 0) return -1;
   const long rounds = p.splits > 1 ? 1 : (p.tiles + target_ctas - 1) / target_ctas;
-  return few_fixed + (double)rounds * p.kb_per_split * few_k_block < many;
+  const double busy = fmin(1.0, (double)p.tiles * p.splits / target_ctas), rows = Chunks(M).rows / 192.0;
+  const double few = 3.8 + 0.98 * busy + (double)rounds * p.kb_per_split * (0.29 + 0.06 * busy) + 3.72 * rows +
+                     (p.splits > 1 ? rows * (0.85 * busy + 5.13 / p.splits) : 0.0) + 0.15 * w_us;
+  return 1.02 * few < many;
 }
 
 #ifdef DSP_STAMPS

@@ -53,7 +53,11 @@ def test_more_rows_than_a_tile(M, N, K, bias, resid, swiglu):
 
 
 @pytest.mark.parametrize("M,N,K,few", [(137, 1536, 8960, True), (137, 17920, 1536, False), (536, 1536, 8960, True),
-                                       (536, 2048, 1536, False), (2048, 1536, 8960, False), (4500, 1536, 1536, False)])
+                                       (536, 2048, 1536, False), (2048, 1536, 8960, False), (4500, 1536, 1536, False),
+                                       # where the other kernel was measured a tenth slower or more
+                                       (384, 2048, 1536, False), (384, 1536, 1536, True), (900, 512, 4096, True),
+                                       (300, 3584, 18944, True), (385, 3584, 18944, False), (1152, 1536, 8960, True),
+                                       (1500, 1536, 8960, False), (384, 4608, 3584, True), (450, 4096, 4096, False)])
 def test_which_kernel_runs(M, N, K, few):
     from dispec_b200.ops import tuning
     assert tuning.rows_in_chunks_is_faster(M, N, K, torch.device(DEV)) is few
