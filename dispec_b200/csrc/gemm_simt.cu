@@ -153,20 +153,25 @@ template <typename TOut>
 __global__ void __launch_bounds__(256)
 bf16_kernel(const bf16* __restrict__ A, long lda, const bf16* __restrict__ W, const bf16* __restrict__ bias,
             const TOut* __restrict__ residual, long ldr, TOut* __restrict__ C, long ldc, int M, int N, int K) {
-  __shared__ float as[BF_K][BF_M + 4], ws[BF_K][BF_N + 4];
-  const int tid = threadIdx.x, m0 = blockIdx.y * BF_M, n0 = blockIdx.x * BF_N;
+  __shared__ float as[BF_K][BF_M + 4];
+  __shared__ float ws[BF_K][BF_N + 4];
+  const int tid = threadIdx.x;
+  const int m0 = blockIdx.y * BF_M, n0 = blockIdx.x * BF_N;
   const int tx = tid % 16, ty = tid / 16;  // outputs rows ty * 4 .., columns tx * 4 ..
   float acc[BF_T][BF_T];
 #pragma unroll
   for (int i = 0; i < BF_T; ++i)
 #pragma unroll
     for (int j = 0; j < BF_T; ++j) acc[i][j] = 0.f;
+
   for (int k0 = 0; k0 < K; k0 += BF_K) {
 #pragma unroll
     for (int e = 0; e < BF_M * BF_K / 256; ++e) {
-      const int idx = tid + e * 256, r = idx / BF_K, c = idx % BF_K, m = m0 + r, n = n0 + r, k = k0 + c;
-      as[c][r] = m < M && k < K ? to_f32(A[(size_t)m * lda + k]) : 0.f;
-      ws[c][r] = n < N && k < K ? to_f32(W[(size_t)n * K + k]) : 0.f;
+      const int idx = tid + e * 256;
+      const int r = idx / BF_K, c = idx % BF_K;
+      const int m = m0 + r, n = n0 + r, k = k0 + c;
+      as[c][r] = (m < M && k < K) ? to_f32(A[(size_t)m * lda + k]) : 0.f;
+      ws[c][r] = (n < N && k < K) ? to_f32(W[(size_t)n * K + k]) : 0.f;
     }
     __syncthreads();
 #pragma unroll
@@ -184,12 +189,19 @@ bf16_kernel(const bf16* __restrict__ A, long lda, const bf16* __restrict__ W, co
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < BF_T; ++i)
+  for (int i = 0; i < BF_T; ++i) {
+    const int m = m0 + ty * BF_T + i;
+    if (m >= M) continue;
 #pragma unroll
     for (int j = 0; j < BF_T; ++j) {
-      const int m = m0 + ty * BF_T + i, n = n0 + tx * BF_T + j;
-      if (m < M && n < N) finish(acc[i][j], bias, residual, ldr, C, ldc, m, n);
+      const int n = n0 + tx * BF_T + j;
+      if (n >= N) continue;
+      float v = acc[i][j];
+      if (bias) v += to_f32(bias[n]);
+      if (residual) v += to_f32(residual[(size_t)m * ldr + n]);
+      C[(size_t)m * ldc + n] = from_f32<TOut>(v);
     }
+  }
 }
 
 template <typename TOut>
