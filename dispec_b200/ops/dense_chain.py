@@ -102,6 +102,10 @@ def run_layers(model, ctx, x: torch.Tensor) -> bool:
         cache = ctx.cache_view(model.placement[model.call_cache[i]], call.write)
         rot = m.position_encoding.rotation()
         keys, values = cache.key_pool, cache.value_pool
+        # weights are kept as a source handed them over; where one begins off a 16-byte address, its product is one that
+        # the parts choose
+        if (m.w_qkv.data_ptr() | m.w_o.data_ptr() | f.w_gate_up.data_ptr() | f.w_down.data_ptr()) % 16:
+            return False
         _LAYER.pack_into(table, i * _LAYER.size, address(m.w_qkv), address(m.b_qkv), address(m.w_o), address(m.b_o),
                          address(f.w_gate_up), address(f.w_down), address(b.mixer_norm.weight),
                          address(b.ffn_norm.weight), address(keys), address(values), address(cache.page_table),

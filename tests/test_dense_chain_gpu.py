@@ -72,3 +72,55 @@ def test_from_captured_steps():
 @pytest.mark.parametrize("changes", [dict(intermediate_size=232), dict(head_dim=24)])
 def test_sizes_that_stay_with_the_parts(changes):
     assert not model_of(**changes).dense_chain
+
+
+def test_weights_off_sixteen_bytes_stay_with_the_parts():
+    """A source may serve views of one slab at any offset: the parts' products take them, the chain's do not."""
+    from dispec_b200.ops.library import LaunchCounter
+    model = model_of()
+    for part, name in ((model.layers[0].mixer, "w_o"), (model.layers[-1].feed_forward, "w_down")):
+        w = getattr(part, name)
+        slab = torch.empty(w.numel() + 3, dtype=w.dtype, device=w.device)
+        slab[3:].copy_(w.flatten())
+        setattr(part, name, slab[3:].view(w.shape))
+    n0 = LaunchCounter.n
+    mine, _ = run(model, True, [70, 9], 2, 16)
+    n1 = LaunchCounter.n
+    parts, _ = run(model, False, [70, 9], 2, 16)
+    assert LaunchCounter.n - n1 == n1 - n0
+    for a, b in zip(mine, parts):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("prompts,stored", [([137], 0), ([536], 0), ([700, 40], 0), ([1900], 0), ([24, 5], 4200), ([300], 9000)])
+def test_same_bits_at_the_sizes_where_c_chooses(prompts, stored):
+    """Two layers of the 1.5B sizes: few-row products above 128 rows, products that let their successor start late, norms a
+    warp a row, and (``stored``) a single token whose keys are cut into ranges beyond a cluster."""
+    from dispec_b200.engine import ModelRunner, SeqEntry
+    from dispec_b200.ops import attention as A, tuning
+    dev = torch.device(DEV)
+    model = model_of(hidden_size=1536, intermediate_size=8960, num_hidden_layers=2, num_attention_heads=12,
+                     num_key_value_heads=2, head_dim=128, max_position_embeddings=16384)
+    assert model.dense_chain
+    T = sum(prompts) + (stored > 0)
+    assert tuning.rows_in_chunks_is_faster(T, 1536, 8960, dev) is (T <= 1152) and 2 * 1536 * 8960 >= tuning.STREAM_LATE_TRIGGER_BYTES
+    if stored:
+        splits = A.choose_splits(1, 2, stored + 1, dev)
+        assert A.choose_outer(1, 2, stored + 1, splits, dev) > 1
+    vocab, out = model.spec.vocab_size, []
+    for chain in (True, False):
+        model.dense_chain = chain
+        runner = ModelRunner(model, page_size=16, num_pages=(stored + sum(prompts)) // 16 + 40, max_num_seqs=4)
+        entries = []
+        if stored:
+            runner.admit("long")
+            ids = ru.random_ids(stored + 1, vocab, 11)
+            for at in range(0, stored, 1500):
+                runner.step([SeqEntry("long", ids[at:min(stored, at + 1500)], at)])
+            entries.append(SeqEntry("long", ids[stored:], stored, [0]))
+        for i, n in enumerate(prompts):
+            runner.admit(i)
+            entries.append(SeqEntry(i, ru.random_ids(n, vocab, 20 + i), 0, [n - 1, n // 2]))
+        out.append(runner.step(entries).clone())
+        runner.check_device()
+    assert torch.equal(*out) and out[0].isfinite().all()
