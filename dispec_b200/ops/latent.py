@@ -260,8 +260,11 @@ def latent_attention_prompts(ctx, q: torch.Tensor, q_head_stride: int, qr_off: i
     assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1 and gate.shape == out.shape)
     _checked_sink(sink, num_heads)
     lib = L.latent_prompt_library(dim, vdim)
-    new = lambda columns: torch.empty((expanded_room(rows), columns), dtype=torch.bfloat16, device=q.device)[:rows]
+    room = expanded_room(rows)
+    new = lambda columns: torch.empty((room, columns), dtype=torch.bfloat16, device=q.device)
     c_rows, r_rows, kv = new(R), new(PROMPT_ROT_DIM), new(num_heads * (dim + vdim))
+    if room != rows:
+        c_rows, kv = c_rows[:rows], kv[:rows]
     bad = torch.empty((S, max_tiles), dtype=torch.int64, device=q.device)
     L.check(lib.dsp_latent_gather(
         L.ptr(c_pool), L.ptr(r_pool), L.ptr(page_table), page_table.stride(0), L.ptr(ctx.q_start), L.ptr(ctx.ctx_len),

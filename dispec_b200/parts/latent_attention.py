@@ -100,19 +100,22 @@ class LatentAttention(JoinableMixer):
     def _expanded_bytes(self, ctx, q, c_pool, r_pool, out, gate) -> int:
         """Bytes of working memory with which the step's portions of prompts run on expanded keys and values; 0: they
         stay on the latents."""
-        H, d, r, dv, R, first = self.num_heads, self.dim, self.rot_dim, self.vdim, self.kv_rank, ctx.num_decode_seqs
-        if not (latent_ops.prompt_operands_fit(q, d + r, d, c_pool, r_pool, out, gate)
-                and latent_ops.PROMPT_TOKENS_PER_TILE in ctx.attention_tiles
-                and latent_ops.mma_supported(R, r, c_pool.dtype) and latent_ops.mma_tokens_per_tile(H) in ctx.attention_tiles):
+        H, d, r, dv, R = self.num_heads, self.dim, self.rot_dim, self.vdim, self.kv_rank
+        key = ("expanded_latents", H, d, dv, R, self.window)  # the layers of a step ask the same
+        need = ctx.scratch.get(key)
+        if need is None:
+            need, first = 0, ctx.num_decode_seqs
+            spans = ctx.host_q_len[first:], ctx.host_ctx_len[first:]
+            if (latent_ops.PROMPT_TOKENS_PER_TILE in ctx.attention_tiles and latent_ops.mma_supported(R, r, c_pool.dtype)
+                    and latent_ops.mma_tokens_per_tile(H) in ctx.attention_tiles):
+                need = latent_ops.expanded_bytes(*spans, H, d, dv, R, self.window)
+                if need > latent_ops.PROMPT_MAX_BYTES or not latent_ops.expanded_is_faster(
+                        *spans, H, d + dv, R, self.window, tuning.sm_count(q.device)):
+                    need = 0
+            ctx.scratch[key] = need
+        if not (need and latent_ops.prompt_operands_fit(q, d + r, d, c_pool, r_pool, out, gate) and ctx.storage.room_beside(need)):
             return 0
-        spans = ctx.host_q_len[first:], ctx.host_ctx_len[first:]
-        need = latent_ops.expanded_bytes(*spans, H, d, dv, R, self.window)
-        if need > latent_ops.PROMPT_MAX_BYTES:
-            return 0
-        key = ("expanded_is_faster", H, d + dv, R, self.window)  # the layers of a step ask the same
-        if key not in ctx.scratch:
-            ctx.scratch[key] = latent_ops.expanded_is_faster(*spans, H, d + dv, R, self.window, tuning.sm_count(q.device))
-        return need if ctx.scratch[key] and ctx.storage.room_beside(need) else 0
+        return need
 
     def heads(self, ctx, down, cache, state, out):
         H, d, r, dv, R, Q = self.num_heads, self.dim, self.rot_dim, self.vdim, self.kv_rank, self.q_rank
