@@ -4,7 +4,7 @@
 // every head), which costs 2,176 operations a query, key and head but needs no memory: right for single tokens,
 // whose time is the reading of the cache.  A portion of a prompt pays 3.4 times the operations of keys and
 // values of 128 + 64 and 128, on mma.sync.  Here the latents of the portion's keys are gathered from the pages
-// (dsp_latent_gather), one ordinary product expands them to every head's keys and values, rows
+// (latent_gather_kernel), one ordinary product expands them to every head's keys and values, rows
 // [key of head 0 | key of head 1 | ... | value of head 0 | ...], and this kernel runs over those rows.
 //
 // A tile is 128 tokens of one sequence and one head.  Roles as in attn_tcgen05.cu, one CTA per tile:
@@ -551,20 +551,15 @@ latent_gather_kernel(const bf16* __restrict__ c_pool, const bf16* __restrict__ r
     }
   }
 }
-}  // namespace
 
 // Latents [rows, R] and rotated parts [rows, 64] of the keys that the portions of prompts (sequences singles ..
 // singles + portions - 1) see, one sequence after the other; bad [portions][max_tiles].
-extern "C" int dsp_latent_gather(const void* c_pool, const void* r_pool, const int* page_table, int pt_stride,
-                                 const int* q_start, const int* ctx_len, int singles, int portions, int window,
-                                 void* c_rows, void* r_rows, void* bad, int max_tiles, int R, int page_size,
-                                 int num_pages, cudaStream_t stream) {
-  if (portions == 0) return 0;
-  DSP_REQUIRE(R > 0 && R % 8 == 0 && max_tiles > 0 && portions <= 65535 && page_size > 0, "dsp_latent_gather: R=%d, portions=%d", R, portions);
+int gather(const void* c_pool, const void* r_pool, const int* page_table, int pt_stride, const int* q_start,
+           const int* ctx_len, int singles, int portions, int window, void* c_rows, void* r_rows, void* bad, int max_tiles,
+           int R, int page_size, int num_pages, int* err, cudaStream_t stream) {
+  DSP_REQUIRE(R > 0 && R % 8 == 0 && max_tiles > 0 && portions <= 65535 && page_size > 0, "dsp_latent_prompts: R=%d, portions=%d", R, portions);
   DSP_REQUIRE(((uintptr_t)c_pool | (uintptr_t)r_pool | (uintptr_t)c_rows | (uintptr_t)r_rows) % 16 == 0,
-              "dsp_latent_gather: rows must be 16-byte aligned");
-  int* err = dsp_device_error_ptr();
-  DSP_REQUIRE(err != nullptr, "dsp_latent_gather: no device error word");
+              "dsp_latent_prompts: rows must be 16-byte aligned");
   DSP_CUDA(launch_plain(latent_gather_kernel, dim3(max_tiles, portions), dim3(GATHER_THREADS), 0, stream,
                         (const bf16*)c_pool, (const bf16*)r_pool, page_table, pt_stride, q_start, ctx_len, singles, window,
                         (bf16*)c_rows, (bf16*)r_rows, (unsigned long long*)bad, max_tiles, R, DR, page_size, num_pages, err));
@@ -572,19 +567,65 @@ extern "C" int dsp_latent_gather(const void* c_pool, const void* r_pool, const i
 }
 
 // kv [rows, H * (DK + DV)]: every head's unrotated key, then every head's value, of the rows gathered above.
-extern "C" int dsp_attn_latent_prompt(const void* q, long q_stride, int q_head_stride, int qr_off, const float* inv_freq,
-                                      int rot, int layout, float mag, const void* kv, const void* r_rows, long rows,
-                                      const int* q_start, const int* ctx_len, const int* tile_seq, const int* tile_tok0,
-                                      int tile_offset, int num_tiles, int singles, int window, const void* bad,
-                                      int max_tiles, void* out, long out_stride, const float* gate, long ldg,
-                                      const float* sink, int H, float scale, cudaStream_t stream) {
-  if (num_tiles <= 0) return 0;
-  DSP_REQUIRE(H > 0 && num_tiles <= 65535 && rows > 0 && scale > 0.f, "dsp_attn_latent_prompt: %d heads, %d tiles", H, num_tiles);
-  DSP_REQUIRE(rot >= 0 && rot <= DR && rot % 2 == 0 && (rot == 0 || inv_freq) && (layout == 0 || layout == 1) && window >= 0,
-              "dsp_attn_latent_prompt: rot=%d layout=%d window=%d", rot, layout, window);
-  DSP_REQUIRE(q_stride % 8 == 0 && q_head_stride % 8 == 0 && qr_off % 8 == 0 && out_stride % 8 == 0 &&
-                  ((uintptr_t)q | (uintptr_t)kv | (uintptr_t)r_rows | (uintptr_t)out) % 16 == 0,
-              "dsp_attn_latent_prompt: operands must be 16-byte aligned with strides in whole 16-byte pieces");
+int attention(const Params& p, const void* kv, const void* r_rows, long rows, int num_tiles, int H, cudaStream_t stream) {
+  DSP_REQUIRE(H > 0 && num_tiles <= 65535 && rows > 0 && p.scale_log2 > 0.f, "dsp_latent_prompts: %d heads, %d tiles", H, num_tiles);
+  DSP_REQUIRE(p.rot >= 0 && p.rot <= DR && p.rot % 2 == 0 && (p.rot == 0 || p.inv_freq) && (p.layout == 0 || p.layout == 1) && p.window >= 0,
+              "dsp_latent_prompts: rot=%d layout=%d window=%d", p.rot, p.layout, p.window);
+  DSP_REQUIRE(p.q_stride % 8 == 0 && p.q_head_stride % 8 == 0 && p.qr_off % 8 == 0 && p.out_stride % 8 == 0 &&
+                  ((uintptr_t)p.q | (uintptr_t)kv | (uintptr_t)r_rows | (uintptr_t)p.out) % 16 == 0,
+              "dsp_latent_prompts: operands must be 16-byte aligned with strides in whole 16-byte pieces");
+  const long columns = (long)H * (DK + DV);
+  CUtensorMap map_k, map_r, map_v;
+  DSP_REQUIRE(make_map_k_blocks(&map_k, kv, rows, columns, columns, BN, DK / 64) &&
+                  make_map_k_blocks(&map_v, kv, rows, columns, columns, BN, DV / 64) &&
+                  make_map(&map_r, r_rows, rows, DR, DR, BN),
+              "dsp_latent_prompts: cannot encode the tensor maps");
+  DSP_CUDA(cudaFuncSetAttribute(attn_latent_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  DSP_CUDA(launch_plain(attn_latent_prompt_kernel, dim3(H, num_tiles), dim3(THREADS), SMEM_BYTES, stream, p, map_k, map_r, map_v));
+  return 0;
+}
+}  // namespace
+
+extern "C" {
+int dsp_gemm_stream(const void* A, long lda, const void* W, const void* bias, const void* residual, long ldr, void* C,
+                    long ldc, int M, int N, int K, int out_dtype, int target_ctas, int epilogue, long late_trigger_bytes,
+                    const void* norm_src, long ld_src, float norm_eps, const void* gain2, void* C2, long ldc2,
+                    cudaStream_t stream);
+int dsp_gemm_tcgen05(const void* A, long lda, const void* W, const void* bias, const void* residual, long ldr, void* C,
+                     long ldc, int M, int N, int K, int out_dtype, int pair_mode, int epilogue, cudaStream_t stream);
+int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas);
+}
+
+// The three launches of a layer behind one call (called one by one from Python, with an allocation each, they cost
+// the host some 30 us more than the three launches on the latents, and short portions are bound by the host): gathers the
+// latents of the `rows` keys, expands them by `w_kv` [H * (DK + DV), R], on the product that ops/gemm.py would choose,
+// and attends.  `work`: 2 room (R + 64 + H (DK + DV)) + 8 portions max_tiles bytes, room >= rows a multiple of 64.
+extern "C" int dsp_latent_prompts(const void* c_pool, const void* r_pool, const int* page_table, int pt_stride,
+                                  const int* q_start, const int* ctx_len, int singles, int portions, int window,
+                                  const void* w_kv, void* work, long rows, long room, int max_tiles, int R, int page_size,
+                                  int num_pages, const void* q, long q_stride, int q_head_stride, int qr_off,
+                                  const float* inv_freq, int rot, int layout, float mag, const int* tile_seq,
+                                  const int* tile_tok0, int num_tiles, void* out, long out_stride, const float* gate,
+                                  long ldg, const float* sink, int H, float scale, int target_ctas, int always_few,
+                                  long late_trigger_bytes, cudaStream_t stream) {
+  if (portions <= 0 || num_tiles <= 0) return 0;
+  DSP_REQUIRE(rows > 0 && rows <= room && room % 64 == 0 && room < (1l << 31), "dsp_latent_prompts: %ld rows in room for %ld", rows, room);
+  int* err = dsp_device_error_ptr();
+  DSP_REQUIRE(err != nullptr, "dsp_latent_prompts: no device error word");
+  const int columns = H * (DK + DV);
+  bf16* c_rows = (bf16*)work;
+  bf16* r_rows = c_rows + room * R;
+  bf16* kv = r_rows + room * DR;
+  void* bad = kv + room * columns;
+  int rc = gather(c_pool, r_pool, page_table, pt_stride, q_start, ctx_len, singles, portions, window, c_rows, r_rows, bad,
+                  max_tiles, R, page_size, num_pages, err, stream);
+  if (rc != 0) return rc;
+  const int few = rows <= always_few ? 1 : dsp_gemm_few_rows_faster((int)rows, columns, R, target_ctas);
+  if (few < 0) return few;
+  rc = few ? dsp_gemm_stream(c_rows, R, w_kv, nullptr, nullptr, 0, kv, columns, (int)rows, columns, R, DSP_BF16, target_ctas, 0,
+                             late_trigger_bytes, nullptr, 0, 0.f, nullptr, nullptr, 0, stream)
+           : dsp_gemm_tcgen05(c_rows, R, w_kv, nullptr, nullptr, 0, kv, columns, (int)rows, columns, R, DSP_BF16, 1, 0, stream);
+  if (rc != 0) return rc;
   Params p;
   p.q = (const bf16*)q;
   p.q_stride = q_stride;
@@ -598,7 +639,7 @@ extern "C" int dsp_attn_latent_prompt(const void* q, long q_stride, int q_head_s
   p.ctx_len = ctx_len;
   p.tile_seq = tile_seq;
   p.tile_tok0 = tile_tok0;
-  p.tile_offset = tile_offset;
+  p.tile_offset = singles;
   p.singles = singles;
   p.window = window;
   p.bad = (const unsigned long long*)bad;
@@ -609,15 +650,6 @@ extern "C" int dsp_attn_latent_prompt(const void* q, long q_stride, int q_head_s
   p.ldg = ldg;
   p.sink = sink;
   p.scale_log2 = scale * 1.4426950408889634f;
-  p.err = dsp_device_error_ptr();
-  DSP_REQUIRE(p.err != nullptr, "dsp_attn_latent_prompt: no device error word");
-  const long columns = (long)H * (DK + DV);
-  CUtensorMap map_k, map_r, map_v;
-  DSP_REQUIRE(make_map_k_blocks(&map_k, kv, rows, columns, columns, BN, DK / 64) &&
-                  make_map_k_blocks(&map_v, kv, rows, columns, columns, BN, DV / 64) &&
-                  make_map(&map_r, r_rows, rows, DR, DR, BN),
-              "dsp_attn_latent_prompt: cannot encode the tensor maps");
-  DSP_CUDA(cudaFuncSetAttribute(attn_latent_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  DSP_CUDA(launch_plain(attn_latent_prompt_kernel, dim3(H, num_tiles), dim3(THREADS), SMEM_BYTES, stream, p, map_k, map_r, map_v));
-  return 0;
+  p.err = err;
+  return attention(p, kv, r_rows, rows, num_tiles, H, stream);
 }

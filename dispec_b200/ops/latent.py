@@ -247,7 +247,7 @@ def latent_attention_prompts(ctx, q: torch.Tensor, q_head_stride: int, qr_off: i
     """The attention of the step's portions of prompts, with the value map applied, into their rows of ``out``
     [T, H * vdim] (bfloat16).  ``w_kv`` [H * (dim + vdim), R]: every head's key map, then every head's value
     map; the latents of the keys the portions see are gathered from the pages and expanded by one product."""
-    from dispec_b200.ops import gemm
+    from dispec_b200.ops import gemm, tuning
     num_pages, _, page_size, R = c_pool.shape
     n_dec = ctx.num_decode_seqs
     q_lens, ctx_lens = ctx.host_q_len[n_dec:], ctx.host_ctx_len[n_dec:]
@@ -259,24 +259,18 @@ def latent_attention_prompts(ctx, q: torch.Tensor, q_head_stride: int, qr_off: i
     assert page_table.dtype == torch.int32 and page_table.stride(1) == 1
     assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1 and gate.shape == out.shape)
     _checked_sink(sink, num_heads)
-    lib = L.latent_prompt_library(dim, vdim)
     room = expanded_room(rows)
-    new = lambda columns: torch.empty((room, columns), dtype=torch.bfloat16, device=q.device)
-    c_rows, r_rows, kv = new(R), new(PROMPT_ROT_DIM), new(num_heads * (dim + vdim))
-    if room != rows:
-        c_rows, kv = c_rows[:rows], kv[:rows]
-    bad = torch.empty((S, max_tiles), dtype=torch.int64, device=q.device)
-    L.check(lib.dsp_latent_gather(
-        L.ptr(c_pool), L.ptr(r_pool), L.ptr(page_table), page_table.stride(0), L.ptr(ctx.q_start), L.ptr(ctx.ctx_len),
-        n_dec, S, int(window), L.ptr(c_rows), L.ptr(r_rows), L.ptr(bad), max_tiles, R, page_size, num_pages,
-        L.stream_handle()))
-    gemm.linear(c_rows, w_kv, out=kv)
+    work = torch.empty(room * (R + PROMPT_ROT_DIM + num_heads * (dim + vdim)) + 4 * S * max_tiles, dtype=torch.bfloat16,
+                       device=q.device)
     tile_seq, tile_tok0, n_tiles = ctx.attention_tiles[PROMPT_TOKENS_PER_TILE]
-    L.check(lib.dsp_attn_latent_prompt(
+    L.check(L.latent_prompt_library(dim, vdim).dsp_latent_prompts(
+        L.ptr(c_pool), L.ptr(r_pool), L.ptr(page_table), page_table.stride(0), L.ptr(ctx.q_start), L.ptr(ctx.ctx_len),
+        n_dec, S, int(window), L.ptr(w_kv), L.ptr(work), L.i64(rows), L.i64(room), max_tiles, R, page_size, num_pages,
         L.ptr(q), L.i64(q.stride(0)), q_head_stride, qr_off, L.ptr(inv_freq), rot, _LAYOUTS[layout], L.f32(magnitude),
-        L.ptr(kv), L.ptr(r_rows), L.i64(rows), L.ptr(ctx.q_start), L.ptr(ctx.ctx_len), L.ptr(tile_seq), L.ptr(tile_tok0),
-        n_dec, n_tiles - n_dec, n_dec, int(window), L.ptr(bad), max_tiles, L.ptr(out), L.i64(out.stride(0)), L.ptr(gate),
-        L.i64(gate.stride(0) if gate is not None else 0), L.ptr(sink), num_heads, L.f32(scale), L.stream_handle()))
+        L.ptr(tile_seq), L.ptr(tile_tok0), n_tiles - n_dec, L.ptr(out), L.i64(out.stride(0)), L.ptr(gate),
+        L.i64(gate.stride(0) if gate is not None else 0), L.ptr(sink), num_heads, L.f32(scale),
+        tuning.stream_target_ctas(q.device), gemm.STREAM_MAX_ROWS, L.i64(tuning.STREAM_LATE_TRIGGER_BYTES),
+        L.stream_handle()), launches=3)
 
 
 def head_products_supported(x: torch.Tensor, head_stride: int, w: torch.Tensor) -> bool:
