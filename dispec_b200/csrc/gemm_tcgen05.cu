@@ -587,7 +587,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 }  // namespace
 
 // bfloat16 A [M, K] (row stride lda) and W [N, K] (contiguous); C and residual bfloat16 or float32.
-// pair_mode 0: single CTAs; 1: CTA pairs; 2, 3: pairs with tiles 192, 256 wide (comparisons).
+// pair_mode 0: single CTAs; 1: CTA pairs.
 // epilogue 1: SwiGLU (2: gelu in its tanh form instead of silu) over W rows alternating in blocks of 16 (16 gate rows, their 16 up rows):
 // C is [M, N/2], no bias, no residual.
 extern "C" int dsp_gemm_tcgen05(const void* A, long lda, const void* W, const void* bias, const void* residual,
@@ -629,7 +629,7 @@ extern "C" int dsp_gemm_tcgen05(const void* A, long lda, const void* W, const vo
     const long pairs_avail = num_sms / 2;
     const long m_tiles2 = (M + 2 * BM - 1) / (2 * BM);
     auto rounds = [&](int bn) { return ((long)((N + bn - 1) / bn) * m_tiles2 + pairs_avail - 1) / pairs_avail; };
-    const int bnp = pair_mode == 2 ? 192 : pair_mode == 3 ? 256 : 0.92 * rounds(192) < rounds(256) ? 192 : 256;
+    const int bnp = 0.92 * rounds(192) < rounds(256) ? 192 : 256;
     e.k_boxes = (make_map_k_blocks(&map_a, A, M, K, lda, BM, SUB) && make_map_k_blocks(&map_w, W, N, K, K, bnp / 2, SUB)) ? 1 : 0;
     if (!e.k_boxes) {
       DSP_REQUIRE(make_map(&map_a, A, M, K, lda, BM), "dsp_gemm_tcgen05: cannot encode the tensor map of A");
