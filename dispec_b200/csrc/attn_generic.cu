@@ -1,11 +1,11 @@
 // Causal grouped-query attention over the paged key/value cache, all arithmetic in 32-bit.
 //
-// One block per (query token, KV head); the G = H / KVH query heads of the group share every
-// key and value load.  The query at absolute position p sees keys b with
+// The G = H / KVH query heads of a group, and in heads of up to 128 dimensions several tokens of a portion as
+// well, share every key and value load (the two kernels: below).  The query at absolute position p sees keys b with
 //     max(0, p - window + 1) <= b <= p        (window == 0: every key from 0)
 // which is the lower-right aligned causal mask for a portion of a prompt on top of cached
 // tokens, and a single decoded token alike.  Online softmax (running max m, running sum l)
-// over tiles of 128 keys.  Keys have D dimensions and values Dv (the pools have their own widths).
+// over tiles of 128 or 64 keys.  Keys have D dimensions and values Dv (the pools have their own widths).
 // With `mask_mode` 1 the number `window` is a chunk size instead: position p sees the keys of its own
 // chunk, floor(p / size) * size <= b <= p (chunks counted from position 0 of the sequence).
 // With `keep_first` = F the keys b < F are seen as well, however far behind the window they lie.

@@ -5,8 +5,8 @@
 // one FMA chain over k = 0..K-1 in ascending order, so a row's result does not depend on
 // which other rows are in the batch, nor on which of the kernels below computes it.
 //
-// Two kernels for floats, both fed by 16-byte asynchronous copies a few stages ahead, and one for bfloat16.  `few_rows_kernel` (up to 16 rows)
-// streams W: it is bound by the bytes of W, or, where N is small, by the chain itself (K dependent FMAs of
+// Two kernels for floats, both fed by 16-byte asynchronous copies a few stages ahead, and one for bfloat16
+// (`bf16_kernel`).  `few_rows_kernel` (up to 16 rows) streams W: it is bound by the bytes of W, or, where N is small, by the chain itself (K dependent FMAs of
 // four cycles).  4 rows x 17,920 x 1,536: 44 us (210 with one 64 x 64 tile, single-float loads and no copies
 // ahead); x 1,536 x 8,960: 62 us (1,056).
 // `tile_kernel` holds BM x BN outputs in the registers of a block, 8 x 8 down to 4 x 2 a thread; it is bound

@@ -3,11 +3,12 @@
 // the fifth-generation tensor cores, and of portions of a few hundred rows where the output is narrow.
 //
 // Roles are swapped: 128 rows of W are the M side of tcgen05.mma, the few rows of A (padded to
-// 16, 32, 64, 128 or 192; more are cut into chunks of equal size, tiles of their own) its N side, so the accumulator in tensor memory is 128 lanes (rows of W) by a
-// few columns (rows of A).  One thread streams W tiles of 128 rows x 64 k (16 KB a request)
-// and the matching slice of A by TMA into a ring of 4 to 5 stages (two CTAs per SM, about 180 KB
-// on its way per SM, which plain loads cannot keep in flight); one thread issues the products; four warps read
-// the accumulator, apply the epilogue and store.  With programmatic dependent launch the first
+// 16, 32, 64, 128 or 192; more are cut into chunks of equal size, tiles of their own) its N side, so the
+// accumulator in tensor memory is 128 lanes (rows of W) by a few columns (rows of A).  One thread streams W
+// tiles of 128 rows x 64 k (16 KB a request) and the matching slice of A by TMA into a ring of 4 to 5 stages
+// (two CTAs per SM up to 64 rows of A, about 180 KB on its way per SM, which plain loads cannot keep in
+// flight); one to four threads issue the products; four warps (eight above 64 rows of A) read the
+// accumulator, apply the epilogue and store.  With programmatic dependent launch the first
 // W tiles are requested before the kernel waits for its predecessor.
 //
 // K is split across a thread-block cluster (up to 8 CTAs) when there are too few 128-row blocks
@@ -37,7 +38,7 @@ using namespace tc;
 constexpr int ROWS_W = 128, BK = 64, UMMA_K = 16;
 constexpr int W_BYTES = ROWS_W * BK * 2;
 // warp 0: TMA; then ISSUERS warps whose first lanes issue the products (the first of them also owns
-// the tensor memory); then four epilogue warps
+// the tensor memory); then four epilogue warps, eight where a CTA has an SM to itself
 constexpr int MAX_SPLITS = 8;
 enum { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_GEGLU = 2 };
 
@@ -370,8 +371,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
   }
 
-  // ---- epilogue.  Thread (quarter, lane) of the four epilogue warps owns W row 32 * quarter + lane of
-  // the block (a warp reaches the 32 lanes of tensor memory that its index modulo 4 names).
+  // ---- epilogue.  Thread (quarter, lane) of an epilogue warp owns W row 32 * quarter + lane of the block (a warp
+  // reaches the 32 lanes of tensor memory that its index modulo 4 names; of eight warps, two share a quarter and take
+  // the windows of the accumulator in turn).
   const int quarter = warp & 3;
   const int row = quarter * 32 + lane;
   const bool swiglu = a.epilogue != EPI_PLAIN, gelu = a.epilogue == EPI_GEGLU;
