@@ -179,8 +179,9 @@ rmsnorm_vec_kernel(T* __restrict__ x, const T* __restrict__ delta, const T* __re
   }
 }
 
-// The same with a warp a row, for many rows: no barrier, every row of a wave on its way at once.  bfloat16 only: a warp adds
-// a row's squares in another order than a block, and a 32-bit row must not depend on how many there are.
+// The same with a warp a row, for many rows: no barrier, every row of a wave on its way at once.  A row's squares are added
+// in the order of the block above (piece i belongs to the block's thread i % 256; its warps' sums one after the other), so
+// the results have the same bits: a row does not depend on how many there are.
 constexpr int RMS_WARPS = 4;
 template <typename T, int VPL>
 __global__ void __launch_bounds__(32 * RMS_WARPS)
@@ -201,7 +202,10 @@ rmsnorm_rows_kernel(T* __restrict__ x, const T* __restrict__ delta, const T* __r
 #pragma unroll
   for (int j = 0; j < VPL; ++j)
     if (lane + j * 32 < nvec) wv[j] = __ldg(reinterpret_cast<const uint4*>(w) + lane + j * 32);
-  float ss = 0.f;
+  constexpr int WARPS = VPL < 8 ? VPL : 8;  // of the block's eight, those that have pieces
+  float part[WARPS];
+#pragma unroll
+  for (int j = 0; j < WARPS; ++j) part[j] = 0.f;
 #pragma unroll
   for (int j = 0; j < VPL; ++j) {
     T* e = reinterpret_cast<T*>(&v[j]);
@@ -213,9 +217,12 @@ rmsnorm_rows_kernel(T* __restrict__ x, const T* __restrict__ delta, const T* __r
       if (write_back) xr[lane + j * 32] = v[j];
     }
 #pragma unroll
-    for (int k = 0; k < N; ++k) ss += to_f32(e[k]) * to_f32(e[k]);
+    for (int k = 0; k < N; ++k) part[j % 8] += to_f32(e[k]) * to_f32(e[k]);
   }
-  const float rstd = rsqrtf(warp_sum(ss) / (float)hidden + eps);
+  float total = 0.f;
+#pragma unroll
+  for (int j = 0; j < WARPS; ++j) total += warp_sum(part[j]);
+  const float rstd = rsqrtf(total / (float)hidden + eps);
   uint4* yr = reinterpret_cast<uint4*>(y + (size_t)r * hidden);
 #pragma unroll
   for (int j = 0; j < VPL; ++j) {
@@ -239,10 +246,10 @@ static bool launch_rmsnorm_vec(void* x, const void* delta, const void* w, void* 
   const uintptr_t bits = (uintptr_t)x | (uintptr_t)delta | (uintptr_t)w | (uintptr_t)y;
   if (bits % 16 != 0) return false;
   const int nvec = hidden / N;
-  // A warp a row from 12 rows an SM on.  Block and warp a row, us of a launch among others, rows from memory: 1,024 rows of
-  // 1,024 2.4 and 2.9, of 1,536 2.9 and 3.8; 2,048 rows of 256 3.4 and 2.3, of 1,536 4.5 and 4.4, of 3,072 7.9 and 7.3;
-  // 4,500 rows of 1,536 8.3 and 6.7, of 3,072 14.9 and 12.8.  Up to 3,072: twelve pieces of the row and of the gains a lane are
-  // what its registers hold (at 3,584 a launch with the gains read first took 223 and was the slower one).
+  // A warp a row from 12 rows an SM on.  Block and warp a row, us of a launch among others, rows from memory: 2,048 rows
+  // of 256 3.4 and 2.4, of 1,536 4.5 and 4.45 (from the L2 4.5 and 4.0), of 3,072 7.9 and 7.8; 4,500 rows of 1,536 8.4 and
+  // 6.9, of 3,072 14.7 and 13.4; below, 1,024 rows of 1,536, 2.8 and 3.8.  Up to 3,072: twelve pieces of the row and of the
+  // gains a lane are what its registers hold (at 3,584 they took 223, and the launch was the slower one).
   if constexpr (sizeof(T) == 2) if (n_rows >= 12 * (dsp_num_sms() > 0 ? dsp_num_sms() : 148) && nvec <= 12 * 32) {
     const dim3 grid((n_rows + RMS_WARPS - 1) / RMS_WARPS);
 #define DSP_RMS_ROWS(V) launch_pdl(rmsnorm_rows_kernel<T, V>, grid, dim3(32 * RMS_WARPS), 0, stream, (T*)x, (const T*)delta, (const T*)w, (T*)y, rows, n_rows, hidden, eps, write_back)

@@ -135,13 +135,15 @@ def test_attention_of_a_token_does_not_depend_on_its_portion(H, G_heads, D, wind
         assert torch.equal(parts.view(torch.int32), whole), cut
 
 
-@pytest.mark.parametrize("hidden", [8, 512, 768, 772, 1536])
-def test_rms_norm_of_a_row_does_not_depend_on_the_others(hidden):
+@pytest.mark.parametrize("dtype,hidden", [(torch.float32, h) for h in (8, 512, 768, 772, 1536)]
+                         + [(torch.bfloat16, h) for h in (8, 256, 1024, 1032, 1536, 1544, 2048, 2056, 3072, 3080)])
+def test_rms_norm_of_a_row_does_not_depend_on_the_others(dtype, hidden):
     from dispec_b200 import ops
-    x, w = rnd((2500, hidden), 41), rnd((hidden,), 42)
-    whole = ops.rms_norm(x, w, 1e-6)
+    x, w, delta = rnd((2500, hidden), 41).to(dtype), rnd((hidden,), 42).to(dtype), rnd((2500, hidden), 43).to(dtype)
+    whole, summed = ops.rms_norm(x, w, 1e-6), ops.rms_norm(x, w, 1e-6, delta=delta)
     for n in (1, 3, 592, 1775, 1776):
         assert torch.equal(ops.rms_norm(x[:n].contiguous(), w, 1e-6), whole[:n]), n
+        assert torch.equal(ops.rms_norm(x[:n].contiguous(), w, 1e-6, delta=delta[:n].contiguous()), summed[:n]), n
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 3, 5), (7, 64, 17), (64, 65, 33), (65, 130, 15), (3, 1000, 515)])
