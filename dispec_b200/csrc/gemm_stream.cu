@@ -294,80 +294,89 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   if (C::PUSH && splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 
   if (warp == 0) {
-    if (lane == 0) {
-      // the CTA's work as one flat sequence of (block of W, k block) items
-      const int my_tiles = blockIdx.x < n_tiles ? (n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-      const int total = my_tiles * num_kb;
-      const int first = total < C::STAGES ? total : C::STAGES;
-      auto w_row = [&](int it) { return ((int)blockIdx.x + (it / num_kb) * (int)gridDim.x) / (C::CHUNKED ? ch.count : 1) * ROWS_W; };
-      auto x_row = [&](int it) { return C::CHUNKED ? ((int)blockIdx.x + (it / num_kb) * (int)gridDim.x) % ch.count * ch.rows : 0; };
-      auto k_of = [&](int it) { return (kb_begin + it % num_kb) * BK; };
-      // W does not depend on the kernel before this one: the ring is filled with W tiles first,
-      // then the kernel waits for its predecessor and sends the matching slices of A after them
-      // W is read once per call and is far larger than the L2 over a step: its lines leave first
-      // (with several chunks of rows it is read as often as there are chunks, and stays)
-      const uint64_t once = !C::CHUNKED || ch.count == 1 ? l2_policy_evict_first() : l2_policy_evict_normal();
-      for (int it = 0; it < first; ++it) {
+    // the CTA's work as one flat sequence of (block of W, k block) items
+    const bool leader = elect_one();
+    const int my_tiles = blockIdx.x < n_tiles ? (n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+    const int total = my_tiles * num_kb;
+    const int first = total < C::STAGES ? total : C::STAGES;
+    // W does not depend on the kernel before this one: the ring is filled with W tiles first,
+    // then the kernel waits for its predecessor and sends the matching slices of A after them
+    // W is read once per call and is far larger than the L2 over a step: its lines leave first
+    // (with several chunks of rows it is read as often as there are chunks, and stays)
+    const uint64_t once = !C::CHUNKED || ch.count == 1 ? l2_policy_evict_first() : l2_policy_evict_normal();
+    struct Item {  // a place in the sequence: block of k, tile
+      int kb, tile;
+    };
+    auto advance = [&](Item& i) {
+      if (++i.kb == num_kb) i.kb = 0, i.tile += (int)gridDim.x;
+    };
+    auto k_of = [&](const Item& i) { return (kb_begin + i.kb) * BK; };
+    auto w_row = [&](const Item& i) { return i.tile / (C::CHUNKED ? ch.count : 1) * ROWS_W; };
+    auto x_row = [&](const Item& i) { return C::CHUNKED ? i.tile % ch.count * ch.rows : 0; };
+    Item w_item = {0, (int)blockIdx.x}, x_item = w_item;
+    for (int it = 0; it < first; ++it, advance(w_item)) {
+      const int k = k_of(w_item), w = w_row(w_item);
+      if (leader) {
         mbar_expect_tx(&full_bar[it], C::STAGE_BYTES);
-        tma_load_2d_hint(smem + it * C::STAGE_BYTES, &map_w, &full_bar[it], k_of(it), w_row(it), once);
+        tma_load_2d_hint(smem + it * C::STAGE_BYTES, &map_w, &full_bar[it], k, w, once);
       }
-      STAMP(10);  // the ring's first tiles of W are requested
-      pdl_wait();
-      STAMP(1);  // the predecessor is complete
-      for (int it = 0; it < first; ++it)
-        tma_load_2d(smem + it * C::STAGE_BYTES + W_BYTES, &map_x, &full_bar[it], k_of(it), x_row(it));
-      for (int it = first; it < total; ++it) {
-        const int s = it % C::STAGES;
-        const uint32_t phase = (it / C::STAGES) & 1;
-        if (!mbar_wait(&empty_bar[s], phase ^ 1)) {
-          failed = 1;
-          break;
-        }
-        mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
-        unsigned char* dst = smem + s * C::STAGE_BYTES;
-        tma_load_2d_hint(dst, &map_w, &full_bar[s], k_of(it), w_row(it), once);
-        tma_load_2d(dst + W_BYTES, &map_x, &full_bar[s], k_of(it), x_row(it));
-      }
-      STAMP(7);  // the last tile of W is requested
-      if (a.late_trigger) pdl_launch_dependents();
     }
+    if (lane == 0) STAMP(10);  // the ring's first tiles of W are requested
+    pdl_wait();
+    if (lane == 0) STAMP(1);  // the predecessor is complete
+    for (int it = 0; it < first; ++it, advance(x_item)) {
+      const int k = k_of(x_item), x = x_row(x_item);
+      if (leader) tma_load_2d(smem + it * C::STAGE_BYTES + W_BYTES, &map_x, &full_bar[it], k, x);
+    }
+    int s = 0, phase = 0;
+    for (int it = first; it < total; ++it, advance(x_item)) {
+      if (!mbar_wait(&empty_bar[s], phase)) {
+        failed = 1;
+        break;
+      }
+      unsigned char* dst = smem + s * C::STAGE_BYTES;
+      const int k = k_of(x_item), w = w_row(x_item), x = x_row(x_item);
+      if (leader) {
+        mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
+        tma_load_2d_hint(dst, &map_w, &full_bar[s], k, w, once);
+        tma_load_2d(dst + W_BYTES, &map_x, &full_bar[s], k, x);
+      }
+      if (++s == C::STAGES) s = 0, phase ^= 1;
+    }
+    if (lane == 0) STAMP(7);  // the last tile of W is requested
+    if (a.late_trigger) pdl_launch_dependents();
   } else if (warp <= C::ISSUERS) {
-    if (lane == 0) {
-      // issuer j owns the k steps j, j + ISSUERS, ... of every k block and the partial accumulator j
-      const int j = warp - 1;
-      const uint32_t idesc = umma_idesc(ROWS_W, NB);
-      int it = 0, local = 0;
-      for (int tile = blockIdx.x; tile < n_tiles && !failed; tile += gridDim.x, ++local) {
-        const int buf = local & 1;
-        if (!mbar_wait(&accum_empty[buf], ((local >> 1) & 1) ^ 1)) {
-          failed = 1;
-          break;
-        }
+    // issuer j owns the k steps j, j + ISSUERS, ... of every k block and the partial accumulator j
+    const bool leader = elect_one();
+    const int j = warp - 1;
+    const uint32_t idesc = umma_idesc(ROWS_W, NB);
+    int s = 0, phase = 0, local = 0;
+    for (int tile = blockIdx.x; tile < n_tiles && !failed; tile += gridDim.x, ++local) {
+      const int buf = local & 1;
+      bool ok = mbar_wait(&accum_empty[buf], ((local >> 1) & 1) ^ 1);
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + (uint32_t)(buf * C::ACC_COLS + j * NB);
+      for (int kb = 0; kb < num_kb && ok; ++kb) {
+        ok = mbar_wait(&full_bar[s], phase);
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + (uint32_t)(buf * C::ACC_COLS + j * NB);
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % C::STAGES;
-          const uint32_t phase = (it / C::STAGES) & 1;
-          if (!mbar_wait(&full_bar[s], phase)) {
-            failed = 1;
-            break;
-          }
-          tc_fence_after();
-          if (it == 0 && j == 0) STAMP(2);  // the first stage (W tile and slice of A) has landed
-          const uint32_t w_addr = smem_u32(smem + s * C::STAGE_BYTES);
-          const uint32_t x_addr = w_addr + W_BYTES;
-          static_assert(BK / UMMA_K % C::ISSUERS == 0, "every issuer takes part in every k block");
+        if (kb == 0 && local == 0 && j == 0 && lane == 0) STAMP(2);  // the first stage (W tile and slice of A) has landed
+        const uint64_t w = umma_desc(smem_u32(smem + s * C::STAGE_BYTES) + j * 32), x = w + (W_BYTES >> 4);
+        static_assert(BK / UMMA_K % C::ISSUERS == 0, "every issuer takes part in every k block");
+        if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K / C::ISSUERS; ++k) {
-            const int step = j + k * C::ISSUERS;
-            umma(tmem_d, umma_desc(w_addr + step * 32), umma_desc(x_addr + step * 32), idesc, (kb | k) != 0);
-          }
+          for (int k = 0; k < BK / UMMA_K / C::ISSUERS; ++k)
+            umma(tmem_d, w + k * C::ISSUERS * 2, x + k * C::ISSUERS * 2, idesc, (kb | k) != 0);
           umma_commit(&empty_bar[s]);
         }
-        if (failed) break;
-        umma_commit(&accum_full[buf]);
-        if (j == 0) STAMP(3);  // the last product of a block is issued
+        if (++s == C::STAGES) s = 0, phase ^= 1;
       }
+      if (!ok) {
+        failed = 1;
+        break;
+      }
+      if (leader) umma_commit(&accum_full[buf]);
+      if (j == 0 && lane == 0) STAMP(3);  // the last product of a block is issued
     }
   }
 
