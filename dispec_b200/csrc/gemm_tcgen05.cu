@@ -179,69 +179,65 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
   if (warp == 0) {
     // ---- TMA producer: the ring runs on across tiles
-    if (lane == 0) {
-      // The weights do not depend on the kernel before: the first ring of W tiles is asked for
-      // while that kernel still runs.  A comes from it, so A waits.
-      const int ahead = num_kb < STAGES ? num_kb : STAGES;
-      for (int kb = 0; kb < ahead; ++kb) {
+    // The weights do not depend on the kernel before: the first ring of W tiles is asked for
+    // while that kernel still runs.  A comes from it, so A waits.
+    const bool leader = elect_one();
+    const int ahead = num_kb < STAGES ? num_kb : STAGES;
+    for (int kb = 0; kb < ahead; ++kb) {
+      if (leader) {
         mbar_expect_tx(&full_bar[kb], STAGE_BYTES);
-        tma_load_2d(smem + kb * STAGE_BYTES + A_BYTES, &map_w, &full_bar[kb], kb * BK,
-                    ((int)blockIdx.x % n_tiles) * BN);
+        tma_load_2d(smem + kb * STAGE_BYTES + A_BYTES, &map_w, &full_bar[kb], kb * BK, ((int)blockIdx.x % n_tiles) * BN);
       }
-      pdl_wait();
-      int it = 0;
-      for (int tile = blockIdx.x; tile < num_tiles && !failed; tile += gridDim.x) {
-        const int m0 = (tile / n_tiles) * BM, n0 = (tile % n_tiles) * BN;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t phase = (it / STAGES) & 1;
-          unsigned char* a_dst = smem + s * STAGE_BYTES;
-          if (it >= ahead) {
-            if (!mbar_wait(&empty_bar[s], phase ^ 1)) {
-              failed = 1;
-              break;
-            }
+    }
+    pdl_wait();
+    int it = 0, s = 0, phase = 1;
+    for (int tile = blockIdx.x; tile < num_tiles && !failed; tile += gridDim.x) {
+      const int m0 = (tile / n_tiles) * BM, n0 = (tile % n_tiles) * BN;
+      for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        unsigned char* a_dst = smem + s * STAGE_BYTES;
+        if (it >= ahead) {
+          if (!mbar_wait(&empty_bar[s], phase)) {
+            failed = 1;
+            break;
+          }
+          if (leader) {
             mbar_expect_tx(&full_bar[s], STAGE_BYTES);
             tma_load_2d(a_dst + A_BYTES, &map_w, &full_bar[s], kb * BK, n0);
           }
-          tma_load_2d(a_dst, &map_a, &full_bar[s], kb * BK, m0);
         }
+        if (leader) tma_load_2d(a_dst, &map_a, &full_bar[s], kb * BK, m0);
+        if (++s == STAGES) s = 0, phase ^= 1;
       }
     }
   } else if (warp == 1) {
     // ---- MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc(BM, BN);
-      int it = 0, local = 0;
-      for (int tile = blockIdx.x; tile < num_tiles && !failed; tile += gridDim.x, ++local) {
-        const int buf = local & 1;
-        // the epilogue must have emptied this accumulator (two tiles ago)
-        if (!mbar_wait(&accum_empty[buf], ((local >> 1) & 1) ^ 1)) {
-          failed = 1;
-          break;
-        }
+    const bool leader = elect_one();
+    const uint32_t idesc = umma_idesc(BM, BN);
+    int s = 0, phase = 0, local = 0;
+    for (int tile = blockIdx.x; tile < num_tiles && !failed; tile += gridDim.x, ++local) {
+      const int buf = local & 1;
+      // the epilogue must have emptied this accumulator (two tiles ago)
+      bool ok = mbar_wait(&accum_empty[buf], ((local >> 1) & 1) ^ 1);
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
+      for (int kb = 0; kb < num_kb && ok; ++kb) {
+        ok = mbar_wait(&full_bar[s], phase);
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t phase = (it / STAGES) & 1;
-          if (!mbar_wait(&full_bar[s], phase)) {
-            failed = 1;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
-          const uint32_t b_addr = a_addr + A_BYTES;
+        const uint64_t a_desc = umma_desc(smem_u32(smem + s * STAGE_BYTES)), b_desc = a_desc + (A_BYTES >> 4);
+        if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            // the next 16 k of a 128-byte swizzled row: 32 bytes further
-            umma(tmem_d, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), idesc, (kb | k) != 0);
-          }
+          for (int k = 0; k < BK / UMMA_K; ++k)  // the next 16 k of a 128-byte swizzled row: 32 bytes further
+            umma(tmem_d, a_desc + k * 2, b_desc + k * 2, idesc, (kb | k) != 0);
           umma_commit(&empty_bar[s]);  // the stage is free once these products have read it
         }
-        if (failed) break;
-        umma_commit(&accum_full[buf]);
+        if (++s == STAGES) s = 0, phase ^= 1;
       }
+      if (!ok) {
+        failed = 1;
+        break;
+      }
+      if (leader) umma_commit(&accum_full[buf]);
     }
   } else {
     // ---- epilogue warps 2..5: warp w owns accumulator lanes 32 (w % 4) .. +31
@@ -444,92 +440,86 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const uint32_t tmem_base = tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // as in the one-CTA kernel: the first ring of W tiles is asked for before the wait.  A ring
-      // slot holds SUB k blocks of A, then SUB k blocks of this CTA's half of W; with the
-      // three-dimensional maps one request brings all SUB blocks of an operand (and counts the
-      // bytes of all SUB, zero-filled beyond K), else one request per k block
-      const int num_steps = (num_kb + SUB - 1) / SUB;  // ring slots per tile
-      const int ahead = num_steps < STAGES2 ? num_steps : STAGES2;
-      auto slot_bytes = [&](int st) {
-        const int subs = num_kb - st * SUB < SUB ? num_kb - st * SUB : SUB;
-        return 2 * STAGE_P * (e.k_boxes ? SUB : subs);
-      };
-      auto load_w = [&](unsigned char* slot, uint64_t* bar, int st, int w0) {
-        unsigned char* dst = slot + SUB * A_BYTES;
-        if (e.k_boxes) {
-          tma_load_3d_pair(dst, &map_w, bar, 0, w0, st * SUB);
-        } else {
-          for (int u = 0; u < SUB && st * SUB + u < num_kb; ++u)
-            tma_load_2d_pair(dst + u * B_HALF, &map_w, bar, (st * SUB + u) * BK, w0);
-        }
-      };
-      auto load_a = [&](unsigned char* slot, uint64_t* bar, int st, int m0) {
-        if (e.k_boxes) {
-          tma_load_3d_pair(slot, &map_a, bar, 0, m0, st * SUB);
-        } else {
-          for (int u = 0; u < SUB && st * SUB + u < num_kb; ++u)
-            tma_load_2d_pair(slot + u * A_BYTES, &map_a, bar, (st * SUB + u) * BK, m0);
-        }
-      };
-      for (int st = 0; st < ahead; ++st) {
-        if (rank == 0) mbar_expect_tx(&full_bar[st], slot_bytes(st));
-        load_w(smem + st * SUB * STAGE_P, &full_bar[st], st, ((pair / m_tiles) % n_tiles) * BNP + (int)rank * (BNP / 2));
+    // as in the one-CTA kernel: the first ring of W tiles is asked for before the wait.  A ring
+    // slot holds SUB k blocks of A, then SUB k blocks of this CTA's half of W; with the
+    // three-dimensional maps one request brings all SUB blocks of an operand (and counts the
+    // bytes of all SUB, zero-filled beyond K), else one request per k block
+    const bool leader = elect_one();
+    const int num_steps = (num_kb + SUB - 1) / SUB;  // ring slots per tile
+    const int ahead = num_steps < STAGES2 ? num_steps : STAGES2;
+    auto slot_bytes = [&](int st) {
+      const int subs = num_kb - st * SUB < SUB ? num_kb - st * SUB : SUB;
+      return 2 * STAGE_P * (e.k_boxes ? SUB : subs);
+    };
+    auto load = [&](const CUtensorMap* map, unsigned char* dst, int bytes, uint64_t* bar, int st, int row0) {
+      if (e.k_boxes) {
+        tma_load_3d_pair(dst, map, bar, 0, row0, st * SUB);
+      } else {
+        for (int u = 0; u < SUB && st * SUB + u < num_kb; ++u) tma_load_2d_pair(dst + u * bytes, map, bar, (st * SUB + u) * BK, row0);
       }
-      pdl_wait();
-      int it = 0;
-      for (int tile = pair; tile < num_tiles && !failed; tile += num_pairs) {
-        const int m0 = (tile % m_tiles) * 2 * BM + (int)rank * BM;
-        const int w0 = (tile / m_tiles) * BNP + (int)rank * (BNP / 2);
-        for (int st = 0; st < num_steps; ++st, ++it) {
-          const int s = it % STAGES2;
-          const uint32_t phase = (it / STAGES2) & 1;
-          unsigned char* slot = smem + s * SUB * STAGE_P;
-          if (it >= ahead) {
-            if (!mbar_wait(&empty_bar[s], phase ^ 1)) {
-              failed = 1;
-              break;
-            }
-            if (rank == 0) mbar_expect_tx(&full_bar[s], slot_bytes(st));
-            load_w(slot, &full_bar[s], st, w0);
-          }
-          load_a(slot, &full_bar[s], st, m0);
-        }
+    };
+    for (int st = 0; st < ahead; ++st) {
+      const int w0 = ((pair / m_tiles) % n_tiles) * BNP + (int)rank * (BNP / 2);
+      if (leader) {
+        if (rank == 0) mbar_expect_tx(&full_bar[st], slot_bytes(st));
+        load(&map_w, smem + st * SUB * STAGE_P + SUB * A_BYTES, B_HALF, &full_bar[st], st, w0);
       }
     }
-  } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
-      const uint32_t idesc = umma_idesc(2 * BM, BNP);  // M 256 across the pair
-      int it = 0, local = 0;
-      for (int tile = pair; tile < num_tiles && !failed; tile += num_pairs, ++local) {
-        const int buf = local & 1;
-        if (!mbar_wait(&accum_empty[buf], ((local >> 1) & 1) ^ 1)) {
-          failed = 1;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t tmem_d = tmem_base + (uint32_t)(buf * 256);
-        const int num_steps = (num_kb + SUB - 1) / SUB;
-        for (int st = 0; st < num_steps; ++st, ++it) {
-          const int s = it % STAGES2;
-          const uint32_t phase = (it / STAGES2) & 1;
-          if (!mbar_wait(&full_bar[s], phase)) {
+    pdl_wait();
+    int it = 0, s = 0, phase = 1;
+    for (int tile = pair; tile < num_tiles && !failed; tile += num_pairs) {
+      const int m0 = (tile % m_tiles) * 2 * BM + (int)rank * BM;
+      const int w0 = (tile / m_tiles) * BNP + (int)rank * (BNP / 2);
+      for (int st = 0; st < num_steps; ++st, ++it) {
+        unsigned char* slot = smem + s * SUB * STAGE_P;
+        if (it >= ahead) {
+          if (!mbar_wait(&empty_bar[s], phase)) {
             failed = 1;
             break;
           }
+          if (leader) {
+            if (rank == 0) mbar_expect_tx(&full_bar[s], slot_bytes(st));
+            load(&map_w, slot + SUB * A_BYTES, B_HALF, &full_bar[s], st, w0);
+          }
+        }
+        if (leader) load(&map_a, slot, A_BYTES, &full_bar[s], st, m0);
+        if (++s == STAGES2) s = 0, phase ^= 1;
+      }
+    }
+  } else if (warp == 1) {
+    if (rank == 0) {
+      const bool leader = elect_one();
+      const uint32_t idesc = umma_idesc(2 * BM, BNP);  // M 256 across the pair
+      const int num_steps = (num_kb + SUB - 1) / SUB;
+      int s = 0, phase = 0, local = 0;
+      for (int tile = pair; tile < num_tiles && !failed; tile += num_pairs, ++local) {
+        const int buf = local & 1;
+        bool ok = mbar_wait(&accum_empty[buf], ((local >> 1) & 1) ^ 1);
+        tc_fence_after();
+        const uint32_t tmem_d = tmem_base + (uint32_t)(buf * 256);
+        for (int st = 0; st < num_steps && ok; ++st) {
+          ok = mbar_wait(&full_bar[s], phase);
+          if (!ok) break;
           tc_fence_after();
           const int subs = num_kb - st * SUB < SUB ? num_kb - st * SUB : SUB;
-          for (int u = 0; u < subs; ++u) {
-            const uint32_t a_addr = smem_u32(smem + s * SUB * STAGE_P + u * A_BYTES);
-            const uint32_t b_addr = smem_u32(smem + s * SUB * STAGE_P + SUB * A_BYTES + u * B_HALF);
+          const uint64_t a_desc = umma_desc(smem_u32(smem + s * SUB * STAGE_P)), b_desc = a_desc + (SUB * A_BYTES >> 4);
+          if (leader) {
 #pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k)
-              umma_pair(tmem_d, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), idesc, (st | u | k) != 0);
+            for (int u = 0; u < SUB; ++u) {
+              if (u >= subs) break;
+#pragma unroll
+              for (int k = 0; k < BK / UMMA_K; ++k)
+                umma_pair(tmem_d, a_desc + (u * (A_BYTES >> 4) + k * 2), b_desc + (u * (B_HALF >> 4) + k * 2), idesc, (st | u | k) != 0);
+            }
+            umma_commit_pair(&empty_bar[s]);
           }
-          umma_commit_pair(&empty_bar[s]);
+          if (++s == STAGES2) s = 0, phase ^= 1;
         }
-        if (failed) break;
-        umma_commit_pair(&accum_full[buf]);
+        if (!ok) {
+          failed = 1;
+          break;
+        }
+        if (leader) umma_commit_pair(&accum_full[buf]);
       }
     }
   } else {
