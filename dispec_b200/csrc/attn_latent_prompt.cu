@@ -202,33 +202,36 @@ attn_latent_prompt_kernel(const Params p, const __grid_constant__ CUtensorMap ma
   }
 
   if (warp == 0) {
-    if (lane == 0) {
-      for (int i = 0; i < n_kt; ++i) {
-        const int s = i % K_STAGES;
-        if (!mbar_wait(&k_empty[s], ((i / K_STAGES) & 1) ^ 1)) {
-          failed = 1;
-          break;
-        }
-        const int row = row0 + (kt_begin + i) * BN;
+    const bool leader = elect_one();
+    for (int i = 0; i < n_kt; ++i) {
+      const int s = i % K_STAGES;
+      if (!mbar_wait(&k_empty[s], ((i / K_STAGES) & 1) ^ 1)) {
+        failed = 1;
+        break;
+      }
+      const int row = row0 + (kt_begin + i) * BN;
+      if (leader) {
         mbar_expect_tx(&k_full[s], K_BYTES);
         tma_load_3d(k_s + s * K_BYTES, &map_k, &k_full[s], 0, row, head * (DK / 64));
         tma_load_2d(k_s + s * K_BYTES + DK / 64 * SLICE, &map_r, &k_full[s], 0, row);
       }
     }
   } else if (warp == V_WARP) {
-    if (lane == 0) {
-      for (int i = 0; i < n_kt; ++i) {
-        const int s = i % V_STAGES;
-        if (!mbar_wait(&v_empty[s], ((i / V_STAGES) & 1) ^ 1)) {
-          failed = 1;
-          break;
-        }
+    const bool leader = elect_one();
+    for (int i = 0; i < n_kt; ++i) {
+      const int s = i % V_STAGES;
+      if (!mbar_wait(&v_empty[s], ((i / V_STAGES) & 1) ^ 1)) {
+        failed = 1;
+        break;
+      }
+      if (leader) {
         mbar_expect_tx(&v_full[s], V_BYTES);
         tma_load_3d(v_s + s * V_BYTES, &map_v, &v_full[s], 0, row0 + (kt_begin + i) * BN, H * (DK / 64) + head * (DV / 64));
       }
     }
   } else if (warp == 1 || warp == S1_WARP) {
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       const uint32_t idesc_s = umma_idesc(BM, BN);
       const uint64_t k_desc0 = umma_desc(smem_u32(k_s)), qr_desc = umma_desc(smem_u32(qr_s));
       bool ok = mbar_wait(&q_ready, 0);
@@ -241,20 +244,23 @@ attn_latent_prompt_kernel(const Params p, const __grid_constant__ CUtensorMap ma
         tc_fence_after();
         const uint64_t k_desc = k_desc0 + (uint64_t)(s * (K_BYTES >> 4));
         const uint32_t tmem_s = tmem_base + (uint32_t)((a & 1) * S_COLS);
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < DK / 16; ++k)
-          umma_a_tmem(tmem_s, tmem_base + (uint32_t)(Q_COL + k * 8),
-                      k_desc + (uint64_t)(((k >> 2) * SLICE + (k & 3) * 32) >> 4), idesc_s, k != 0);
+          for (int k = 0; k < DK / 16; ++k)
+            umma_a_tmem(tmem_s, tmem_base + (uint32_t)(Q_COL + k * 8),
+                        k_desc + (uint64_t)(((k >> 2) * SLICE + (k & 3) * 32) >> 4), idesc_s, k != 0);
 #pragma unroll
-        for (int k = 0; k < DR / 16; ++k)
-          umma(tmem_s, qr_desc + (uint64_t)(k * 2), k_desc + (uint64_t)((DK / 64 * SLICE + k * 32) >> 4), idesc_s, 1);
-        umma_commit(&s_full[a & 1]);
-        umma_commit(&k_empty[s]);
+          for (int k = 0; k < DR / 16; ++k)
+            umma(tmem_s, qr_desc + (uint64_t)(k * 2), k_desc + (uint64_t)((DK / 64 * SLICE + k * 32) >> 4), idesc_s, 1);
+          umma_commit(&s_full[a & 1]);
+          umma_commit(&k_empty[s]);
+        }
       }
       if (!ok) failed = 1;
     }
   } else if (warp == PV_WARP) {
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       const uint32_t idesc_o = umma_idesc(BM, DV) | (1u << 16);  // B (values) is N-major
       const uint64_t v_desc0 = umma_desc_mn(smem_u32(v_s), SLICE);
       bool ok = true;
@@ -264,12 +270,14 @@ attn_latent_prompt_kernel(const Params p, const __grid_constant__ CUtensorMap ma
         if (!ok) break;
         tc_fence_after();
         const uint64_t v_desc = v_desc0 + (uint64_t)(st * (V_BYTES >> 4));
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < BN / 16; ++k)
-          umma_a_tmem(tmem_base + (uint32_t)(O_COL + g * DV), tmem_base + (uint32_t)(P_COL + g * P_COLS + k * 8),
-                      v_desc + (uint64_t)(k * 128), idesc_o, (b >= 2) || k != 0);
-        umma_commit(&v_empty[st]);
-        umma_commit(&o_done[g]);
+          for (int k = 0; k < BN / 16; ++k)
+            umma_a_tmem(tmem_base + (uint32_t)(O_COL + g * DV), tmem_base + (uint32_t)(P_COL + g * P_COLS + k * 8),
+                        v_desc + (uint64_t)(k * 128), idesc_o, (b >= 2) || k != 0);
+          umma_commit(&v_empty[st]);
+          umma_commit(&o_done[g]);
+        }
       }
       if (!ok) failed = 1;
     }

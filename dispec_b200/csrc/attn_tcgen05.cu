@@ -10,8 +10,8 @@
 //   warp 0      issues the TMA loads of the K tiles and of the V tiles, each into a ring of its own: a
 //               K tile is free again when its scores are complete, a V tile two softmax iterations
 //               later, when its output product is;
-//   warps 1, 11 one thread each issues the score products S[i] = Q K[i]^T of one softmax group;
-//   warp 10     one thread issues the output products O[i % 2] += P[i] V[i];
+//   warps 1, 11 issue the score products S[i] = Q K[i]^T of one softmax group;
+//   warp 10     issues the output products O[i % 2] += P[i] V[i];
 //   warps 2..9  two softmax groups of four warps.  Group g owns the key tiles i = g, g + 2, ...: its own
 //               score buffer S[g], output accumulator O[g] and P[g] in tensor memory and its own
 //               running maximum and sum, so the two groups never exchange anything until the end
@@ -304,10 +304,9 @@ attn_tcgen05_kernel(const Params p, int tile_offset, const __grid_constant__ CUt
     }
   } else if (warp == 1 || warp == S1_WARP) {
     // ---- issuers of the score products: warp 1 for the tiles of softmax group 0, warp S1_WARP for
-    // those of group 1.  One thread for both spent 340 cycles per tile on barriers that were long
-    // complete and 700 on issuing eight products and two commits, and these 1,250 cycles a tile,
-    // in one thread, were the kernel's pace.
-    if (lane == 0) {
+    // those of group 1 (one warp for both was the kernel's pace while a single thread ran its loop)
+    {
+      const bool leader = elect_one();
       const uint32_t idesc_s = umma_idesc(BM, BN);
       // descriptors are linear in the address: the tile's base once, a constant per k step
       const uint64_t k_desc0 = umma_desc(smem_u32(k_s));
@@ -316,13 +315,15 @@ attn_tcgen05_kernel(const Params p, int tile_offset, const __grid_constant__ CUt
         tc_fence_after();
         const uint64_t k_desc = k_desc0 + (uint64_t)(s * (KV_BYTES >> 4));
         const uint32_t tmem_s = tmem_base + (uint32_t)((i & 1) * S_COLS);
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (uint32_t)(k >> 2), in = (uint32_t)(k & 3) * 32u;
-          umma_a_tmem(tmem_s, tmem_base + (uint32_t)(Q_COL + k * 8), k_desc + ((off * KV_SLICE + in) >> 4), idesc_s, k != 0);
+          for (int k = 0; k < D / 16; ++k) {
+            const uint32_t off = (uint32_t)(k >> 2), in = (uint32_t)(k & 3) * 32u;
+            umma_a_tmem(tmem_s, tmem_base + (uint32_t)(Q_COL + k * 8), k_desc + ((off * KV_SLICE + in) >> 4), idesc_s, k != 0);
+          }
+          umma_commit(&s_full[i & 1]);
+          umma_commit(&k_empty[s]);
         }
-        umma_commit(&s_full[i & 1]);
-        umma_commit(&k_empty[s]);
       };
       // The scores of tile a need K[a] and, from the group's second tile on, that the group has
       // read S[a % 2] (tile a - 2).
@@ -337,7 +338,8 @@ attn_tcgen05_kernel(const Params p, int tile_offset, const __grid_constant__ CUt
     }
   } else if (warp == PV_WARP) {
     // ---- issuer of the output products: O[g] += P[b] V[b] needs P[b] (written, O rescaled, dead value rows zeroed)
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       const uint32_t idesc_o = umma_idesc(BM, D) | (1u << 16);  // B (values) is N-major
       const uint64_t v_desc0 = umma_desc_mn(smem_u32(v_s), KV_SLICE);
       bool ok = true;
@@ -347,12 +349,14 @@ attn_tcgen05_kernel(const Params p, int tile_offset, const __grid_constant__ CUt
         if (!ok) break;
         tc_fence_after();
         const uint64_t v_desc = v_desc0 + (uint64_t)(st * (KV_BYTES >> 4));
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < BN / 16; ++k)
-          umma_a_tmem(tmem_base + (uint32_t)(O_COL + g * D), tmem_base + (uint32_t)(P_COL + g * P_COLS + k * 8),
-                      v_desc + (uint64_t)(k * 128), idesc_o, (b >= 2) || k != 0);
-        umma_commit(&v_empty[st]);
-        umma_commit(&o_done[g]);
+          for (int k = 0; k < BN / 16; ++k)
+            umma_a_tmem(tmem_base + (uint32_t)(O_COL + g * D), tmem_base + (uint32_t)(P_COL + g * P_COLS + k * 8),
+                        v_desc + (uint64_t)(k * 128), idesc_o, (b >= 2) || k != 0);
+          umma_commit(&v_empty[st]);
+          umma_commit(&o_done[g]);
+        }
       }
       if (!ok) failed = 1;
     }
