@@ -28,6 +28,7 @@ CORE_SOURCES = [
     "elementwise.cu",
     "norm32.cu",
     "gemm_simt.cu",
+    "gemm_split.cu",
     "gemm_tcgen05.cu",
     "gemm_stream.cu",
     "attn_generic.cu",

@@ -1,7 +1,7 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]) (+ residual[M,N]) on the 32-bit FMA units.
 //
-// This is the matrix product of the true 32-bit path (no tensor cores, no reduced-precision
-// mode) and the catch-all for sizes the tensor-core kernels refuse.  Every output element is
+// This is the catch-all for sizes the tensor-core kernels refuse, and the product of floats of short
+// rows (gemm_split.cu takes the others).  Every output element is
 // one FMA chain over k = 0..K-1 in ascending order, so a row's result does not depend on
 // which other rows are in the batch, nor on which of the kernels below computes it.
 //

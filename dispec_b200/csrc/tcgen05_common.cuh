@@ -300,6 +300,18 @@ inline bool make_map(CUtensorMap* map, const void* base, long rows, long K, long
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+// rows x K floats, row stride ld elements; box of 32 k x box_rows rows, 128-byte swizzle, zero fill outside the matrix
+inline bool make_map_f32(CUtensorMap* map, const void* base, long rows, long K, long ld, int box_rows) {
+  EncodeTiled fn = encode_fn();
+  if (fn == nullptr) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  cuuint32_t box[2] = {32u, (cuuint32_t)box_rows};
+  cuuint32_t elem[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, elem,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 // The same matrix seen as (64 of k, rows, K / 64 blocks of k): one box of (64, box_rows, k_blocks)
 // brings several k blocks of a row tile with a single request, laid out as consecutive tiles of
 // [box_rows][64] (a request costs the TMA unit about 200 cycles whatever its size: measured 41 bytes

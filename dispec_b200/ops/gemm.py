@@ -1,7 +1,9 @@
 """y = x W^T (+ bias) (+ residual): the one matrix product the model uses.
 
-float32: the FMA kernel (``dsp_gemm_simt``), always; no tensor cores, no reduced-precision
-mode, one FMA chain per output so that a row does not depend on its batch.
+float32: every operand cut into three bfloat16 pieces that add up to it, whose products run on the
+tensor cores and are summed in 32 bits (``dsp_gemm_split``: closer to 64 bits than a chain of 32-bit
+FMAs); the FMA kernel (``dsp_gemm_simt``) for short K and for matrices that TMA cannot read.  Which of
+the two runs is decided by the matrix alone, and a row does not depend on its batch in either.
 bfloat16: the weight-streaming tcgen05 kernel for up to 128 rows (decoding and the rows whose
 logits are wanted); above that the persistent tcgen05/TMA kernel of this package, except that narrow
 products at a few hundred rows stay with the weight-streaming kernel where
@@ -23,6 +25,7 @@ from dispec_b200.ops import library as L
 from dispec_b200.ops import tuning
 
 STREAM_MAX_ROWS = 128  # rows up to which the weight-streaming kernel always runs
+SPLIT_MIN_K = 512  # length of a product of floats from which the tensor cores are used
 NORM_SPLIT_MAX_ROWS = 64  # rows up to which a norm is split over two products
 
 
@@ -77,6 +80,16 @@ def _simt(x, w, bias, residual, out, tile: int = -1):
     return out
 
 
+def _split(x, w, bias, residual, out):
+    """The product of floats on the tensor cores, operands cut into three bfloat16 pieces."""
+    M, K = x.shape
+    L.check(L.core().dsp_gemm_split(
+        L.ptr(x), L.i64(x.stride(0)), L.ptr(w), L.ptr(bias), L.ptr(residual),
+        L.i64(residual.stride(0) if residual is not None else 0), L.ptr(out), L.i64(out.stride(0)),
+        M, w.shape[0], K, L.stream_handle()))
+    return out
+
+
 def _tcgen05(x, w, bias, residual, out, pairs: bool = True, epilogue=EPI_PLAIN):
     """The many-row product; ``pairs``: CTA pairs (cta_group::2), the default, or single CTAs."""
     M, K = x.shape
@@ -107,6 +120,14 @@ def _stream(x, w, bias, residual, out, epilogue=EPI_PLAIN, target_ctas: int | No
         ctypes.c_float(norm.eps if norm is not None else 0.0), L.ptr(gain2), L.ptr(out2),
         L.i64(out2.stride(0) if out2 is not None else 0), L.stream_handle()))
     return out
+
+
+def split_supported(w: torch.Tensor) -> bool:
+    """Whether a product of floats runs on the tensor cores: by its matrix alone, so that a row has the same bits
+    alone and among others.  Below ``SPLIT_MIN_K`` the fixed latencies of that kernel are longer than the FMA chain:
+    264 rows x 1,024 x 128 17.4 us for 11.0, 4 rows x 256 x 256 12.3 for 8.2; 33 rows x 200 x 516 15.4 for 15.1, 97 rows
+    x 1,000 x 1,000 16.4 for 24.6."""
+    return w.shape[1] >= SPLIT_MIN_K and w.shape[1] % 4 == 0 and w.data_ptr() % 16 == 0
 
 
 def tcgen05_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -209,7 +230,7 @@ def linear(x, w: torch.Tensor, bias: torch.Tensor | None = None,
         return result()
     if x.dtype == torch.float32:
         assert out_dtype == torch.float32
-        _simt(x, w, bias, residual, out)
+        (_split if split_supported(w) and backend != "simt" else _simt)(x, w, bias, residual, out)
         return result()
     if backend is None:
         if stream_supported(M, K, x, w):
