@@ -32,6 +32,14 @@
 // prompt leaves an SM one block: eight warps hide one another's latencies), the groups' results meet in
 // shared memory and leave one round later.  Single tokens: transformed as they are staged, in one kernel,
 // the lanes of a warp cover all the rows.
+// Longer steps are cut into segments of 64 tokens or more that run side by side, the first of a request from its state and the
+// others from zero.  What a state in front of a segment adds is linear in it:
+//     o_t += (S_in)^T (P_t q_t),   S_out = A S_in + S_local,   P_t the product of the segment's a up to t, A the last of them
+// so a scan over a request's segments gives every S_in, and a product of P_t q_t (which the segments' first blocks write
+// down as they go) with S_in completes the outputs.  In a segment a warp covers all state rows of eight columns and adds
+// within itself.  2,500 tokens of two requests, 12 heads of 128 x 128: 297 us (FORGET_GATE) and 252 (FIXED_DECAY) walked
+// in one piece by 192 blocks of which an SM held one or two; segments 118, scan 16, product 39 (all four blocks of an SM
+// busy, the FMA pipe two fifths).
 // State rows beyond 256 take a kernel of their own with one column a thread.  A request whose first row
 // carries a negative position (a padding row of a captured step) is skipped: its state slot belongs to
 // someone else.
@@ -75,7 +83,30 @@ struct RecurrenceArgs {
   int slices;            // threads per column (a power of two, at most 32)
   int cols_per_block;    // threads / slices
   int tokens_per_round;
+  // segments of seg_len tokens (null and 0 without): number q_start[s] / seg_len + s + j is the j-th of request s
+  float* seg_state;  // [segments, H, dim, vdim]: the state behind it, later the one in front of it
+  float* seg_decay;  // [segments, H, dim]: the product of its decays
+  float* seg_q;      // [T, H * dim]: P_t q_t
+  int S, seg_len;
 };
+
+struct Segment {
+  int seq, index, t0, t1;
+  bool only;  // the request has no other
+};
+// Segment `number`; false where there is none.
+__device__ __forceinline__ bool find_segment(const RecurrenceArgs& p, int number, Segment& g) {
+  int lo = 0, hi = p.S;  // the last request whose first segment is not beyond `number`
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (p.q_start[mid] / p.seg_len + mid <= number) lo = mid; else hi = mid;
+  }
+  const int a = p.q_start[lo], b = p.q_start[lo + 1];
+  g.seq = lo, g.index = number - (a / p.seg_len + lo);
+  g.t0 = a + g.index * p.seg_len, g.t1 = min(b, g.t0 + p.seg_len);
+  g.only = b - a <= p.seg_len;
+  return g.index >= 0 && g.t0 < b && p.positions[a] >= 0;
+}
 
 // sigmoid(z)^power by way of ln sigmoid(z) = -(ln(1 + e^-|z|) + max(-z, 0))
 __device__ __forceinline__ float sigmoid_power(float z, float power) {
@@ -137,7 +168,7 @@ __device__ __forceinline__ void transform(const RecurrenceArgs& p, int token, in
 
 // ready[t][0] = q, [1] = b, [2] = a (FORGET_GATE and KEY_DECAY), each [H * dim].  A thread keeps its channel and walks
 // over tokens blockIdx.y, blockIdx.y + gridDim.y, ...: from a running index every element paid two 64-bit divisions
-// (2,500 tokens of 12 heads of 128: 38.6 us, now 31.3).
+// (2,500 tokens of 12 heads of 128: 38.6 us, now 31.3; four tokens at a time 35.7).
 __global__ void __launch_bounds__(256) recurrence_prepare_kernel(const RecurrenceArgs p, int T) {
   const int hd = p.H * p.dim, planes = p.mode == FORGET_GATE ? 3 : 2;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -401,30 +432,38 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
 // the state's rows (padded); every output is the sum of the groups' results, which meet in shared memory.
 constexpr int TILE_STAGES = 3, BATCH = 8;
 
-template <int SLICES, int PAIRS, int PARTS, int WARPS, bool STREAMED, int KIND>
+template <int SLICES, int PAIRS, int PARTS, int WARPS, bool STREAMED, int KIND, bool SEGMENTS>
 struct Tile {
   static constexpr bool gate = KIND == VECTOR_DECAY, per_token = KIND == TOKEN_DECAY;
   static constexpr int planes = gate ? 3 : 2;
   static constexpr int part_rows = SLICES * 2 * PAIRS;                       // state rows of a group of warps
   static constexpr int rows = part_rows * PARTS;                             // state rows, padded
   static constexpr int cols = WARPS / PARTS * (32 / SLICES) * 4;             // value columns of a block
-  static constexpr int round = rows <= 128 ? 16 : 8;                         // tokens staged together
+  static constexpr int round = rows <= 128 && !SEGMENTS ? 16 : 8;            // tokens staged together
   static constexpr int stage = planes * round * rows + round * cols + (per_token ? 2 * round : 0);
   static constexpr int meet = PARTS == 1 ? 0 : 2 * PARTS * round * cols;     // the groups' results of two rounds
   static constexpr int stages = STREAMED ? TILE_STAGES : 1;
   static constexpr size_t smem = sizeof(float) * (stages * stage + meet);
 };
 
-template <int SLICES, int PAIRS, int PARTS, int WARPS, bool STREAMED, int KIND>
-__global__ void __launch_bounds__(32 * WARPS, 2)
+template <int SLICES, int PAIRS, int PARTS, int WARPS, bool STREAMED, int KIND, bool SEGMENTS>
+__global__ void __launch_bounds__(32 * WARPS, SEGMENTS ? 4 : 2)
 recurrence_tile_kernel(const RecurrenceArgs p) {
-  using L = Tile<SLICES, PAIRS, PARTS, WARPS, STREAMED, KIND>;
+  using L = Tile<SLICES, PAIRS, PARTS, WARPS, STREAMED, KIND, SEGMENTS>;
   constexpr bool gate = L::gate, per_token = L::per_token;
   constexpr int DP = L::rows, C = L::cols, R = L::round, planes = L::planes;
   extern __shared__ __align__(16) float tile_smem[];
-  const int seq = blockIdx.z, head = blockIdx.y;
-  const int t0 = p.q_start[seq], t1 = p.q_start[seq + 1];
-  if (t1 <= t0 || p.positions[t0] < 0) return;
+  const int head = blockIdx.y;
+  int seq = blockIdx.z, t0, t1;
+  bool fresh = false, onward = false;  // it begins with a state of zeros; more segments follow or came before
+  if constexpr (SEGMENTS) {
+    Segment g;
+    if (!find_segment(p, blockIdx.z, g)) return;
+    seq = g.seq, t0 = g.t0, t1 = g.t1, fresh = g.index > 0, onward = !g.only;
+  } else {
+    t0 = p.q_start[seq], t1 = p.q_start[seq + 1];
+    if (t1 <= t0 || p.positions[t0] < 0) return;
+  }
   const int tid = threadIdx.x, lane = tid & 31, slice = lane % SLICES;
   constexpr int TILE_THREADS = 32 * WARPS, PART_WARPS = WARPS / PARTS;
   const int part = (tid >> 5) / PART_WARPS;  // this warp's group of state rows
@@ -437,18 +476,22 @@ recurrence_tile_kernel(const RecurrenceArgs p) {
   const bool v_wide = whole && p.v_off % 4 == 0 && p.vdim % 4 == 0;
   const int hd = p.H * p.dim, group0 = (head / p.heads_per_group) * p.dim;
 
-  // 2 PAIRS neighbouring state rows of columns col0 .. col0 + 3
+  // 2 PAIRS state rows of columns col0 .. col0 + 3, in pieces of four neighbours (two with one pair), the slices' pieces
+  // side by side: what the lanes of a warp read of q, b and a together is contiguous
   float* sp = p.state + (((size_t)p.state_slot[seq] * p.H + head) * p.dim) * p.vdim;
   const bool s_wide = p.vdim % 4 == 0;
-  const int row0 = part * L::part_rows + slice * 2 * PAIRS;
+  constexpr int PIECE = PAIRS >= 2 ? 2 : 1;  // pairs of a piece
+  static_assert(PAIRS % PIECE == 0, "whole pieces");
+  const int row0 = part * L::part_rows + slice * 2 * PIECE;
+  auto row_of = [&](int k) { return row0 + k / PIECE * (SLICES * 2 * PIECE) + k % PIECE * 2; };  // first row of pair k
   f32x2 S[PAIRS][4];  // [pair of rows 2k, 2k + 1][column]
 #pragma unroll
   for (int k = 0; k < PAIRS; ++k) {
     float s[2][4] = {};
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int i = row0 + 2 * k + h;
-      if (i >= p.dim || col0 >= p.vdim) continue;
+      const int i = row_of(k) + h;
+      if (fresh || i >= p.dim || col0 >= p.vdim) continue;
       const float* src = sp + (size_t)i * p.vdim + col0;
       if (s_wide) {
         const float4 v = *reinterpret_cast<const float4*>(src);
@@ -464,6 +507,14 @@ recurrence_tile_kernel(const RecurrenceArgs p) {
   }
   const float decay = KIND == SCALAR_DECAY ? p.decay[head] : 0.f;
   const float skip = per_token ? p.skip[head] : 0.f;
+
+  // the product of this segment's decays so far; the lanes of one group of columns write P_t q_t down
+  const bool notes = SEGMENTS && fresh && blockIdx.x == 0 && cg == 0;
+  f32x2 product[SEGMENTS ? PAIRS : 1];
+  if constexpr (SEGMENTS) {
+#pragma unroll
+    for (int k = 0; k < PAIRS; ++k) product[k] = pack2f(1.f, 1.f);
+  }
 
   // rows and columns beyond the head's own stay zero in every stage: written here and never again
   if (DP > p.dim || (int)(blockIdx.x + 1) * C > p.vdim) {
@@ -550,15 +601,44 @@ recurrence_tile_kernel(const RecurrenceArgs p) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) v2[c] = pack2f(v[c], v[c]);
           const f32x2 all2 = pack2f(a_all, a_all);
+          f32x2 q_of[PAIRS], b_of[PAIRS], a_of[PAIRS];
+#pragma unroll
+          for (int e = 0; e < PAIRS; e += PIECE) {
+            const float* at = qs + r * DP + e / PIECE * (SLICES * 2 * PIECE);
+            if constexpr (PIECE == 2) {
+              const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(at), y = *reinterpret_cast<const ulonglong2*>(at + R * DP);
+              q_of[e] = x.x, q_of[e + 1] = x.y, b_of[e] = y.x, b_of[e + 1] = y.y;
+              if constexpr (gate) {
+                const ulonglong2 z = *reinterpret_cast<const ulonglong2*>(at + 2 * R * DP);
+                a_of[e] = z.x, a_of[e + 1] = z.y;
+              } else {
+                a_of[e] = a_of[e + 1] = all2;
+              }
+            } else {
+              q_of[e] = *reinterpret_cast<const f32x2*>(at), b_of[e] = *reinterpret_cast<const f32x2*>(at + R * DP);
+              a_of[e] = all2;
+              if constexpr (gate) a_of[e] = *reinterpret_cast<const f32x2*>(at + 2 * R * DP);
+            }
+          }
 #pragma unroll
           for (int e = 0; e < PAIRS; ++e) {
-            const f32x2* at = reinterpret_cast<const f32x2*>(qs + r * DP) + e;
-            const f32x2 qe = at[0], be = at[R * DP / 2], ae = gate ? at[R * DP] : all2;
+            const f32x2 qe = q_of[e], be = b_of[e], ae = a_of[e];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
               f32x2& s = S[e][c];
               s = fma2(ae, s, mul2(be, v2[c]));
               o2[c] = e == 0 ? mul2(s, qe) : fma2(s, qe, o2[c]);
+            }
+            if constexpr (SEGMENTS) {
+              if (notes) {
+                product[e] = mul2(product[e], ae);
+                float x, y;
+                unpack2f(mul2(product[e], qe), x, y);
+                const int i = row_of(e);
+                float* dst = p.seg_q + (size_t)(base + r) * hd + (size_t)head * p.dim + i;
+                if (i < p.dim) dst[0] = x;
+                if (i + 1 < p.dim) dst[1] = y;
+              }
             }
           }
 #pragma unroll
@@ -675,6 +755,20 @@ recurrence_tile_kernel(const RecurrenceArgs p) {
     __syncthreads();
     flush(t0 + (t1 - t0 - 1) / R * R);
   }
+  if constexpr (SEGMENTS) {
+    if (notes) {
+      float* dst = p.seg_decay + ((size_t)blockIdx.z * p.H + head) * p.dim;
+#pragma unroll
+      for (int k = 0; k < PAIRS; ++k) {
+        float x, y;
+        unpack2f(product[k], x, y);
+        const int i = row_of(k);
+        if (i < p.dim) dst[i] = x;
+        if (i + 1 < p.dim) dst[i + 1] = y;
+      }
+    }
+    if (onward) sp = p.seg_state + ((size_t)blockIdx.z * p.H + head) * p.dim * p.vdim;
+  }
 #pragma unroll
   for (int k = 0; k < PAIRS; ++k) {
     float s[2][4];
@@ -682,7 +776,7 @@ recurrence_tile_kernel(const RecurrenceArgs p) {
     for (int c = 0; c < 4; ++c) unpack2f(S[k][c], s[0][c], s[1][c]);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int i = row0 + 2 * k + h;
+      const int i = row_of(k) + h;
       if (i >= p.dim || col0 >= p.vdim) continue;
       float* dst = sp + (size_t)i * p.vdim + col0;
       if (s_wide) {
@@ -696,26 +790,141 @@ recurrence_tile_kernel(const RecurrenceArgs p) {
   }
 }
 
-template <int SLICES, int PAIRS, int PARTS, int WARPS, bool STREAMED, int KIND>
-int launch_tile_kind(const RecurrenceArgs& a, int S, cudaStream_t stream) {
-  using L = Tile<SLICES, PAIRS, PARTS, WARPS, STREAMED, KIND>;
+// The states in front of a request's segments (in place of those behind them) and the request's own state.  A thread
+// an element; the next segment's is on its way while one is added.
+__global__ void __launch_bounds__(256) segment_scan_kernel(const RecurrenceArgs p) {
+  const int seq = blockIdx.z, head = blockIdx.y, e = blockIdx.x * 256 + threadIdx.x;
+  const int a = p.q_start[seq], n = p.q_start[seq + 1] - a, size = p.dim * p.vdim;
+  if (n <= p.seg_len || p.positions[a] < 0 || e >= size) return;
+  const int first = a / p.seg_len + seq, count = (n + p.seg_len - 1) / p.seg_len, row = e / p.vdim;
+  const size_t step = (size_t)p.H * size, dstep = (size_t)p.H * p.dim;
+  float* at = p.seg_state + ((size_t)first * p.H + head) * size + e;
+  const float* decay = p.seg_decay + ((size_t)first * p.H + head) * p.dim + row;
+  float running = *at, next = at[step], d = decay[dstep];
+  for (int j = 1; j < count; ++j) {
+    at += step, decay += dstep;
+    const float local = next, mine = d;
+    if (j + 1 < count) next = at[step], d = decay[dstep];
+    *at = running;
+    running = fmaf(mine, running, local);
+  }
+  p.state[((size_t)p.state_slot[seq] * p.H + head) * size + e] = running;
+}
+
+// o_t += S_in^T (P_t q_t) for a segment's tokens and 128 columns of a head: 256 threads of 8 x 4 outputs, 64 tokens and
+// 32 state rows at a time, the next ones on their way while these are multiplied.
+constexpr int CARRY_TOKENS = 64, SLAB = 32, CARRY_COLS = 128;
+__global__ void __launch_bounds__(256, 2) segment_carry_kernel(const RecurrenceArgs p) {
+  __shared__ __align__(16) float qs[CARRY_TOKENS][SLAB + 4], ss[SLAB][CARRY_COLS];
+  Segment g;
+  if (!find_segment(p, blockIdx.z, g) || g.index == 0) return;
+  const int head = blockIdx.y, col0 = blockIdx.x * CARRY_COLS, tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+  const int hd = p.H * p.dim;
+  const bool wide = p.dim % 4 == 0 && p.vdim % 4 == 0 && p.ldo % 4 == 0 && ((uintptr_t)p.out & 15) == 0;
+  const float* state = p.seg_state + ((size_t)blockIdx.z * p.H + head) * p.dim * p.vdim;
+  auto load4 = [&](const float* src, int there) {  // the first `there` of four floats, zeros behind them
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (wide) {
+      if (there > 0) v = *reinterpret_cast<const float4*>(src);
+    } else {
+      if (there > 0) v.x = src[0];
+      if (there > 1) v.y = src[1];
+      if (there > 2) v.z = src[2];
+      if (there > 3) v.w = src[3];
+    }
+    return v;
+  };
+  constexpr int QN = CARRY_TOKENS * SLAB / 1024, SN = SLAB * CARRY_COLS / 1024;  // fours a thread fetches of a slab
+  for (int t0 = g.t0; t0 < g.t1; t0 += CARRY_TOKENS) {
+    const int n = min(CARRY_TOKENS, g.t1 - t0);
+    const float* q = p.seg_q + (size_t)t0 * hd + (size_t)head * p.dim;
+    float4 q_next[QN], s_next[SN];
+    auto fetch = [&](int k0) {
+#pragma unroll
+      for (int i = 0; i < QN; ++i) {
+        const int r = (tid >> 3) + 32 * i, k = k0 + (tid & 7) * 4;
+        q_next[i] = load4(q + (size_t)r * hd + k, r < n ? p.dim - k : 0);
+      }
+#pragma unroll
+      for (int i = 0; i < SN; ++i) {
+        const int k = k0 + (tid >> 5) + 8 * i, c = col0 + (tid & 31) * 4;
+        s_next[i] = load4(state + (size_t)k * p.vdim + c, k < p.dim ? p.vdim - c : 0);
+      }
+    };
+    float acc[8][4] = {};
+    fetch(0);
+    for (int k0 = 0; k0 < p.dim; k0 += SLAB) {
+      __syncthreads();  // the slab before has been read
+#pragma unroll
+      for (int i = 0; i < QN; ++i) *reinterpret_cast<float4*>(&qs[(tid >> 3) + 32 * i][(tid & 7) * 4]) = q_next[i];
+#pragma unroll
+      for (int i = 0; i < SN; ++i) *reinterpret_cast<float4*>(&ss[(tid >> 5) + 8 * i][(tid & 31) * 4]) = s_next[i];
+      __syncthreads();
+      if (k0 + SLAB < p.dim) fetch(k0 + SLAB);
+#pragma unroll
+      for (int k = 0; k < SLAB; k += 4) {
+        float4 y[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j] = *reinterpret_cast<const float4*>(&ss[k + j][4 * tx]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {  // a warp has the same eight tokens: one address
+          const float4 x = *reinterpret_cast<const float4*>(&qs[ty * 8 + i][k]);
+          const float w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            acc[i][0] = fmaf(w[j], y[j].x, acc[i][0]);
+            acc[i][1] = fmaf(w[j], y[j].y, acc[i][1]);
+            acc[i][2] = fmaf(w[j], y[j].z, acc[i][2]);
+            acc[i][3] = fmaf(w[j], y[j].w, acc[i][3]);
+          }
+        }
+      }
+    }
+    const int there = p.vdim - (col0 + 4 * tx);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = ty * 8 + i;
+      if (r >= n || there <= 0) break;
+      float* dst = p.out + (size_t)(t0 + r) * p.ldo + (size_t)head * p.vdim + col0 + 4 * tx;
+      float4 o = load4(dst, there);
+      o.x += acc[i][0], o.y += acc[i][1], o.z += acc[i][2], o.w += acc[i][3];
+      if (wide) {
+        *reinterpret_cast<float4*>(dst) = o;
+      } else {
+        dst[0] = o.x;
+        if (there > 1) dst[1] = o.y;
+        if (there > 2) dst[2] = o.z;
+        if (there > 3) dst[3] = o.w;
+      }
+    }
+  }
+}
+
+template <int SLICES, int PAIRS, int PARTS, int WARPS, bool STREAMED, int KIND, bool SEGMENTS>
+int launch_tile_kind(const RecurrenceArgs& a, int S, int segments, cudaStream_t stream) {
+  using L = Tile<SLICES, PAIRS, PARTS, WARPS, STREAMED, KIND, SEGMENTS>;
+  auto kernel = recurrence_tile_kernel<SLICES, PAIRS, PARTS, WARPS, STREAMED, KIND, SEGMENTS>;
   static bool configured = false;
   if (!configured) {
-    DSP_CUDA(cudaFuncSetAttribute(recurrence_tile_kernel<SLICES, PAIRS, PARTS, WARPS, STREAMED, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)L::smem));
+    DSP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem));
     configured = true;
   }
-  const dim3 grid((a.vdim + L::cols - 1) / L::cols, a.H, S);
-  recurrence_tile_kernel<SLICES, PAIRS, PARTS, WARPS, STREAMED, KIND><<<grid, 32 * WARPS, L::smem, stream>>>(a);
+  const dim3 grid((a.vdim + L::cols - 1) / L::cols, a.H, SEGMENTS ? segments : S);
+  kernel<<<grid, 32 * WARPS, L::smem, stream>>>(a);
   DSP_CHECK_LAUNCH("dsp_linear_recurrence");
+  if constexpr (SEGMENTS) {
+    segment_scan_kernel<<<dim3((a.dim * a.vdim + 255) / 256, a.H, S), 256, 0, stream>>>(a);
+    segment_carry_kernel<<<dim3((a.vdim + CARRY_COLS - 1) / CARRY_COLS, a.H, segments), 256, 0, stream>>>(a);
+    DSP_CHECK_LAUNCH("dsp_linear_recurrence (segments)");
+  }
   return 0;
 }
 
-template <int SLICES, int PAIRS, int PARTS, int WARPS, bool STREAMED>
-int launch_tile(const RecurrenceArgs& a, int S, cudaStream_t stream) {
-  if (a.mode == STEP_DECAY) return launch_tile_kind<SLICES, PAIRS, PARTS, WARPS, STREAMED, TOKEN_DECAY>(a, S, stream);
-  if (a.mode == FIXED_DECAY) return launch_tile_kind<SLICES, PAIRS, PARTS, WARPS, STREAMED, SCALAR_DECAY>(a, S, stream);
-  return launch_tile_kind<SLICES, PAIRS, PARTS, WARPS, STREAMED, VECTOR_DECAY>(a, S, stream);
+template <int SLICES, int PAIRS, int PARTS, int WARPS, bool STREAMED, bool SEGMENTS = false>
+int launch_tile(const RecurrenceArgs& a, int S, cudaStream_t stream, int segments = 0) {
+  if (a.mode == STEP_DECAY) return launch_tile_kind<SLICES, PAIRS, PARTS, WARPS, STREAMED, TOKEN_DECAY, SEGMENTS>(a, S, segments, stream);
+  if (a.mode == FIXED_DECAY) return launch_tile_kind<SLICES, PAIRS, PARTS, WARPS, STREAMED, SCALAR_DECAY, SEGMENTS>(a, S, segments, stream);
+  return launch_tile_kind<SLICES, PAIRS, PARTS, WARPS, STREAMED, VECTOR_DECAY, SEGMENTS>(a, S, segments, stream);
 }
 
 template <int ROWS, int TPR, int KIND>
@@ -741,7 +950,8 @@ int launch(const RecurrenceArgs& a, int S, size_t smem, cudaStream_t stream) {
 
 // scratch: null (one kernel, tokens transformed as they are staged) or room for [T, planes, H * dim]
 // floats, planes = 2 with one decay for all rows, else 3 (a first kernel transforms every token, the
-// recurrence streams); STEP_DECAY takes none.
+// recurrence streams); STEP_DECAY takes none.  segment_scratch: null, or room for the segments of at most 256 state
+// rows, `segment` tokens each: (T / segment + S) * H * dim * (vdim + 1) + T * H * dim floats.
 extern "C" int dsp_linear_recurrence(const void* proj, int proj_dtype, long ld, int q_off, int k_off,
                                      int v_off, int mode, int H, int dim, int vdim, const float* decay,
                                      const float* inv_freq, int rot, float key_scale, int act,
@@ -749,7 +959,8 @@ extern "C" int dsp_linear_recurrence(const void* proj, int proj_dtype, long ld, 
                                      const float* gate_map, int low_off, int rank, float q_scale, float power,
                                      const float* steps, const float* skip, int heads_per_group, float* state,
                                      const int* state_slot, const int* q_start, const int* positions,
-                                     float* out, long ldo, int S, int T, float* scratch, cudaStream_t stream) {
+                                     float* out, long ldo, int S, int T, float* scratch, float* segment_scratch, int segment,
+                                     cudaStream_t stream) {
   if (S == 0 || T == 0) return 0;
   DSP_REQUIRE(proj && state && state_slot && q_start && positions && out, "dsp_linear_recurrence: missing operand");
   DSP_REQUIRE(H > 0 && H <= 65535 && S <= 65535, "dsp_linear_recurrence: H=%d, S=%d outside the grid", H, S);
@@ -778,6 +989,12 @@ extern "C" int dsp_linear_recurrence(const void* proj, int proj_dtype, long ld, 
   a.steps = steps; a.skip = skip; a.heads_per_group = mode == STEP_DECAY ? heads_per_group : 1;
   a.state = state; a.state_slot = state_slot; a.q_start = q_start; a.positions = positions;
   a.out = out; a.ldo = ldo; a.ready = scratch;
+  DSP_REQUIRE(!segment_scratch || segment > 0, "dsp_linear_recurrence: segments of %d tokens", segment);
+  a.S = S; a.seg_len = segment;
+  const int segments = segment_scratch ? T / segment + S : 0;  // as many numbers as segments may have
+  a.seg_state = segment_scratch;
+  a.seg_decay = a.seg_state ? a.seg_state + (size_t)segments * H * dim * vdim : nullptr;
+  a.seg_q = a.seg_state ? a.seg_decay + (size_t)segments * H * dim : nullptr;
   // one column a thread, 32 threads a column, 16 or 32 state rows a thread (beyond 256 state rows)
   const bool tiled = dim <= 256;
   const int slices = 32, rows = (dim + slices - 1) / slices;
@@ -801,6 +1018,14 @@ extern "C" int dsp_linear_recurrence(const void* proj, int proj_dtype, long ld, 
     const int fill = (sms > 0 ? sms : 148) * 8 / across + 1, down = T < fill ? T : fill;
     recurrence_prepare_kernel<<<dim3(across, down < 65535 ? down : 65535), 256, 0, stream>>>(a, T);
     DSP_CHECK_LAUNCH("dsp_linear_recurrence (first kernel)");
+  }
+  if (segment_scratch) {
+    DSP_REQUIRE(tiled && (scratch || mode == STEP_DECAY), "dsp_linear_recurrence: segments of tokens that are not prepared, or of %d state rows", dim);
+    DSP_REQUIRE(segments <= 65535, "dsp_linear_recurrence: %d segments", segments);
+    if (dim <= 32) return launch_tile<8, 2, 1, 4, true, true>(a, S, stream, segments);
+    if (dim <= 64) return launch_tile<16, 2, 1, 4, true, true>(a, S, stream, segments);
+    if (dim <= 128) return launch_tile<16, 4, 1, 4, true, true>(a, S, stream, segments);
+    return launch_tile<32, 4, 1, 4, true, true>(a, S, stream, segments);
   }
   if (scratch || (mode == STEP_DECAY && T > 2 * S)) {  // portions of prompts
     if (dim <= 32) return launch_tile<8, 1, 2, 8, true>(a, S, stream);

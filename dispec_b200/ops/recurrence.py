@@ -8,6 +8,10 @@ import torch
 from dispec_b200.ops import library as L
 
 FIXED_DECAY, FORGET_GATE, KEY_DECAY, STEP_DECAY = 0, 1, 2, 3
+SEGMENT = 64  # tokens of a request that run side by side with its others (at least)
+_MAX_SEGMENTS = 128  # longer segments rather than more of them: they fill the SMs, and a state is kept for each
+SEGMENTS_MIN_TOKENS = 192  # tokens of a step, beyond two a request, from which its requests are cut into segments
+_SEGMENTS_MAX_ROWS = 256
 
 
 def linear_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, mode: int, num_heads: int,
@@ -59,12 +63,23 @@ def linear_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, mo
     if T > 2 * S and mode != STEP_DECAY:
         planes = 2 if mode == FIXED_DECAY else 3
         scratch = torch.empty((T, planes, num_heads * dim), dtype=torch.float32, device=proj.device)
+    # longer steps: segments of the requests side by side, if there is room for their states
+    segment_scratch, segment = None, SEGMENT
+    if T - 2 * S >= SEGMENTS_MIN_TOKENS and dim <= _SEGMENTS_MAX_ROWS:
+        while T // segment > _MAX_SEGMENTS:
+            segment *= 2
+        try:
+            segment_scratch = torch.empty((T // segment + S) * num_heads * dim * (vdim + 1) + T * num_heads * dim,
+                                          dtype=torch.float32, device=proj.device)
+        except torch.OutOfMemoryError:
+            pass
     L.check(lib.dsp_linear_recurrence(
         L.ptr(proj), L.dtype_code(proj.dtype), L.i64(proj.stride(0)), q_off, k_off, v_off, mode, num_heads, dim,
         vdim, L.ptr(decay), L.ptr(inv_freq), rot, L.f32(key_scale), int(silu_inputs), L.ptr(gate_bias), L.ptr(lower),
         L.ptr(gate_map), low_off, rank, L.f32(q_scale), L.f32(power), L.ptr(steps), L.ptr(skip), heads_per_group, L.ptr(state),
         L.ptr(state_slot), L.ptr(q_start), L.ptr(positions), L.ptr(out), L.i64(out.stride(0)), S, T,
-        L.ptr(scratch), L.stream_handle()))
+        L.ptr(scratch), L.ptr(segment_scratch), segment, L.stream_handle()),
+        launches=1 + (scratch is not None) + 2 * (segment_scratch is not None))
     return out
 
 
