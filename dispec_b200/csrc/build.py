@@ -30,6 +30,7 @@ CORE_SOURCES = [
     "gemm_simt.cu",
     "gemm_split.cu",
     "gemm_tcgen05.cu",
+    "gemm_pairs.cu",
     "gemm_stream.cu",
     "attn_generic.cu",
     "attn_combine.cu",

@@ -23,6 +23,9 @@ int dsp_gemm_stream(const void* A, long lda, const void* W, const void* bias, co
 int dsp_gemm_tcgen05(const void* A, long lda, const void* W, const void* bias, const void* residual, long ldr, void* C,
                      long ldc, int M, int N, int K, int out_dtype, int pair_mode, int epilogue, cudaStream_t stream);
 int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas);
+int dsp_gemm_pairs(const void* A, long lda, const void* W, const void* bias, const void* residual, long ldr, void* C, long ldc,
+                   int M, int N, int K, int out_dtype, int epilogue, int splits, int chunks, cudaStream_t stream);
+int dsp_gemm_pairs_faster(int M, int N, int K, int target_ctas);
 int dsp_attn_combine(const float* part_o, const float* part_ml, void* out, long out_stride, int num_tokens, int H, int D,
                      int splits, int dtype, cudaStream_t stream);
 }
@@ -84,6 +87,11 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
                      float eps, const void* gain, void* scaled_out, bool* prepared) -> int {
     const void* residual = add ? C : nullptr;
     if (prepared) *prepared = false;
+    if (T > s.always_few) {
+      const int pairs = dsp_gemm_pairs_faster(T, N, K, (int)s.target_ctas);
+      if (pairs < 0) return pairs;
+      if (pairs) return dsp_gemm_pairs(A, K, W, bias, residual, add ? N : 0, C, N, T, N, K, DSP_BF16, 0, 0, 0, stream);
+    }
     const int few = T <= s.always_few ? 1 : dsp_gemm_few_rows_faster(T, N, K, (int)s.target_ctas);
     if (few < 0) return few;
     if (few) {
@@ -97,6 +105,8 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
     return dsp_gemm_tcgen05(A, K, W, bias, residual, add ? N : 0, C, N, T, N, K, DSP_BF16, 1, 0, stream);
   };
 
+  const int pairs_gate_up = T > s.always_few ? dsp_gemm_pairs_faster(T, 2 * inter, hidden, (int)s.target_ctas) : 0;
+  if (pairs_gate_up < 0) return pairs_gate_up;
   bool ready = false;  // scaled_b holds x times the next norm1's gain
   for (long i = 0; i < s.layers; ++i) {
     const DspDenseLayer& l = layers[i];
@@ -146,6 +156,9 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
                                2 * inter, hidden, DSP_BF16, (int)s.target_ctas, (int)s.epilogue, s.late_trigger_bytes,
                                normed ? s.x : nullptr, normed ? hidden : 0, normed ? (float)l.eps2 : 0.f, nullptr, nullptr,
                                0, stream));
+    else if (pairs_gate_up)
+      DSP_STEP(dsp_gemm_pairs(s.h, hidden, l.w_gate_up, nullptr, nullptr, 0, s.act, inter, T, 2 * inter, hidden, DSP_BF16,
+                              (int)s.epilogue, 0, 0, stream));
     else
       DSP_STEP(dsp_gemm_tcgen05(s.h, hidden, l.w_gate_up, nullptr, nullptr, 0, s.act, inter, T, 2 * inter, hidden,
                                 DSP_BF16, 1, (int)s.epilogue, stream));

@@ -849,8 +849,7 @@ Plan make_plan(int M, int N, int K, int out_dtype, int target_ctas, bool may_spl
 // 17.5 / 15.0 / 34 us and 11.5 / 12.5 / 19.0 / 43 / 86 at 129 rows; 12.9 / 11.7 / 30 / 20.5 / 62 and 11.6 / 12.9 / 25 / 44 / 89 at
 // 384; 15.1 / 12.9 / 37 / 27 / 109 and 11.7 / 12.9 / 32 / 44 / 89 at 536; 15.6 / 15.6 / 64 / 37 / 204 and 12.9 / 13.1 / 44 /
 // 46 / 106 at 1,016.
-extern "C" int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas) {
-  if (M <= 0 || N <= 0 || K <= 0 || target_ctas <= 0) return 0;
+extern "C" int dsp_gemm_row_estimates(int M, int N, int K, int target_ctas, double* few, double* many) {
   const int k_blocks = (K + BK - 1) / BK;
   const double w_us = 2.0 * N * K / 6.5e6;  // W at the memory's rate
   // the many-row kernel: the rounds of its tiles over the CTA pairs, of the width that it would choose
@@ -859,16 +858,22 @@ extern "C" int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas) {
   auto many_rounds = [&](int width) { return (many_tiles(width) + pairs - 1) / pairs; };
   const int width = 0.92 * many_rounds(192) < many_rounds(256) ? 192 : 256;
   const double many_busy = fmin(1.0, (double)many_tiles(width) / pairs);
-  const double many = 5.0 + many_rounds(width) * (1.2 + k_blocks * (0.23 + 0.056 * many_busy)) + 0.44 * w_us;
+  *many = 5.0 + many_rounds(width) * (1.2 + k_blocks * (0.23 + 0.056 * many_busy)) + 0.44 * w_us;
   // this one: a k block costs more while more CTAs stream; storing a tile, and the partial rows a split sends and adds,
   // go with the rows of a tile
   const Plan p = make_plan(M, N, K, DSP_BF16, target_ctas, N % 4 == 0);
   if (p.splits == 0) return -1;
   const long rounds = p.splits > 1 ? 1 : (p.tiles + target_ctas - 1) / target_ctas;
   const double busy = fmin(1.0, (double)p.tiles * p.splits / target_ctas), rows = Chunks(M).rows / 192.0;
-  const double few = 3.8 + 0.98 * busy + (double)rounds * p.kb_per_split * (0.29 + 0.06 * busy) + 3.72 * rows +
+  *few = 3.8 + 0.98 * busy + (double)rounds * p.kb_per_split * (0.29 + 0.06 * busy) + 3.72 * rows +
                      (p.splits > 1 ? rows * (0.85 * busy + 5.13 / p.splits) : 0.0) + 0.15 * w_us;
-  return 1.02 * few < many;
+  return 0;
+}
+extern "C" int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas) {
+  if (M <= 0 || N <= 0 || K <= 0 || target_ctas <= 0) return 0;
+  double few = 0.0, many = 0.0;
+  const int rc = dsp_gemm_row_estimates(M, N, K, target_ctas, &few, &many);
+  return rc != 0 ? rc : 1.02 * few < many;
 }
 
 #ifdef DSP_STAMPS

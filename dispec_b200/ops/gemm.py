@@ -5,9 +5,10 @@ tensor cores and are summed in 32 bits (``dsp_gemm_split``: closer to 64 bits th
 FMAs); the FMA kernel (``dsp_gemm_simt``) for short K and for matrices that TMA cannot read.  Which of
 the two runs is decided by the matrix alone, and a row does not depend on its batch in either.
 bfloat16: the weight-streaming tcgen05 kernel for up to 128 rows (decoding and the rows whose
-logits are wanted); above that the persistent tcgen05/TMA kernel of this package, except that narrow
-products at a few hundred rows stay with the weight-streaming kernel where
-``tuning.rows_in_chunks_is_faster`` says so (the many-row kernel does not split K).  Operands
+logits are wanted); above that the persistent tcgen05/TMA kernel of this package, except that, mostly
+at some hundred rows, the kernel on CTA pairs with swapped roles runs where ``tuning.pairs_are_faster``
+says so (it splits K, and cuts the rows into equal chunks) and the weight-streaming kernel where
+``tuning.rows_in_chunks_is_faster`` does.  Operands
 those kernels cannot take (a width that is no multiple of 8) go to the FMA kernel when there
 are at most 64 rows or 32-bit logits are wanted, and otherwise to the library matrix product
 (cuBLAS through torch.mm), which is where the reference engine itself calls a library
@@ -90,6 +91,16 @@ def _split(x, w, bias, residual, out):
     return out
 
 
+def _pairs(x, w, bias, residual, out, epilogue=EPI_PLAIN, splits: int = 0, chunks: int = 0):
+    """The product of some hundred rows on CTA pairs; ``splits``, ``chunks``: instead of its own choice (comparisons)."""
+    M, K = x.shape
+    L.check(L.core().dsp_gemm_pairs(
+        L.ptr(x), L.i64(x.stride(0)), L.ptr(w), L.ptr(bias), L.ptr(residual),
+        L.i64(residual.stride(0) if residual is not None else 0), L.ptr(out), L.i64(out.stride(0)),
+        M, w.shape[0], K, L.dtype_code(out.dtype), epilogue, splits, chunks, L.stream_handle()))
+    return out
+
+
 def _tcgen05(x, w, bias, residual, out, pairs: bool = True, epilogue=EPI_PLAIN):
     """The many-row product; ``pairs``: CTA pairs (cta_group::2), the default, or single CTAs."""
     M, K = x.shape
@@ -135,6 +146,14 @@ def tcgen05_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def pairs_supported(x: torch.Tensor, w: torch.Tensor, bias, residual, out: torch.Tensor) -> bool:
+    """Whether the operands of a product let the kernel on CTA pairs finish four outputs of a row at a time."""
+    vec = lambda t, n: t is None or (t.stride(0) % 4 == 0 and t.data_ptr() % n == 0)
+    width = 4 * out.element_size()
+    return (tcgen05_supported(x, w) and w.shape[0] % 4 == 0 and vec(out, width) and vec(residual, width)
+            and (bias is None or bias.data_ptr() % 8 == 0))
+
+
 def stream_supported(M: int, K: int, x: torch.Tensor, w: torch.Tensor) -> bool:
     return (M <= STREAM_MAX_ROWS and K % 8 == 0 and x.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
@@ -168,6 +187,8 @@ def linear_gate_up_swiglu(x, w_interleaved, out=None, act: str = "silu"):
         out = torch.empty((M, N // 2), dtype=x.dtype, device=x.device)
     epilogue = {"silu": EPI_SWIGLU, "gelu_tanh": EPI_GEGLU}[act]
     if M > STREAM_MAX_ROWS:
+        if pairs_supported(x, w_interleaved, None, None, out) and tuning.pairs_are_faster(M, N, x.shape[1], x.device):
+            return _pairs(x, w_interleaved, None, None, out, epilogue=epilogue)
         return _tcgen05(x, w_interleaved, None, None, out, epilogue=epilogue)
     return _stream(x, w_interleaved, None, None, out, epilogue=epilogue, norm=norm)
 
@@ -193,8 +214,8 @@ def linear(x, w: torch.Tensor, bias: torch.Tensor | None = None,
            out: torch.Tensor | None = None, backend: str | None = None, then_norm=None):
     """x [M, K] (row stride free, unit column stride), w [N, K] contiguous, bias [N],
     residual [M, N] of the output type.  Output type: ``out_dtype`` (default: x's);
-    bfloat16 inputs may produce float32 (logits).  ``backend``: "stream", "tcgen05", "library"
-    or "simt" instead of the choice described at the top of this file.
+    bfloat16 inputs may produce float32 (logits).  ``backend``: "stream", "tcgen05", "pairs",
+    "library" or "simt" instead of the choice described at the top of this file.
 
     ``x`` may be ``NormedRows`` (a norm still to be applied): the few-row kernel takes it apart
     where it can, otherwise the norm kernel runs first.  ``then_norm`` = (weight, eps) of the
@@ -235,6 +256,8 @@ def linear(x, w: torch.Tensor, bias: torch.Tensor | None = None,
     if backend is None:
         if stream_supported(M, K, x, w):
             backend = "stream"
+        elif M > STREAM_MAX_ROWS and pairs_supported(x, w, bias, residual, out) and tuning.pairs_are_faster(M, N, K, x.device):
+            backend = "pairs"
         elif (M > STREAM_MAX_ROWS and stream_supported(STREAM_MAX_ROWS, K, x, w)
               and tuning.rows_in_chunks_is_faster(M, N, K, x.device, STREAM_MAX_ROWS)):
             backend = "stream"  # (a norm after it runs as a kernel)
@@ -254,6 +277,8 @@ def linear(x, w: torch.Tensor, bias: torch.Tensor | None = None,
         return result(scaled)
     if backend == "tcgen05":
         _tcgen05(x, w, bias, residual, out)
+    elif backend == "pairs":
+        _pairs(x, w, bias, residual, out)
     elif backend == "library":
         _library(x, w, bias, residual, out)
     elif backend == "simt":

@@ -58,6 +58,21 @@ def _few_rows_faster(M: int, N: int, K: int, sms: int) -> bool:
     return bool(answer)
 
 
+def pairs_are_faster(M: int, N: int, K: int, device=None) -> bool:
+    """Whether the product on CTA pairs with swapped roles beats the few-row and the many-row product at M rows; the
+    estimate stands beside the kernel (``dsp_gemm_pairs_faster`` in csrc/gemm_pairs.cu)."""
+    return _pairs_faster(M, N, K, sm_count(device))
+
+
+@functools.lru_cache(maxsize=4096)
+def _pairs_faster(M: int, N: int, K: int, sms: int) -> bool:
+    from dispec_b200.ops import library
+    answer = library.core().dsp_gemm_pairs_faster(M, N, K, STREAM_CTAS_PER_SM * sms)
+    if answer < 0:  # (an exception is not kept by the cache)
+        library.check(answer, launches=0)
+    return bool(answer)
+
+
 # ---- attention of single tokens (attn_mma.cu, decode kernel) ---------------------------------
 ATTN_CTAS_PER_SM = 2  # resident CTAs the decode launch aims for
 CLUSTER_MAX_SPLITS = 8  # key splits of one row that merge on chip (one thread-block cluster)
