@@ -7,7 +7,7 @@
 // accumulator in tensor memory is 128 lanes (rows of W) by a few columns (rows of A).  One thread streams W
 // tiles of 128 rows x 64 k (16 KB a request) and the matching slice of A by TMA into a ring of 4 to 5 stages
 // (two CTAs per SM up to 64 rows of A, about 180 KB on its way per SM, which plain loads cannot keep in
-// flight); one to four threads issue the products; four warps (eight above 64 rows of A) read the
+// flight); one warp issues the products; four warps (eight above 64 rows of A) read the
 // accumulator, apply the epilogue and store.  With programmatic dependent launch the first
 // W tiles are requested before the kernel waits for its predecessor.
 //
@@ -37,8 +37,8 @@ namespace {
 using namespace tc;
 constexpr int ROWS_W = 128, BK = 64, UMMA_K = 16;
 constexpr int W_BYTES = ROWS_W * BK * 2;
-// warp 0: TMA; then ISSUERS warps whose first lanes issue the products (the first of them also owns
-// the tensor memory); then four epilogue warps, eight where a CTA has an SM to itself
+// warp 0: TMA; warp 1: issues the products and owns the tensor memory; then four epilogue warps, eight where a CTA has
+// an SM to itself
 constexpr int MAX_SPLITS = 8;
 enum { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_GEGLU = 2 };
 
@@ -50,30 +50,18 @@ template <int NB> struct Cfg {
   // dependent launch) fills its ring with W while this kernel's CTA is still streaming
   // (128 and 192 rows of A: one CTA per SM; at 192 the ring must also hold the partial tile and the inbox of a K split)
   static constexpr int STAGES = NB == 64 ? 4 : 5;
-  // One thread's turn of the ring (wait for the stage, fence, four products, commit) takes about
-  // 0.3 us, of which the tensor pipe is busy a third (a product of 128 x 16 x 16 every 55 cycles from
-  // one issuing thread, every 39 from two: `bench.py --only mma-rate`); a W tile of 16 KB per 0.3 us is
-  // 55 GB/s, which is what an SM's share of the memory bandwidth delivers.  The four k steps of a k
-  // block therefore belong to ISSUERS threads of different warps, each with a partial accumulator of
-  // its own, so that their turns overlap; the epilogue adds the partial accumulators up in a fixed
-  // order.  Measured on the captured decode step at 8 rows: first stage to last product 0.96 -> 0.7 us
-  // on the small products, 8.1 -> 7.6 us on gate/up, 5.75 -> 4.7 us on down.  (Whole k blocks dealt
-  // to five issuers that own a stage of the ring each measured 1 % slower on the whole step.)  Two
-  // CTAs share the SM's 512 columns of tensor memory.
-  // (at 128 rows of A a product of 128 x 128 x 16 keeps the pipe busy for the 64 cycles one thread
-  // needs to issue it: one issuer, no partial accumulators)
-  static constexpr int PARTS = NB == 16 ? 4 : NB <= 64 ? 2 : 1;
-  static constexpr int ISSUERS = PARTS;
-  static constexpr int FIRST_EPI_WARP = 1 + ISSUERS;
+  // One warp issues the products.  (While a single thread ran that loop, its turn of the ring took 0.3 us, as long as a
+  // tile takes to arrive, and up to 64 rows of A the k steps of a block were dealt to two or four threads with partial
+  // accumulators of their own; with the loop run by whole warps that costs more than it gives: decode steps at 1, 8 and
+  // 64 rows 913, 941 and 1,697 us with them, 910, 937 and 1,690 without.)
   // two epilogue warps per quarter of the lanes where a CTA has an SM to itself: they take the windows of the
   // accumulator (the rows of a K split) in turn
   static constexpr int EPI_GROUPS = NB <= 64 ? 1 : 2, EPI_WARPS = 4 * EPI_GROUPS;
-  static constexpr int THREADS = 32 * (1 + ISSUERS + EPI_WARPS);
+  static constexpr int FIRST_EPI_WARP = 2, THREADS = 32 * (FIRST_EPI_WARP + EPI_WARPS);
   static constexpr int MIN_CTAS = NB <= 64 ? 2 : 1;  // CTAs per SM the registers are held down for
   // the epilogue takes the accumulator in windows of at most 64 columns (rows of A): what a thread holds at once
   static constexpr int WINDOW = NB <= 64 ? NB : 64;
-  static constexpr int ACC_COLS = PARTS * NB;  // one accumulator buffer
-  static constexpr int TMEM_COLS = 2 * ACC_COLS < 32 ? 32 : 2 * ACC_COLS <= 256 ? 2 * ACC_COLS : 512;  // a power of two
+  static constexpr int TMEM_COLS = 2 * NB <= 256 ? 2 * NB : 512;  // two accumulators, a power of two
   // K split over a cluster: every CTA sends the rows of its partial tile to the CTA that finishes
   // them (row m to rank m % splits), into an inbox of [source rank][rows per CTA][128] floats.  Up
   // to 16 rows of A (at most 16 + 8 rows of inbox) it has room of its own behind the ring
@@ -197,45 +185,15 @@ __device__ __forceinline__ float square_sum8(const uint4 u) {
   return ss;
 }
 
-// The accumulator of this thread's W row: the partial accumulators added in a fixed order.
-// NB columns from taddr on; the PARTS partial accumulators lie part_stride columns apart.
-template <int NB, int PARTS>
-__device__ __forceinline__ void load_accumulator(uint32_t taddr, uint32_t part_stride, uint32_t (&v)[NB]) {
+// NB columns of the accumulator of this thread's W row.
+template <int NB>
+__device__ __forceinline__ void load_accumulator(uint32_t taddr, uint32_t (&v)[NB]) {
   if constexpr (NB == 16) {
-    // the partial accumulators lie side by side: one load of PARTS x 16 columns, one wait
-    static_assert(PARTS == 4 || PARTS == 2, "loads of 32 or 64 columns");
-    uint32_t all[PARTS * 16];
-    if constexpr (PARTS == 4) {
-      tmem_ld32_nowait(taddr, reinterpret_cast<uint32_t(&)[32]>(all[0]));
-      tmem_ld32_nowait(taddr + 32, reinterpret_cast<uint32_t(&)[32]>(all[32]));
-      tmem_ld_wait();
-    } else {
-      tmem_ld32(taddr, reinterpret_cast<uint32_t(&)[32]>(all[0]));
-    }
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      float sum = __uint_as_float(all[c]);
-#pragma unroll
-      for (int p = 1; p < PARTS; ++p) sum += __uint_as_float(all[p * 16 + c]);
-      v[c] = __float_as_uint(sum);
-    }
-  } else if constexpr (PARTS == 1) {
+    tmem_ld16(taddr, v);
+  } else {
 #pragma unroll
     for (int c0 = 0; c0 < NB; c0 += 32) tmem_ld32_nowait(taddr + (uint32_t)c0, reinterpret_cast<uint32_t(&)[32]>(v[c0]));
     tmem_ld_wait();
-  } else {
-    // 32 columns of every partial accumulator per trip to the tensor memory (a load and its wait
-    // take a few hundred nanoseconds: they are not taken one after the other)
-    static_assert(PARTS == 2, "two partial accumulators");
-#pragma unroll
-    for (int c0 = 0; c0 < NB; c0 += 32) {
-      uint32_t part[32];
-      tmem_ld32_nowait(taddr + (uint32_t)c0, reinterpret_cast<uint32_t(&)[32]>(v[c0]));
-      tmem_ld32_nowait(taddr + part_stride + (uint32_t)c0, part);
-      tmem_ld_wait();
-#pragma unroll
-      for (int c = 0; c < 32; ++c) v[c0 + c] = __float_as_uint(__uint_as_float(v[c0 + c]) + __uint_as_float(part[c]));
-    }
   }
 }
 
@@ -269,17 +227,17 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], C::ISSUERS);
+      mbar_init(&empty_bar[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&accum_full[b], C::ISSUERS);
+      mbar_init(&accum_full[b], 1);
       mbar_init(&accum_empty[b], C::EPI_WARPS);
     }
     mbar_init(&inbox_bar, 1);
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {  // the first issuer warp owns the tensor memory
+  if (warp == 1) {  // the issuing warp owns the tensor memory
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                  "r"(C::TMEM_COLS)
                  : "memory");
@@ -345,28 +303,24 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     if (lane == 0) STAMP(7);  // the last tile of W is requested
     if (a.late_trigger) pdl_launch_dependents();
-  } else if (warp <= C::ISSUERS) {
-    // issuer j owns the k steps j, j + ISSUERS, ... of every k block and the partial accumulator j
+  } else if (warp == 1) {
     const bool leader = elect_one();
-    const int j = warp - 1;
     const uint32_t idesc = umma_idesc(ROWS_W, NB);
     int s = 0, phase = 0, local = 0;
     for (int tile = blockIdx.x; tile < n_tiles && !failed; tile += gridDim.x, ++local) {
       const int buf = local & 1;
       bool ok = mbar_wait(&accum_empty[buf], ((local >> 1) & 1) ^ 1);
       tc_fence_after();
-      const uint32_t tmem_d = tmem_base + (uint32_t)(buf * C::ACC_COLS + j * NB);
+      const uint32_t tmem_d = tmem_base + (uint32_t)(buf * NB);
       for (int kb = 0; kb < num_kb && ok; ++kb) {
         ok = mbar_wait(&full_bar[s], phase);
         if (!ok) break;
         tc_fence_after();
-        if (kb == 0 && local == 0 && j == 0 && lane == 0) STAMP(2);  // the first stage (W tile and slice of A) has landed
-        const uint64_t w = umma_desc(smem_u32(smem + s * C::STAGE_BYTES) + j * 32), x = w + (W_BYTES >> 4);
-        static_assert(BK / UMMA_K % C::ISSUERS == 0, "every issuer takes part in every k block");
+        if (kb == 0 && local == 0 && lane == 0) STAMP(2);  // the first stage (W tile and slice of A) has landed
+        const uint64_t w = umma_desc(smem_u32(smem + s * C::STAGE_BYTES)), x = w + (W_BYTES >> 4);
         if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K / C::ISSUERS; ++k)
-            umma(tmem_d, w + k * C::ISSUERS * 2, x + k * C::ISSUERS * 2, idesc, (kb | k) != 0);
+          for (int k = 0; k < BK / UMMA_K; ++k) umma(tmem_d, w + k * 2, x + k * 2, idesc, (kb | k) != 0);  // 32 bytes a step
           umma_commit(&empty_bar[s]);
         }
         if (++s == C::STAGES) s = 0, phase ^= 1;
@@ -376,7 +330,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         break;
       }
       if (leader) umma_commit(&accum_full[buf]);
-      if (j == 0 && lane == 0) STAMP(3);  // the last product of a block is issued
+      if (lane == 0) STAMP(3);  // the last product of a block is issued
     }
   }
 
@@ -496,7 +450,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&accum_empty[buf])) : "memory");
         for (int h0 = mine; h0 < NB && h0 < rows; h0 += STEP) {
         uint32_t v[WIN];
-        load_accumulator<WIN, C::PARTS>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * C::ACC_COLS + h0), NB, v);
+        load_accumulator<WIN>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * NB + h0), v);
         if (h0 + STEP >= NB || h0 + STEP >= rows) {  // the last window: the accumulator is free again
           tc_fence_before();
           __syncwarp();
@@ -643,7 +597,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       if (threadIdx.x == 32 * C::FIRST_EPI_WARP) STAMP(4);  // the accumulator is complete
       for (int h0 = C::EPI_GROUPS == 1 ? 0 : C::WINDOW * (ew >> 2); h0 < NB && h0 < rows; h0 += C::WINDOW * C::EPI_GROUPS) {
         uint32_t v[C::WINDOW];
-        load_accumulator<C::WINDOW, C::PARTS>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)h0, NB, v);
+        load_accumulator<C::WINDOW>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)h0, v);
 #pragma unroll
         for (int m = 0; m < C::WINDOW; ++m) tile[(h0 + m) * ROWS_W + row] = __uint_as_float(v[m]);
       }
