@@ -25,6 +25,8 @@
 // Two kernels.  `attn_rows_kernel` takes heads of up to 128 dimensions in rows of whole 16-byte (bfloat16: 8-byte)
 // pieces: several tokens of a portion share every key and value, which pass through shared memory.
 // `attn_generic_kernel` takes the rest, one block per (query token, KV head).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -200,11 +202,11 @@ attn_generic_kernel(const T* __restrict__ q, long q_stride, const T* __restrict_
 // the result (the same rows, so the running maximum and sum stay in its registers); the keys of the next tile
 // are on their way while the values of this one are summed, and the other way round.
 //
-// What bounds it: shared-memory reads (eight 16-byte reads a thread per 64 products of the scores, twelve per
-// 128 of the sums).  260 tokens of a prompt beside four single tokens at 330, 12 heads of 128 on 2 KV heads:
-// 93 us; 112 with the page table read and indices divided for every copied piece, 299 with a block per token whose
-// threads each walk a key of their own through global memory.
-constexpr int TILE_KEYS = 64, MAX_DIM = 128;
+// What bounds it: the latencies of a tile, one after the other (a block alone on an SM takes 7 us a tile of 16 rows, 11 of
+// 32, the FMA units 1 and 2).  260 tokens of a prompt beside four single tokens at 330, 12 heads of 128 on 2 KV heads:
+// 55 us; 75 with 128 threads and runs of 32 rows whatever their number (69 with 256 threads, 63 with the longest runs
+// first), 93 before that, 299 with a block per token whose threads each walk a key of their own through global memory.
+constexpr int TILE_KEYS = 64, MAX_DIM = 128, ROW_THREADS = 256;
 
 struct RowsArgs {
   const void *q, *k_pool, *v_pool;
@@ -239,7 +241,7 @@ __device__ __forceinline__ void wait_groups() { asm volatile("cp.async.wait_grou
 template <typename T, int R, int TY>
 __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0, int n, int pos0, int seq, int kvh,
                                           int g0, int gn) {
-  constexpr int TX = THREADS / TY, RI = R / TY, KJ = TILE_KEYS / TX, DJ = MAX_DIM / (4 * TX), LP = TILE_KEYS + 4;
+  constexpr int TX = ROW_THREADS / TY, RI = R / TY, KJ = TILE_KEYS / TX, DJ = MAX_DIM / (4 * TX), LP = TILE_KEYS + 4;
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int D = a.D, Dv = a.Dv, LK = D + 4, LV = Dv + 4, G = a.H / a.KVH, rows = n * gn;
   float* qs = smem;                     // [R][LK]
@@ -259,7 +261,7 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
   auto tile_start = [&](int i) { return (i < nfront ? i : first + i - nfront) * TILE_KEYS; };
 
   __syncthreads();  // (a block of several groups of heads: the last one's reads are done)
-  for (int i = tid; i < R * (D / 4); i += THREADS) {
+  for (int i = tid; i < R * (D / 4); i += ROW_THREADS) {
     const int r = i / (D / 4), d = i % (D / 4) * 4;
     const bool there = r < rows;
     const T* src = (const T*)a.q;
@@ -285,7 +287,7 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
   auto bring = [&](int i, const T* pool, int width, float* to, int ld) {
     if (lane < width / 4) {
 #pragma unroll 2
-      for (int j = warp; j < TILE_KEYS; j += THREADS / 32) {
+      for (int j = warp; j < TILE_KEYS; j += ROW_THREADS / 32) {
         const long at = slot[(i & 1) * TILE_KEYS + j];
         bring4(to + j * ld + lane * 4, at >= 0 ? pool + at * width + lane * 4 : pool, at >= 0);
       }
@@ -326,13 +328,26 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
       float4 x[RI];
 #pragma unroll
       for (int i = 0; i < RI; ++i) x[i] = *reinterpret_cast<const float4*>(qs + (ty + i * TY) * LK + d);
+      float4 y[KJ];
 #pragma unroll
-      for (int j = 0; j < KJ; ++j) {
-        const float4 y = *reinterpret_cast<const float4*>(ks + (tx + j * TX) * LK + d);
+      for (int j = 0; j < KJ; ++j) y[j] = *reinterpret_cast<const float4*>(ks + (tx + j * TX) * LK + d);
+      // dimension after dimension over all sums: neighbouring instructions do not wait for one another
 #pragma unroll
-        for (int i = 0; i < RI; ++i)
-          s[i][j] = fmaf(x[i].w, y.w, fmaf(x[i].z, y.z, fmaf(x[i].y, y.y, fmaf(x[i].x, y.x, s[i][j]))));
-      }
+      for (int j = 0; j < KJ; ++j)
+#pragma unroll
+        for (int i = 0; i < RI; ++i) s[i][j] = fmaf(x[i].x, y[j].x, s[i][j]);
+#pragma unroll
+      for (int j = 0; j < KJ; ++j)
+#pragma unroll
+        for (int i = 0; i < RI; ++i) s[i][j] = fmaf(x[i].y, y[j].y, s[i][j]);
+#pragma unroll
+      for (int j = 0; j < KJ; ++j)
+#pragma unroll
+        for (int i = 0; i < RI; ++i) s[i][j] = fmaf(x[i].z, y[j].z, s[i][j]);
+#pragma unroll
+      for (int j = 0; j < KJ; ++j)
+#pragma unroll
+        for (int i = 0; i < RI; ++i) s[i][j] = fmaf(x[i].w, y[j].w, s[i][j]);
     }
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
@@ -379,31 +394,34 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
     // where some row does not see every key, a key that a row does not see (weight -0) must not reach it: 0 times a
     // value that is no number is none either
     const bool all_seen = kt + TILE_KEYS - 1 <= pos0 && kt >= lowest(last);
+    auto add_values = [&](auto some_hidden) {
 #pragma unroll 2
-    for (int j = 0; j < TILE_KEYS; j += 4) {
-      float p[RI][4];
+      for (int j = 0; j < TILE_KEYS; j += 4) {
+        float p[RI][4];
 #pragma unroll
-      for (int i = 0; i < RI; ++i) {
-        const float4 v = *reinterpret_cast<const float4*>(ps + (ty + i * TY) * LP + j);
-        p[i][0] = v.x, p[i][1] = v.y, p[i][2] = v.z, p[i][3] = v.w;
-      }
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-#pragma unroll
-        for (int dj = 0; dj < DJ; ++dj) {
-          const int d = (tx + dj * TX) * 4;
-          if (d >= Dv) continue;
-          const float4 v = *reinterpret_cast<const float4*>(vs + (j + e) * LV + d);
-#pragma unroll
-          for (int i = 0; i < RI; ++i) {
-            if (!all_seen && __float_as_uint(p[i][e]) == 0x80000000u) continue;
-            acc[i][4 * dj] = fmaf(p[i][e], v.x, acc[i][4 * dj]);
-            acc[i][4 * dj + 1] = fmaf(p[i][e], v.y, acc[i][4 * dj + 1]);
-            acc[i][4 * dj + 2] = fmaf(p[i][e], v.z, acc[i][4 * dj + 2]);
-            acc[i][4 * dj + 3] = fmaf(p[i][e], v.w, acc[i][4 * dj + 3]);
-          }
+        for (int i = 0; i < RI; ++i) {
+          const float4 v = *reinterpret_cast<const float4*>(ps + (ty + i * TY) * LP + j);
+          p[i][0] = v.x, p[i][1] = v.y, p[i][2] = v.z, p[i][3] = v.w;
         }
-    }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int dj = 0; dj < DJ; ++dj) {
+            const int d = (tx + dj * TX) * 4;
+            if (d >= Dv) continue;
+            const float4 v = *reinterpret_cast<const float4*>(vs + (j + e) * LV + d);
+#pragma unroll
+            for (int i = 0; i < RI; ++i) {
+              if (decltype(some_hidden)::value && __float_as_uint(p[i][e]) == 0x80000000u) continue;
+              acc[i][4 * dj] = fmaf(p[i][e], v.x, acc[i][4 * dj]);
+              acc[i][4 * dj + 1] = fmaf(p[i][e], v.y, acc[i][4 * dj + 1]);
+              acc[i][4 * dj + 2] = fmaf(p[i][e], v.z, acc[i][4 * dj + 2]);
+              acc[i][4 * dj + 3] = fmaf(p[i][e], v.w, acc[i][4 * dj + 3]);
+            }
+          }
+      }
+    };
+    if (all_seen) add_values(std::false_type{}); else add_values(std::true_type{});
     __syncthreads();  // the values have been read
     if (t + 1 < ntiles) bring_values(t + 1); else end_group();
   }
@@ -433,7 +451,7 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
   if (a.turn_freq) {
     __syncthreads();
     const int half = Dv / 2;
-    for (int i = tid; i < rows * Dv; i += THREADS) {
+    for (int i = tid; i < rows * Dv; i += ROW_THREADS) {
       const int r = i / Dv, d = i % Dv, mth = d < half ? d : d - half;
       float sn, cn;
       sincosf((float)(pos0 + r / gn) * a.turn_freq[mth], &sn, &cn);
@@ -444,31 +462,37 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
   }
 }
 
-constexpr int ROWS = 32, FEW_ROWS = 8;
+constexpr int FEW_ROWS = 8;
 
-template <typename T>
-__global__ void __launch_bounds__(THREADS) attn_rows_kernel(const RowsArgs a) {
+template <typename T, int ROWS>
+__global__ void __launch_bounds__(ROW_THREADS) attn_rows_kernel(const RowsArgs a) {
   extern __shared__ __align__(16) float rows_smem[];
-  const int t0 = blockIdx.x, kvh = blockIdx.y, pos0 = a.positions[t0];
+  const int t0 = (int)gridDim.x - 1 - (int)blockIdx.x, kvh = blockIdx.y, pos0 = a.positions[t0];  // the longest first
   if (pos0 < 0) return;
   const int seq = a.seq_of_token[t0], G = a.H / a.KVH, per = max(1, ROWS / G);
   if (pos0 % per && t0 > 0 && a.seq_of_token[t0 - 1] == seq && a.positions[t0 - 1] == pos0 - 1) return;  // inside a run
   int n = 1;
   while (n < per && (pos0 + n) % per && t0 + n < a.T && a.seq_of_token[t0 + n] == seq && a.positions[t0 + n] == pos0 + n) ++n;
   if (n * G <= FEW_ROWS)
-    attn_rows<T, FEW_ROWS, 4>(a, rows_smem, t0, n, pos0, seq, kvh, 0, G);
+    attn_rows<T, FEW_ROWS, 8>(a, rows_smem, t0, n, pos0, seq, kvh, 0, G);
   else
-    for (int g0 = 0; g0 < G; g0 += ROWS) attn_rows<T, ROWS, 8>(a, rows_smem, t0, n, pos0, seq, kvh, g0, min(ROWS, G - g0));
+    for (int g0 = 0; g0 < G; g0 += ROWS) attn_rows<T, ROWS, 16>(a, rows_smem, t0, n, pos0, seq, kvh, g0, min(ROWS, G - g0));
 }
 
-template <typename T>
+template <typename T, int ROWS>
 int launch_rows(const RowsArgs& a, cudaStream_t stream) {
   const size_t smem = (size_t)((ROWS + TILE_KEYS) * (a.D + 4) + TILE_KEYS * (a.Dv + 4) + ROWS * (TILE_KEYS + 4)) * sizeof(float) +
                       2 * TILE_KEYS * sizeof(long);
-  DSP_CUDA(cudaFuncSetAttribute(attn_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  attn_rows_kernel<T><<<dim3(a.T, a.KVH), THREADS, smem, stream>>>(a);
+  DSP_CUDA(cudaFuncSetAttribute(attn_rows_kernel<T, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  attn_rows_kernel<T, ROWS><<<dim3(a.T, a.KVH), ROW_THREADS, smem, stream>>>(a);
   DSP_CHECK_LAUNCH("dsp_attn_generic");
   return 0;
+}
+// Runs of half the tokens where those that fill 32 rows leave SMs idle: a block's time is that of its own tiles.
+template <typename T>
+int launch_rows(const RowsArgs& a, cudaStream_t stream) {
+  const int G = a.H / a.KVH, per = G < 32 ? 32 / G : 1;
+  return (long)(a.T / per + 1) * a.KVH <= 2 * dsp_num_sms() ? launch_rows<T, 16>(a, stream) : launch_rows<T, 32>(a, stream);
 }
 
 // Whether rows of `width` elements at `stride` from `p` consist of whole pieces of four elements.
