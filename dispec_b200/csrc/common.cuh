@@ -175,3 +175,26 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
   for (int w = 0; w < nwarps; ++w) total = fmaxf(total, scratch[w]);
   return total;
 }
+
+__device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
+
+// xIELU with the factors ap = softplus(p), an = 1/2 + softplus(q):
+//   z > 0:  ap z^2 + z / 2;   z <= 0:  an (exp(z) - 1 - z) + z / 2
+// exp(z) - 1 - z by its series from -1 on, z^2 (1/2! + z/3! + .. + z^9/11!), which is off by 2^-27 of it at -1, and from
+// the exponential below, where it is at least exp(-1): no cancellation in either, and no branch.  Against 64 bits, rms of
+// the relative error, this and by way of expm1f: 2.6e-8 and 6.5e-8 in (-0.1, 0), 4.3e-8 and 1.1e-7 in (-0.5, -0.1),
+// 1.8e-7 both in (-1, -0.5), 1.5e-7 both in (-10, -2).
+__device__ __forceinline__ float xielu_f(float z, float ap, float an) {
+  const float x = fmaxf(z, -1.f);
+  float s = fmaf(x, 1.f / 39916800.f, 1.f / 3628800.f);
+  s = fmaf(x, s, 1.f / 362880.f);
+  s = fmaf(x, s, 1.f / 40320.f);
+  s = fmaf(x, s, 1.f / 5040.f);
+  s = fmaf(x, s, 1.f / 720.f);
+  s = fmaf(x, s, 1.f / 120.f);
+  s = fmaf(x, s, 1.f / 24.f);
+  s = fmaf(x, s, 1.f / 6.f);
+  s = fmaf(x, s, 0.5f);
+  const float g = z < -1.f ? expf(z) - 1.f - z : z * z * s;
+  return fmaf(z > 0.f ? ap * z : an, z > 0.f ? z : g, 0.5f * z);
+}

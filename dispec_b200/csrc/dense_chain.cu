@@ -24,7 +24,7 @@ int dsp_gemm_tcgen05(const void* A, long lda, const void* W, const void* bias, c
                      long ldc, int M, int N, int K, int out_dtype, int pair_mode, int epilogue, cudaStream_t stream);
 int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas);
 int dsp_gemm_pairs(const void* A, long lda, const void* W, const void* bias, const void* residual, long ldr, void* C, long ldc,
-                   int M, int N, int K, int out_dtype, int epilogue, int splits, int chunks, cudaStream_t stream);
+                   int M, int N, int K, int out_dtype, int epilogue, const float* act, int splits, int chunks, cudaStream_t stream);
 int dsp_gemm_pairs_faster(int M, int N, int K, int target_ctas);
 int dsp_attn_combine(const float* part_o, const float* part_ml, void* out, long out_stride, int num_tokens, int H, int D,
                      int splits, int dtype, cudaStream_t stream);
@@ -90,7 +90,7 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
     if (T > s.always_few) {
       const int pairs = dsp_gemm_pairs_faster(T, N, K, (int)s.target_ctas);
       if (pairs < 0) return pairs;
-      if (pairs) return dsp_gemm_pairs(A, K, W, bias, residual, add ? N : 0, C, N, T, N, K, DSP_BF16, 0, 0, 0, stream);
+      if (pairs) return dsp_gemm_pairs(A, K, W, bias, residual, add ? N : 0, C, N, T, N, K, DSP_BF16, 0, nullptr, 0, 0, stream);
     }
     const int few = T <= s.always_few ? 1 : dsp_gemm_few_rows_faster(T, N, K, (int)s.target_ctas);
     if (few < 0) return few;
@@ -158,7 +158,7 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
                                0, stream));
     else if (pairs_gate_up)
       DSP_STEP(dsp_gemm_pairs(s.h, hidden, l.w_gate_up, nullptr, nullptr, 0, s.act, inter, T, 2 * inter, hidden, DSP_BF16,
-                              (int)s.epilogue, 0, 0, stream));
+                              (int)s.epilogue, nullptr, 0, 0, stream));
     else
       DSP_STEP(dsp_gemm_tcgen05(s.h, hidden, l.w_gate_up, nullptr, nullptr, 0, s.act, inter, T, 2 * inter, hidden,
                                 DSP_BF16, 1, (int)s.epilogue, stream));

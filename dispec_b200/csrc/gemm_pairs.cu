@@ -26,10 +26,11 @@ constexpr int STAGING = EPI_GROUPS * 32 * ROWS_W * 4;  // a chunk of 32 columns 
 constexpr int TMEM_COLS = 512;                // two accumulators of up to 256 columns
 constexpr int SMEM = SLOTS * SUB * (W_BYTES + MAX_COLS / 2 * BK * 2) + STAGING + 1024;
 constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;  // clears the lowest bit of the CTA rank of a shared::cluster address
-enum { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_GEGLU = 2 };
+enum { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_GEGLU = 2, EPI_XIELU = 3 };
 
 struct Args {
   int epilogue;
+  const float* act;  // the two raw parameters of xIELU
   const bf16* bias;
   const void* residual;
   long ldr;
@@ -102,6 +103,10 @@ __device__ __forceinline__ void store4(bf16* p, float4 v) { *reinterpret_cast<ui
 __device__ __forceinline__ float unit_times(float gate, float up, bool gelu) {
   const float y = gelu ? 2.f * 0.7978845608028654f * fmaf(0.044715f * gate * gate, gate, gate) : gate;
   return __fdividef(gate, 1.f + __expf(-y)) * up;
+}
+
+__device__ __forceinline__ float4 xielu4(float4 z, float ap, float an) {
+  return make_float4(xielu_f(z.x, ap, an), xielu_f(z.y, ap, an), xielu_f(z.z, ap, an), xielu_f(z.w, ap, an));
 }
 
 // Four outputs of a row, this lane's n0 + 4 lane .. + 3, from their sums.
@@ -275,6 +280,7 @@ gemm_pairs_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       }
       float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f), res4[8];
       if (a.bias && n4 < a.N) bias4 = load4(a.bias + n4);
+      const float ap = a.act ? softplus_f(a.act[0]) : 0.f, an = a.act ? 0.5f + softplus_f(a.act[1]) : 0.f;
       auto fetch_residual = [&](int c0) {  // of the rows this warp finishes in the chunk at c0
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -301,7 +307,14 @@ gemm_pairs_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         float4 x[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(staging + (8 * ew + i) * ROWS_W + 4 * lane);
-        if (a.epilogue != EPI_PLAIN) {
+        if (a.epilogue == EPI_XIELU) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int m = c0 + 8 * ew + i;
+            const float4 y = xielu4(x[i], ap, an);
+            if (m < rows && n4 < a.N) store4(reinterpret_cast<TOut*>(a.C) + (size_t)(m0 + m) * a.ldc + n4, y);
+          }
+        } else if (a.epilogue != EPI_PLAIN) {
 #pragma unroll
           for (int i = 0; i < 8; i += 2) {
             const int m = c0 + 8 * ew + i;
@@ -338,6 +351,7 @@ gemm_pairs_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       const int rows = min(a.chunk_rows, a.M - m0), n4 = n0 + 4 * lane;
       float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
       if (a.bias && n4 < a.N) bias4 = load4(a.bias + n4);
+      const float ap = a.act ? softplus_f(a.act[0]) : 0.f, an = a.act ? 0.5f + softplus_f(a.act[1]) : 0.f;
       uint32_t from[MAX_SPLITS];
 #pragma unroll
       for (int sp = 0; sp < MAX_SPLITS; ++sp) from[sp] = sp < a.splits ? mapa_u32(smem_u32(smem) + lane * 16, 2 * sp + half) : 0;
@@ -365,9 +379,10 @@ gemm_pairs_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int m = split + a.splits * (r0 + i);
-          if (a.epilogue == EPI_PLAIN) finish_row<TOut>(a, x[i], m0 + m, m < rows, n4, bias4, res4[i]);
+          if (a.epilogue == EPI_XIELU) x[i] = xielu4(x[i], ap, an);
+          if (a.epilogue == EPI_PLAIN || a.epilogue == EPI_XIELU) finish_row<TOut>(a, x[i], m0 + m, m < rows, n4, bias4, res4[i]);
         }
-        if (a.epilogue != EPI_PLAIN) {
+        if (a.epilogue == EPI_SWIGLU || a.epilogue == EPI_GEGLU) {
 #pragma unroll
           for (int i = 0; i < 4; i += 2) {
             const int m = split + a.splits * (r0 + i);
@@ -498,16 +513,18 @@ extern "C" int dsp_gemm_pairs_faster(int M, int N, int K, int target_ctas) {
 }
 
 // Operands as dsp_gemm_tcgen05 takes them; N, ldc and ldr multiples of 4, C and residual on 16 bytes (bfloat16: 8),
-// bias on 8.  splits, chunks: pairs that share a tile's K, chunks of rows (0: by the estimate).
+// bias on 8.  epilogue 3: xIELU of every output, its two raw parameters in `act` (null otherwise).  splits, chunks: pairs that share a tile's K, chunks of rows (0: by the estimate).
 extern "C" int dsp_gemm_pairs(const void* A, long lda, const void* W, const void* bias, const void* residual, long ldr, void* C,
-                              long ldc, int M, int N, int K, int out_dtype, int epilogue, int splits, int chunks, cudaStream_t stream) {
+                              long ldc, int M, int N, int K, int out_dtype, int epilogue, const float* act,
+                              int splits, int chunks, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   DSP_REQUIRE(K > 0 && K % 8 == 0 && lda % 8 == 0, "dsp_gemm_pairs: K=%d and the row stride must be multiples of 8", K);
   DSP_REQUIRE(((uintptr_t)A % 16) == 0 && ((uintptr_t)W % 16) == 0, "dsp_gemm_pairs: operands must be 16-byte aligned");
   DSP_REQUIRE(out_dtype == DSP_BF16 || out_dtype == DSP_F32, "dsp_gemm_pairs: unknown output dtype %d", out_dtype);
-  DSP_REQUIRE(epilogue >= EPI_PLAIN && epilogue <= EPI_GEGLU, "dsp_gemm_pairs: unknown epilogue %d", epilogue);
-  DSP_REQUIRE(epilogue == EPI_PLAIN || (N % 32 == 0 && bias == nullptr && residual == nullptr),
-              "dsp_gemm_pairs: the SwiGLU epilogue needs N in whole blocks of 32 and no bias or residual");
+  DSP_REQUIRE(epilogue >= EPI_PLAIN && epilogue <= EPI_XIELU, "dsp_gemm_pairs: unknown epilogue %d", epilogue);
+  DSP_REQUIRE(epilogue == EPI_PLAIN || ((epilogue == EPI_XIELU || N % 32 == 0) && bias == nullptr && residual == nullptr),
+              "dsp_gemm_pairs: an activation takes no bias or residual, and a gated one N in whole blocks of 32");
+  DSP_REQUIRE((epilogue == EPI_XIELU) == (act != nullptr), "dsp_gemm_pairs: xIELU and its parameters come together");
   const uintptr_t mask = out_dtype == DSP_F32 ? 15 : 7;
   DSP_REQUIRE(N % 4 == 0 && ldc % 4 == 0 && ((uintptr_t)C & mask) == 0 && (residual == nullptr || (ldr % 4 == 0 && ((uintptr_t)residual & mask) == 0)) &&
                   (bias == nullptr || ((uintptr_t)bias & 7) == 0),
@@ -517,7 +534,7 @@ extern "C" int dsp_gemm_pairs(const void* A, long lda, const void* W, const void
   const Plan p = make_plan(M, N, K, splits, chunks);
   if (p.splits == 0) return -1;
   DSP_REQUIRE(p.us >= 0.0, "dsp_gemm_pairs: no plan for M=%d, N=%d, K=%d in %d splits and %d chunks", M, N, K, splits, chunks);
-  Args a = {epilogue, (const bf16*)bias, residual, ldr, C, ldc, M, N, K, p.cols, p.chunk_rows, p.chunks, p.splits, p.slots_per_split, 0};
+  Args a = {epilogue, act, (const bf16*)bias, residual, ldr, C, ldc, M, N, K, p.cols, p.chunk_rows, p.chunks, p.splits, p.slots_per_split, 0};
   CUtensorMap map_a, map_w;
   a.k_boxes = make_map_k_blocks(&map_a, A, M, K, lda, p.cols / 2, SUB) && make_map_k_blocks(&map_w, W, N, K, K, ROWS_W, SUB);
   if (!a.k_boxes) {

@@ -158,16 +158,12 @@ head_norm_gate_wide_kernel(const float* __restrict__ o, long ldo, const float* _
   }
 }
 
-__device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
-
-// xIELU with the two raw parameters (p, q) read from the device:
-//   z > 0:  softplus(p) z^2 + z / 2
-//   z <= 0: (1/2 + softplus(q)) (exp(z) - 1 - z) + z / 2
+// xIELU (`xielu_f`) with the two raw parameters (p, q) read from the device.
 __global__ void __launch_bounds__(256)
 xielu_kernel(const void* __restrict__ z, int z_dtype, long ldz, const float* __restrict__ pq,
              void* __restrict__ y, int y_dtype, long ldy, long rows, int cols) {
   const float ap = softplus_f(pq[0]), an = 0.5f + softplus_f(pq[1]);
-  auto act = [&](float v) { return v > 0.f ? fmaf(ap * v, v, 0.5f * v) : fmaf(an, expm1f(v) - v, 0.5f * v); };
+  auto act = [&](float v) { return xielu_f(v, ap, an); };
   const long n = rows * cols;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const long r = i / cols;
@@ -187,7 +183,7 @@ __global__ void __launch_bounds__(128)
 xielu_rows_kernel(const float* __restrict__ z, long ldz, const float* __restrict__ pq, bf16* __restrict__ y, long ldy,
                   long rows, int cols) {
   const float ap = softplus_f(pq[0]), an = 0.5f + softplus_f(pq[1]);
-  auto act = [&](float v) { return v > 0.f ? fmaf(ap * v, v, 0.5f * v) : fmaf(an, expm1f(v) - v, 0.5f * v); };
+  auto act = [&](float v) { return xielu_f(v, ap, an); };
   const int c0 = (blockIdx.x * GROUPS * blockDim.x + threadIdx.x) * 4, step = blockDim.x * 4;
   for (long r = blockIdx.y; r < rows; r += gridDim.y) {
     const float* src = z + (size_t)r * ldz;

@@ -66,7 +66,7 @@ class NormedRows:
         return (x is not None and x.dtype == torch.bfloat16 and M <= NORM_SPLIT_MAX_ROWS
                 and self.source.stride(1) == 1 and self.source.stride(0) % 8 == 0
                 and self.source.data_ptr() % 16 == 0 and stream_supported(M, K, x, w))
-EPI_PLAIN, EPI_SWIGLU, EPI_GEGLU = 0, 1, 2
+EPI_PLAIN, EPI_SWIGLU, EPI_GEGLU, EPI_XIELU = 0, 1, 2, 3
 SWIGLU_BLOCK = 16  # gate/up rows alternate in blocks of this many for the fused epilogue
 
 
@@ -91,13 +91,13 @@ def _split(x, w, bias, residual, out):
     return out
 
 
-def _pairs(x, w, bias, residual, out, epilogue=EPI_PLAIN, splits: int = 0, chunks: int = 0):
-    """The product of some hundred rows on CTA pairs; ``splits``, ``chunks``: instead of its own choice (comparisons)."""
+def _pairs(x, w, bias, residual, out, epilogue=EPI_PLAIN, splits: int = 0, chunks: int = 0, act: torch.Tensor | None = None):
+    """The product of some hundred rows on CTA pairs; ``act``: the raw parameters of ``EPI_XIELU``; ``splits``, ``chunks``: instead of its own choice (comparisons)."""
     M, K = x.shape
     L.check(L.core().dsp_gemm_pairs(
         L.ptr(x), L.i64(x.stride(0)), L.ptr(w), L.ptr(bias), L.ptr(residual),
         L.i64(residual.stride(0) if residual is not None else 0), L.ptr(out), L.i64(out.stride(0)),
-        M, w.shape[0], K, L.dtype_code(out.dtype), epilogue, splits, chunks, L.stream_handle()))
+        M, w.shape[0], K, L.dtype_code(out.dtype), epilogue, L.ptr(act), splits, chunks, L.stream_handle()))
     return out
 
 
@@ -191,6 +191,26 @@ def linear_gate_up_swiglu(x, w_interleaved, out=None, act: str = "silu"):
             return _pairs(x, w_interleaved, None, None, out, epilogue=epilogue)
         return _tcgen05(x, w_interleaved, None, None, out, epilogue=epilogue)
     return _stream(x, w_interleaved, None, None, out, epilogue=epilogue, norm=norm)
+
+
+XIELU_MAX_ROWS = 1024  # rows up to which xIELU is formed in the epilogue of the product before it
+
+
+def linear_xielu(x: torch.Tensor, w: torch.Tensor, params: torch.Tensor) -> torch.Tensor:
+    """xIELU(x W^T), the activation formed in 32 bits from the 32-bit sums and rounded to x's type (``params``: its two raw
+    parameters, float32); the same bits in the product's epilogue, where the kernel on CTA pairs takes the operands, and in
+    a kernel of its own behind the product.  The epilogue saves writing and reading the sums and a launch, but takes longer
+    than the products of its tile.  us, fused and not, w 8,960 x 1,536: 137 rows 17 and 27, 300 23 and 36, 536 36 and 35,
+    1,016 48 and 52, 2,500 101 and 106; w 4,096 x 1,024: 1,016 rows 27 and 36, 2,500 59 and 47."""
+    from dispec_b200.ops.norm32 import xielu
+    M, N = x.shape[0], w.shape[0]
+    if STREAM_MAX_ROWS < M <= XIELU_MAX_ROWS and x.dtype == w.dtype == torch.bfloat16:
+        out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+        if pairs_supported(x, w, None, None, out):
+            assert w.shape[1] == x.shape[1] and x.stride(1) == 1 and w.is_contiguous()
+            assert params.dtype == torch.float32 and params.numel() == 2 and params.is_contiguous() and params.is_cuda
+            return _pairs(x, w, None, None, out, epilogue=EPI_XIELU, act=params)
+    return xielu(linear(x, w, out_dtype=torch.float32), params, x.dtype)
 
 
 def _library(x, w, bias, residual, out):

@@ -9,7 +9,7 @@ from __future__ import annotations
 import torch
 
 from dispec_b200 import ops
-from dispec_b200.ops import norm32 as norm32_ops
+from dispec_b200.ops import gemm as gemm_ops
 from dispec_b200.parts.base import FeedForward, TensorSpec
 from dispec_b200.registry import register_part
 
@@ -28,5 +28,4 @@ class XIELUFeedForward(FeedForward):
         self.w_up, self.w_down, self.act = tensors["up.weight"], tensors["down.weight"], tensors["act"]
 
     def forward(self, ctx, x):
-        z = ops.linear(x, self.w_up, out_dtype=torch.float32)
-        return ops.linear(norm32_ops.xielu(z, self.act, x.dtype), self.w_down, out_dtype=torch.float32)
+        return ops.linear(gemm_ops.linear_xielu(x, self.w_up, self.act), self.w_down, out_dtype=torch.float32)

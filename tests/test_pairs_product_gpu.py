@@ -57,3 +57,19 @@ def test_the_choice_and_what_it_refuses():
         with pytest.raises(library.KernelError, match="rows of four outputs"):
             gemm._pairs(x, w, None, None, out)
         assert torch.allclose(gemm.linear(x, w, out=out).float(), (x.double() @ w.double().T).float(), atol=2e-2, rtol=1e-2)
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 260, 136), (300, 1024, 1024), (1024, 512, 64), (1025, 512, 64)])
+def test_xielu_in_the_epilogue_and_behind_the_product(M, N, K):
+    from dispec_b200.ops import gemm, library, norm32
+    x, w, params = rnd((M, K), 7, 3.0), rnd((N, K), 8, K ** -0.5), torch.tensor([0.3, -0.7], device=DEV)
+    out = gemm.linear_xielu(x, w, params)
+    assert library.device_error() == 0
+    z = x.double() @ w.double().T
+    p, q = torch.nn.functional.softplus(params.double())
+    ref = torch.where(z > 0, p * z * z, (0.5 + q) * (torch.expm1(z.clamp(max=0)) - z)) + z / 2
+    # the sums within 1e-5, a slope of at most 2 p |z| + 1/2 + q, one rounding to bfloat16
+    assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * (2 * p * z.abs() + 1.5)).all()
+    if M <= 1024:
+        sums = gemm._pairs(x, w, None, None, torch.empty((M, N), device=DEV))
+        assert torch.equal(out, norm32.xielu(sums, params, torch.bfloat16))
