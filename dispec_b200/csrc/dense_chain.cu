@@ -80,6 +80,20 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
     ++count;                    \
   } while (0)
 
+  // The kernel of a product, asked once for each of the layers' sizes (an answer takes the host about two microseconds).
+  enum { MANY = 0, FEW = 1, PAIRS = 2 };
+  struct { int N, K, kernel; } chosen[8];
+  int num_chosen = 0;
+  auto choose = [&](int N, int K) -> int {
+    if (T <= s.always_few) return FEW;
+    for (int i = 0; i < num_chosen; ++i)
+      if (chosen[i].N == N && chosen[i].K == K) return chosen[i].kernel;
+    int kernel = dsp_gemm_pairs_faster(T, N, K, (int)s.target_ctas);
+    if (kernel == 1) kernel = PAIRS;
+    else if (kernel == 0) kernel = dsp_gemm_few_rows_faster(T, N, K, (int)s.target_ctas);
+    if (kernel >= 0 && num_chosen < 8) chosen[num_chosen++] = {N, K, kernel};
+    return kernel;
+  };
   // C = A W^T (+ bias) (+ C): the kernel that ops/gemm.py chooses.  `scaled`, `eps`: A is x under a norm still to be
   // applied, `scaled` those rows times its gain.  `gain`, `scaled_out`: the norm after this product, where its kernel
   // can prepare it; *prepared says whether it did.
@@ -87,14 +101,10 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
                      float eps, const void* gain, void* scaled_out, bool* prepared) -> int {
     const void* residual = add ? C : nullptr;
     if (prepared) *prepared = false;
-    if (T > s.always_few) {
-      const int pairs = dsp_gemm_pairs_faster(T, N, K, (int)s.target_ctas);
-      if (pairs < 0) return pairs;
-      if (pairs) return dsp_gemm_pairs(A, K, W, bias, residual, add ? N : 0, C, N, T, N, K, DSP_BF16, 0, nullptr, 0, 0, stream);
-    }
-    const int few = T <= s.always_few ? 1 : dsp_gemm_few_rows_faster(T, N, K, (int)s.target_ctas);
-    if (few < 0) return few;
-    if (few) {
+    const int kernel = choose(N, K);
+    if (kernel < 0) return kernel;
+    if (kernel == PAIRS) return dsp_gemm_pairs(A, K, W, bias, residual, add ? N : 0, C, N, T, N, K, DSP_BF16, 0, nullptr, 0, 0, stream);
+    if (kernel == FEW) {
       const bool prepare = gain && scaled_out;
       if (prepared) *prepared = prepare;
       return dsp_gemm_stream(scaled ? scaled : A, K, W, bias, residual, add ? N : 0, C, N, T, N, K, DSP_BF16,

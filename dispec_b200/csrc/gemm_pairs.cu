@@ -454,6 +454,23 @@ struct Plan {
   int cols, chunk_rows, chunks, splits, slots_per_split, clusters;
   double us;  // estimate; negative: none (the message is set where `splits` is 0)
 };
+Plan make_plan(int M, int N, int K, int force_splits, int force_chunks);
+// The plan of a size, of which the thread's last few are remembered: the layers of a step ask for the same ones.
+Plan plan_of(int M, int N, int K, int splits, int chunks) {
+  struct Known {
+    int M, N, K, device;
+    Plan plan;
+  };
+  static thread_local Known known[8] = {};
+  static thread_local int next = 0;
+  int device = 0;
+  if (splits != 0 || chunks != 0 || cudaGetDevice(&device) != cudaSuccess) return make_plan(M, N, K, splits, chunks);
+  for (const Known& k : known)
+    if (k.M == M && k.N == N && k.K == K && k.device == device) return k.plan;
+  const Plan p = make_plan(M, N, K, 0, 0);
+  if (p.splits > 0 && p.us >= 0.0) known[next++ & 7] = {M, N, K, device, p};
+  return p;
+}
 // Chunks of rows and splits of K by an estimate in microseconds, fitted on launches that follow one another in a graph
 // and read W from memory: 15 shapes from 2,304 x 768 to 37,888 x 3,584, 72 to 2,048 rows, every split and number of chunks
 // (rms error 5 %).  A ring slot costs more the more columns and the more pairs are busy, a tile its epilogue.
@@ -507,7 +524,7 @@ extern "C" int dsp_gemm_pairs_faster(int M, int N, int K, int target_ctas) {
   double few = 0.0, many = 0.0;
   const int rc = dsp_gemm_row_estimates(M, N, K, target_ctas, &few, &many);
   if (rc != 0) return rc;
-  const Plan p = make_plan(M, N, K, 0, 0);
+  const Plan p = plan_of(M, N, K, 0, 0);
   if (p.splits == 0) return -1;
   return p.us > 0.0 && p.us < 0.93 * (few < many ? few : many);
 }
@@ -531,7 +548,7 @@ extern "C" int dsp_gemm_pairs(const void* A, long lda, const void* W, const void
               "dsp_gemm_pairs: rows of four outputs (N=%d, ldc=%ld)", N, ldc);
   int* err = dsp_device_error_ptr();
   DSP_REQUIRE(err != nullptr, "dsp_gemm_pairs: no device error word");
-  const Plan p = make_plan(M, N, K, splits, chunks);
+  const Plan p = plan_of(M, N, K, splits, chunks);
   if (p.splits == 0) return -1;
   DSP_REQUIRE(p.us >= 0.0, "dsp_gemm_pairs: no plan for M=%d, N=%d, K=%d in %d splits and %d chunks", M, N, K, splits, chunks);
   Args a = {epilogue, act, (const bf16*)bias, residual, ldr, C, ldc, M, N, K, p.cols, p.chunk_rows, p.chunks, p.splits, p.slots_per_split, 0};

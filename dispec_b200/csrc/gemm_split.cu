@@ -405,7 +405,7 @@ extern "C" int dsp_gemm_split(const float* A, long lda, const float* W, const fl
   g.chunks = (M + MAX_ROWS - 1) / MAX_ROWS;
   g.chunk_rows = (M + g.chunks - 1) / g.chunks;
   g.chunks = (M + g.chunk_rows - 1) / g.chunk_rows;
-  g.a_wide = lda % 4 == 0 && ((uintptr_t)A & 15) == 0;
+  g.a_wide = lda % 4 == 0 && lda >= K && ((uintptr_t)A & 15) == 0;  // (rows that overlap are no tensor map's)
   // K is split where there are few blocks of W, by their number alone: a row's sums must not depend on how many rows
   // there are.  As many times as leaves clusters that fit beside one another with three chunks of rows (36 clusters of
   // four did not: 264 rows x 1,536 x 8,960 115 us for 68 in three; nor 48 of three: x 2,048 x 1,536 41)

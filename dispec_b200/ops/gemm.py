@@ -148,9 +148,9 @@ def tcgen05_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 def pairs_supported(x: torch.Tensor, w: torch.Tensor, bias, residual, out: torch.Tensor) -> bool:
     """Whether the operands of a product let the kernel on CTA pairs finish four outputs of a row at a time."""
-    vec = lambda t, n: t is None or (t.stride(0) % 4 == 0 and t.data_ptr() % n == 0)
     width = 4 * out.element_size()
-    return (tcgen05_supported(x, w) and w.shape[0] % 4 == 0 and vec(out, width) and vec(residual, width)
+    return (w.shape[0] % 4 == 0 and out.stride(0) % 4 == 0 and out.data_ptr() % width == 0 and tcgen05_supported(x, w)
+            and (residual is None or (residual.stride(0) % 4 == 0 and residual.data_ptr() % width == 0))
             and (bias is None or bias.data_ptr() % 8 == 0))
 
 
@@ -187,7 +187,7 @@ def linear_gate_up_swiglu(x, w_interleaved, out=None, act: str = "silu"):
         out = torch.empty((M, N // 2), dtype=x.dtype, device=x.device)
     epilogue = {"silu": EPI_SWIGLU, "gelu_tanh": EPI_GEGLU}[act]
     if M > STREAM_MAX_ROWS:
-        if pairs_supported(x, w_interleaved, None, None, out) and tuning.pairs_are_faster(M, N, x.shape[1], x.device):
+        if tuning.pairs_are_faster(M, N, x.shape[1], x.device) and pairs_supported(x, w_interleaved, None, None, out):
             return _pairs(x, w_interleaved, None, None, out, epilogue=epilogue)
         return _tcgen05(x, w_interleaved, None, None, out, epilogue=epilogue)
     return _stream(x, w_interleaved, None, None, out, epilogue=epilogue, norm=norm)
@@ -276,7 +276,7 @@ def linear(x, w: torch.Tensor, bias: torch.Tensor | None = None,
     if backend is None:
         if stream_supported(M, K, x, w):
             backend = "stream"
-        elif M > STREAM_MAX_ROWS and pairs_supported(x, w, bias, residual, out) and tuning.pairs_are_faster(M, N, K, x.device):
+        elif M > STREAM_MAX_ROWS and tuning.pairs_are_faster(M, N, K, x.device) and pairs_supported(x, w, bias, residual, out):
             backend = "pairs"
         elif (M > STREAM_MAX_ROWS and stream_supported(STREAM_MAX_ROWS, K, x, w)
               and tuning.rows_in_chunks_is_faster(M, N, K, x.device, STREAM_MAX_ROWS)):
