@@ -203,12 +203,15 @@ def linear_xielu(x: torch.Tensor, w: torch.Tensor, params: torch.Tensor) -> torc
     than the products of its tile.  us, fused and not, w 8,960 x 1,536: 137 rows 17 and 27, 300 23 and 36, 536 36 and 35,
     1,016 48 and 52, 2,500 101 and 106; w 4,096 x 1,024: 1,016 rows 27 and 36, 2,500 59 and 47."""
     from dispec_b200.ops.norm32 import xielu
+    if not (x.is_cuda and w.is_cuda and params.is_cuda):
+        raise L.KernelError("linear_xielu: CUDA tensors only (there is no CPU path)")
+    assert x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1], (x.shape, w.shape)
+    assert x.stride(1) == 1 and w.is_contiguous() and x.dtype == w.dtype
     M, N = x.shape[0], w.shape[0]
-    if STREAM_MAX_ROWS < M <= XIELU_MAX_ROWS and x.dtype == w.dtype == torch.bfloat16:
+    if STREAM_MAX_ROWS < M <= XIELU_MAX_ROWS and x.dtype == torch.bfloat16:
         out = torch.empty((M, N), dtype=x.dtype, device=x.device)
         if pairs_supported(x, w, None, None, out):
-            assert w.shape[1] == x.shape[1] and x.stride(1) == 1 and w.is_contiguous()
-            assert params.dtype == torch.float32 and params.numel() == 2 and params.is_contiguous() and params.is_cuda
+            assert params.dtype == torch.float32 and params.numel() == 2 and params.is_contiguous()
             return _pairs(x, w, None, None, out, epilogue=EPI_XIELU, act=params)
     return xielu(linear(x, w, out_dtype=torch.float32), params, x.dtype)
 
