@@ -81,17 +81,19 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
   } while (0)
 
   // The kernel of a product, asked once for each of the layers' sizes (an answer takes the host about two microseconds).
+  // The one on CTA pairs reads four biases at a time: a bias that does not begin on eight bytes goes to the others.
   enum { MANY = 0, FEW = 1, PAIRS = 2 };
-  struct { int N, K, kernel; } chosen[8];
+  struct { int N, K, kernel; bool fours; } chosen[8];
   int num_chosen = 0;
-  auto choose = [&](int N, int K) -> int {
+  auto choose = [&](int N, int K, const void* bias) -> int {
     if (T <= s.always_few) return FEW;
+    const bool fours = ((uintptr_t)bias & 7) == 0;
     for (int i = 0; i < num_chosen; ++i)
-      if (chosen[i].N == N && chosen[i].K == K) return chosen[i].kernel;
-    int kernel = dsp_gemm_pairs_faster(T, N, K, (int)s.target_ctas);
+      if (chosen[i].N == N && chosen[i].K == K && chosen[i].fours == fours) return chosen[i].kernel;
+    int kernel = fours ? dsp_gemm_pairs_faster(T, N, K, (int)s.target_ctas) : 0;
     if (kernel == 1) kernel = PAIRS;
     else if (kernel == 0) kernel = dsp_gemm_few_rows_faster(T, N, K, (int)s.target_ctas);
-    if (kernel >= 0 && num_chosen < 8) chosen[num_chosen++] = {N, K, kernel};
+    if (kernel >= 0 && num_chosen < 8) chosen[num_chosen++] = {N, K, kernel, fours};
     return kernel;
   };
   // C = A W^T (+ bias) (+ C): the kernel that ops/gemm.py chooses.  `scaled`, `eps`: A is x under a norm still to be
@@ -101,7 +103,7 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
                      float eps, const void* gain, void* scaled_out, bool* prepared) -> int {
     const void* residual = add ? C : nullptr;
     if (prepared) *prepared = false;
-    const int kernel = choose(N, K);
+    const int kernel = choose(N, K, bias);
     if (kernel < 0) return kernel;
     if (kernel == PAIRS) return dsp_gemm_pairs(A, K, W, bias, residual, add ? N : 0, C, N, T, N, K, DSP_BF16, 0, nullptr, 0, 0, stream);
     if (kernel == FEW) {

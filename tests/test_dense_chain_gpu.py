@@ -92,6 +92,22 @@ def test_weights_off_sixteen_bytes_stay_with_the_parts():
         assert torch.equal(a, b)
 
 
+def test_a_bias_off_eight_bytes():
+    """At sizes where the product on CTA pairs is chosen, which takes no such bias: another kernel runs, as in the parts."""
+    from dispec_b200.ops import gemm, tuning
+    model = model_of(hidden_size=1536, intermediate_size=2048, num_attention_heads=12, num_key_value_heads=2, head_dim=128)
+    mixer = model.layers[0].mixer
+    slab = torch.empty(1536 + 1, dtype=torch.bfloat16, device=DEV).normal_()
+    mixer.b_o = slab[1:]
+    assert model.dense_chain and tuning.pairs_are_faster(536, 1536, 1536)
+    x = torch.zeros((536, 1536), dtype=torch.bfloat16, device=DEV)
+    assert gemm.pairs_supported(x, mixer.w_o, None, x, x) and not gemm.pairs_supported(x, mixer.w_o, mixer.b_o, x, x)
+    mine, _ = run(model, True, [500, 36], 2, 16)
+    parts, _ = run(model, False, [500, 36], 2, 16)
+    for a, b in zip(mine, parts):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("prompts,stored", [([137], 0), ([536], 0), ([700, 40], 0), ([1900], 0), ([24, 5], 4200), ([300], 9000)])
 def test_same_bits_at_the_sizes_where_c_chooses(prompts, stored):
     """Two layers of the 1.5B sizes: few-row products above 128 rows, products that let their successor start late, norms a
