@@ -50,10 +50,11 @@ template <int NB> struct Cfg {
   // dependent launch) fills its ring with W while this kernel's CTA is still streaming
   // (128 and 192 rows of A: one CTA per SM; at 192 the ring must also hold the partial tile and the inbox of a K split)
   static constexpr int STAGES = NB == 64 ? 4 : 5;
-  // One warp issues the products.  (While a single thread ran that loop, its turn of the ring took 0.3 us, as long as a
-  // tile takes to arrive, and up to 64 rows of A the k steps of a block were dealt to two or four threads with partial
-  // accumulators of their own; with the loop run by whole warps that costs more than it gives: decode steps at 1, 8 and
-  // 64 rows 913, 941 and 1,697 us with them, 910, 937 and 1,690 without.)
+  // One warp issues the products, step k of every block into partial accumulator k % PARTS; the epilogue adds these in a
+  // fixed order.  The tensor cores cut sums off, so that shorter chains of sums are closer to 64 bits: relative error of
+  // 32-bit results x 2,048 columns, 8 rows, K 1,536 / 8,960 / 18,944: 8.6e-8 / 2.6e-7 / 5.5e-7 with four, 1.8e-7 / 1.1e-6 / 2.5e-6
+  // in one accumulator; 64 rows 1.1e-7 / 5.3e-7 / 1.2e-6 with two.
+  static constexpr int PARTS = NB == 16 ? 4 : NB <= 64 ? 2 : 1;
   // two epilogue warps per quarter of the lanes where a CTA has an SM to itself: they take the windows of the
   // accumulator (the rows of a K split) in turn
   static constexpr int EPI_GROUPS = NB <= 64 ? 1 : 2, EPI_WARPS = 4 * EPI_GROUPS;
@@ -61,7 +62,8 @@ template <int NB> struct Cfg {
   static constexpr int MIN_CTAS = NB <= 64 ? 2 : 1;  // CTAs per SM the registers are held down for
   // the epilogue takes the accumulator in windows of at most 64 columns (rows of A): what a thread holds at once
   static constexpr int WINDOW = NB <= 64 ? NB : 64;
-  static constexpr int TMEM_COLS = 2 * NB <= 256 ? 2 * NB : 512;  // two accumulators, a power of two
+  static constexpr int ACC_COLS = PARTS * NB;  // one accumulator buffer
+  static constexpr int TMEM_COLS = 2 * ACC_COLS <= 256 ? 2 * ACC_COLS : 512;  // two of them, a power of two
   // K split over a cluster: every CTA sends the rows of its partial tile to the CTA that finishes
   // them (row m to rank m % splits), into an inbox of [source rank][rows per CTA][128] floats.  Up
   // to 16 rows of A (at most 16 + 8 rows of inbox) it has room of its own behind the ring
@@ -185,15 +187,40 @@ __device__ __forceinline__ float square_sum8(const uint4 u) {
   return ss;
 }
 
-// NB columns of the accumulator of this thread's W row.
-template <int NB>
-__device__ __forceinline__ void load_accumulator(uint32_t taddr, uint32_t (&v)[NB]) {
+// The accumulator of this thread's W row: NB columns from taddr on, the PARTS partial accumulators (part_stride columns
+// apart) added in a fixed order.
+template <int NB, int PARTS>
+__device__ __forceinline__ void load_accumulator(uint32_t taddr, uint32_t part_stride, uint32_t (&v)[NB]) {
   if constexpr (NB == 16) {
-    tmem_ld16(taddr, v);
-  } else {
+    // they lie side by side: 64 columns, one wait
+    static_assert(PARTS == 4, "four partial accumulators");
+    uint32_t all[PARTS * 16];
+    tmem_ld32_nowait(taddr, reinterpret_cast<uint32_t(&)[32]>(all[0]));
+    tmem_ld32_nowait(taddr + 32, reinterpret_cast<uint32_t(&)[32]>(all[32]));
+    tmem_ld_wait();
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      float sum = __uint_as_float(all[c]);
+#pragma unroll
+      for (int p = 1; p < PARTS; ++p) sum += __uint_as_float(all[p * 16 + c]);
+      v[c] = __float_as_uint(sum);
+    }
+  } else if constexpr (PARTS == 1) {
 #pragma unroll
     for (int c0 = 0; c0 < NB; c0 += 32) tmem_ld32_nowait(taddr + (uint32_t)c0, reinterpret_cast<uint32_t(&)[32]>(v[c0]));
     tmem_ld_wait();
+  } else {
+    // 32 columns of both per trip to the tensor memory (a load and its wait take a few hundred nanoseconds)
+    static_assert(PARTS == 2, "two partial accumulators");
+#pragma unroll
+    for (int c0 = 0; c0 < NB; c0 += 32) {
+      uint32_t part[32];
+      tmem_ld32_nowait(taddr + (uint32_t)c0, reinterpret_cast<uint32_t(&)[32]>(v[c0]));
+      tmem_ld32_nowait(taddr + part_stride + (uint32_t)c0, part);
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < 32; ++c) v[c0 + c] = __float_as_uint(__uint_as_float(v[c0 + c]) + __uint_as_float(part[c]));
+    }
   }
 }
 
@@ -311,7 +338,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       const int buf = local & 1;
       bool ok = mbar_wait(&accum_empty[buf], ((local >> 1) & 1) ^ 1);
       tc_fence_after();
-      const uint32_t tmem_d = tmem_base + (uint32_t)(buf * NB);
+      const uint32_t tmem_d = tmem_base + (uint32_t)(buf * C::ACC_COLS);
       for (int kb = 0; kb < num_kb && ok; ++kb) {
         ok = mbar_wait(&full_bar[s], phase);
         if (!ok) break;
@@ -320,7 +347,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint64_t w = umma_desc(smem_u32(smem + s * C::STAGE_BYTES)), x = w + (W_BYTES >> 4);
         if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) umma(tmem_d, w + k * 2, x + k * 2, idesc, (kb | k) != 0);  // 32 bytes a step
+          for (int k = 0; k < BK / UMMA_K; ++k)  // 32 bytes a step
+            umma(tmem_d + (uint32_t)(k % C::PARTS * NB), w + k * 2, x + k * 2, idesc, kb != 0 || k >= C::PARTS);
           umma_commit(&empty_bar[s]);
         }
         if (++s == C::STAGES) s = 0, phase ^= 1;
@@ -450,7 +478,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&accum_empty[buf])) : "memory");
         for (int h0 = mine; h0 < NB && h0 < rows; h0 += STEP) {
         uint32_t v[WIN];
-        load_accumulator<WIN>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * NB + h0), v);
+        load_accumulator<WIN, C::PARTS>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * C::ACC_COLS + h0), NB, v);
         if (h0 + STEP >= NB || h0 + STEP >= rows) {  // the last window: the accumulator is free again
           tc_fence_before();
           __syncwarp();
@@ -597,7 +625,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       if (threadIdx.x == 32 * C::FIRST_EPI_WARP) STAMP(4);  // the accumulator is complete
       for (int h0 = C::EPI_GROUPS == 1 ? 0 : C::WINDOW * (ew >> 2); h0 < NB && h0 < rows; h0 += C::WINDOW * C::EPI_GROUPS) {
         uint32_t v[C::WINDOW];
-        load_accumulator<C::WINDOW>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)h0, v);
+        load_accumulator<C::WINDOW, C::PARTS>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)h0, NB, v);
 #pragma unroll
         for (int m = 0; m < C::WINDOW; ++m) tile[(h0 + m) * ROWS_W + row] = __uint_as_float(v[m]);
       }
