@@ -1,8 +1,9 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]) (+ residual[M,N]), floats in and out, on the fifth-generation tensor
 // cores: the matrix product of the true 32-bit path.
 //
-// An operand is the sum of three bfloat16 values, x = x1 + x2 + x3 exactly (8 + 8 + 8 bits, each piece the rounded
-// rest of the one before), and of the nine products of pieces the six largest are formed: a1 w1, and a1 w2, a2 w1,
+// An operand times 2^24 is the sum of three bfloat16 values, x1 + x2 + x3 exactly (8 + 8 + 8 bits, each piece the rounded
+// rest of the one before; the lowest bit of any float is 2^-149, so that no piece is smaller than the normal numbers), and
+// of the nine products of pieces the six largest are formed: a1 w1, and a1 w2, a2 w1,
 // a2 w2, a1 w3, a3 w1; what is left out is below 2^-24 of a product.  The a1 w1 of 128 k are summed in tensor
 // memory, then added to 32-bit sums in registers (rounded to nearest, where the tensor cores cut sums off); the five
 // small products, 2^-8 of them, are summed in tensor memory over all of K and added at the end.
@@ -25,10 +26,10 @@
 // alone, the pieces are summed in the same order for every width of a chunk, and so a row has the same bits alone and
 // among others.
 //
-// Where the pieces do not hold, the result says so: an infinity or NaN among the operands, or one too large for a
-// bfloat16, gives NaN (x - x1 = -inf or NaN); sums beyond 2^100 are not trusted, nor are sums below 2^-60, whose small
-// products may have been flushed (operands whose third piece is below 2^-126 lose at most 2^-126 each).  Such a
-// result is formed again as one chain of 32-bit FMAs.
+// Where the pieces do not hold, the result says so: an infinity or NaN among the operands, or one from 2^104 on, whose
+// first piece is no bfloat16, gives NaN (x - x1 = -inf or NaN); sums from 2^76 on are not trusted, being near the end of
+// the range of the scaled ones.  Such a result is formed again as one chain of 32-bit FMAs; so is one below 2^-60, whose
+// bits are then those of gemm_simt.cu down to the subnormal numbers.
 //
 // Launched plainly, and every wait on an mbarrier is bounded; a wait that runs out is recorded in the device error word.
 #include <cooperative_groups.h>
@@ -75,8 +76,14 @@ struct Args {
   int a_wide;  // rows of A are whole 16-byte pieces
 };
 
-// two floats as three pairs of bfloat16 values that add up to them
+// of an operand, of a sum of products (two operands an instruction; without, the product is up to 2.5 % faster and the
+// second and third pieces of operands below 2^-110 lose bits)
+constexpr float SCALE = 0x1p24f, UNSCALE = 0x1p-48f;
+
+// two floats times 2^24 as three pairs of bfloat16 values that add up to them
 __device__ __forceinline__ void cut2(float x, float y, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+  asm("{\n\t.reg .b64 t, s;\n\tmov.b64 t, {%0, %1};\n\tmov.b64 s, {%2, %2};\n\tmul.rn.f32x2 t, t, s;\n\tmov.b64 {%0, %1}, t;\n\t}"
+      : "+f"(x), "+f"(y) : "f"(SCALE));
   p1 = pack2(x, y);
   x -= __uint_as_float(p1 << 16), y -= __uint_as_float(p1 & 0xffff0000u);
   p2 = pack2(x, y);
@@ -108,8 +115,9 @@ __device__ __noinline__ float chain(const float* a, const float* w, int K) {
   return s;
 }
 __device__ __forceinline__ float finish(const Args& g, float v, int m, int n) {
+  v *= UNSCALE;
   const float size = fabsf(v);
-  if (!(size < 0x1p100f) || (size < 0x1p-60f && v != 0.f)) v = chain(g.A + (size_t)m * g.lda, g.W + (size_t)n * g.K, g.K);
+  if (!(size < 0x1p76f) || (size < 0x1p-60f && v != 0.f)) v = chain(g.A + (size_t)m * g.lda, g.W + (size_t)n * g.K, g.K);
   if (g.bias) v += g.bias[n];
   if (g.residual) v += g.residual[(size_t)m * g.ldr + n];
   return v;

@@ -1,0 +1,49 @@
+"""The product of floats whose operands are cut into bfloat16 pieces, at the ends of the range of operands."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+U = 2.0 ** -24
+
+
+def rnd(shape, seed):
+    return torch.randn(shape, generator=torch.Generator().manual_seed(seed)).to(DEV)
+
+
+@pytest.mark.parametrize("M,N", [(3, 300), (40, 9000)])  # K split and not
+@pytest.mark.parametrize("ex,ew", [(-118, 60), (-126, 90), (-138, 100), (60, -118), (90, -126), (-112, 50), (-30, 60), (75, -60)])
+def test_small_operands_against_large_ones(M, N, ex, ew):
+    """No bit of an operand is lost, down to the smallest: pieces of subnormal size would not hold it."""
+    from dispec_b200.ops import gemm
+    K = 512
+    x, w = rnd((M, K), 1) * 2.0 ** ex, rnd((N, K), 2) * 2.0 ** ew
+    out = gemm._split(x, w, None, None, torch.empty((M, N), device=DEV))
+    ref, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    # as in test_split_product_gpu.py, or where a result is formed as one chain, its K sums
+    bound = torch.where(ref.abs() < 2.0 ** -59, 2.0 * K, 4 + 16 + K / 128 + 12) * U * size
+    assert ((out.double() - ref).abs() <= bound).all()
+
+
+def test_rows_of_very_different_sizes():
+    """A row of tiny values among others, a matrix with a huge row: each result as if it were alone."""
+    from dispec_b200.ops import gemm
+    x, w = rnd((24, 1536), 3), rnd((640, 1536), 4)
+    x[5] *= 2.0 ** -115
+    x[7, ::2] *= 2.0 ** -120
+    w[9] *= 2.0 ** 70
+    w[11, 1::2] *= 2.0 ** -130
+    out = gemm._split(x, w, None, None, torch.empty((24, 640), device=DEV))
+    chain = gemm._simt(x, w, None, None, torch.empty((24, 640), device=DEV))
+    ref, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    error = ((out.double() - ref).abs() / size).max()
+    assert error <= (4 + 16 + 12 + 12) * U or error <= ((chain.double() - ref).abs() / size).max()
+
+
+def test_products_that_underflow():
+    """Results near the smallest numbers are those of the chain of FMAs."""
+    from dispec_b200.ops import gemm
+    for e in (-64, -70, -73, -74):
+        x, w = rnd((8, 512), 5).abs() * 2.0 ** e, rnd((256, 512), 6).abs() * 2.0 ** e
+        out, chain = (f(x, w, None, None, torch.empty((8, 256), device=DEV)) for f in (gemm._split, gemm._simt))
+        assert torch.equal(out, chain) and (e < -73 or bool((out != 0).all()))
