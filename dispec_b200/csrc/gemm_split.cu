@@ -108,10 +108,25 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       : "memory");
 }
 
-// One result as one chain of 32-bit FMAs over ascending k.
+// One result as one chain of 32-bit FMAs (K a multiple of 4, w on 16 bytes).  Sixteen operands of each side are on their
+// way at a time, and a chain that is no number any more ends: rows that hold a NaN cost a few loads each.
 __device__ __noinline__ float chain(const float* a, const float* w, int K) {
   float s = 0.f;
-  for (int k = 0; k < K; ++k) s = fmaf(a[k], w[k], s);
+  int k = 0;
+  for (; k + 16 <= K && s == s; k += 16) {
+    float x[16];
+    float4 y[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) y[j] = *reinterpret_cast<const float4*>(w + k + 4 * j);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = a[k + j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      s = fmaf(x[4 * j], y[j].x, s), s = fmaf(x[4 * j + 1], y[j].y, s);
+      s = fmaf(x[4 * j + 2], y[j].z, s), s = fmaf(x[4 * j + 3], y[j].w, s);
+    }
+  }
+  for (; k < K && s == s; ++k) s = fmaf(a[k], w[k], s);
   return s;
 }
 __device__ __forceinline__ float finish(const Args& g, float v, int m, int n) {

@@ -47,3 +47,25 @@ def test_products_that_underflow():
         x, w = rnd((8, 512), 5).abs() * 2.0 ** e, rnd((256, 512), 6).abs() * 2.0 ** e
         out, chain = (f(x, w, None, None, torch.empty((8, 256), device=DEV)) for f in (gemm._split, gemm._simt))
         assert torch.equal(out, chain) and (e < -73 or bool((out != 0).all()))
+
+
+def test_rows_without_numbers_are_not_slow():
+    """A result that is no number is formed again one by one; all of them together take no more than some ten times the
+    product (rows of a step that hold nothing are computed with the others)."""
+    from dispec_b200.ops import gemm
+    x, w = rnd((264, 1536), 7), rnd((4096, 1536), 8)
+    out = torch.empty((264, 4096), device=DEV)
+
+    def ms(a):
+        gemm._split(a, w, None, None, out)
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        gemm._split(a, w, None, None, out)
+        end.record()
+        end.synchronize()
+        return start.elapsed_time(end)
+
+    usual = min(ms(x) for _ in range(5))
+    assert ms(torch.full_like(x, float("nan"))) < 12 * usual and bool(out.isnan().all())
+    x[100, 3] = float("nan")
+    assert ms(x) < 3 * usual and bool(out[100].isnan().all()) and bool(out[99].isfinite().all())
