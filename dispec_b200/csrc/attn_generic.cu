@@ -204,9 +204,9 @@ attn_generic_kernel(const T* __restrict__ q, long q_stride, const T* __restrict_
 //
 // What bounds it: the latencies of a tile, one after the other (a block alone on an SM takes 7 us a tile of 16 rows, 11 of
 // 32, the FMA units 1 and 2).  260 tokens of a prompt beside four single tokens at 330, 12 heads of 128 on 2 KV heads:
-// 55 us; 75 with 128 threads and runs of 32 rows whatever their number (69 with 256 threads, 63 with the longest runs
-// first), 93 before that, 299 with a block per token whose threads each walk a key of their own through global memory.
-constexpr int TILE_KEYS = 64, MAX_DIM = 128, ROW_THREADS = 256;
+// 55 us; 75 with 128 threads and runs of 32 rows (`rows_kernel` has the other sizes), 299 with a block per token whose
+// threads each walk a key of their own through global memory.
+constexpr int TILE_KEYS = 64, MAX_DIM = 128;
 
 struct RowsArgs {
   const void *q, *k_pool, *v_pool;
@@ -237,11 +237,11 @@ __device__ __forceinline__ void end_group() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void wait_groups() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// R rows on a grid of TY x TX threads.
-template <typename T, int R, int TY>
+// R rows on a grid of TY x TX of NT threads.
+template <typename T, int R, int TY, int NT>
 __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0, int n, int pos0, int seq, int kvh,
                                           int g0, int gn) {
-  constexpr int TX = ROW_THREADS / TY, RI = R / TY, KJ = TILE_KEYS / TX, DJ = MAX_DIM / (4 * TX), LP = TILE_KEYS + 4;
+  constexpr int TX = NT / TY, RI = R / TY, KJ = TILE_KEYS / TX, DJ = MAX_DIM / (4 * TX), LP = TILE_KEYS + 4;
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int D = a.D, Dv = a.Dv, LK = D + 4, LV = Dv + 4, G = a.H / a.KVH, rows = n * gn;
   float* qs = smem;                     // [R][LK]
@@ -261,7 +261,7 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
   auto tile_start = [&](int i) { return (i < nfront ? i : first + i - nfront) * TILE_KEYS; };
 
   __syncthreads();  // (a block of several groups of heads: the last one's reads are done)
-  for (int i = tid; i < R * (D / 4); i += ROW_THREADS) {
+  for (int i = tid; i < R * (D / 4); i += NT) {
     const int r = i / (D / 4), d = i % (D / 4) * 4;
     const bool there = r < rows;
     const T* src = (const T*)a.q;
@@ -287,7 +287,7 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
   auto bring = [&](int i, const T* pool, int width, float* to, int ld) {
     if (lane < width / 4) {
 #pragma unroll 2
-      for (int j = warp; j < TILE_KEYS; j += ROW_THREADS / 32) {
+      for (int j = warp; j < TILE_KEYS; j += NT / 32) {
         const long at = slot[(i & 1) * TILE_KEYS + j];
         bring4(to + j * ld + lane * 4, at >= 0 ? pool + at * width + lane * 4 : pool, at >= 0);
       }
@@ -451,7 +451,7 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
   if (a.turn_freq) {
     __syncthreads();
     const int half = Dv / 2;
-    for (int i = tid; i < rows * Dv; i += ROW_THREADS) {
+    for (int i = tid; i < rows * Dv; i += NT) {
       const int r = i / Dv, d = i % Dv, mth = d < half ? d : d - half;
       float sn, cn;
       sincosf((float)(pos0 + r / gn) * a.turn_freq[mth], &sn, &cn);
@@ -464,8 +464,8 @@ __device__ __forceinline__ void attn_rows(const RowsArgs& a, float* smem, int t0
 
 constexpr int FEW_ROWS = 8;
 
-template <typename T, int ROWS>
-__global__ void __launch_bounds__(ROW_THREADS) attn_rows_kernel(const RowsArgs a) {
+template <typename T, int ROWS, int NT>
+__global__ void __launch_bounds__(NT) attn_rows_kernel(const RowsArgs a) {
   extern __shared__ __align__(16) float rows_smem[];
   const int t0 = (int)gridDim.x - 1 - (int)blockIdx.x, kvh = blockIdx.y, pos0 = a.positions[t0];  // the longest first
   if (pos0 < 0) return;
@@ -474,25 +474,47 @@ __global__ void __launch_bounds__(ROW_THREADS) attn_rows_kernel(const RowsArgs a
   int n = 1;
   while (n < per && (pos0 + n) % per && t0 + n < a.T && a.seq_of_token[t0 + n] == seq && a.positions[t0 + n] == pos0 + n) ++n;
   if (n * G <= FEW_ROWS)
-    attn_rows<T, FEW_ROWS, 8>(a, rows_smem, t0, n, pos0, seq, kvh, 0, G);
+    attn_rows<T, FEW_ROWS, NT / 32, NT>(a, rows_smem, t0, n, pos0, seq, kvh, 0, G);
   else
-    for (int g0 = 0; g0 < G; g0 += ROWS) attn_rows<T, ROWS, 16>(a, rows_smem, t0, n, pos0, seq, kvh, g0, min(ROWS, G - g0));
+    for (int g0 = 0; g0 < G; g0 += ROWS) attn_rows<T, ROWS, NT / 16, NT>(a, rows_smem, t0, n, pos0, seq, kvh, g0, min(ROWS, G - g0));
 }
 
-template <typename T, int ROWS>
+template <typename T, int ROWS, int NT>
 int launch_rows(const RowsArgs& a, cudaStream_t stream) {
   const size_t smem = (size_t)((ROWS + TILE_KEYS) * (a.D + 4) + TILE_KEYS * (a.Dv + 4) + ROWS * (TILE_KEYS + 4)) * sizeof(float) +
                       2 * TILE_KEYS * sizeof(long);
-  DSP_CUDA(cudaFuncSetAttribute(attn_rows_kernel<T, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  attn_rows_kernel<T, ROWS><<<dim3(a.T, a.KVH), ROW_THREADS, smem, stream>>>(a);
+  DSP_CUDA(cudaFuncSetAttribute(attn_rows_kernel<T, ROWS, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  attn_rows_kernel<T, ROWS, NT><<<dim3(a.T, a.KVH), NT, smem, stream>>>(a);
   DSP_CHECK_LAUNCH("dsp_attn_generic");
   return 0;
 }
-// Runs of half the tokens where those that fill 32 rows leave SMs idle: a block's time is that of its own tiles.
+// Rows of a run and threads of a block, by the blocks that a step of `singles` single tokens and portions of the other
+// tokens gives; the bits are the same.  A block's time is that of its tiles, one after the other: runs of 16 rows while all
+// their blocks are on the SMs together (two on one), for heads of which a group fills no more; many single tokens of up to
+// 8 rows share the SMs better with 128 threads, and so do many blocks of up to 96 dimensions, of which three fit an SM then.
+// us with 16 rows and 256 threads / 32 and 256 / 32 and 128, behind 600 keys: 12 heads of 128 on 2, 264 tokens 154 / 200 /
+// 211, 400 tokens 263 / 236 / 242; 40 on 2, 128 tokens 267 / 179 / 183; 16 heads of 64 on 8, 800 tokens 370 / 368 / 295; at 600
+// keys each: 64 single tokens of 32 heads of 128 on 8 145 / 143 / 133, one 49 / 48 / 55.
+enum { RUNS_16 = 0, RUNS_32 = 1, RUNS_32_NARROW = 2 };
+int rows_kernel(int T, int singles, int H, int KVH, int D, int Dv, int sms) {
+  const int G = H / KVH;
+  auto blocks = [&](int rows) {
+    const int per = G < rows ? rows / G : 1;
+    return (long)KVH * (singles + (T - singles + per - 1) / per);
+  };
+  const long alone = (long)KVH * singles, runs = blocks(32);
+  if (G <= FEW_ROWS && alone > sms && 2 * alone >= runs) return RUNS_32_NARROW;
+  if (G <= 16 && (singles == T || blocks(16) <= 2l * sms)) return RUNS_16;
+  return runs > 2l * sms && D + Dv <= 192 ? RUNS_32_NARROW : RUNS_32;
+}
 template <typename T>
-int launch_rows(const RowsArgs& a, cudaStream_t stream) {
-  const int G = a.H / a.KVH, per = G < 32 ? 32 / G : 1;
-  return (long)(a.T / per + 1) * a.KVH <= 2 * dsp_num_sms() ? launch_rows<T, 16>(a, stream) : launch_rows<T, 32>(a, stream);
+int launch_rows(const RowsArgs& a, int singles, cudaStream_t stream) {
+  const int sms = dsp_num_sms();
+  switch (rows_kernel(a.T, singles, a.H, a.KVH, a.D, a.Dv, sms > 0 ? sms : 148)) {
+    case RUNS_16: return launch_rows<T, 16, 256>(a, stream);
+    case RUNS_32: return launch_rows<T, 32, 256>(a, stream);
+    default: return launch_rows<T, 32, 128>(a, stream);
+  }
 }
 
 // Whether rows of `width` elements at `stride` from `p` consist of whole pieces of four elements.
@@ -501,10 +523,16 @@ bool whole_pieces(const void* p, long stride, int width, int dtype) {
 }
 }  // namespace
 
+// Which kernel runs (0: runs of 16 rows, 1: of 32, 2: of 32 on 128 threads).
+extern "C" int dsp_attn_rows_choice(int T, int singles, int H, int KVH, int D, int Dv, int sms) {
+  return rows_kernel(T, singles, H, KVH, D, Dv, sms);
+}
+
+// singles: of the T tokens, so many are the only ones of their request (what is known of them decides how the work is cut).
 extern "C" int dsp_attn_generic(const void* q, long q_stride, const void* k_pool,
                                 const void* v_pool, const int* page_table, int pt_stride,
                                 const int* positions, const int* seq_of_token, void* out,
-                                long out_stride, int T, int H, int KVH, int D, int Dv, int page_size,
+                                long out_stride, int T, int singles, int H, int KVH, int D, int Dv, int page_size,
                                 int num_pages, int window, int mask_mode, int keep_first, float scale,
                                 int sink, const float* sink_values, const float* turn_freq, const float* gate, long ldg, int dtype, int out_dtype,
                                 cudaStream_t stream) {
@@ -518,6 +546,7 @@ extern "C" int dsp_attn_generic(const void* q, long q_stride, const void* k_pool
   DSP_REQUIRE(keep_first >= 0, "dsp_attn_generic: keep_first=%d", keep_first);
   DSP_REQUIRE(!gate || !turn_freq, "dsp_attn_generic: results are gated or turned back, not both");
   DSP_REQUIRE(!turn_freq || Dv % 2 == 0, "dsp_attn_generic: values of an odd width %d cannot be turned", Dv);
+  DSP_REQUIRE(singles >= 0 && singles <= T, "dsp_attn_generic: %d single tokens of %d", singles, T);
   int* err = dsp_device_error_ptr();
   DSP_REQUIRE(err != nullptr, "dsp_attn_generic: no device error word");
   if ((dtype == DSP_F32 || dtype == DSP_BF16) && D <= MAX_DIM && Dv <= MAX_DIM && whole_pieces(q, q_stride, D, dtype) &&
@@ -525,7 +554,7 @@ extern "C" int dsp_attn_generic(const void* q, long q_stride, const void* k_pool
     const RowsArgs a = {q, k_pool, v_pool, page_table, positions, seq_of_token, out, sink_values, turn_freq, gate,
                         q_stride, out_stride, ldg, pt_stride, T, H, KVH, D, Dv, page_size, num_pages, window, mask_mode,
                         keep_first, sink, out_dtype, scale, err};
-    return dtype == DSP_F32 ? launch_rows<float>(a, stream) : launch_rows<bf16>(a, stream);
+    return dtype == DSP_F32 ? launch_rows<float>(a, singles, stream) : launch_rows<bf16>(a, singles, stream);
   }
   const size_t smem = (size_t)(GCHUNK * D + GCHUNK * THREADS + (turn_freq ? GCHUNK * Dv : 0)) * sizeof(float) +
                       THREADS * sizeof(long);
