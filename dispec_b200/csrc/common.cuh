@@ -73,6 +73,13 @@ inline bool pdl_enabled() {
   return state == 1;
 }
 
+// The current device, by which what is asked once is remembered (-1: not known, or beyond the tables).
+constexpr int MAX_DEVICES = 64;
+inline int current_device() {
+  int device = -1;
+  return cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < MAX_DEVICES ? device : -1;
+}
+
 // Asks, once per kernel, for the largest shared-memory carveout.  The kernels of a step differ
 // widely in the shared memory they use; with one carveout for all of them the SMs are not
 // reconfigured between consecutive kernels.

@@ -408,12 +408,15 @@ template <typename TOut>
 cudaError_t launch(int clusters, int splits, const CUtensorMap& map_a, const CUtensorMap& map_w, const Args& a, int* err,
                    cudaStream_t stream, int* fit) {
   auto kernel = gemm_pairs_kernel<TOut>;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  static std::atomic<bool> configured[MAX_DEVICES] = {};
+  const int device = current_device();
+  if (device < 0) return cudaErrorInvalidDevice;
+  if (!configured[device].load(std::memory_order_relaxed)) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
-    prefer_max_shared(reinterpret_cast<const void*>(kernel));
-    configured = true;
+    configured[device].store(true, std::memory_order_relaxed);
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(clusters * 2 * splits, 1, 1);
@@ -433,60 +436,70 @@ cudaError_t launch(int clusters, int splits, const CUtensorMap& map_a, const CUt
   return cudaLaunchKernelEx(&cfg, kernel, map_a, map_w, a, err);
 }
 
-// Clusters of `splits` pairs that the device holds at once (0: not known, the message is set).  A cluster stays
-// inside a group of SMs, so fewer large ones fit than there are SMs.
-int max_clusters(int splits) {
-  static std::atomic<int> known[MAX_SPLITS + 1] = {};
-  int n = known[splits].load(std::memory_order_relaxed);
-  if (n > 0) return n;
-  const CUtensorMap none = {};
-  const cudaError_t e = launch<bf16>(1, splits, none, none, Args{}, nullptr, nullptr, &n);
-  if (e != cudaSuccess || n <= 0) {
-    dsp_set_error("dsp_gemm_pairs: how many clusters of %d pairs fit is not known (%s)", splits, cudaGetErrorString(e));
-    cudaGetLastError();
-    return 0;
+// fits[s]: clusters of s pairs that the device holds at once (a cluster stays inside a group of SMs, so fewer large ones fit
+// than there are SMs; 0: none does).  Asked once a device; an answer that does not come is an error of this call (false,
+// with the message set) and nothing that is remembered.
+struct Fits {
+  int of[MAX_SPLITS + 1];
+};
+bool clusters_that_fit(Fits& fits) {
+  static std::atomic<int> known[MAX_DEVICES][MAX_SPLITS + 1] = {};  // one more than the answer, 0: not asked
+  const int device = current_device();
+  for (int splits = 1; splits <= MAX_SPLITS; ++splits) {
+    int n = device < 0 ? 0 : known[device][splits].load(std::memory_order_relaxed) - 1;
+    if (device < 0 || n < 0) {
+      n = 0;
+      const CUtensorMap none = {};
+      const cudaError_t e = launch<bf16>(1, splits, none, none, Args{}, nullptr, nullptr, &n);
+      if (e != cudaSuccess) {
+        dsp_set_error("dsp_gemm_pairs: how many clusters of %d pairs fit is not known (%s)", splits, cudaGetErrorString(e));
+        cudaGetLastError();
+        return false;
+      }
+      known[device][splits].store(n + 1, std::memory_order_relaxed);
+    }
+    fits.of[splits] = n;
   }
-  known[splits].store(n, std::memory_order_relaxed);
-  return n;
+  return true;
 }
 
 struct Plan {
   int cols, chunk_rows, chunks, splits, slots_per_split, clusters;
   double us;  // estimate; negative: none (the message is set where `splits` is 0)
 };
-Plan make_plan(int M, int N, int K, int force_splits, int force_chunks);
+Plan make_plan(int M, int N, int K, const Fits& fits, int force_splits, int force_chunks);
 // The plan of a size, of which the thread's last few are remembered: the layers of a step ask for the same ones.
 Plan plan_of(int M, int N, int K, int splits, int chunks) {
   struct Known {
     int M, N, K, device;
     Plan plan;
   };
-  static thread_local Known known[8] = {};
+  constexpr int KEPT = 32;
+  static thread_local Known known[KEPT] = {};
   static thread_local int next = 0;
-  int device = 0;
-  if (splits != 0 || chunks != 0 || cudaGetDevice(&device) != cudaSuccess) return make_plan(M, N, K, splits, chunks);
-  for (const Known& k : known)
-    if (k.M == M && k.N == N && k.K == K && k.device == device) return k.plan;
-  const Plan p = make_plan(M, N, K, 0, 0);
-  if (p.splits > 0 && p.us >= 0.0) known[next++ & 7] = {M, N, K, device, p};
+  const int device = current_device();
+  const bool chosen = splits == 0 && chunks == 0 && device >= 0;
+  if (chosen)
+    for (const Known& k : known)
+      if (k.M == M && k.N == N && k.K == K && k.device == device) return k.plan;
+  Fits fits;
+  if (!clusters_that_fit(fits)) return Plan{0, 0, 0, 0, 0, 0, -1.0};
+  const Plan p = make_plan(M, N, K, fits, splits, chunks);
+  if (chosen && p.us >= 0.0) known[next++ % KEPT] = {M, N, K, device, p};
   return p;
 }
 // Chunks of rows and splits of K by an estimate in microseconds, fitted on launches that follow one another in a graph
 // and read W from memory: 15 shapes from 2,304 x 768 to 37,888 x 3,584, 72 to 2,048 rows, every split and number of chunks
 // (rms error 5 %).  A ring slot costs more the more columns and the more pairs are busy, a tile its epilogue.
-Plan make_plan(int M, int N, int K, int force_splits, int force_chunks) {
+Plan make_plan(int M, int N, int K, const Fits& fits, int force_splits, int force_chunks) {
   Plan best = {};
   best.us = -1.0, best.splits = 1;
   const int blocks = (N + 2 * ROWS_W - 1) / (2 * ROWS_W), slots = (K + SUB * BK - 1) / (SUB * BK);
-  const int least = (M + MAX_COLS - 1) / MAX_COLS, pairs = max_clusters(1);
+  const int least = (M + MAX_COLS - 1) / MAX_COLS, pairs = fits.of[1];
   const double w_us = 2.0 * N * K / 6.5e6;  // W at the memory's rate
   for (int splits = 1; splits <= MAX_SPLITS; ++splits) {
-    const int fit = max_clusters(splits);
-    if (fit == 0) {
-      best.splits = 0, best.us = -1.0;
-      return best;
-    }
-    if (force_splits > 0 && splits != force_splits) continue;
+    const int fit = fits.of[splits];
+    if (fit <= 0 || (force_splits > 0 && splits != force_splits)) continue;
     if (splits > 1 && slots < 2 * splits) break;
     for (int chunks = least; chunks < least + 3; ++chunks) {
       if (force_chunks > 0 && chunks != force_chunks) continue;
@@ -527,6 +540,17 @@ extern "C" int dsp_gemm_pairs_faster(int M, int N, int K, int target_ctas) {
   const Plan p = plan_of(M, N, K, 0, 0);
   if (p.splits == 0) return -1;
   return p.us > 0.0 && p.us < 0.93 * (few < many ? few : many);
+}
+
+// The plan of a size where fits[0..3] clusters of one to four pairs fit: pairs that share a tile, chunks of rows, clusters
+// launched (1: there is none).
+extern "C" int dsp_gemm_pairs_plan(int M, int N, int K, const int* fits, int* plan) {
+  Fits f = {};
+  for (int s = 1; s <= MAX_SPLITS; ++s) f.of[s] = fits[s - 1];
+  const Plan p = make_plan(M, N, K, f, 0, 0);
+  if (p.us < 0.0) return 1;
+  plan[0] = p.splits, plan[1] = p.chunks, plan[2] = p.clusters;
+  return 0;
 }
 
 // Operands as dsp_gemm_tcgen05 takes them; N, ldc and ldr multiples of 4, C and residual on 16 bytes (bfloat16: 8),

@@ -10,3 +10,32 @@ def test_an_answer_that_does_not_come_is_an_error_each_time():
     for _ in range(2):
         with pytest.raises(library.KernelError, match="how many clusters"):
             tuning._few_rows_faster(300, 1536, 8960, 148)
+
+
+def pairs_plan(M, N, K, fits):
+    import ctypes
+    from dispec_b200.ops import library
+    plan = (ctypes.c_int * 3)()
+    rc = library.core().dsp_gemm_pairs_plan(M, N, K, (ctypes.c_int * 4)(*fits), plan)
+    return None if rc else tuple(plan)
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 1536, 8960), (137, 512, 4096), (536, 1536, 1536)])
+def test_pairs_of_a_device_that_holds_fewer_clusters(M, N, K):
+    """A cluster size of which the device holds none is not planned with, and hides none of the others."""
+    splits, _, clusters = pairs_plan(M, N, K, [74, 36, 22, 16])
+    assert splits > 1
+    for held in range(1, 4):
+        fits = [74, 36, 22, 16][:held] + [0] * (4 - held)
+        splits, chunks, clusters = pairs_plan(M, N, K, fits)
+        assert 1 <= splits <= held and 0 < clusters <= fits[splits - 1] and chunks >= -(-M // 256)
+    assert pairs_plan(M, N, K, [0, 0, 0, 0]) is None
+    assert pairs_plan(M, N, K, [0, 36, 0, 0])[0] == 2
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the question has an answer here")
+def test_a_cluster_query_that_fails_is_an_error():
+    import ctypes
+    from dispec_b200.ops import library
+    with pytest.raises(library.KernelError, match="how many clusters"):
+        library.check(library.core().dsp_gemm_pairs_faster(300, 1536, 8960, 148))
