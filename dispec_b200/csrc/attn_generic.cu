@@ -488,29 +488,32 @@ int launch_rows(const RowsArgs& a, cudaStream_t stream) {
   DSP_CHECK_LAUNCH("dsp_attn_generic");
   return 0;
 }
-// Rows of a run and threads of a block, by the blocks that a step of `singles` single tokens and portions of the other
-// tokens gives; the bits are the same.  A block's time is that of its tiles, one after the other: runs of 16 rows while all
-// their blocks are on the SMs together (two on one), for heads of which a group fills no more; many single tokens of up to
-// 8 rows share the SMs better with 128 threads, and so do many blocks of up to 96 dimensions, of which three fit an SM then.
-// us with 16 rows and 256 threads / 32 and 256 / 32 and 128, behind 600 keys: 12 heads of 128 on 2, 264 tokens 154 / 200 /
-// 211, 400 tokens 263 / 236 / 242; 40 on 2, 128 tokens 267 / 179 / 183; 16 heads of 64 on 8, 800 tokens 370 / 368 / 295; at 600
-// keys each: 64 single tokens of 32 heads of 128 on 8 145 / 143 / 133, one 49 / 48 / 55.
+// Rows of a run and threads of a block, by the blocks that a step gives: `singles` single tokens, portions of the other
+// tokens, `longest` the tokens of its longest context (0: not known).  The bits are the same.  A block's time is that of its
+// tiles, one after the other, and a portion that begins a prompt has half as many as its last block has: runs of 16 rows
+// while the step takes no longer than its longest block (two of them on an SM), for heads of which a group fills no more;
+// many single tokens of up to 8 rows share the SMs better with 128 threads, and so do many blocks of up to 96 dimensions,
+// of which three fit an SM then.  us with 16 rows and 256 threads / 32 and 256 / 32 and 128: 12 heads of 128 on 2, 264 tokens
+// behind 600 keys 154 / 200 / 211, 400 behind 600 263 / 236 / 242, 500 alone 95 / 120 / 126; 40 on 2, 128 behind 600 267 / 179 /
+// 183; 16 heads of 64 on 8, 800 behind 600 370 / 368 / 295; single tokens at 600 keys, 32 heads of 128 on 8, 64 of them 145 /
+// 143 / 133, one 49 / 48 / 55.
 enum { RUNS_16 = 0, RUNS_32 = 1, RUNS_32_NARROW = 2 };
-int rows_kernel(int T, int singles, int H, int KVH, int D, int Dv, int sms) {
-  const int G = H / KVH;
+int rows_kernel(int T, int singles, int longest, int H, int KVH, int D, int Dv, int sms) {
+  const int G = H / KVH, rest = T - singles;
+  const double share = longest > 0 ? 1.0 - 0.5 * (rest < longest ? rest : longest) / longest : 1.0;  // of a portion's block
   auto blocks = [&](int rows) {
     const int per = G < rows ? rows / G : 1;
-    return (long)KVH * (singles + (T - singles + per - 1) / per);
+    return KVH * (singles + share * ((rest + per - 1) / per));
   };
-  const long alone = (long)KVH * singles, runs = blocks(32);
-  if (G <= FEW_ROWS && alone > sms && 2 * alone >= runs) return RUNS_32_NARROW;
-  if (G <= 16 && (singles == T || blocks(16) <= 2l * sms)) return RUNS_16;
-  return runs > 2l * sms && D + Dv <= 192 ? RUNS_32_NARROW : RUNS_32;
+  const double alone = (double)KVH * singles, runs = blocks(32);
+  if (G <= FEW_ROWS && alone > sms && 2.0 * alone >= runs) return RUNS_32_NARROW;
+  if (G <= 16 && (rest == 0 || blocks(16) <= 2.0 * sms)) return RUNS_16;
+  return runs > 1.9 * sms && D + Dv <= 192 ? RUNS_32_NARROW : RUNS_32;
 }
 template <typename T>
-int launch_rows(const RowsArgs& a, int singles, cudaStream_t stream) {
+int launch_rows(const RowsArgs& a, int singles, int longest, cudaStream_t stream) {
   const int sms = dsp_num_sms();
-  switch (rows_kernel(a.T, singles, a.H, a.KVH, a.D, a.Dv, sms > 0 ? sms : 148)) {
+  switch (rows_kernel(a.T, singles, longest, a.H, a.KVH, a.D, a.Dv, sms > 0 ? sms : 148)) {
     case RUNS_16: return launch_rows<T, 16, 256>(a, stream);
     case RUNS_32: return launch_rows<T, 32, 256>(a, stream);
     default: return launch_rows<T, 32, 128>(a, stream);
@@ -524,15 +527,16 @@ bool whole_pieces(const void* p, long stride, int width, int dtype) {
 }  // namespace
 
 // Which kernel runs (0: runs of 16 rows, 1: of 32, 2: of 32 on 128 threads).
-extern "C" int dsp_attn_rows_choice(int T, int singles, int H, int KVH, int D, int Dv, int sms) {
-  return rows_kernel(T, singles, H, KVH, D, Dv, sms);
+extern "C" int dsp_attn_rows_choice(int T, int singles, int longest, int H, int KVH, int D, int Dv, int sms) {
+  return rows_kernel(T, singles, longest, H, KVH, D, Dv, sms);
 }
 
-// singles: of the T tokens, so many are the only ones of their request (what is known of them decides how the work is cut).
+// singles: of the T tokens, so many are the only ones of their request; longest: tokens of the longest context (0: not
+// known).  They decide how the work is cut.
 extern "C" int dsp_attn_generic(const void* q, long q_stride, const void* k_pool,
                                 const void* v_pool, const int* page_table, int pt_stride,
                                 const int* positions, const int* seq_of_token, void* out,
-                                long out_stride, int T, int singles, int H, int KVH, int D, int Dv, int page_size,
+                                long out_stride, int T, int singles, int longest, int H, int KVH, int D, int Dv, int page_size,
                                 int num_pages, int window, int mask_mode, int keep_first, float scale,
                                 int sink, const float* sink_values, const float* turn_freq, const float* gate, long ldg, int dtype, int out_dtype,
                                 cudaStream_t stream) {
@@ -554,7 +558,7 @@ extern "C" int dsp_attn_generic(const void* q, long q_stride, const void* k_pool
     const RowsArgs a = {q, k_pool, v_pool, page_table, positions, seq_of_token, out, sink_values, turn_freq, gate,
                         q_stride, out_stride, ldg, pt_stride, T, H, KVH, D, Dv, page_size, num_pages, window, mask_mode,
                         keep_first, sink, out_dtype, scale, err};
-    return dtype == DSP_F32 ? launch_rows<float>(a, singles, stream) : launch_rows<bf16>(a, singles, stream);
+    return dtype == DSP_F32 ? launch_rows<float>(a, singles, longest, stream) : launch_rows<bf16>(a, singles, longest, stream);
   }
   const size_t smem = (size_t)(GCHUNK * D + GCHUNK * THREADS + (turn_freq ? GCHUNK * Dv : 0)) * sizeof(float) +
                       THREADS * sizeof(long);

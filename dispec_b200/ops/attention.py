@@ -38,7 +38,7 @@ def paged_attention_generic(q: torch.Tensor, q_stride: int, k_pool: torch.Tensor
                             num_kv_heads: int, head_dim: int, window: int, scale: float,
                             sink: bool = False, chunked: bool = False, sink_values: torch.Tensor | None = None,
                             turn_freq: torch.Tensor | None = None, keep_first: int = 0,
-                            gate: torch.Tensor | None = None, num_single: int = 0) -> torch.Tensor:
+                            gate: torch.Tensor | None = None, num_single: int = 0, max_keys: int = 0) -> torch.Tensor:
     """32-bit arithmetic kernel, any value size up to 512 and any group size.
 
     q: element (t, h, d) at q.data_ptr + (t * q_stride + h * D + d); out: [T, H * Dv], Dv being the
@@ -51,7 +51,8 @@ def paged_attention_generic(q: torch.Tensor, q_stride: int, k_pool: torch.Tensor
     [H]) that key's score is the head's own number, unscaled.  ``turn_freq`` (float32 [Dv/2]):
     every head's result is turned back, pair (m, m + Dv/2) by -p * turn_freq[m].  ``gate`` (float32, shaped like
     ``out``): every result is multiplied by the sigmoid of its gate value.  ``num_single``: tokens that are the only ones of
-    their request, as far as the host knows (it decides how the work is cut, no bits).
+    their request, ``max_keys``: the longest context of the step, as far as the host knows (they decide how the work is
+    cut, no bits).
     """
     assert q.is_cuda and k_pool.is_cuda, "CUDA tensors only (there is no CPU path)"
     T = positions.shape[0]
@@ -67,7 +68,7 @@ def paged_attention_generic(q: torch.Tensor, q_stride: int, k_pool: torch.Tensor
     L.check(L.core().dsp_attn_generic(
         L.ptr(q), L.i64(q_stride), L.ptr(k_pool), L.ptr(v_pool), L.ptr(page_table),
         page_table.stride(0), L.ptr(positions), L.ptr(seq_of_token), L.ptr(out),
-        L.i64(out.stride(0)), T, num_single, num_heads, num_kv_heads, head_dim, dv, page_size, num_pages,
+        L.i64(out.stride(0)), T, num_single, max_keys, num_heads, num_kv_heads, head_dim, dv, page_size, num_pages,
         window, int(bool(chunked) and window > 0), int(keep_first), L.f32(scale), int(bool(sink)), L.ptr(sink_values),
         L.ptr(turn_freq), L.ptr(gate), L.i64(gate.stride(0) if gate is not None else 0), L.dtype_code(q.dtype),
         L.dtype_code(out.dtype), L.stream_handle()))
@@ -316,7 +317,7 @@ def paged_attention(ctx, q: torch.Tensor, q_stride: int, cache, out: torch.Tenso
         raise L.KernelError("single tokens were left unrotated for a kernel that is not in use")
     return paged_attention_generic(q, q_stride, cache.key_pool, cache.value_pool, cache.page_table,
                                    ctx.positions, ctx.seq_of_token, out, num_heads, num_kv_heads,
-                                   head_dim, window, scale, num_single=ctx.num_decode_seqs)
+                                   head_dim, window, scale, num_single=ctx.num_decode_seqs, max_keys=ctx.max_ctx_len)
 
 
 def qkv_rotate_store(qkv: torch.Tensor, positions: torch.Tensor, seq_of_token: torch.Tensor, cache,
@@ -487,4 +488,4 @@ def sink_paged_attention(ctx, q: torch.Tensor, cache, out: torch.Tensor, num_hea
                                    ctx.positions, ctx.seq_of_token, out, num_heads, num_kv_heads, key_dim,
                                    window, scale, sink=sink, chunked=chunked, sink_values=sink_values,
                                    turn_freq=turn_freq, keep_first=keep_first, gate=gate,
-                                   num_single=ctx.num_decode_seqs)
+                                   num_single=ctx.num_decode_seqs, max_keys=ctx.max_ctx_len)

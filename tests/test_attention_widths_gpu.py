@@ -24,7 +24,7 @@ def test_requests_of_one_token_and_portions(H, KVH, D, kernels):
 
     def run(lo, hi, num_single):
         out = torch.full((hi - lo, H * D), float("nan"), device=DEV)
-        used.add(L.core().dsp_attn_rows_choice(hi - lo, num_single, H, KVH, D, D, 148))
+        used.add(L.core().dsp_attn_rows_choice(hi - lo, num_single, 0, H, KVH, D, D, 148))
         return A.paged_attention_generic(q[lo:hi], H * D, kp, vp, table, positions[lo:hi], request[lo:hi], out, H, KVH, D, 0,
                                          D ** -0.5, num_single=num_single)
 
