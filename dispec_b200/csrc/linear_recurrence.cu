@@ -32,17 +32,18 @@
 // prompt leaves an SM one block: eight warps hide one another's latencies), the groups' results meet in
 // shared memory and leave one round later.  Single tokens: transformed as they are staged, in one kernel,
 // the lanes of a warp cover all the rows.
-// Longer steps are cut into segments of 64 tokens or more that run side by side, the first of a request from its state and the
-// others from zero.  What a state in front of a segment adds is linear in it:
+// A long request is cut into segments of 64 tokens or more that run side by side, the first from its state and the others
+// from zero.  What a state in front of a segment adds is linear in it:
 //     o_t += (S_in)^T (P_t q_t),   S_out = A S_in + S_local,   P_t the product of the segment's a up to t, A the last of them
 // so a scan over a request's segments gives every S_in, and a product of P_t q_t (which the segments' first blocks write
 // down as they go) with S_in completes the outputs.  In a segment a warp covers all state rows of eight columns and adds
-// within itself.  2,500 tokens of two requests, 12 heads of 128 x 128: 297 us (FORGET_GATE) and 252 (FIXED_DECAY) walked
-// in one piece by 192 blocks of which an SM held one or two; segments 118, scan 16, product 39 (all four blocks of an SM
-// busy, the FMA pipe two fifths).
+// within itself.  Whether a request is cut, and into what, depends on its own tokens of the step and on the sizes of its
+// heads alone (ops/recurrence.py has the rule and what it measured): its bits are the same alone and among others.
 // State rows beyond 256 take a kernel of their own with one column a thread.  A request whose first row
 // carries a negative position (a padding row of a captured step) is skipped: its state slot belongs to
 // someone else.
+#include <limits.h>
+
 #include <type_traits>
 
 #include "common.cuh"
@@ -83,29 +84,40 @@ struct RecurrenceArgs {
   int slices;            // threads per column (a power of two, at most 32)
   int cols_per_block;    // threads / slices
   int tokens_per_round;
-  // segments of seg_len tokens (null and 0 without): number q_start[s] / seg_len + s + j is the j-th of request s
-  float* seg_state;  // [segments, H, dim, vdim]: the state behind it, later the one in front of it
-  float* seg_decay;  // [segments, H, dim]: the product of its decays
-  float* seg_q;      // [T, H * dim]: P_t q_t
-  int S, seg_len;
+  // Requests of seg_min tokens and more (a multiple of SEGMENT; INT_MAX: none) are cut into at most seg_max segments.
+  // `heads` heads from head0 on are in the workspace together.
+  float* seg_state;  // [segments, heads, dim, vdim]: the state behind it, later the one in front of it
+  float* seg_decay;  // [segments, heads, dim]: the product of its decays
+  float* seg_q;      // [T, heads * dim]: P_t q_t
+  int S, seg_min, seg_max, head0, heads;
 };
+
+constexpr int SEGMENT = 64;
+// The length of the segments of a request of n tokens.
+__host__ __device__ inline int segment_length(int n, int most) {
+  int len = SEGMENT;
+  while (n > (long)len * most) len *= 2;
+  return len;
+}
+// The number of the first segment of a request whose first row is `row`: with r = seg_min / SEGMENT, row (r + 1) / seg_min.
+// A request of n >= seg_min tokens has ceil(n / SEGMENT) segments or fewer, no more than n (r + 1) / seg_min rounded down, so
+// that numbers do not meet; requests that are not cut take none.
+__host__ __device__ inline long first_segment(long row, int seg_min) { return row * (seg_min / SEGMENT + 1) / seg_min; }
 
 struct Segment {
   int seq, index, t0, t1;
-  bool only;  // the request has no other
 };
 // Segment `number`; false where there is none.
 __device__ __forceinline__ bool find_segment(const RecurrenceArgs& p, int number, Segment& g) {
   int lo = 0, hi = p.S;  // the last request whose first segment is not beyond `number`
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (p.q_start[mid] / p.seg_len + mid <= number) lo = mid; else hi = mid;
+    if (first_segment(p.q_start[mid], p.seg_min) <= number) lo = mid; else hi = mid;
   }
-  const int a = p.q_start[lo], b = p.q_start[lo + 1];
-  g.seq = lo, g.index = number - (a / p.seg_len + lo);
-  g.t0 = a + g.index * p.seg_len, g.t1 = min(b, g.t0 + p.seg_len);
-  g.only = b - a <= p.seg_len;
-  return g.index >= 0 && g.t0 < b && p.positions[a] >= 0;
+  const int a = p.q_start[lo], b = p.q_start[lo + 1], len = segment_length(b - a, p.seg_max);
+  g.seq = lo, g.index = number - (int)first_segment(a, p.seg_min);
+  g.t0 = a + g.index * len, g.t1 = min(b, g.t0 + len);
+  return b - a >= p.seg_min && g.index >= 0 && g.t0 < b && p.positions[a] >= 0;
 }
 
 // sigmoid(z)^power by way of ln sigmoid(z) = -(ln(1 + e^-|z|) + max(-z, 0))
@@ -453,16 +465,16 @@ recurrence_tile_kernel(const RecurrenceArgs p) {
   constexpr bool gate = L::gate, per_token = L::per_token;
   constexpr int DP = L::rows, C = L::cols, R = L::round, planes = L::planes;
   extern __shared__ __align__(16) float tile_smem[];
-  const int head = blockIdx.y;
+  const int head = (SEGMENTS ? p.head0 : 0) + blockIdx.y;
   int seq = blockIdx.z, t0, t1;
-  bool fresh = false, onward = false;  // it begins with a state of zeros; more segments follow or came before
+  bool fresh = false;  // it begins with a state of zeros
   if constexpr (SEGMENTS) {
     Segment g;
     if (!find_segment(p, blockIdx.z, g)) return;
-    seq = g.seq, t0 = g.t0, t1 = g.t1, fresh = g.index > 0, onward = !g.only;
+    seq = g.seq, t0 = g.t0, t1 = g.t1, fresh = g.index > 0;
   } else {
     t0 = p.q_start[seq], t1 = p.q_start[seq + 1];
-    if (t1 <= t0 || p.positions[t0] < 0) return;
+    if (t1 <= t0 || t1 - t0 >= p.seg_min || p.positions[t0] < 0) return;
   }
   const int tid = threadIdx.x, lane = tid & 31, slice = lane % SLICES;
   constexpr int TILE_THREADS = 32 * WARPS, PART_WARPS = WARPS / PARTS;
@@ -635,7 +647,7 @@ recurrence_tile_kernel(const RecurrenceArgs p) {
                 float x, y;
                 unpack2f(mul2(product[e], qe), x, y);
                 const int i = row_of(e);
-                float* dst = p.seg_q + (size_t)(base + r) * hd + (size_t)head * p.dim + i;
+                float* dst = p.seg_q + ((size_t)(base + r) * p.heads + blockIdx.y) * p.dim + i;
                 if (i < p.dim) dst[0] = x;
                 if (i + 1 < p.dim) dst[1] = y;
               }
@@ -757,7 +769,7 @@ recurrence_tile_kernel(const RecurrenceArgs p) {
   }
   if constexpr (SEGMENTS) {
     if (notes) {
-      float* dst = p.seg_decay + ((size_t)blockIdx.z * p.H + head) * p.dim;
+      float* dst = p.seg_decay + ((size_t)blockIdx.z * p.heads + blockIdx.y) * p.dim;
 #pragma unroll
       for (int k = 0; k < PAIRS; ++k) {
         float x, y;
@@ -767,7 +779,7 @@ recurrence_tile_kernel(const RecurrenceArgs p) {
         if (i + 1 < p.dim) dst[i + 1] = y;
       }
     }
-    if (onward) sp = p.seg_state + ((size_t)blockIdx.z * p.H + head) * p.dim * p.vdim;
+    sp = p.seg_state + ((size_t)blockIdx.z * p.heads + blockIdx.y) * p.dim * p.vdim;
   }
 #pragma unroll
   for (int k = 0; k < PAIRS; ++k) {
@@ -793,13 +805,14 @@ recurrence_tile_kernel(const RecurrenceArgs p) {
 // The states in front of a request's segments (in place of those behind them) and the request's own state.  A thread
 // an element; the next segment's is on its way while one is added.
 __global__ void __launch_bounds__(256) segment_scan_kernel(const RecurrenceArgs p) {
-  const int seq = blockIdx.z, head = blockIdx.y, e = blockIdx.x * 256 + threadIdx.x;
+  const int seq = blockIdx.z, h = blockIdx.y, e = blockIdx.x * 256 + threadIdx.x;
   const int a = p.q_start[seq], n = p.q_start[seq + 1] - a, size = p.dim * p.vdim;
-  if (n <= p.seg_len || p.positions[a] < 0 || e >= size) return;
-  const int first = a / p.seg_len + seq, count = (n + p.seg_len - 1) / p.seg_len, row = e / p.vdim;
-  const size_t step = (size_t)p.H * size, dstep = (size_t)p.H * p.dim;
-  float* at = p.seg_state + ((size_t)first * p.H + head) * size + e;
-  const float* decay = p.seg_decay + ((size_t)first * p.H + head) * p.dim + row;
+  if (n < p.seg_min || p.positions[a] < 0 || e >= size) return;
+  const int len = segment_length(n, p.seg_max), count = (n + len - 1) / len, row = e / p.vdim;
+  const size_t first = (size_t)first_segment(a, p.seg_min) * p.heads + h;
+  const size_t step = (size_t)p.heads * size, dstep = (size_t)p.heads * p.dim;
+  float* at = p.seg_state + first * size + e;
+  const float* decay = p.seg_decay + first * p.dim + row;
   float running = *at, next = at[step], d = decay[dstep];
   for (int j = 1; j < count; ++j) {
     at += step, decay += dstep;
@@ -808,7 +821,7 @@ __global__ void __launch_bounds__(256) segment_scan_kernel(const RecurrenceArgs 
     *at = running;
     running = fmaf(mine, running, local);
   }
-  p.state[((size_t)p.state_slot[seq] * p.H + head) * size + e] = running;
+  p.state[((size_t)p.state_slot[seq] * p.H + p.head0 + h) * size + e] = running;
 }
 
 // o_t += S_in^T (P_t q_t) for a segment's tokens and 128 columns of a head: 256 threads of 8 x 4 outputs, 64 tokens and
@@ -818,10 +831,10 @@ __global__ void __launch_bounds__(256, 2) segment_carry_kernel(const RecurrenceA
   __shared__ __align__(16) float qs[CARRY_TOKENS][SLAB + 4], ss[SLAB][CARRY_COLS];
   Segment g;
   if (!find_segment(p, blockIdx.z, g) || g.index == 0) return;
-  const int head = blockIdx.y, col0 = blockIdx.x * CARRY_COLS, tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-  const int hd = p.H * p.dim;
+  const int head = p.head0 + blockIdx.y, col0 = blockIdx.x * CARRY_COLS, tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+  const int hd = p.heads * p.dim;  // of a row of P_t q_t
   const bool wide = p.dim % 4 == 0 && p.vdim % 4 == 0 && p.ldo % 4 == 0 && ((uintptr_t)p.out & 15) == 0;
-  const float* state = p.seg_state + ((size_t)blockIdx.z * p.H + head) * p.dim * p.vdim;
+  const float* state = p.seg_state + ((size_t)blockIdx.z * p.heads + blockIdx.y) * p.dim * p.vdim;
   auto load4 = [&](const float* src, int there) {  // the first `there` of four floats, zeros behind them
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (wide) {
@@ -837,7 +850,7 @@ __global__ void __launch_bounds__(256, 2) segment_carry_kernel(const RecurrenceA
   constexpr int QN = CARRY_TOKENS * SLAB / 1024, SN = SLAB * CARRY_COLS / 1024;  // fours a thread fetches of a slab
   for (int t0 = g.t0; t0 < g.t1; t0 += CARRY_TOKENS) {
     const int n = min(CARRY_TOKENS, g.t1 - t0);
-    const float* q = p.seg_q + (size_t)t0 * hd + (size_t)head * p.dim;
+    const float* q = p.seg_q + (size_t)t0 * hd + (size_t)blockIdx.y * p.dim;
     float4 q_next[QN], s_next[SN];
     auto fetch = [&](int k0) {
 #pragma unroll
@@ -909,13 +922,19 @@ int launch_tile_kind(const RecurrenceArgs& a, int S, int segments, cudaStream_t 
     DSP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem));
     configured = true;
   }
-  const dim3 grid((a.vdim + L::cols - 1) / L::cols, a.H, SEGMENTS ? segments : S);
-  kernel<<<grid, 32 * WARPS, L::smem, stream>>>(a);
-  DSP_CHECK_LAUNCH("dsp_linear_recurrence");
+  const int across = (a.vdim + L::cols - 1) / L::cols;
   if constexpr (SEGMENTS) {
-    segment_scan_kernel<<<dim3((a.dim * a.vdim + 255) / 256, a.H, S), 256, 0, stream>>>(a);
-    segment_carry_kernel<<<dim3((a.vdim + CARRY_COLS - 1) / CARRY_COLS, a.H, segments), 256, 0, stream>>>(a);
-    DSP_CHECK_LAUNCH("dsp_linear_recurrence (segments)");
+    RecurrenceArgs g = a;
+    for (g.head0 = 0; g.head0 < a.H; g.head0 += a.heads) {  // as many heads as the workspace holds
+      const int n = a.heads < a.H - g.head0 ? a.heads : a.H - g.head0;
+      kernel<<<dim3(across, n, segments), 32 * WARPS, L::smem, stream>>>(g);
+      segment_scan_kernel<<<dim3((a.dim * a.vdim + 255) / 256, n, S), 256, 0, stream>>>(g);
+      segment_carry_kernel<<<dim3((a.vdim + CARRY_COLS - 1) / CARRY_COLS, n, segments), 256, 0, stream>>>(g);
+      DSP_CHECK_LAUNCH("dsp_linear_recurrence (segments)");
+    }
+  } else {
+    kernel<<<dim3(across, a.H, S), 32 * WARPS, L::smem, stream>>>(a);
+    DSP_CHECK_LAUNCH("dsp_linear_recurrence");
   }
   return 0;
 }
@@ -948,10 +967,16 @@ int launch(const RecurrenceArgs& a, int S, size_t smem, cudaStream_t stream) {
 }
 }  // namespace
 
+// Floats of the workspace for the segments of `heads` heads of a step of T tokens.
+extern "C" long dsp_linear_recurrence_segment_floats(int T, int heads, int dim, int vdim, int segment_min) {
+  return (first_segment(T, segment_min) + 1) * heads * dim * (vdim + 1) + (long)T * heads * dim;
+}
+
 // scratch: null (one kernel, tokens transformed as they are staged) or room for [T, planes, H * dim]
 // floats, planes = 2 with one decay for all rows, else 3 (a first kernel transforms every token, the
-// recurrence streams); STEP_DECAY takes none.  segment_scratch: null, or room for the segments of at most 256 state
-// rows, `segment` tokens each: (T / segment + S) * H * dim * (vdim + 1) + T * H * dim floats.
+// recurrence streams); STEP_DECAY takes none.  segment_scratch: null, or room for the segments of `segment_heads` heads (at
+// most 128 state rows) at a time, dsp_linear_recurrence_segment_floats.  Requests of segment_min tokens and more are then cut
+// into at most max_segments; all_long: there is no other.
 extern "C" int dsp_linear_recurrence(const void* proj, int proj_dtype, long ld, int q_off, int k_off,
                                      int v_off, int mode, int H, int dim, int vdim, const float* decay,
                                      const float* inv_freq, int rot, float key_scale, int act,
@@ -959,8 +984,8 @@ extern "C" int dsp_linear_recurrence(const void* proj, int proj_dtype, long ld, 
                                      const float* gate_map, int low_off, int rank, float q_scale, float power,
                                      const float* steps, const float* skip, int heads_per_group, float* state,
                                      const int* state_slot, const int* q_start, const int* positions,
-                                     float* out, long ldo, int S, int T, float* scratch, float* segment_scratch, int segment,
-                                     cudaStream_t stream) {
+                                     float* out, long ldo, int S, int T, float* scratch, float* segment_scratch,
+                                     int segment_heads, int segment_min, int max_segments, int all_long, cudaStream_t stream) {
   if (S == 0 || T == 0) return 0;
   DSP_REQUIRE(proj && state && state_slot && q_start && positions && out, "dsp_linear_recurrence: missing operand");
   DSP_REQUIRE(H > 0 && H <= 65535 && S <= 65535, "dsp_linear_recurrence: H=%d, S=%d outside the grid", H, S);
@@ -989,12 +1014,20 @@ extern "C" int dsp_linear_recurrence(const void* proj, int proj_dtype, long ld, 
   a.steps = steps; a.skip = skip; a.heads_per_group = mode == STEP_DECAY ? heads_per_group : 1;
   a.state = state; a.state_slot = state_slot; a.q_start = q_start; a.positions = positions;
   a.out = out; a.ldo = ldo; a.ready = scratch;
-  DSP_REQUIRE(!segment_scratch || segment > 0, "dsp_linear_recurrence: segments of %d tokens", segment);
-  a.S = S; a.seg_len = segment;
-  const int segments = segment_scratch ? T / segment + S : 0;  // as many numbers as segments may have
-  a.seg_state = segment_scratch;
-  a.seg_decay = a.seg_state ? a.seg_state + (size_t)segments * H * dim * vdim : nullptr;
-  a.seg_q = a.seg_state ? a.seg_decay + (size_t)segments * H * dim : nullptr;
+  a.S = S; a.head0 = 0;
+  a.seg_min = INT_MAX; a.seg_max = max_segments; a.heads = segment_heads;
+  a.seg_state = a.seg_decay = a.seg_q = nullptr;
+  long segments = 0;  // as many numbers as segments may have
+  if (segment_scratch) {
+    DSP_REQUIRE(segment_heads > 0 && segment_min >= 2 * SEGMENT && segment_min % SEGMENT == 0 && max_segments > 1,
+                "dsp_linear_recurrence: %d segments at most of requests from %d tokens on, %d heads at a time", max_segments, segment_min, segment_heads);
+    segments = first_segment(T, segment_min) + 1;
+    DSP_REQUIRE(segments <= 65535, "dsp_linear_recurrence: %ld segments", segments);
+    a.seg_min = segment_min;
+    a.seg_state = segment_scratch;
+    a.seg_decay = a.seg_state + (size_t)segments * segment_heads * dim * vdim;
+    a.seg_q = a.seg_decay + (size_t)segments * segment_heads * dim;
+  }
   // one column a thread, 32 threads a column, 16 or 32 state rows a thread (beyond 256 state rows)
   const bool tiled = dim <= 256;
   const int slices = 32, rows = (dim + slices - 1) / slices;
@@ -1020,12 +1053,12 @@ extern "C" int dsp_linear_recurrence(const void* proj, int proj_dtype, long ld, 
     DSP_CHECK_LAUNCH("dsp_linear_recurrence (first kernel)");
   }
   if (segment_scratch) {
-    DSP_REQUIRE(tiled && (scratch || mode == STEP_DECAY), "dsp_linear_recurrence: segments of tokens that are not prepared, or of %d state rows", dim);
-    DSP_REQUIRE(segments <= 65535, "dsp_linear_recurrence: %d segments", segments);
-    if (dim <= 32) return launch_tile<8, 2, 1, 4, true, true>(a, S, stream, segments);
-    if (dim <= 64) return launch_tile<16, 2, 1, 4, true, true>(a, S, stream, segments);
-    if (dim <= 128) return launch_tile<16, 4, 1, 4, true, true>(a, S, stream, segments);
-    return launch_tile<32, 4, 1, 4, true, true>(a, S, stream, segments);
+    DSP_REQUIRE(dim <= 128 && (scratch || mode == STEP_DECAY), "dsp_linear_recurrence: segments of tokens that are not prepared, or of %d state rows", dim);
+    const int n = (int)segments;
+    const int rc = dim <= 32   ? launch_tile<8, 2, 1, 4, true, true>(a, S, stream, n)
+                   : dim <= 64 ? launch_tile<16, 2, 1, 4, true, true>(a, S, stream, n)
+                               : launch_tile<16, 4, 1, 4, true, true>(a, S, stream, n);
+    if (rc != 0 || all_long) return rc;
   }
   if (scratch || (mode == STEP_DECAY && T > 2 * S)) {  // portions of prompts
     if (dim <= 32) return launch_tile<8, 1, 2, 8, true>(a, S, stream);

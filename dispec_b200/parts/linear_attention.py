@@ -89,8 +89,8 @@ class Retention(_MatrixStateMixer):
             raise ValueError(f"retention turns pairs (i, i + rot/2) only, not the {rot.layout!r} layout")
         o = rec_ops.linear_recurrence(
             proj, 0, H * d, 2 * H * d, rec_ops.FIXED_DECAY, H, d, dv, state.buffer, state.slots, ctx.q_start,
-            ctx.positions, decay=self.decay, inv_freq=rot.inv_freq if rot is not None else None,
-            rot=rot.rotary_dim if rot is not None else 0, key_scale=d ** -0.5)
+            ctx.positions, host_q_len=getattr(ctx, "host_q_len", None), decay=self.decay,
+            inv_freq=rot.inv_freq if rot is not None else None, rot=rot.rotary_dim if rot is not None else 0, key_scale=d ** -0.5)
         gated = norm32_ops.head_norm_gate(o, H, self.eps, x.dtype, gate=proj[:, 2 * H * d + H * dv:])
         return ops.linear(gated, self.w_o, out_dtype=torch.float32)
 
@@ -116,7 +116,7 @@ class HGRN2(_MatrixStateMixer):
         proj = ops.linear(x, self.w_in, out_dtype=torch.float32)  # [T, q | f | v]
         o = rec_ops.linear_recurrence(
             proj, 0, H * d, 2 * H * d, rec_ops.FORGET_GATE, H, d, dv, state.buffer, state.slots, ctx.q_start,
-            ctx.positions, gate_bias=self.f_bias, lower=self.lower)
+            ctx.positions, host_q_len=getattr(ctx, "host_q_len", None), gate_bias=self.f_bias, lower=self.lower)
         normed = norm32_ops.head_norm_gate(o, H, self.eps, x.dtype, gain=self.gain)
         return ops.linear(normed, self.w_o, out_dtype=torch.float32)
 
@@ -149,7 +149,7 @@ class Lightning(_MatrixStateMixer):
         proj = ops.linear(x, self.w_in, out_dtype=torch.float32)  # [T, q | k | v | g]
         o = rec_ops.linear_recurrence(
             proj, 0, H * d, 2 * H * d, rec_ops.FIXED_DECAY, H, d, dv, state.buffer, state.slots, ctx.q_start,
-            ctx.positions, decay=self.decay, silu_inputs=True)
+            ctx.positions, host_q_len=getattr(ctx, "host_q_len", None), decay=self.decay, silu_inputs=True)
         gated = norm32_ops.head_norm_gate(o, 1, self.eps, x.dtype, gain=self.gain,
                                           gate=proj[:, 2 * H * d + H * dv:], gate_kind="sigmoid")
         return ops.linear(gated, self.w_o, out_dtype=torch.float32)
@@ -183,8 +183,8 @@ class GatedLinearAttention(_MatrixStateMixer):
         v_off, g_off = 2 * H * d, 2 * H * d + H * dv
         o = rec_ops.linear_recurrence(
             proj, 0, H * d, v_off, rec_ops.KEY_DECAY, H, d, dv, state.buffer, state.slots, ctx.q_start, ctx.positions,
-            gate_map=self.gate_map, gate_bias=self.gate_bias, low_off=g_off + H * dv, q_scale=d ** -0.5,
-            power=1.0 / self.tau)
+            host_q_len=getattr(ctx, "host_q_len", None), gate_map=self.gate_map, gate_bias=self.gate_bias,
+            low_off=g_off + H * dv, q_scale=d ** -0.5, power=1.0 / self.tau)
         gated = norm32_ops.head_norm_gate(o, H, self.eps, x.dtype, gain=self.gain, gate=proj[:, g_off:g_off + H * dv])
         return ops.linear(gated, self.w_o, out_dtype=torch.float32)
 

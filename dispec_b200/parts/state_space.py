@@ -62,6 +62,7 @@ class StateSpaceDual(JoinableMixer):
         xbc, steps = conv_ops.conv_steps(z, inner, self.w_conv, self.b_conv, state[1].buffer if self.taps > 1 else None, ctx,
                                          step_offset=inner + self.channels, step_bias=self.step_bias, a_log=self.a_log)
         y = rec_ops.linear_recurrence(xbc, inner + G * N, inner, 0, rec_ops.STEP_DECAY, H, N, dv, state[0].buffer,
-                                      state[0].slots, ctx.q_start, ctx.positions, steps=steps, skip=self.skip, num_groups=G)
+                                      state[0].slots, ctx.q_start, ctx.positions, steps=steps, skip=self.skip, num_groups=G,
+                                      host_q_len=getattr(ctx, "host_q_len", None))
         norm32_ops.head_norm_gate(y, self.norm_groups, self.eps, out.dtype, gain=self.gain, gate=z[:, :inner],
                                   gate_first=True, out=out)
