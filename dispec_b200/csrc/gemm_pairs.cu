@@ -25,7 +25,6 @@ constexpr int EPI_GROUPS = 2, EPI_WARPS = 4 * EPI_GROUPS, THREADS = 32 * (2 + EP
 constexpr int STAGING = EPI_GROUPS * 32 * ROWS_W * 4;  // a chunk of 32 columns as floats for each group
 constexpr int TMEM_COLS = 512;                // two accumulators of up to 256 columns
 constexpr int SMEM = SLOTS * SUB * (W_BYTES + MAX_COLS / 2 * BK * 2) + STAGING + 1024;
-constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;  // clears the lowest bit of the CTA rank of a shared::cluster address
 enum { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_GEGLU = 2, EPI_XIELU = 3 };
 
 struct Args {
@@ -42,44 +41,6 @@ struct Args {
   int k_boxes;                   // one request brings both blocks of k of an operand
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint64_t* leader_bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-          smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(leader_bar) & PEER_BIT_MASK), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, uint64_t* leader_bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
-          smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(leader_bar) & PEER_BIT_MASK), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8, %9, %10, %11, %12}, p;\n\t}" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-      : "memory");
-}
-// arrives on the barrier at this offset in both CTAs of the pair (`mask`) once the products issued so far are done
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-      "h"(mask)
-      : "memory");
-}
 __device__ __forceinline__ void mbar_arrive_on(uint64_t* bar, uint32_t rank) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mapa_u32(smem_u32(bar), rank)) : "memory");
 }
@@ -97,13 +58,6 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
 }
 __device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 __device__ __forceinline__ void store4(bf16* p, float4 v) { *reinterpret_cast<uint2*>(p) = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w)); }
-
-// silu(gate) * up, or the tanh form of gelu(gate) times up (0.5 (1 + tanh(y)) = 1 / (1 + exp(-2 y))), on the hardware's
-// exponential and reciprocal
-__device__ __forceinline__ float unit_times(float gate, float up, bool gelu) {
-  const float y = gelu ? 2.f * 0.7978845608028654f * fmaf(0.044715f * gate * gate, gate, gate) : gate;
-  return __fdividef(gate, 1.f + __expf(-y)) * up;
-}
 
 __device__ __forceinline__ float4 xielu4(float4 z, float ap, float an) {
   return make_float4(xielu_f(z.x, ap, an), xielu_f(z.y, ap, an), xielu_f(z.z, ap, an), xielu_f(z.w, ap, an));

@@ -137,22 +137,6 @@ __device__ __forceinline__ void finish(const Args& a, float v, int m, int n) {
     reinterpret_cast<TOut*>(a.C2)[(size_t)m * a.ldc2 + n] = from_f32<TOut>(to_f32(out) * __bfloat162float(a.gain2[n]));
 }
 
-// silu(gate) * up for the bfloat16 model.  One warp per scheduler runs the epilogue, so its length
-// in instructions is its time: the hardware's exponential and reciprocal (a few units in the last
-// place of 32 bits, far below the output's rounding) instead of the library's sequences, which at
-// 64 rows of A made the epilogue of the gate/up product 3.9 us long.
-__device__ __forceinline__ float silu_times(float gate, float up) {
-  return __fdividef(gate, 1.f + __expf(-gate)) * up;
-}
-// the tanh form of gelu(gate), times up: 0.5 (1 + tanh(y)) = 1 / (1 + exp(-2 y))
-__device__ __forceinline__ float gelu_times(float gate, float up) {
-  const float y = 0.7978845608028654f * fmaf(0.044715f * gate * gate, gate, gate);
-  return __fdividef(gate, 1.f + __expf(-2.f * y)) * up;
-}
-__device__ __forceinline__ float unit_times(float gate, float up, bool gelu) {
-  return gelu ? gelu_times(gate, up) : silu_times(gate, up);
-}
-
 // four consecutive values of a row, as 32-bit floats
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 load4(const bf16* p) {

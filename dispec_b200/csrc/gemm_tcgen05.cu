@@ -40,21 +40,6 @@ struct Epilogue {
   int k_boxes;  // the tensor maps are the three-dimensional ones: one request brings SUB k blocks (pair kernel)
 };
 
-// silu(gate) * up of the bfloat16 model on the hardware's exponential and reciprocal (a few units in
-// the last place of 32 bits, far below the output's rounding): four epilogue warps, one per
-// scheduler, run 128 of these per thread and tile, and their length in instructions is their time
-__device__ __forceinline__ float silu_times(float gate, float up) {
-  return __fdividef(gate, 1.f + __expf(-gate)) * up;
-}
-// the tanh form of gelu(gate), times up: 0.5 (1 + tanh(y)) = 1 / (1 + exp(-2 y))
-__device__ __forceinline__ float gelu_times(float gate, float up) {
-  const float y = 0.7978845608028654f * fmaf(0.044715f * gate * gate, gate, gate);
-  return __fdividef(gate, 1.f + __expf(-2.f * y)) * up;
-}
-__device__ __forceinline__ float unit_times(float gate, float up, bool gelu) {
-  return gelu ? gelu_times(gate, up) : silu_times(gate, up);
-}
-
 template <typename TOut>
 __device__ __forceinline__ void store_row_chunk(const Epilogue& e, const uint32_t (&v)[32], int row, int col) {
   if (row >= e.M || col >= e.N) return;
@@ -341,47 +326,6 @@ __device__ __forceinline__ void store_row_chunk_with(const Epilogue& e, const ui
 
 constexpr int STAGES2 = 3;   // ring slots of the pair kernel, SUB k blocks each
 constexpr int SUB = 2;       // k blocks per ring slot: one barrier round trip of the issuing thread per 128 of k
-constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;       // clears the CTA-rank bit of a shared::cluster address
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint64_t* leader_bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(leader_bar) & PEER_BIT_MASK), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, uint64_t* leader_bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(leader_bar) & PEER_BIT_MASK), "r"(c0), "r"(c1),
-        "r"(c2)
-      : "memory");
-}
-__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8, %9, %10, %11, %12}, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u),
-        "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-      : "memory");
-}
-// arrives on the barrier at this offset in both CTAs of the pair once the products issued so far are done
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-      ::"r"(smem_u32(bar)), "h"((uint16_t)3)
-      : "memory");
-}
 __device__ __forceinline__ void mbar_arrive_on_leader(uint64_t* bar) {
   asm volatile(
       "{\n\t.reg .b32 remote;\n\t"
@@ -511,7 +455,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
               for (int k = 0; k < BK / UMMA_K; ++k)
                 umma_pair(tmem_d, a_desc + (u * (A_BYTES >> 4) + k * 2), b_desc + (u * (B_HALF >> 4) + k * 2), idesc, (st | u | k) != 0);
             }
-            umma_commit_pair(&empty_bar[s]);
+            umma_commit_pair(&empty_bar[s], 3);
           }
           if (++s == STAGES2) s = 0, phase ^= 1;
         }
@@ -519,7 +463,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           failed = 1;
           break;
         }
-        if (leader) umma_commit_pair(&accum_full[buf]);
+        if (leader) umma_commit_pair(&accum_full[buf], 3);
       }
     }
   } else {

@@ -62,10 +62,8 @@ __device__ __forceinline__ bool mbar_wait_both(uint64_t* bar_a, uint32_t parity_
 }
 
 // True in one lane of a warp that calls it as one.  The loops that request tiles and issue products are run by whole
-// warps, and this lane alone makes the requests: with the loop itself under `if (lane == 0)` the compiler knows none of
-// its values to be the same for the whole warp, and moves every descriptor and address of every instruction into the
-// uniform registers that these instructions take their operands from (measured on products of 128 x 16 x 16 with the
-// first operand in tensor memory: 110 cycles from one to the next, without it less than the tensor cores take).
+// warps, and this lane alone makes the requests (with the loop itself under `if (lane == 0)` 110 cycles went by from one
+// product of 128 x 16 x 16 with its first operand in tensor memory to the next; so, less than the tensor cores take).
 __device__ __forceinline__ bool elect_one() {
   uint32_t one;
   asm volatile(
@@ -74,6 +72,57 @@ __device__ __forceinline__ bool elect_one() {
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(one));
   return one != 0;
+}
+
+// ---- CTA pairs (cta_group::2).  Loads of both CTAs arrive on the leader's barrier, whose address has the lowest bit of
+// the CTA rank clear.
+constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint64_t* leader_bar, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+          smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(leader_bar) & PEER_BIT_MASK), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, uint64_t* leader_bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+          smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(leader_bar) & PEER_BIT_MASK), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8, %9, %10, %11, %12}, p;\n\t}" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      : "memory");
+}
+// arrives on the barrier at this offset in the CTAs of `mask` (both of the pair) once the products issued so far are done
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+      "h"(mask)
+      : "memory");
+}
+
+// silu(gate) * up, or the tanh form of gelu(gate) times up (0.5 (1 + tanh(y)) = 1 / (1 + exp(-2 y))), on the hardware's
+// exponential and reciprocal: a few units in the last place of 32 bits, far below the rounding of the bfloat16 outputs that
+// the epilogues form, whose length in instructions is their time (64 rows of a gate/up product with the library's
+// sequences: 3.9 us).
+__device__ __forceinline__ float unit_times(float gate, float up, bool gelu) {
+  const float y = gelu ? 2.f * 0.7978845608028654f * fmaf(0.044715f * gate * gate, gate, gate) : gate;
+  return __fdividef(gate, 1.f + __expf(-y)) * up;
 }
 
 // address of the same shared-memory location in CTA `rank` of the cluster
