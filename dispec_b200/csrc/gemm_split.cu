@@ -34,6 +34,8 @@
 // Launched plainly, and every wait on an mbarrier is bounded; a wait that runs out is recorded in the device error word.
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "tcgen05_common.cuh"
 
 namespace cg = cooperative_groups;
@@ -391,12 +393,14 @@ int launch(const CUtensorMap& map_w, const Args& g, int tiles, int splits, int s
   auto kernel = gemm_split_kernel<NB>;
   CUtensorMap map_a = map_w;  // not used where A's rows are no whole pieces
   DSP_REQUIRE(!g.a_wide || make_map_f32(&map_a, g.A, g.M, g.K, g.lda, NB), "dsp_gemm_split: cannot encode the tensor map of A");
-  static bool configured = false;
-  if (!configured) {
+  static std::atomic<bool> configured[MAX_DEVICES] = {};
+  const int device = current_device();
+  DSP_REQUIRE(device >= 0, "dsp_gemm_split: the current device is not known");
+  if (!configured[device].load(std::memory_order_relaxed)) {
     DSP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<NB>::SMEM));
-    configured = true;
+    DSP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    configured[device].store(true, std::memory_order_relaxed);
   }
-  prefer_max_shared(reinterpret_cast<const void*>(kernel));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(splits > 1 || tiles < sms ? tiles : sms, splits, 1);
   cfg.blockDim = dim3(THREADS, 1, 1);
