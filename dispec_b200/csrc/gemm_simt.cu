@@ -297,7 +297,8 @@ int launch_few(const void* A, long lda, const void* W, const void* bias, const v
   return 0;
 }
 
-// Cycles a block takes per k (measured at 1,965 MHz, K 8,960 and 1,536): with an SM to itself, and its share of an
+// Cycles a block takes per k (measured at 1,965 MHz, K 8,960 and 1,536; aligned floats come with K below 1,536, the others
+// with any): with an SM to itself, and its share of an
 // SM that holds as many as fit.  The larger tiles need fewer shared-memory reads per product (128 x 128: 195 cycles
 // of which 128 are the FMA units' own), the smaller ones reach more SMs when there are few outputs.
 struct Tile {

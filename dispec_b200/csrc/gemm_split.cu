@@ -434,10 +434,15 @@ extern "C" int dsp_gemm_split(const float* A, long lda, const float* W, const fl
   g.chunks = (M + g.chunk_rows - 1) / g.chunk_rows;
   g.a_wide = lda % 4 == 0 && lda >= K && ((uintptr_t)A & 15) == 0;  // (rows that overlap are no tensor map's)
   // K is split where there are few blocks of W, by their number alone: a row's sums must not depend on how many rows
-  // there are.  As many times as leaves clusters that fit beside one another with three chunks of rows (36 clusters of
-  // four did not: 264 rows x 1,536 x 8,960 115 us for 68 in three; nor 48 of three: x 2,048 x 1,536 41)
+  // there are.  Up to 14 blocks as many times as leaves clusters that fit beside one another with three chunks of rows
+  // (36 clusters of four do not); from there on with one chunk (33 clusters of four, 45 of three, 74 of two): not
+  // split from 23 blocks on and in two parts below, one row x 3,072 x 2,048 took 26.9 us, in four 11.6 (chain of FMAs 15.6),
+  // x 2,048 x 1,536 13.8 and 10.0 (10.9), x 8,960 x 3,072 39.7 and about 26 in two (31.9); 264 rows x 3,072 x 2,048 45 and 49 (103),
+  // x 2,048 x 1,536 23 and 29 (62).  Where it is still behind the chain: up to 4 rows x 9,300 to 12,000 and 19,000 to 24,000, at
+  // most 23.2 us for 18.5.
   const int blocks = (N + ROWS_W - 1) / ROWS_W, kb_total = (K + BK - 1) / BK;
-  int splits = 44 / blocks < MAX_SPLITS ? 44 / blocks : MAX_SPLITS;
+  int splits = blocks <= 14 ? 44 / blocks : blocks <= 32 ? 4 : blocks <= 44 ? 3 : blocks <= 72 ? 2 : 1;
+  if (splits > MAX_SPLITS) splits = MAX_SPLITS;
   if (splits > kb_total / 8) splits = kb_total / 8;
   if (splits < 1) splits = 1;
   g.kb_per_split = (kb_total + splits - 1) / splits;

@@ -2,7 +2,7 @@
 
 float32: every operand cut into three bfloat16 pieces that add up to it, whose products run on the
 tensor cores and are summed in 32 bits (``dsp_gemm_split``: closer to 64 bits than a chain of 32-bit
-FMAs); the FMA kernel (``dsp_gemm_simt``) for short K and for matrices that TMA cannot read.  Which of
+FMAs); the FMA kernel (``dsp_gemm_simt``) for K below 1,536 and for matrices that TMA cannot read.  Which of
 the two runs is decided by the matrix alone, and a row does not depend on its batch in either.
 bfloat16: the weight-streaming tcgen05 kernel for up to 128 rows (decoding and the rows whose
 logits are wanted); above that the persistent tcgen05/TMA kernel of this package, except that, mostly
@@ -26,7 +26,7 @@ from dispec_b200.ops import library as L
 from dispec_b200.ops import tuning
 
 STREAM_MAX_ROWS = 128  # rows up to which the weight-streaming kernel always runs
-SPLIT_MIN_K = 512  # length of a product of floats from which the tensor cores are used
+SPLIT_MIN_K = 1536  # length of a product of floats from which the tensor cores are used
 NORM_SPLIT_MAX_ROWS = 64  # rows up to which a norm is split over two products
 
 
@@ -135,9 +135,11 @@ def _stream(x, w, bias, residual, out, epilogue=EPI_PLAIN, target_ctas: int | No
 
 def split_supported(w: torch.Tensor) -> bool:
     """Whether a product of floats runs on the tensor cores: by its matrix alone, so that a row has the same bits
-    alone and among others.  Below ``SPLIT_MIN_K`` the fixed latencies of that kernel are longer than the FMA chain:
-    264 rows x 1,024 x 128 17.4 us for 11.0, 4 rows x 256 x 256 12.3 for 8.2; 33 rows x 200 x 516 15.4 for 15.1, 97 rows
-    x 1,000 x 1,000 16.4 for 24.6."""
+    alone and among others.  Below ``SPLIT_MIN_K`` a few rows wait longer for that kernel's fixed latencies than for the
+    FMA chain: 4 rows x 1,536 x 512 8.0 us for 4.4, x 1,024 9.5 for 7.9, x 1,280 10.3 for 9.6, x 1,536 11.4 for 11.3 (264 rows
+    14 and 18, 15 and 33, 17 and 41, 18 and 49); nor is it always closer to 64 bits there (products of two lognormal
+    operands of sigma 2, K 256 / 512 / 1,024: 7.5e-7 / 7.1e-7 / 9.1e-7 off for 3.4e-7 / 3.7e-7 / 6.8e-7 of the chain; from
+    1,280 on it is, with eight distributions tried)."""
     return w.shape[1] >= SPLIT_MIN_K and w.shape[1] % 4 == 0 and w.data_ptr() % 16 == 0
 
 

@@ -39,3 +39,13 @@ def test_a_cluster_query_that_fails_is_an_error():
     from dispec_b200.ops import library
     with pytest.raises(library.KernelError, match="how many clusters"):
         library.check(library.core().dsp_gemm_pairs_faster(300, 1536, 8960, 148))
+
+
+@pytest.mark.parametrize("N,K,split", [(64, 512, False), (1536, 1024, False), (4096, 1532, False), (1, 1536, True), (1536, 1538, False),
+                                       (3072, 2048, True)])
+def test_which_products_of_floats_run_on_the_tensor_cores(N, K, split):
+    from dispec_b200.ops import gemm
+    w = torch.zeros((N, K))
+    assert w.data_ptr() % 16 == 0 and gemm.split_supported(w) == split
+    shifted = torch.zeros(N * K + 1)[1:].view(N, K)
+    assert not gemm.split_supported(shifted)

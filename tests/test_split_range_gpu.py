@@ -69,3 +69,31 @@ def test_rows_without_numbers_are_not_slow():
     assert ms(torch.full_like(x, float("nan"))) < 12 * usual and bool(out.isnan().all())
     x[100, 3] = float("nan")
     assert ms(x) < 3 * usual and bool(out[100].isnan().all()) and bool(out[99].isfinite().all())
+
+
+@pytest.mark.parametrize("N,K", [(512, 1536), (2048, 1536), (3072, 2048), (4096, 4096), (8960, 1536), (14336, 2048)])
+def test_few_rows_are_not_slower_than_the_chain(N, K):
+    """A matrix goes to the same kernel for every number of rows, so that one row must not pay for many."""
+    from dispec_b200.ops import gemm
+    x, w = rnd((1, K), 9), rnd((N, K), 10)
+    assert gemm.split_supported(w)
+    out = torch.empty((1, N), device=DEV)
+
+    def us(f):
+        f(x, w, None, None, out)
+        torch.cuda.synchronize()
+        graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=stream):
+            for _ in range(20):
+                f(x, w, None, None, out)
+        times = []
+        for _ in range(5):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            graph.replay()
+            end.record()
+            end.synchronize()
+            times.append(50 * start.elapsed_time(end))
+        return min(times)
+
+    assert us(gemm._split) < 1.25 * us(gemm._simt)
