@@ -25,7 +25,7 @@ int dsp_gemm_tcgen05(const void* A, long lda, const void* W, const void* bias, c
 int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas);
 int dsp_gemm_pairs(const void* A, long lda, const void* W, const void* bias, const void* residual, long ldr, void* C, long ldc,
                    int M, int N, int K, int out_dtype, int epilogue, const float* act, int splits, int chunks, cudaStream_t stream);
-int dsp_gemm_pairs_faster(int M, int N, int K, int target_ctas);
+int dsp_gemm_pairs_faster(int M, int N, int K, int target_ctas, int result);
 int dsp_attn_combine(const float* part_o, const float* part_ml, void* out, long out_stride, int num_tokens, int H, int D,
                      int splits, int dtype, cudaStream_t stream);
 }
@@ -90,7 +90,7 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
     const bool fours = ((uintptr_t)bias & 7) == 0;
     for (int i = 0; i < num_chosen; ++i)
       if (chosen[i].N == N && chosen[i].K == K && chosen[i].fours == fours) return chosen[i].kernel;
-    int kernel = fours ? dsp_gemm_pairs_faster(T, N, K, (int)s.target_ctas) : 0;
+    int kernel = fours ? dsp_gemm_pairs_faster(T, N, K, (int)s.target_ctas, 0) : 0;
     if (kernel == 1) kernel = PAIRS;
     else if (kernel == 0) kernel = dsp_gemm_few_rows_faster(T, N, K, (int)s.target_ctas);
     if (kernel >= 0 && num_chosen < 8) chosen[num_chosen++] = {N, K, kernel, fours};
@@ -117,7 +117,7 @@ extern "C" int dsp_dense_layers(const DspDenseStep* step, const DspDenseLayer* l
     return dsp_gemm_tcgen05(A, K, W, bias, residual, add ? N : 0, C, N, T, N, K, DSP_BF16, 1, 0, stream);
   };
 
-  const int pairs_gate_up = T > s.always_few ? dsp_gemm_pairs_faster(T, 2 * inter, hidden, (int)s.target_ctas) : 0;
+  const int pairs_gate_up = T > s.always_few ? dsp_gemm_pairs_faster(T, 2 * inter, hidden, (int)s.target_ctas, 2) : 0;
   if (pairs_gate_up < 0) return pairs_gate_up;
   bool ready = false;  // scaled_b holds x times the next norm1's gain
   for (long i = 0; i < s.layers; ++i) {

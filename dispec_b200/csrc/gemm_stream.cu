@@ -815,31 +815,69 @@ Plan make_plan(int M, int N, int K, int out_dtype, int target_ctas, bool may_spl
 // 17.5 / 15.0 / 34 us and 11.5 / 12.5 / 19.0 / 43 / 86 at 129 rows; 12.9 / 11.7 / 30 / 20.5 / 62 and 11.6 / 12.9 / 25 / 44 / 89 at
 // 384; 15.1 / 12.9 / 37 / 27 / 109 and 11.7 / 12.9 / 32 / 44 / 89 at 536; 15.6 / 15.6 / 64 / 37 / 204 and 12.9 / 13.1 / 44 /
 // 46 / 106 at 1,016.
-extern "C" int dsp_gemm_row_estimates(int M, int N, int K, int target_ctas, double* few, double* many) {
+namespace {
+struct ManyTiles {  // of the many-row kernel, of the width that it would choose
+  bool narrow;
+  long rounds;
+  double busy;
+};
+ManyTiles many_tiles(int M, int N, int target_ctas) {
+  const long pairs = target_ctas / 2 > 0 ? target_ctas / 2 : 1;
+  auto tiles = [&](int width) { return (long)((M + 255) / 256) * ((N + width - 1) / width); };
+  auto rounds = [&](int width) { return (tiles(width) + pairs - 1) / pairs; };
+  const bool narrow = 0.92 * rounds(192) < rounds(256);
+  const int width = narrow ? 192 : 256;
+  return {narrow, rounds(width), fmin(1.0, (double)tiles(width) / pairs)};
+}
+}  // namespace
+extern "C" int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas) {
+  if (M <= 0 || N <= 0 || K <= 0 || target_ctas <= 0) return 0;
   const int k_blocks = (K + BK - 1) / BK;
   const double w_us = 2.0 * N * K / 6.5e6;  // W at the memory's rate
-  // the many-row kernel: the rounds of its tiles over the CTA pairs, of the width that it would choose
-  const long pairs = target_ctas / 2 > 0 ? target_ctas / 2 : 1;
-  auto many_tiles = [&](int width) { return (long)((M + 255) / 256) * ((N + width - 1) / width); };
-  auto many_rounds = [&](int width) { return (many_tiles(width) + pairs - 1) / pairs; };
-  const int width = 0.92 * many_rounds(192) < many_rounds(256) ? 192 : 256;
-  const double many_busy = fmin(1.0, (double)many_tiles(width) / pairs);
-  *many = 5.0 + many_rounds(width) * (1.2 + k_blocks * (0.23 + 0.056 * many_busy)) + 0.44 * w_us;
+  const ManyTiles t = many_tiles(M, N, target_ctas);
+  const double many = 5.0 + t.rounds * (1.2 + k_blocks * (0.23 + 0.056 * t.busy)) + 0.44 * w_us;
   // this one: a k block costs more while more CTAs stream; storing a tile, and the partial rows a split sends and adds,
   // go with the rows of a tile
   const Plan p = make_plan(M, N, K, DSP_BF16, target_ctas, N % 4 == 0);
   if (p.splits == 0) return -1;
   const long rounds = p.splits > 1 ? 1 : (p.tiles + target_ctas - 1) / target_ctas;
   const double busy = fmin(1.0, (double)p.tiles * p.splits / target_ctas), rows = Chunks(M).rows / 192.0;
-  *few = 3.8 + 0.98 * busy + (double)rounds * p.kb_per_split * (0.29 + 0.06 * busy) + 3.72 * rows +
+  const double few = 3.8 + 0.98 * busy + (double)rounds * p.kb_per_split * (0.29 + 0.06 * busy) + 3.72 * rows +
                      (p.splits > 1 ? rows * (0.85 * busy + 5.13 / p.splits) : 0.0) + 0.15 * w_us;
-  return 0;
+  return 1.02 * few < many;
 }
-extern "C" int dsp_gemm_few_rows_faster(int M, int N, int K, int target_ctas) {
-  if (M <= 0 || N <= 0 || K <= 0 || target_ctas <= 0) return 0;
-  double few = 0.0, many = 0.0;
-  const int rc = dsp_gemm_row_estimates(M, N, K, target_ctas, &few, &many);
-  return rc != 0 ? rc : 1.02 * few < many;
+
+// The time of whichever of the two runs where the product on CTA pairs does not (for a gated product that is always the
+// many-row one), and the blocks of k that it sums one after the other.  result: 0 bfloat16, 1 32 bits, 2 gated.  A fit of its
+// own on 26 numbers of rows from 130 to 2,048 at each of 44 shapes from 512 x 512 to 37,888 x 3,584 (rms error 9 to 11 %); the
+// rule above was fitted on the kernels of before whole warps ran their loops, and is left as it is: which of these two kernels
+// runs decides how far 32-bit results are from 64 bits.
+extern "C" int dsp_gemm_other_rows(int M, int N, int K, int target_ctas, int result, double* us, int* k_blocks_in_a_row) {
+  static constexpr double FEW[2][11] = {{5.404, 0.329, 0.139, 0.036, -0.283, 1.846, 5.233, 0.362, 3.326, 0.127, -1.701},
+                                        {3.973, -0.144, 0.133, 0.041, 0.416, 2.561, 4.808, 0.378, 2.308, 0.130, -0.043}};
+  static constexpr double MANY[3][7] = {{5.044, 1.522, 0.274, 0.044, 0.385, -1.297, -0.046},
+                                        {6.159, 3.865, 0.272, 0.045, 0.417, -2.197, -0.044},
+                                        {5.054, 0.850, 0.271, 0.049, 0.340, -1.233, -0.044}};
+  const int k_blocks = (K + BK - 1) / BK;
+  const double w_us = 2.0 * N * K / 6.5e6;
+  const int few = result == 2 ? 0 : dsp_gemm_few_rows_faster(M, N, K, target_ctas);
+  if (few < 0) return few;
+  if (few) {
+    const Plan p = make_plan(M, N, K, DSP_BF16, target_ctas, N % 4 == 0);
+    if (p.splits == 0) return -1;
+    const double rounds = p.splits > 1 ? 1 : (p.tiles + target_ctas - 1) / target_ctas, kb = p.kb_per_split;
+    const double busy = fmin(1.0, (double)p.tiles * p.splits / target_ctas), rows = Chunks(M).rows / 192.0, split = p.splits > 1;
+    const double* c = FEW[result];
+    *us = c[0] + c[1] * busy + rounds * kb * (c[2] + c[3] * busy + c[9] * rows) + rows * (c[4] + split * (c[5] * busy + c[6] / p.splits)) +
+          c[7] * w_us + rounds * (c[8] * rows + c[10]);
+    *k_blocks_in_a_row = p.kb_per_split;
+  } else {
+    const ManyTiles t = many_tiles(M, N, target_ctas);
+    const double* c = MANY[result];
+    *us = c[0] + t.rounds * (c[1] + k_blocks * (c[2] + c[3] * t.busy) + t.narrow * (c[5] + c[6] * k_blocks)) + c[4] * w_us;
+    *k_blocks_in_a_row = k_blocks;
+  }
+  return 0;
 }
 
 #ifdef DSP_STAMPS

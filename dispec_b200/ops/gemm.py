@@ -6,9 +6,8 @@ FMAs); the FMA kernel (``dsp_gemm_simt``) for K below 1,536 and for matrices tha
 the two runs is decided by the matrix alone, and a row does not depend on its batch in either.
 bfloat16: the weight-streaming tcgen05 kernel for up to 128 rows (decoding and the rows whose
 logits are wanted); above that the persistent tcgen05/TMA kernel of this package, except that, mostly
-at some hundred rows, the kernel on CTA pairs with swapped roles runs where ``tuning.pairs_are_faster``
-says so (it splits K, and cuts the rows into equal chunks) and the weight-streaming kernel where
-``tuning.rows_in_chunks_is_faster`` does.  Operands
+at some hundred rows, the kernel on CTA pairs with swapped roles (it splits K, and cuts the rows into
+equal chunks) or the weight-streaming kernel runs where ``tuning.many_rows_product`` says so.  Operands
 those kernels cannot take (a width that is no multiple of 8) go to the FMA kernel when there
 are at most 64 rows or 32-bit logits are wanted, and otherwise to the library matrix product
 (cuBLAS through torch.mm), which is where the reference engine itself calls a library
@@ -150,8 +149,12 @@ def tcgen05_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 def pairs_supported(x: torch.Tensor, w: torch.Tensor, bias, residual, out: torch.Tensor) -> bool:
     """Whether the operands of a product let the kernel on CTA pairs finish four outputs of a row at a time."""
+    return tcgen05_supported(x, w) and _whole_fours(w, bias, residual, out)
+
+
+def _whole_fours(w: torch.Tensor, bias, residual, out: torch.Tensor) -> bool:
     width = 4 * out.element_size()
-    return (w.shape[0] % 4 == 0 and out.stride(0) % 4 == 0 and out.data_ptr() % width == 0 and tcgen05_supported(x, w)
+    return (w.shape[0] % 4 == 0 and out.stride(0) % 4 == 0 and out.data_ptr() % width == 0
             and (residual is None or (residual.stride(0) % 4 == 0 and residual.data_ptr() % width == 0))
             and (bias is None or bias.data_ptr() % 8 == 0))
 
@@ -189,7 +192,8 @@ def linear_gate_up_swiglu(x, w_interleaved, out=None, act: str = "silu"):
         out = torch.empty((M, N // 2), dtype=x.dtype, device=x.device)
     epilogue = {"silu": EPI_SWIGLU, "gelu_tanh": EPI_GEGLU}[act]
     if M > STREAM_MAX_ROWS:
-        if tuning.pairs_are_faster(M, N, x.shape[1], x.device) and pairs_supported(x, w_interleaved, None, None, out):
+        if (tuning.many_rows_product(M, N, x.shape[1], tuning.GATED_RESULT, x.device) == "pairs"
+                and _whole_fours(w_interleaved, None, None, out)):
             return _pairs(x, w_interleaved, None, None, out, epilogue=epilogue)
         return _tcgen05(x, w_interleaved, None, None, out, epilogue=epilogue)
     return _stream(x, w_interleaved, None, None, out, epilogue=epilogue, norm=norm)
@@ -281,13 +285,11 @@ def linear(x, w: torch.Tensor, bias: torch.Tensor | None = None,
     if backend is None:
         if stream_supported(M, K, x, w):
             backend = "stream"
-        elif M > STREAM_MAX_ROWS and tuning.pairs_are_faster(M, N, K, x.device) and pairs_supported(x, w, bias, residual, out):
-            backend = "pairs"
-        elif (M > STREAM_MAX_ROWS and stream_supported(STREAM_MAX_ROWS, K, x, w)
-              and tuning.rows_in_chunks_is_faster(M, N, K, x.device, STREAM_MAX_ROWS)):
-            backend = "stream"  # (a norm after it runs as a kernel)
-        elif M > STREAM_MAX_ROWS and tcgen05_supported(x, w):
-            backend = "tcgen05"
+        elif M > STREAM_MAX_ROWS and tcgen05_supported(x, w):  # ("stream": a norm after it runs as a kernel)
+            result_kind = tuning.FLOAT32_RESULT if out_dtype == torch.float32 else tuning.BF16_RESULT
+            backend = tuning.many_rows_product(M, N, K, result_kind, x.device)
+            if backend == "pairs" and not _whole_fours(w, bias, residual, out):
+                backend = "stream" if tuning.rows_in_chunks_is_faster(M, N, K, x.device, STREAM_MAX_ROWS) else "tcgen05"
         elif M > STREAM_MAX_ROWS and out_dtype == torch.bfloat16:
             backend = "library"
         else:

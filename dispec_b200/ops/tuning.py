@@ -58,19 +58,35 @@ def _few_rows_faster(M: int, N: int, K: int, sms: int) -> bool:
     return bool(answer)
 
 
-def pairs_are_faster(M: int, N: int, K: int, device=None) -> bool:
-    """Whether the product on CTA pairs with swapped roles beats the few-row and the many-row product at M rows; the
+BF16_RESULT, FLOAT32_RESULT, GATED_RESULT = 0, 1, 2  # what the time of a product is fitted for
+
+
+def pairs_are_faster(M: int, N: int, K: int, device=None, result: int = BF16_RESULT) -> bool:
+    """Whether the product on CTA pairs with swapped roles beats the one that runs otherwise at M rows; the
     estimate stands beside the kernel (``dsp_gemm_pairs_faster`` in csrc/gemm_pairs.cu)."""
-    return _pairs_faster(M, N, K, sm_count(device))
+    return _pairs_faster(M, N, K, sm_count(device), result)
 
 
 @functools.lru_cache(maxsize=4096)
-def _pairs_faster(M: int, N: int, K: int, sms: int) -> bool:
+def _pairs_faster(M: int, N: int, K: int, sms: int, result: int) -> bool:
     from dispec_b200.ops import library
-    answer = library.core().dsp_gemm_pairs_faster(M, N, K, STREAM_CTAS_PER_SM * sms)
+    answer = library.core().dsp_gemm_pairs_faster(M, N, K, STREAM_CTAS_PER_SM * sms, result)
     if answer < 0:  # (an exception is not kept by the cache)
         library.check(answer, launches=0)
     return bool(answer)
+
+
+def many_rows_product(M: int, N: int, K: int, result: int, device) -> str:
+    """The kernel of a bfloat16 product of more rows than the few-row kernel always takes: "pairs", "stream" or "tcgen05"
+    (a product of a step asks once, for its size and kind of result)."""
+    return _many_rows_product(M, N, K, result, sm_count(device))
+
+
+@functools.lru_cache(maxsize=4096)
+def _many_rows_product(M: int, N: int, K: int, result: int, sms: int) -> str:
+    if _pairs_faster(M, N, K, sms, result):
+        return "pairs"
+    return "stream" if result != GATED_RESULT and _few_rows_faster(M, N, K, sms) else "tcgen05"
 
 
 # ---- attention of single tokens (attn_mma.cu, decode kernel) ---------------------------------

@@ -38,7 +38,7 @@ def test_a_cluster_query_that_fails_is_an_error():
     import ctypes
     from dispec_b200.ops import library
     with pytest.raises(library.KernelError, match="how many clusters"):
-        library.check(library.core().dsp_gemm_pairs_faster(300, 1536, 8960, 148))
+        library.check(library.core().dsp_gemm_pairs_faster(300, 1536, 8960, 148, 0))
 
 
 @pytest.mark.parametrize("N,K,split", [(64, 512, False), (1536, 1024, False), (4096, 1532, False), (1, 1536, True), (1536, 1538, False),
