@@ -480,12 +480,13 @@ Plan make_plan(int M, int N, int K, const Fits& fits, int force_splits, int forc
 
 extern "C" int dsp_gemm_other_rows(int M, int N, int K, int target_ctas, int result, double* us, int* k_blocks_in_a_row);
 
-// The time of this product for a bfloat16 result (0), one of 32 bits (1) or a gated one (2),
+// The time of this product for a bfloat16 result (0), one of 32 bits (1), a gated one (2) or one that xIELU is applied to (3),
 // fitted as dsp_gemm_other_rows is; rms error 7 %.
 static double time_us(const Plan& p, int N, int K, int target_ctas, int result) {
-  static constexpr double FIT[3][11] = {{4.592, -1.518, 0.131, 0.208, 0.319, -0.049, 4.186, 0.642, -1.413, 0.411, 3.534},
+  static constexpr double FIT[4][11] = {{4.592, -1.518, 0.131, 0.208, 0.319, -0.049, 4.186, 0.642, -1.413, 0.411, 3.534},
                                         {5.056, -1.721, 0.144, 0.188, 0.282, 0.016, 3.055, 0.356, -0.941, 0.418, 4.389},
-                                        {4.822, -1.399, 0.123, 0.212, 0.345, -0.063, 3.618, 0.362, 0.201, 0.391, 2.827}};
+                                        {4.822, -1.399, 0.123, 0.212, 0.345, -0.063, 3.618, 0.362, 0.201, 0.391, 2.827},
+                                        {6.424, -3.517, 0.069, 0.352, 0.613, -0.469, 3.181, 1.244, -7.046, 0.365, 13.721}};
   const long tiles = (long)((N + 2 * ROWS_W - 1) / (2 * ROWS_W)) * p.chunks;
   const double rounds = (double)((tiles + p.clusters - 1) / p.clusters), slots = p.slots_per_split, cols = p.cols / 256.0;
   const double busy = fmin(1.0, 2.0 * tiles * p.splits / target_ctas), split = p.splits > 1;
@@ -495,15 +496,16 @@ static double time_us(const Plan& p, int N, int K, int target_ctas, int result) 
 }
 // Whether this product beats what runs otherwise (-1: not known, the message is set): the few-row or the many-row kernel for
 // results 0 to 2, with a margin for the fits' errors (of 3,432 sizes eight take more than 1.03 of the other kernel's time, at
-// most 1.10; the mean is 0.963 / 0.927 / 0.897 of it).  32-bit results stay where their sums are shorter: the tensor cores cut every one off (300 rows x 2,048
+// most 1.10; the mean is 0.963 / 0.927 / 0.897 of it), and for 3 a product with a 32-bit result and the activation behind it (mean
+// 0.88, at most 1.15).  32-bit results stay where their sums are shorter: the tensor cores cut every one off (300 rows x 2,048
 // x 8,960: 3.2e-6 off 64 bits here, 2.3e-6 in the few-row kernel, which splits K further, 1.0e-5 in the many-row one).  This,
 // few-row and many-row: 536 rows x 1,536 x 1,536 9.8 / 11.8 / 11.8 us, x 17,920 x 1,536 29.0 / 30.7 / 30.5, x 1,536 x 8,960 21.3 /
 // 23.1 / 42.3; 1,016 rows x 3,584 x 18,944 104.5 / 169 / 108, x 2,048 x 1,536 13.6 / 13.2 / 11.3.
 extern "C" int dsp_gemm_pairs_faster(int M, int N, int K, int target_ctas, int result) {
-  if (M <= 0 || M > 2048 || N <= 0 || K <= 0 || target_ctas <= 0 || result < 0 || result > 2) return 0;  // (fitted up to there)
+  if (M <= 0 || M > 2048 || N <= 0 || K <= 0 || target_ctas <= 0 || result < 0 || result > 3) return 0;  // (fitted up to there)
   double other = 0.0;
   int in_a_row = 0;
-  const int rc = dsp_gemm_other_rows(M, N, K, target_ctas, result, &other, &in_a_row);
+  const int rc = dsp_gemm_other_rows(M, N, K, target_ctas, result == 3 ? 1 : result, &other, &in_a_row);
   if (rc != 0) return rc;
   const Plan p = plan_of(M, N, K, 0, 0);
   if (p.splits == 0) return -1;
@@ -511,7 +513,11 @@ extern "C" int dsp_gemm_pairs_faster(int M, int N, int K, int target_ctas, int r
   const double us = time_us(p, N, K, target_ctas, result);
   if (result == 0) return us < 0.955 * other;
   if (result == 2) return us < 0.94 * other;
-  return p.slots_per_split * SUB <= in_a_row && us < 0.94 * other;
+  const bool no_longer_sums = p.slots_per_split * SUB <= in_a_row;
+  if (result == 1) return no_longer_sums && us < 0.94 * other;
+  const double here = time_us(p, N, K, target_ctas, 1);  // of the 32-bit product that the activation would follow
+  const double product = no_longer_sums && here < 0.94 * other ? here : other;
+  return us < 3.22 + 1.063 * product + 1.493e-6 * M * N;
 }
 
 // The plan of a size where fits[0..3] clusters of one to four pairs fit: pairs that share a tile, chunks of rows, clusters

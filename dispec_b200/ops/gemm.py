@@ -199,24 +199,23 @@ def linear_gate_up_swiglu(x, w_interleaved, out=None, act: str = "silu"):
     return _stream(x, w_interleaved, None, None, out, epilogue=epilogue, norm=norm)
 
 
-XIELU_MAX_ROWS = 1024  # rows up to which xIELU is formed in the epilogue of the product before it
-
-
 def linear_xielu(x: torch.Tensor, w: torch.Tensor, params: torch.Tensor) -> torch.Tensor:
     """xIELU(x W^T), the activation formed in 32 bits from the 32-bit sums and rounded to x's type (``params``: its two raw
-    parameters, float32); the same bits in the product's epilogue, where the kernel on CTA pairs takes the operands, and in
-    a kernel of its own behind the product.  The epilogue saves writing and reading the sums and a launch, but takes longer
-    than the products of its tile.  us, fused and not, w 8,960 x 1,536: 137 rows 17 and 27, 300 23 and 36, 536 36 and 35,
-    1,016 48 and 52, 2,500 101 and 106; w 4,096 x 1,024: 1,016 rows 27 and 36, 2,500 59 and 47."""
+    parameters, float32): in the epilogue of the product on CTA pairs, or by a kernel of its own behind a product with a
+    32-bit result, whichever the estimate beside the former says is faster (``tuning.XIELU_RESULT``).  The activation is
+    the same function of the sums in both; the sums are added in the order of the kernel that runs.  us, fused and not, w
+    8,960 x 1,536: 137 rows 16 and 17, 300 21 and 22, 536 34 and 31, 1,016 46 and 49; w 14,336 x 4,096: 536 rows 68 and 82,
+    2,048 171 and 216; w 4,096 x 1,024: 900 rows 30 and 24."""
     from dispec_b200.ops.norm32 import xielu
     if not (x.is_cuda and w.is_cuda and params.is_cuda):
         raise L.KernelError("linear_xielu: CUDA tensors only (there is no CPU path)")
     assert x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1], (x.shape, w.shape)
     assert x.stride(1) == 1 and w.is_contiguous() and x.dtype == w.dtype
     M, N = x.shape[0], w.shape[0]
-    if STREAM_MAX_ROWS < M <= XIELU_MAX_ROWS and x.dtype == torch.bfloat16:
+    if (M > STREAM_MAX_ROWS and x.dtype == torch.bfloat16 and tcgen05_supported(x, w)
+            and tuning.pairs_are_faster(M, N, x.shape[1], x.device, tuning.XIELU_RESULT)):
         out = torch.empty((M, N), dtype=x.dtype, device=x.device)
-        if pairs_supported(x, w, None, None, out):
+        if _whole_fours(w, None, None, out):
             assert params.dtype == torch.float32 and params.numel() == 2 and params.is_contiguous()
             return _pairs(x, w, None, None, out, epilogue=EPI_XIELU, act=params)
     return xielu(linear(x, w, out_dtype=torch.float32), params, x.dtype)

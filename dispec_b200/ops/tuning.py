@@ -58,7 +58,7 @@ def _few_rows_faster(M: int, N: int, K: int, sms: int) -> bool:
     return bool(answer)
 
 
-BF16_RESULT, FLOAT32_RESULT, GATED_RESULT = 0, 1, 2  # what the time of a product is fitted for
+BF16_RESULT, FLOAT32_RESULT, GATED_RESULT, XIELU_RESULT = 0, 1, 2, 3  # what the time of a product is fitted for
 
 
 def pairs_are_faster(M: int, N: int, K: int, device=None, result: int = BF16_RESULT) -> bool:

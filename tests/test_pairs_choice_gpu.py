@@ -18,6 +18,17 @@ def test_the_choice(M, N, K, result, pairs):
     assert (tuning.many_rows_product(M, N, K, result, torch.device(DEV)) == "pairs") == pairs
 
 
+@pytest.mark.parametrize("M,N,K,fused", [(137, 8960, 1536, True), (900, 4096, 1024, False), (900, 14336, 4096, True),
+                                         (2048, 14336, 4096, True), (2500, 8960, 1536, False), (128, 8960, 1536, False)])
+def test_xielu_is_fused_where_that_is_faster(M, N, K, fused, monkeypatch):
+    from dispec_b200.ops import gemm
+    x, w = (torch.ones(s, dtype=torch.bfloat16, device=DEV) for s in ((M, K), (N, K)))
+    asked, pairs = [], gemm._pairs
+    monkeypatch.setattr(gemm, "_pairs", lambda *a, **k: asked.append(k.get("epilogue", 0)) or pairs(*a, **k))
+    gemm.linear_xielu(x, w, torch.tensor([0.3, -0.7], device=DEV))
+    assert (gemm.EPI_XIELU in asked) == fused
+
+
 @pytest.mark.parametrize("M,N,K", [(225, 4608, 3584), (300, 1536, 8960), (193, 1024, 4096), (1153, 512, 2048), (640, 1536, 1536)])
 def test_32_bit_results_lose_nothing(M, N, K):
     """The tensor cores cut every sum off: a kernel that adds more of K one after the other is not chosen for its speed."""
