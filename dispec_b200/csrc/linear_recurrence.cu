@@ -1060,7 +1060,7 @@ extern "C" int dsp_linear_recurrence(const void* proj, int proj_dtype, long ld, 
                                : launch_tile<16, 4, 1, 4, true, true>(a, S, stream, n);
     if (rc != 0 || all_long) return rc;
   }
-  if (scratch || (mode == STEP_DECAY && T > 2 * S)) {  // portions of prompts
+  if (T > 2 * S && (scratch || mode == STEP_DECAY)) {  // portions of prompts (not: a long one beside many single tokens)
     if (dim <= 32) return launch_tile<8, 1, 2, 8, true>(a, S, stream);
     if (dim <= 64) return launch_tile<8, 1, 4, 8, true>(a, S, stream);
     if (dim <= 128) return launch_tile<8, 1, 8, 8, true>(a, S, stream);

@@ -88,6 +88,19 @@ def test_against_one_scan(H, d, dv, monkeypatch):
         at += n
 
 
+@pytest.mark.parametrize("mode", ["gate", "step"])
+def test_a_long_request_beside_many_single_tokens(mode, monkeypatch):
+    """The single tokens have the bits of a step without the long request, whether the host knows the lengths or not."""
+    from dispec_b200.ops import recurrence as R
+    monkeypatch.setattr(R, "SEGMENTS_MIN_TOKENS", 128)
+    monkeypatch.setitem(globals(), "LENS", [200] + [1] * 250)
+    data = inputs(2, 64, 64, mode, 9)
+    together = run(2, 64, 64, mode, list(range(251)), data)
+    assert all(map(same, together, run(2, 64, 64, mode, list(range(251)), data, known=False)))
+    assert all(map(same, together[1:], run(2, 64, 64, mode, list(range(1, 251)), data)))
+    assert same(together[0], run(2, 64, 64, mode, [0], data)[0])
+
+
 def test_memory_that_is_refused_gives_the_same_bits(monkeypatch):
     from dispec_b200.ops import recurrence as R
     monkeypatch.setattr(R, "SEGMENTS_MIN_TOKENS", 128)
