@@ -97,3 +97,19 @@ def test_few_rows_are_not_slower_than_the_chain(N, K):
         return min(times)
 
     assert us(gemm._split) < 1.25 * us(gemm._simt)
+
+
+@pytest.mark.parametrize("K", [1536, 4096, 8960])
+@pytest.mark.parametrize("kind", ["uniform", "lognormal", "squares", "half"])
+def test_operands_of_one_sign(kind, K):
+    """The tensor cores cut sums off, always towards zero: products of one sign must not add that up beyond what a chain of
+    FMAs rounds."""
+    from dispec_b200.ops import gemm
+    g = torch.Generator(device=DEV).manual_seed(K)
+    u = lambda s: torch.randn(s, generator=g, device=DEV)
+    draw = {"uniform": lambda s: torch.rand(s, generator=g, device=DEV), "lognormal": lambda s: torch.exp(2 * u(s)),
+            "squares": lambda s: u(s) ** 2, "half": lambda s: u(s).relu()}[kind]
+    x, w = draw((48, K)), draw((512, K))
+    ref = x.double() @ w.double().T
+    error = lambda f: float((f(x, w, None, None, torch.empty((48, 512), device=DEV)).double() - ref).norm() / ref.norm())
+    assert error(gemm._split) < error(gemm._simt)
