@@ -16,7 +16,7 @@ _sm_count: dict[int, int] = {}
 
 def sm_count(device=None) -> int:
     """Streaming multiprocessors of the device (asked once per device)."""
-    index = torch.device(device).index if device is not None else None
+    index = device.index if isinstance(device, torch.device) else None if device is None else torch.device(device).index
     if index is None:
         index = torch.cuda.current_device()
     if index not in _sm_count:
