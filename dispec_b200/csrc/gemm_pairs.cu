@@ -496,7 +496,7 @@ static double time_us(const Plan& p, int N, int K, int target_ctas, int result) 
 }
 // Whether this product beats what runs otherwise (-1: not known, the message is set): the few-row or the many-row kernel for
 // results 0 to 2, with a margin for the fits' errors (of 3,432 sizes eight take more than 1.03 of the other kernel's time, at
-// most 1.10; the mean is 0.963 / 0.927 / 0.897 of it), and for 3 a product with a 32-bit result and the activation behind it (mean
+// most 1.11; the mean is 0.961 / 0.927 / 0.897 of it), and for 3 a product with a 32-bit result and the activation behind it (mean
 // 0.88, at most 1.15).  32-bit results stay where their sums are shorter: the tensor cores cut every one off (300 rows x 2,048
 // x 8,960: 3.2e-6 off 64 bits here, 2.3e-6 in the few-row kernel, which splits K further, 1.0e-5 in the many-row one).  This,
 // few-row and many-row: 536 rows x 1,536 x 1,536 9.8 / 11.8 / 11.8 us, x 17,920 x 1,536 29.0 / 30.7 / 30.5, x 1,536 x 8,960 21.3 /

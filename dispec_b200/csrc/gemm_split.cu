@@ -3,9 +3,8 @@
 //
 // An operand times 2^24 is the sum of three bfloat16 values, x1 + x2 + x3 exactly (8 + 8 + 8 bits, each piece the rounded
 // rest of the one before; the lowest bit of any float is 2^-149, so that no piece is smaller than the normal numbers), and
-// of the nine products of pieces the six largest are formed: a1 w1, and a1 w2, a2 w1,
-// a2 w2, a1 w3, a3 w1; what is left out is below 2^-24 of a product.  The a1 w1 of 128 k are summed in tensor
-// memory, then added to 32-bit sums in registers (rounded to nearest, where the tensor cores cut sums off); the five
+// of the nine products of pieces the six largest are formed: a1 w1, and a1 w2, a2 w1, a2 w2, a1 w3, a3 w1; what is left
+// out is below 2^-24 of a product.  The a1 w1 of 128 k are summed in tensor memory, then added to 32-bit sums in registers (rounded to nearest, where the tensor cores cut sums off); the five
 // small products, 2^-8 of them, are summed in tensor memory over all of K and added at the end.
 //
 // Roles are swapped as in gemm_stream.cu: 128 rows of W are the lanes, a chunk of up to 96 rows of A the columns.
@@ -18,9 +17,10 @@
 // cycles for 32 k of 96 rows, beside 580 to 660 of the tensor cores.
 //
 // Against 64 bits, relative error of normal operands, this product and the chain of 32-bit FMAs (gemm_simt.cu): 1.3e-7
-// and 7.0e-7 at K 1,536, 1.6e-7 and 1.7e-6 at K 8,960.  us, the same two: 264 rows x 17,920 x 1,536 109 and 381,
-// x 1,536 x 8,960 68 and 274, x 1,536 x 1,536 25 and 55; 4 rows x 17,920 x 1,536 32 and 43, x 1,536 x 8,960 44 and 62;
-// 5 rows x 151,936 x 1,536 169 and 312.
+// and 7.0e-7 at K 1,536, 1.6e-7 and 1.7e-6 at K 8,960; operands of one sign, K 1,536, uniform 1.5e-7 and 5.9e-7, lognormal
+// 6.7e-7 and 8.4e-7, squares 3.0e-7 and 6.0e-7.  us, the same two, launches one after the other: 264
+// rows x 17,920 x 1,536 109 and 380, x 1,536 x 8,960 62 and 268, x 1,536 x 1,536 18 and 49; 4 rows x 17,920 x 1,536 26 and 37, x
+// 1,536 x 8,960 40 and 57, x 151,936 x 1,536 162 and 204.
 //
 // What a result depends on: its row of A, its row of W, N and K.  K is split over a cluster by a rule on N and K
 // alone, the pieces are summed in the same order for every width of a chunk, and so a row has the same bits alone and
