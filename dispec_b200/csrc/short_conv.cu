@@ -129,8 +129,6 @@ __device__ __forceinline__ void keep_inputs(const ConvIn& p, const Turn& r, floa
     hist[(size_t)m * p.channels + c] = input_at(p, r, hist, c, r.n - (p.taps - 1) + m);
 }
 
-__device__ __forceinline__ float softplus_wide(float v) { return v > 20.f ? v + log1pf(expf(-v)) : log1pf(expf(v)); }
-
 constexpr int PER_THREAD = 4;
 
 __global__ void __launch_bounds__(256)
@@ -170,7 +168,7 @@ conv_steps_kernel(const ConvIn p, const float* __restrict__ bias, float* __restr
   }
   if (blockIdx.y == 0)
     for (int h = threadIdx.x; h < heads; h += blockDim.x) {
-      const float step = softplus_wide(ld_any(p.u, p.dtype, (size_t)t * p.ld + step_off + h) + step_bias[h]);
+      const float step = softplus_f(ld_any(p.u, p.dtype, (size_t)t * p.ld + step_off + h) + step_bias[h]);
       steps[((size_t)t * 2) * heads + h] = step;
       steps[((size_t)t * 2 + 1) * heads + h] = expf(-expf(a_log[h]) * step);
     }
@@ -341,7 +339,7 @@ conv_heads_kernel(const ConvIn p, int T, int A, int B, int dim, int vdim, float 
       const int tok = t + idx / H, h = idx % H;
       if (p.positions[tok] < 0) continue;
       steps[(size_t)tok * 2 * H + h] = 1.f / (1.f + expf(-ld_any(p.u, p.dtype, (size_t)tok * p.ld + b_off + h)));
-      steps[((size_t)tok * 2 + 1) * H + h] = -expf(a_log[h]) * softplus_wide(ld_any(p.u, p.dtype, (size_t)tok * p.ld + a_off + h) + step_bias[h]);
+      steps[((size_t)tok * 2 + 1) * H + h] = -expf(a_log[h]) * softplus_f(ld_any(p.u, p.dtype, (size_t)tok * p.ld + a_off + h) + step_bias[h]);
     }
     return;
   }
